@@ -12,6 +12,7 @@
 // The state carried between tiles lives in shared memory (one float per channel and state), so any
 // dstate <= 256 works; states are processed in blocks of kStateBlock with B/C re-staged per block.
 // Steps past seqlen get dt = 0, u = 0, i.e. the identity (1, 0), so the final state is exact.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1062,13 +1063,47 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 template <typename T> int split_segments(const mb200_scan_args &a);
 
-// The channel-parallel kernel keeps at most 16 states per channel in registers and takes its B and C from the input; fewer than
-// kStreamMinChannels channels would leave most of the GPU idle unless the sequence can be cut.
+// The channel-parallel kernel works on tiles of 32 channels of one group.
+int64_t channel_tiles(const mb200_scan_args &a) { return (int64_t)a.batch * a.ngroups * ((a.dim / a.ngroups + kStreamCh - 1) / kStreamCh); }
+
+template <typename T> bool stream_tiles(const mb200_scan_args &a);
+
+// Every row of u, delta, z and the outputs starts on a 16-byte boundary.
+template <typename T>
+bool rows_aligned(const mb200_scan_args &a)
+{
+    constexpr int VEC = 16 / sizeof(T);
+    auto ok = [](const void *p, const int64_t *s) { return aligned16(p) && s[0] % VEC == 0 && s[1] % VEC == 0; };
+    return ok(a.u, a.u_stride) && ok(a.delta, a.delta_stride) && ok(a.out, a.out_stride) && (!a.z || ok(a.z, a.z_stride)) &&
+           (!a.z || !a.out_pregate || ok(a.out_pregate, a.pregate_stride));
+}
+
+// Which calls the channel-parallel kernel serves.  It keeps at most 16 states per channel in registers and takes its B and C from the
+// input; fewer than kStreamMinChannels channels would leave most of the GPU idle unless the sequence can be cut.  Rows that TMA can
+// describe need no more than that.  Where the lanes fetch the rows (stream_tiles is false), a pass is a chain of about 0.11 us per step
+// however few the tiles, and lanes past the end of a group are idle, so that the time-parallel kernel -- which takes 512 steps of a
+// channel at a time -- is often the faster one.  Measured, lanes / time-parallel, us, bf16 and 16 states unless said:
+//   one pass, 999 steps:         2048 channels 105 / 55, 4128: 106 / 101, 5120: 115 / 134; 8 states, 6144: 121 / 109, 8192: 122 / 140
+//   one pass, 133 steps:         1024 channels 21.5 / 24.6; 8 states, 2048: 22 / 20, 3072: 23 / 29
+//   16 segments, 2048 steps:     1008 channels in groups of 24: 64 / 83; 4097 steps, 2048 channels: 163 / 201
+//   8 segments, 1999 steps:      2048 channels 95 / 101, 3072: 151 / 176; 2000 channels in groups of 40 (800 CTAs): 113 / 93
+//   groups that fill half of a tile, one pass, 2048 steps: 8192 channels 329 / 340, fp32 398 / 355; a quarter of a tile: 552 / 342
+//   8 states, rows on 16-byte boundaries (which the time-parallel kernel loads in packets): 7680 channels in groups of 80: 245 / 203,
+//   40960: 780 / 719
 template <typename T>
 bool stream_eligible(const mb200_scan_args &a)
 {
     if (a.dstate > 16 || !a.B_variable || !a.C_variable) return false;
-    return (int64_t)a.batch * a.dim >= kStreamMinChannels || split_segments<T>(a) > 1;
+    const int64_t channels = (int64_t)a.batch * a.dim, tiles = channel_tiles(a);
+    const int nseg = split_segments<T>(a);
+    if (channels < kStreamMinChannels && nseg <= 1) return false;
+    if (stream_tiles<T>(a)) return true;
+    const bool few_states = a.dstate <= 8;
+    if (channels * (few_states ? 24 : sizeof(T) == 4 ? 30 : 32) < tiles * kStreamCh * 16) return false;       // too few live lanes
+    if (few_states && channels >= kStreamMinChannels && rows_aligned<T>(a)) return false;
+    if (nseg > 1) return nseg > 8 || tiles * nseg <= 4 * 148 || channels >= 2688;
+    const int64_t steps = a.seqlen;      // of the chain, against channels of the other kernel
+    return channels >= (few_states ? std::min<int64_t>(7168, 12 * steps + 768) : std::min<int64_t>(4608, 10 * steps - 320));
 }
 
 // ... and its operands can be described to TMA: 16-byte aligned bases and row strides, whole groups of 32 channels, one output.
@@ -1091,17 +1126,16 @@ bool stream_tiles(const mb200_scan_args &a)
 }
 
 // How many segments the sequence is cut into (1 = one pass).  Cutting pays when the channel groups alone leave most
-// of the GPU idle: with G = batch * dim / 32 groups, nseg is the largest power of two with G * nseg CTAs in one wave
+// of the GPU idle: with G tiles of 32 channels, nseg is the largest power of two with G * nseg CTAs in one wave
 // of 9 per SM.  It costs a second pass over every segment but the last, so it is used only from nseg = 8 up (fewer
 // segments measured no faster than one pass), with segments of at least 128 steps, and only when the caller lent
 // scratch for the summaries.
 template <typename T>
 int split_segments(const mb200_scan_args &a)
 {
-    const int64_t groups = (int64_t)a.batch * a.dim / kStreamCh;
-    if (groups <= 0) return 1;
+    const int64_t tiles = channel_tiles(a);
     int nseg = 1;
-    while (nseg < kMaxSegments && groups * nseg * 2 <= 9 * 148 && a.seqlen / (nseg * 2) >= 128) nseg *= 2;
+    while (nseg < kMaxSegments && tiles * nseg * 2 <= 9 * 148 && a.seqlen / (nseg * 2) >= 128) nseg *= 2;
     if (nseg < 8) return 1;
     const size_t need = 3 * sizeof(float) * (size_t)a.batch * nseg * a.dim * a.dstate;
     if (!a.scratch || a.scratch_bytes < need || (reinterpret_cast<uintptr_t>(a.scratch) & 15)) return 1;
@@ -1186,7 +1220,6 @@ int launch_stream(const mb200_scan_args &a, cudaStream_t stream)
 template <typename T>
 int launch_scan(const mb200_scan_args &a, cudaStream_t stream)
 {
-    constexpr int VEC = 16 / sizeof(T);
     const int N = a.dstate;
     const int nblocks = (N + kStateBlock - 1) / kStateBlock;
     const int per_group = a.dim / a.ngroups;
@@ -1195,11 +1228,7 @@ int launch_scan(const mb200_scan_args &a, cudaStream_t stream)
     if (nblocks == 1 && per_group >= 2 * kWarps && (int64_t)a.batch * a.dim >= 8 * kWarps * 2 * 148) cpw = 2;
     const int chans = kWarps * cpw;
     const int npad = N;
-    auto strides_ok = [&](const int64_t *s) { return s[0] % VEC == 0 && s[1] % VEC == 0; };
-    bool io_vec = aligned16(a.u) && aligned16(a.delta) && aligned16(a.out) && strides_ok(a.u_stride) &&
-                  strides_ok(a.delta_stride) && strides_ok(a.out_stride);
-    if (a.z) io_vec = io_vec && aligned16(a.z) && strides_ok(a.z_stride);
-    if (a.z && a.out_pregate) io_vec = io_vec && aligned16(a.out_pregate) && strides_ok(a.pregate_stride);
+    const bool io_vec = rows_aligned<T>(a);
     // staging reads 4 elements at a time: 8 bytes for 16-bit types, 16 for fp32
     const int bc_align = sizeof(T) == 4 ? 16 : 8;
     bool bc_vec = true;
@@ -1211,7 +1240,7 @@ int launch_scan(const mb200_scan_args &a, cudaStream_t stream)
                  a.C_stride[1] % 4 == 0 && a.C_stride[2] % 4 == 0;
     const int vec_flags = (io_vec ? 1 : 0) | (bc_vec ? 2 : 0);
     if (stream_eligible<T>(a)) return launch_stream<T>(a, stream);
-    if (N <= kStateBlock && a.B_variable && a.C_variable) {      // fewer than kStreamMinChannels channels
+    if (N <= kStateBlock && a.B_variable && a.C_variable && (int64_t)a.batch * a.dim < kStreamMinChannels) {
         auto go = [&](auto ch_c) {
             constexpr int CH = decltype(ch_c)::value;
             const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(&scan_few_kernel<T, CH>), (int)sizeof(FewSmem<CH>), a.device);

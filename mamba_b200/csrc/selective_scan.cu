@@ -1188,9 +1188,14 @@ int launch_stream(const mb200_scan_args &a, cudaStream_t stream)
                 if (split.h0) launch_dependent(kernel, grid, threads, smem, stream, a, maps, split);        // after the fold
                 else kernel<<<grid, threads, smem, stream>>>(a, maps, split);
             };
-            if (ctas <= 4 * 148) run(std::integral_constant<int, 4>{}, std::true_type{});
-            else if (ctas <= 6 * 148) run(std::integral_constant<int, 2>{}, std::true_type{});
-            else run(std::integral_constant<int, 2>{}, std::false_type{});
+            // fp32 rows fetched by the lanes take two granules per hand-off, of which shared memory holds three: a single scalar warp would
+            // wait for the last it asked for.  Rows off their 16-byte boundaries need twice the sectors, and the six-warp layout whatever
+            // the grid (us: six, four, three warps; 8 x 5120 channels of 1999 steps: 901, 1466, 1720; 40960 channels in groups of 80, 2048
+            // steps, aligned: 1122, 1073, 1268; 16000 of them, 600 CTAs: 598, 509, -).
+            constexpr bool kLanes32 = sizeof(T) == 4 && !TMA;
+            if (ctas <= 4 * 148 || (kLanes32 && !rows_aligned<T>(a))) run(std::integral_constant<int, 4>{}, std::true_type{});
+            else if (ctas <= 6 * 148 || kLanes32) run(std::integral_constant<int, 2>{}, std::true_type{});
+            else if constexpr (!kLanes32) run(std::integral_constant<int, 2>{}, std::false_type{});
         };
         auto with_ns = [&](auto ns_c) {
             if (tiles) summary ? pick(ns_c, std::true_type{}, std::true_type{}) : pick(ns_c, std::false_type{}, std::true_type{});

@@ -31,6 +31,7 @@ def test_segments_follow_the_tiles(dim, groups, segments):
     (1, 2048, 72, 16, 256), (1, 1920, 72, 16, 128), (1, 2048, 73, 16, 128), (1, 2176, 72, 16, 128), # 8, 15, 16, 17 channels a group
     (2, 64, 72, 16, 64), (1, 1280, 33, 5, 1280),                                                    # one channel a group
     (1, 1040, 2051, 16, 1), (1, 2720, 1027, 16, 1), (1, 2640, 1027, 16, 1),                         # 16 segments; 8, either side
+    (1, 14448, 40, 16, 602), (1, 14448, 41, 16, 602), (1, 21672, 40, 16, 903),                      # many CTAs, aligned and not
 ])
 def test_either_side(dtype, tol, batch, dim, L, N, groups):
     run_both(make_inputs(dim + L, batch, dim, L, N, groups, dtype, has_z=L != 73), tol, f"route b{batch} d{dim} L{L} N{N} G{groups}")

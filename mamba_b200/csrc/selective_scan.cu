@@ -1245,7 +1245,9 @@ int launch_scan(const mb200_scan_args &a, cudaStream_t stream)
                  a.C_stride[1] % 4 == 0 && a.C_stride[2] % 4 == 0;
     const int vec_flags = (io_vec ? 1 : 0) | (bc_vec ? 2 : 0);
     if (stream_eligible<T>(a)) return launch_stream<T>(a, stream);
-    if (N <= kStateBlock && a.B_variable && a.C_variable && (int64_t)a.batch * a.dim < kStreamMinChannels) {
+    // Four warps per channel while that is at most one CTA per SM; beyond, their barriers cost more than the shorter chain saves
+    // (bf16, 777 steps, us, four warps / one: 512 channels of 16 states 27 / 45, 640: 43 / 45; of 8 states 22 / 31, 35 / 31).
+    if (N <= kStateBlock && a.B_variable && a.C_variable && (int64_t)a.batch * a.ngroups * ((per_group + 3) / 4) <= 148) {
         auto go = [&](auto ch_c) {
             constexpr int CH = decltype(ch_c)::value;
             const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(&scan_few_kernel<T, CH>), (int)sizeof(FewSmem<CH>), a.device);

@@ -1,5 +1,5 @@
 """Selective scan on either side of each line between its kernels: tiles with too few live lanes, rows that the lanes fetch in one pass
-or cut into segments, groups of a few channels."""
+or cut into segments, groups of a few channels, four warps per channel or one."""
 import ctypes
 
 import pytest
@@ -32,6 +32,7 @@ def test_segments_follow_the_tiles(dim, groups, segments):
     (2, 64, 72, 16, 64), (1, 1280, 33, 5, 1280),                                                    # one channel a group
     (1, 1040, 2051, 16, 1), (1, 2720, 1027, 16, 1), (1, 2640, 1027, 16, 1),                         # 16 segments; 8, either side
     (1, 14448, 40, 16, 602), (1, 14448, 41, 16, 602), (1, 21672, 40, 16, 903),                      # many CTAs, aligned and not
+    (1, 592, 520, 16, 1), (1, 593, 520, 16, 1), (1, 296, 65, 16, 148), (1, 298, 65, 16, 149),       # four warps per channel, or one
 ])
 def test_either_side(dtype, tol, batch, dim, L, N, groups):
     run_both(make_inputs(dim + L, batch, dim, L, N, groups, dtype, has_z=L != 73), tol, f"route b{batch} d{dim} L{L} N{N} G{groups}")

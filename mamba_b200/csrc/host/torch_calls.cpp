@@ -208,17 +208,17 @@ PyObject *scan_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
     Tensor dz;
     if (z.has()) dz = empty_as(*z);
     if (du.stride(2) != 1 || dd.stride(2) != 1 || (z.has() && dz.stride(2) != 1)) DECLINE();
-    // the fp32 accumulators share one allocation, which the library clears with one memset
-    const int64_t nA = A->numel(), nB = B->numel(), nC = C->numel(), nd = a.dim;
-    auto up = [](int64_t k) { return (k + 63) / 64 * 64; };      // 256-byte steps
-    const Tensor acc = empty({up(nA) + up(nB) + up(nC) + 2 * up(nd)}, at::kFloat, dev);
-    a.accumulators_bytes = acc.numel() * sizeof(float);
-    float *base = static_cast<float *>(acc.data_ptr());
-    const int64_t oB = up(nA), oC = oB + up(nB), oD = oC + up(nC), ob = oD + up(nd);
+    // the fp32 accumulators each in a storage of its own: autograd keeps what it is given as .grad
+    const Tensor dA = empty(A->sizes(), at::kFloat, dev);
+    const Tensor dB = empty(B->sizes(), at::kFloat, dev), dC = empty(C->sizes(), at::kFloat, dev);
+    Tensor dD, db;
+    if (D.has()) dD = empty(D->sizes(), at::kFloat, dev);
+    if (bias.has()) db = empty(bias->sizes(), at::kFloat, dev);
+    auto floats = [](const Tensor &t) { return static_cast<float *>(t.data_ptr()); };
     a.dout = dout.ptr(); a.du = du.data_ptr(); a.ddelta = dd.data_ptr(); a.dz = z.has() ? dz.data_ptr() : nullptr;
-    a.dA = base; a.dB = base + oB; a.dC = base + oC;
-    a.dD = D.has() ? base + oD : nullptr;
-    a.ddelta_bias = bias.has() ? base + ob : nullptr;
+    a.dA = floats(dA); a.dB = floats(dB); a.dC = floats(dC);
+    a.dD = D.has() ? floats(dD) : nullptr;
+    a.ddelta_bias = bias.has() ? floats(db) : nullptr;
     strides(a.dout_stride, *dout, 2);
     strides(a.du_stride, du, 2);
     strides(a.ddelta_stride, dd, 2);
@@ -229,14 +229,12 @@ PyObject *scan_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
     a.scratch = scratch.data_ptr();
     a.scratch_bytes = need;
     if (mb200_selective_scan_bwd(&a, stream_of(*u)) != MB200_OK) DECLINE();
-    auto part = [&](int64_t off, const Tensor &like) { return acc.narrow(0, off, like.numel()).view(like.sizes()); };
-    const Tensor dA = part(0, *A), dB = part(oB, *B).to(B->scalar_type()), dC = part(oC, *C).to(C->scalar_type());
     auto opt = [](bool on, const Tensor &t) -> PyObject * {
         if (on) return wrap(t);
         Py_RETURN_NONE;
     };
-    return Py_BuildValue("(NNNNNNNN)", wrap(du), wrap(dd), wrap(dA), wrap(dB), wrap(dC), opt(D.has(), D.has() ? part(oD, *D) : Tensor()),
-                         opt(z.has(), dz), opt(bias.has(), bias.has() ? part(ob, *bias) : Tensor()));
+    return Py_BuildValue("(NNNNNNNN)", wrap(du), wrap(dd), wrap(dA), wrap(dB.to(B->scalar_type())), wrap(dC.to(C->scalar_type())), opt(D.has(), dD),
+                         opt(z.has(), dz), opt(bias.has(), db));
     GUARD_END
 }
 

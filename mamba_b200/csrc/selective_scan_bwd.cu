@@ -1059,6 +1059,20 @@ __global__ void __launch_bounds__(128, 4) scan_bwd_few_kernel(const mb200_scan_b
     }
 }
 
+// Zeroes the accumulators in one launch, each by a row of the grid.
+struct ClearList {
+    float *p[5];
+    size_t n[5];
+};
+__global__ void __launch_bounds__(256) scan_bwd_clear_kernel(const ClearList l)
+{
+    float *p = l.p[blockIdx.y];
+    const size_t n = l.n[blockIdx.y], first = (size_t)blockIdx.x * 256 + threadIdx.x, step = (size_t)gridDim.x * 256;
+    const size_t packets = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? n / 4 : 0;
+    for (size_t i = first; i < packets; i += step) reinterpret_cast<float4 *>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (size_t i = 4 * packets + first; i < n; i += step) p[i] = 0.f;
+}
+
 bool aligned_to(const void *p, size_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
 
 // Scratch per batch row: the stored states and, above 16 states, the partial sums carried between the passes.  Batch
@@ -1234,12 +1248,10 @@ extern "C" int mb200_selective_scan_bwd(const mb200_scan_bwd_args *args, void *s
         const cudaError_t e = cudaMemsetAsync(a.dA, 0, a.accumulators_bytes, stream);
         if (e != cudaSuccess) return fail(MB200_ERR_LAUNCH, "selective_scan_bwd: memset: %s", cudaGetErrorString(e));
     } else {
-        cudaError_t e = cudaMemsetAsync(a.dA, 0, wn, stream);
-        if (e == cudaSuccess && a.dB && bn) e = cudaMemsetAsync(a.dB, 0, bn, stream);
-        if (e == cudaSuccess && a.dC && cn) e = cudaMemsetAsync(a.dC, 0, cn, stream);
-        if (e == cudaSuccess && a.dD) e = cudaMemsetAsync(a.dD, 0, sizeof(float) * a.dim, stream);
-        if (e == cudaSuccess && a.ddelta_bias) e = cudaMemsetAsync(a.ddelta_bias, 0, sizeof(float) * a.dim, stream);
-        if (e != cudaSuccess) return fail(MB200_ERR_LAUNCH, "selective_scan_bwd: memset: %s", cudaGetErrorString(e));
+        const size_t pn = sizeof(float) * (size_t)a.dim;
+        const ClearList list = {{a.dA, a.dB, a.dC, a.dD, a.ddelta_bias}, {wn / 4, a.dB ? bn / 4 : 0, a.dC ? cn / 4 : 0, a.dD ? pn / 4 : 0, a.ddelta_bias ? pn / 4 : 0}};
+        scan_bwd_clear_kernel<<<dim3(148, 5), 256, 0, stream>>>(list);
+        MB200_CHECK_LAUNCH("selective_scan_bwd: clearing the accumulators");
     }
     if (a.batch == 0 || a.seqlen == 0) return MB200_OK;
     MB200_CHECK_ARG(a.u && a.delta && a.B && a.C && a.dout && a.du && a.ddelta && a.dB && a.dC,

@@ -88,3 +88,21 @@ def test_ssd_and_block(monkeypatch, norm, batch, ngroups, init):
     x, B, C = r(batch, L, H, P), r(batch, L, ngroups, N), r(batch, L, ngroups, N, seed=1)
     both(monkeypatch, lambda: mamba_chunk_scan_combined(x, r(batch, L, H), A, B, C, 64, D=D.half(), z=x, dt_bias=bias, initial_states=h0,
                                                         dt_softplus=True, return_final_states=True))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("variable", [True, False])
+def test_gradients_own_their_storage(dtype, variable):
+    """What autograd hands on may be kept as .grad: no gradient holds the memory, or shares the version counter, of another."""
+    from mamba_b200 import selective_scan_fn
+    b, d, L, N = 2, 8, 300, 4
+    u, delta, z = (r(b, d, L, seed=i).to(dtype).requires_grad_() for i in range(3))
+    B, C = (r(b, 1, N, L, seed=i).to(dtype).requires_grad_() if variable else r(d, N, seed=i).requires_grad_() for i in range(2))
+    A, D, bias = (-torch.exp(r(d, N))).requires_grad_(), r(d).requires_grad_(), (r(d) - 3).requires_grad_()
+    leaves = (u, delta, A, B, C, D, z, bias)
+    grads = torch.autograd.grad(selective_scan_fn(u, delta, A, B, C, D, z, bias, delta_softplus=True), leaves, r(b, d, L, seed=9).to(dtype))
+    for t, g in zip(leaves, grads):
+        assert g.untyped_storage().nbytes() == t.numel() * t.element_size()
+    versions = [g._version for g in grads]
+    grads[5].add_(1)
+    assert [g._version for g in grads] == [v + (i == 5) for i, v in enumerate(versions)]

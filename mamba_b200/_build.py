@@ -16,6 +16,7 @@ OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "libmamba_b200.so")
 HOST_SRC = os.path.join(CSRC, "host", "torch_calls.cpp")
 HOST = os.path.join(PKG, "_host.so")
+HOST_BUILT_FOR = os.path.join(OBJ, "host_built_for.txt")      # host_environment() of the last build of _host.so
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -41,6 +42,26 @@ def _headers():
     hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     hs.append(os.path.join(os.path.dirname(PKG), "include", "mamba_b200.h"))
     return hs
+
+
+def host_environment():
+    """What _host.so has to have been compiled against: it works on PyTorch's C++ objects, whose layout changes between versions."""
+    import torch
+    return f"torch {torch.__version__} cxx11abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} {sys.implementation.cache_tag}"
+
+
+def host_built_for():
+    """host_environment() at the last build of _host.so, or None where that was not recorded."""
+    try:
+        with open(HOST_BUILT_FOR) as f:
+            return f.read().strip()
+    except OSError:
+        return None
+
+
+def host_stale(obj, newest_hdr):
+    return (not os.path.exists(obj) or not os.path.exists(HOST) or os.path.getmtime(obj) < max(os.path.getmtime(HOST_SRC), newest_hdr)
+            or host_built_for() != host_environment())
 
 
 def _host_command(obj):
@@ -73,9 +94,8 @@ def build(force=False, verbose=False):
             cmd = [nvcc, *host, *NVCC_FLAGS, "-c", src, "-o", obj]
             procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, env=env, text=True)))
     host_obj = os.path.join(OBJ, "torch_calls.o")
-    host_stale = force or not os.path.exists(host_obj) or os.path.getmtime(host_obj) < max(os.path.getmtime(HOST_SRC), newest_hdr)
     host_proc = None
-    if host_stale:
+    if force or host_stale(host_obj, newest_hdr):
         host_proc = subprocess.Popen(_host_command(host_obj), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, env=env, text=True)
     for src, p in procs:
         out, _ = p.communicate()
@@ -93,12 +113,13 @@ def build(force=False, verbose=False):
         if host_proc.returncode != 0:
             sys.stderr.write(out)
             raise RuntimeError(f"g++ failed on {HOST_SRC}")
-    if host_stale or not os.path.exists(HOST):
         import torch
         libs = ["-L", os.path.join(os.path.dirname(torch.__file__), "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda",
                 "-lc10"]
         subprocess.check_call([_host_command(host_obj)[0], "-shared", "-Wl,--no-as-needed", "-o", HOST, host_obj, "-L", PKG, "-l:libmamba_b200.so",
                                *libs, "-Wl,-rpath,$ORIGIN"], env=env)
+        with open(HOST_BUILT_FOR, "w") as f:
+            f.write(host_environment() + "\n")
     if logs:
         with open(os.path.join(OBJ, "ptxas.log"), "w") as f:
             for src, out in logs:

@@ -7,6 +7,7 @@ exception.  Nothing here computes anything.
 import ctypes
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -156,14 +157,29 @@ def lib():
 _host = None
 
 
+class _NoNativePath:
+    """Declines every call: the operators then go to the library through ctypes."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def host():
     """The native call path (csrc/host): its functions take an operator's arguments, return its result, or return None when
-    the Python operator has something to check, convert or raise first.  Raises RuntimeError when it has not been built."""
+    the Python operator has something to check, convert or raise first.  Raises RuntimeError when it has not been built.
+    One that was built for another PyTorch is not loaded: its calls would read that one's objects."""
     global _host
     if _host is None:
         if not os.path.exists(HOST_PATH):
             raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m mamba_b200._build`")
         lib()
+        from . import _build
+        built_for = _build.host_built_for()
+        if built_for is not None and built_for != _build.host_environment():
+            warnings.warn(f"{HOST_PATH} was built for {built_for}, this is {_build.host_environment()}: calls take the slower path "
+                          "through ctypes until `python -m mamba_b200._build` has been run")
+            _host = _NoNativePath()
+            return _host
         spec = importlib.util.spec_from_file_location("mamba_b200._host", HOST_PATH)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)

@@ -98,3 +98,16 @@ def test_cpu_tensors_are_rejected():
     s = torch.zeros(1, 4, 8)
     with pytest.raises(RuntimeError, match="CUDA"):
         selective_state_update(s, torch.zeros(1, 4), torch.zeros(1, 4), torch.zeros(4, 8), torch.zeros(1, 8), torch.zeros(1, 8))
+
+
+def test_call_path_of_another_pytorch(built, monkeypatch):
+    """_host.so works on PyTorch's C++ objects: it is rebuilt for another PyTorch, and not loaded until then."""
+    import torch
+    from mamba_b200 import _build, _lib
+    obj = os.path.join(_build.OBJ, "torch_calls.o")
+    assert _build.host_built_for() == _build.host_environment() and not _build.host_stale(obj, 0)
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    assert _build.host_stale(obj, 0)
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.warns(UserWarning, match="torch 99.0"):
+        assert _lib.host().ssd_fwd(1, 2, 3) is None

@@ -1096,11 +1096,13 @@ __global__ void __launch_bounds__(256) ssd_incoming_state_kernel(T *prev16, cons
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-bool mult8(const int64_t *s, int n)
+// TMA can walk a (batch, time, row, element) tensor of 16-bit values: strides in steps of 16 bytes, none of them 0 (a tensor
+// expanded over a dimension).
+bool rows_for_tma(const void *p, const int64_t *s)
 {
-    for (int i = 0; i < n; ++i)
-        if (s[i] % 8) return false;
-    return true;
+    for (int i = 0; i < 3; ++i)
+        if (s[i] <= 0 || s[i] % 8) return false;
+    return aligned16(p);
 }
 
 // ====================================================================================== end states of packed sequences
@@ -1409,20 +1411,19 @@ bool ssd_tc_shape(const mb200_ssd_args &a)
 bool ssd_tc_local_eligible(const mb200_ssd_args &a)
 {
     if (!ssd_tc_shape(a)) return false;
-    if (!aligned16(a.x) || !aligned16(a.B) || !mult8(a.x_stride, 3) || !mult8(a.B_stride, 3)) return false;
+    if (!rows_for_tma(a.x, a.x_stride) || !rows_for_tma(a.B, a.B_stride)) return false;
     const int64_t nc = (a.seqlen + kQ - 1) / kQ;
     if ((int64_t)a.batch * nc * a.nheads * slices(a) > INT32_MAX || nc > 65535) return false;
     return encode_fn() != nullptr;
 }
 
-bool ssd_tc_cb_eligible(const mb200_ssd_args &a) { return a.C && aligned16(a.C) && mult8(a.C_stride, 3); }
+bool ssd_tc_cb_eligible(const mb200_ssd_args &a) { return a.C && rows_for_tma(a.C, a.C_stride); }
 
 bool ssd_tc_output_eligible(const mb200_ssd_args &a)
 {
     if (!ssd_tc_cb_eligible(a)) return false;
-    if (!a.out || !aligned16(a.out) || !mult8(a.out_stride, 3)) return false;
-    if (a.z && (!aligned16(a.z) || !mult8(a.z_stride, 3))) return false;
-    return true;
+    if (!a.out || !rows_for_tma(a.out, a.out_stride)) return false;
+    return !a.z || rows_for_tma(a.z, a.z_stride);
 }
 
 // One head slice of one batch row per CTA: worth it once those fill half of the SMs, or when there are so few chunks that

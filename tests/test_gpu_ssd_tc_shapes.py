@@ -72,3 +72,20 @@ def test_packed_row_on_both_sides_of_the_wide_prefix_sum(L):
         s = slice(int(cu[i]), int(cu[i + 1]))
         assert_close(out[:, s], _fn()(c["x"][:, s], c["dt"][:, s], c["A"], c["B"][:, s], c["C"][:, s], 256, z=c["z"][:, s], **kw), TOL_BF16, f"seq {i}")
     assert _status() == 0
+
+
+@pytest.mark.parametrize("name,dim", [("x", 0), ("z", 0), ("B", 2), ("C", 0), ("C", 2), ("x", 2)])
+def test_expanded_inputs(name, dim):
+    """A tensor expanded over the batch, the heads or the groups (stride 0), which is not for TMA, is read in place all the same."""
+    inp = make(420, 2, 300, 4, 64, 2, 128, torch.bfloat16, init=True)
+    c = {k: _c(v) for k, v in inp.items()}
+    full = c[name].narrow(dim, 0, 1).expand(c[name].shape)
+    c[name], inp[name] = full, full.cpu().contiguous()
+    f = lambda t: None if t is None else t.float()
+    want, wfin = oracle.ssd_chunk_scan(f(inp["x"]), f(inp["dt"]), inp["A"], f(inp["B"]), f(inp["C"]), 256, inp["D"], f(inp["z"]), inp["dt_bias"],
+                                       inp["initial_states"], dt_softplus=True)
+    got, fin = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 256, D=c["D"], z=c["z"], dt_bias=c["dt_bias"], initial_states=c["initial_states"],
+                     dt_softplus=True, return_final_states=True)
+    assert _status() == 0
+    assert_close(got, want, TOL_BF16, f"{name} expanded over {dim}: out")
+    assert_close(fin, wfin, TOL_BF16, f"{name} expanded over {dim}: final states")

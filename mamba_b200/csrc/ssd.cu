@@ -1,4 +1,4 @@
-// Mamba-2 SSD chunked forward for sm_100a: stage kernels that work for every shape and dtype.
+// Mamba-2 SSD chunked forward for sm_100a: the stages, and their kernels for fp32 inputs.
 //
 // Stages (each one launch, all on the caller's stream, handing fp32 intermediates through the
 // caller's scratch buffer):
@@ -8,8 +8,8 @@
 //   4. chunk_cb       CB[m,k] = C_m . B_k   (lower block triangle)
 //   5. chunk_scan     y_m = exp(dA_m) C_m.H_c + sum_{k<=m} CB[m,k] exp(min(dA_m - dA_k,0)) dt_k x_k + D x_m,
 //                     then y_m * silu(z_m)
-// The contractions here run on the fp32 FMA pipes through a 64x64 shared-memory tile loop (tile_gemm), which
-// keeps fp32 inputs exact; the tensor-core kernels for bf16/fp16 live in ssd_tc.cu and replace stages 2 to 5.
+// The contractions here run on the fp32 FMA pipes through a 64x64 shared-memory tile loop (tile_gemm) and serve fp32 inputs.  For
+// bf16/fp16, ssd_tc.cu replaces stages 2 to 5 for the shape that most layers have, and ssd_split.cu stages 2, 4 and 5 for all others.
 #include <algorithm>
 
 #include "ssd_common.cuh"
@@ -23,41 +23,25 @@ constexpr int kLd = 68;       // padded leading dimension of the staged tiles (k
 struct TileSmem { __align__(16) float A[2][kKT * kLd], B[2][kKT * kLd]; };
 
 // Four consecutive elements, in one load where `vec` says that they lie on their own alignment; zeros from `n` on.
-template <typename T> __device__ __forceinline__ float4 load4(const T *p, bool vec, int n)
+__device__ __forceinline__ float4 load4(const float *p, bool vec, int n)
 {
-    if (vec && n >= 4) {
-        if constexpr (sizeof(T) == 4) {
-            return *reinterpret_cast<const float4 *>(p);
-        } else {
-            const uint2 r = *reinterpret_cast<const uint2 *>(p);
-            const T *e = reinterpret_cast<const T *>(&r);
-            return make_float4(to_float(e[0]), to_float(e[1]), to_float(e[2]), to_float(e[3]));
-        }
-    }
-    return make_float4(n > 0 ? to_float(p[0]) : 0.f, n > 1 ? to_float(p[1]) : 0.f, n > 2 ? to_float(p[2]) : 0.f, n > 3 ? to_float(p[3]) : 0.f);
+    if (vec && n >= 4) return *reinterpret_cast<const float4 *>(p);
+    return make_float4(n > 0 ? p[0] : 0.f, n > 1 ? p[1] : 0.f, n > 2 ? p[2] : 0.f, n > 3 ? p[3] : 0.f);
 }
-template <typename T> __device__ __forceinline__ void store4(T *p, bool vec, int n, const float (&v)[4])
+__device__ __forceinline__ void store4(float *p, bool vec, int n, const float (&v)[4])
 {
     if (vec && n >= 4) {
-        if constexpr (sizeof(T) == 4) {
-            *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-        } else {
-            uint2 r;
-            T *e = reinterpret_cast<T *>(&r);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) e[i] = from_float<T>(v[i]);
-            *reinterpret_cast<uint2 *>(p) = r;
-        }
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            if (i < n) p[i] = from_float<T>(v[i]);
+            if (i < n) p[i] = v[i];
     }
 }
 // rows of a (batch, time, group or head, columns) tensor start where load4 can take four at once
-template <typename T> __device__ __forceinline__ bool rows_of_4(const T *p, int64_t s0, int64_t s1, int64_t s2)
+__device__ __forceinline__ bool rows_of_4(const float *p, int64_t s0, int64_t s1, int64_t s2)
 {
-    return (reinterpret_cast<uintptr_t>(p) & (4 * sizeof(T) - 1)) == 0 && ((s0 | s1 | s2) & 3) == 0;
+    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((s0 | s1 | s2) & 3) == 0;
 }
 
 // acc += A[64 x K] * B[K x 64] for the thread's 8x4 patch: rows ty*8.. in pairs (packed fp32 FMAs), columns tx*4...  fa and fb
@@ -256,7 +240,6 @@ __global__ void __launch_bounds__(NW * 32) ssd_cumsum_kernel(const mb200_ssd_arg
 }
 
 // ---- stage 2 ------------------------------------------------------------------------------------
-template <typename T>
 __global__ void __launch_bounds__(kT, 4) ssd_chunk_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb,
                                                              float *states, int nchunks)
 {
@@ -271,8 +254,8 @@ __global__ void __launch_bounds__(kT, 4) ssd_chunk_state_kernel(const mb200_ssd_
     const float *dtc = dtb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
     const float *dAc = dAb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
     const float dA_last = dAc[Q - 1];
-    const T *x = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const T *B = static_cast<const T *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
+    const float *x = static_cast<const float *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
+    const float *B = static_cast<const float *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
     const bool vx = rows_of_4(x, 0, a.x_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
     uint64_t acc[4][4] = {};
     const int seq_last = seq_at(a, b, t0 + len - 1);    // only steps of the chunk's last sequence reach its end state
@@ -368,7 +351,6 @@ __global__ void __launch_bounds__(256) ssd_state_passing_kernel(const mb200_ssd_
 }
 
 // ---- stage 4 ------------------------------------------------------------------------------------
-template <typename T>
 __global__ void __launch_bounds__(kT, 4) ssd_cb_kernel(const mb200_ssd_args a, float *cb, int nchunks)
 {
     __shared__ TileSmem sm;
@@ -379,8 +361,8 @@ __global__ void __launch_bounds__(kT, 4) ssd_cb_kernel(const mb200_ssd_args a, f
     const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, g = blockIdx.z;
     const int t0 = c * Q;
     const int len = min(Q, a.seqlen - t0);
-    const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
-    const T *B = static_cast<const T *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
+    const float *C = static_cast<const float *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
+    const float *B = static_cast<const float *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
     const bool vC = rows_of_4(C, 0, a.C_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
     uint64_t acc[4][4] = {};
     tile_gemm<true, true>(
@@ -403,7 +385,6 @@ __global__ void __launch_bounds__(kT, 4) ssd_cb_kernel(const mb200_ssd_args a, f
 }
 
 // ---- stage 5 ------------------------------------------------------------------------------------
-template <typename T>
 __global__ void __launch_bounds__(kT, 4) ssd_chunk_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb,
                                                             const float *states, const float *cb, int nchunks)
 {
@@ -418,8 +399,8 @@ __global__ void __launch_bounds__(kT, 4) ssd_chunk_scan_kernel(const mb200_ssd_a
     if (m0 >= len) return;
     const float *dtc = dtb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
     const float *dAc = dAb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
-    const T *x = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
+    const float *x = static_cast<const float *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
+    const float *C = static_cast<const float *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
     const float *prev = states + (((int64_t)b * nchunks + c) * a.nheads + h) * (int64_t)P * N;
     const float *cbc = cb + (((int64_t)b * nchunks + c) * a.ngroups + g) * (int64_t)Q * Q;
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -459,8 +440,8 @@ __global__ void __launch_bounds__(kT, 4) ssd_chunk_scan_kernel(const mb200_ssd_a
         },
         [&](int k, int j) { return load4(x + (int64_t)k * a.x_stride[1] + p0 + j, vx, k < kend ? P - p0 - j : 0); }, sm);
 
-    const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + (int64_t)t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] : nullptr;
-    T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + (int64_t)t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2];
+    const float *z = a.z ? static_cast<const float *>(a.z) + (int64_t)b * a.z_stride[0] + (int64_t)t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] : nullptr;
+    float *out = static_cast<float *>(a.out) + (int64_t)b * a.out_stride[0] + (int64_t)t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2];
     const bool vz = z && rows_of_4(z, 0, a.z_stride[1], 0), vo = rows_of_4(out, 0, a.out_stride[1], 0);
     const int p = p0 + tx * 4, np = P - p;
     if (np <= 0) return;
@@ -490,7 +471,6 @@ __global__ void __launch_bounds__(kT, 4) ssd_chunk_scan_kernel(const mb200_ssd_a
 // ---- packed sequences: state after the last token of each one ------------------------------------
 // A 64 x 64 tile of one (sequence, head): the contribution of the sequence's steps inside the chunk that holds its last
 // token, plus the state entering that chunk if the sequence began earlier.
-template <typename T>
 __global__ void __launch_bounds__(kT, 4) ssd_varlen_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, int nchunks)
 {
     __shared__ TileSmem sm;
@@ -506,8 +486,8 @@ __global__ void __launch_bounds__(kT, 4) ssd_varlen_state_kernel(const mb200_ssd
     const float *dtc = dtb + ((int64_t)h * nchunks + c) * Q + (first - t0);
     const float *dAc = dAb + ((int64_t)h * nchunks + c) * Q + (first - t0);
     const float dA_end = empty ? 0.f : dAc[end - 1 - first];
-    const T *x = static_cast<const T *>(a.x) + (int64_t)first * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const T *B = static_cast<const T *>(a.B) + (int64_t)first * a.B_stride[1] + (int64_t)g * a.B_stride[2];
+    const float *x = static_cast<const float *>(a.x) + (int64_t)first * a.x_stride[1] + (int64_t)h * a.x_stride[2];
+    const float *B = static_cast<const float *>(a.B) + (int64_t)first * a.B_stride[1] + (int64_t)g * a.B_stride[2];
     const bool vx = rows_of_4(x, 0, a.x_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
     const int steps = empty ? 0 : end - first;
     uint64_t acc[4][4] = {};
@@ -570,8 +550,6 @@ __global__ void ssd_fold_ranges_kernel(const float *summaries, int64_t record_st
     }
 }
 
-// `a` and `lay` are in the chunks the path works in: the caller's on the general path, kTcChunk on the tensor-core path.
-template <typename T>
 int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {
     char *base = static_cast<char *>(a.scratch);
@@ -606,7 +584,14 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
     // The LOCAL half took the streaming launch but this OUTPUT half cannot use its 16-bit entering states: the
     // scratch holds no fp32 chunk states, so they are formed here before the recurrence.
     const bool local_streamed = !has_local && fused_states && !tc_out;
-    const int tq = (Q + 63) / 64;
+    const bool split = a.io_dtype != MB200_F32;       // the general stages for 16-bit inputs
+    const int tq = (Q + 63) / 64, tp = (a.headdim + 63) / 64, tn = (a.dstate + 63) / 64;
+    auto form_cb = [&]() -> int {
+        if (split) return ssd_split_cb(a, lay, stream);
+        ssd_cb_kernel<<<dim3(tq * tq, a.batch * nc, a.ngroups), kT, 0, stream>>>(a, cb, nc);
+        MB200_CHECK_LAUNCH("ssd chunk_cb");
+        return MB200_OK;
+    };
     auto state_passing = [&](const mb200_ssd_args &p, bool write_prev, void *to16) {
         if (PN % 4 == 0)
             ssd_state_passing_kernel<4><<<dim3((unsigned)((PN / 4 + 255) / 256), a.nheads, a.batch), 256, 0, stream>>>(p, dAb, states, nc, write_prev, to16);
@@ -633,17 +618,16 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
         const cudaError_t ce = a.dt_dtype == MB200_F32 ? cumsum(float{}) : a.dt_dtype == MB200_BF16 ? cumsum(__nv_bfloat16{}) : cumsum(__half{});
         if (ce != cudaSuccess) return fail(MB200_ERR_LAUNCH, "ssd chunk_cumsum: shared memory opt-in: %s", cudaGetErrorString(ce));
         MB200_CHECK_LAUNCH("ssd chunk_cumsum");
-        if (cb_early) {
-            ssd_cb_kernel<T><<<dim3(tq * tq, a.batch * nc, a.ngroups), kT, 0, stream>>>(a, cb, nc);
-            MB200_CHECK_LAUNCH("ssd chunk_cb");
-        }
+        if (cb_early)
+            if (int rc = form_cb()) return rc;
         if (fused_states) {
             if (int rc = ssd_tc_state_stream(a, lay, stream)) return rc;
         } else if (tc_loc) {
             if (int rc = ssd_tc_chunk_state(a, lay, stream)) return rc;
+        } else if (split) {
+            if (int rc = ssd_split_states(a, lay, stream)) return rc;
         } else {
-            ssd_chunk_state_kernel<T><<<dim3(((a.headdim + 63) / 64) * ((a.dstate + 63) / 64), a.batch * nc, a.nheads), kT, 0, stream>>>(
-                a, dtb, dAb, states, nc);
+            ssd_chunk_state_kernel<<<dim3(tp * tn, a.batch * nc, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, nc);
             MB200_CHECK_LAUNCH("ssd chunk_state");
         }
         if (!fused_states && !has_out && (a.final_states || a.range_decay)) {
@@ -672,18 +656,23 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
         if (tc_out) {
             if (int rc = ssd_tc_output(a, lay, fused_states, stream)) return rc;
             if (varlen)
-                if (int rc = ssd_tc_varlen(a, lay, fused_states, stream)) return rc;
+                if (int rc = a.io_dtype == MB200_BF16 ? ssd_tc_varlen(a, lay, fused_states, stream)
+                                                      : ssd_split_varlen(a, lay, fused_states ? SsdStates::np16 : SsdStates::pn16, stream))
+                    return rc;
         } else {
-            if (!cb_ready) {
-                ssd_cb_kernel<T><<<dim3(tq * tq, a.batch * nc, a.ngroups), kT, 0, stream>>>(a, cb, nc);
-                MB200_CHECK_LAUNCH("ssd chunk_cb");
-            }
-            ssd_chunk_scan_kernel<T><<<dim3(tq * ((a.headdim + 63) / 64), a.batch * nc, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, cb, nc);
-            MB200_CHECK_LAUNCH("ssd chunk_scan");
-            if (varlen) {
-                ssd_varlen_state_kernel<T><<<dim3(((a.headdim + 63) / 64) * ((a.dstate + 63) / 64), a.num_seqs, a.nheads), kT, 0, stream>>>(a, dtb, dAb,
-                                                                                                                                          states, nc);
-                MB200_CHECK_LAUNCH("ssd varlen states");
+            if (!cb_ready)
+                if (int rc = form_cb()) return rc;
+            if (split) {
+                if (int rc = ssd_split_scan(a, lay, stream)) return rc;
+                if (varlen)
+                    if (int rc = ssd_split_varlen(a, lay, SsdStates::pn32, stream)) return rc;
+            } else {
+                ssd_chunk_scan_kernel<<<dim3(tq * tp, a.batch * nc, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, cb, nc);
+                MB200_CHECK_LAUNCH("ssd chunk_scan");
+                if (varlen) {
+                    ssd_varlen_state_kernel<<<dim3(tp * tn, a.num_seqs, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, nc);
+                    MB200_CHECK_LAUNCH("ssd varlen states");
+                }
             }
         }
     }
@@ -715,7 +704,7 @@ extern "C" int mb200_ssd_scratch_bytes(const mb200_ssd_args *args, size_t *bytes
     using namespace mb200;
     if (!args || !bytes) return fail(MB200_ERR_BAD_ARG, "ssd_scratch_bytes: NULL argument");
     if (int rc = check_ssd(*args)) return rc;
-    *bytes = ssd_scratch_layout(*args, args->chunk_size).total;
+    *bytes = ssd_scratch_layout(*args).total;
     return MB200_OK;
 }
 
@@ -723,7 +712,7 @@ extern "C" int mb200_ssd_chunk_scan_fwd(const mb200_ssd_args *args, void *stream
 {
     using namespace mb200;
     if (!args) return fail(MB200_ERR_BAD_ARG, "ssd_chunk_scan_fwd: args is NULL");
-    mb200_ssd_args a = *args;
+    const mb200_ssd_args &a = *args;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (int rc = check_ssd(a)) return rc;
     MB200_CHECK_ARG(!(a.phases & MB200_SSD_PHASE_OUTPUT) || a.out || a.seqlen == 0 || a.batch == 0, "ssd: out is NULL");
@@ -755,15 +744,10 @@ extern "C" int mb200_ssd_chunk_scan_fwd(const mb200_ssd_args *args, void *stream
         }
         return MB200_OK;
     }
-    const bool whole = (a.phases & MB200_SSD_PHASE_ALL) == MB200_SSD_PHASE_ALL;
-    const bool tc = whole && ssd_tc_local_eligible(a) && ssd_tc_output_eligible(a);
-    const SsdScratch lay = ssd_scratch_layout(a, tc ? kTcChunk : a.chunk_size);
-    if (tc) a.chunk_size = kTcChunk;        // the layout is in the path's chunks; sizes were checked against the caller's
+    const SsdScratch lay = ssd_scratch_layout(a);
     MB200_CHECK_ARG(a.scratch && a.scratch_bytes >= lay.total, "ssd: scratch too small (%zu < %zu bytes)", a.scratch_bytes, lay.total);
     MB200_CHECK_ARG((reinterpret_cast<uintptr_t>(a.scratch) & 255) == 0, "ssd: scratch must be 256-byte aligned");
-    if (a.io_dtype == MB200_F32) return run_ssd<float>(a, lay, stream);
-    if (a.io_dtype == MB200_BF16) return run_ssd<__nv_bfloat16>(a, lay, stream);
-    return run_ssd<__half>(a, lay, stream);
+    return run_ssd(a, lay, stream);
 }
 
 // ---- the variant that allocates nothing ---------------------------------------------------------------
@@ -777,7 +761,7 @@ extern "C" int mb200_ssd_chunk_scan_fwd_static(const mb200_ssd_args *args, void 
     using namespace mb200;
     if (!args) return fail(MB200_ERR_BAD_ARG, "ssd_chunk_scan_fwd_static: args is NULL");
     if (int rc = check_ssd(*args)) return rc;
-    const size_t need = ssd_scratch_layout(*args, args->chunk_size).total;
+    const size_t need = ssd_scratch_layout(*args).total;
     if (need > MB200_SSD_STATIC_SCRATCH_BYTES)
         return fail(MB200_ERR_BAD_ARG,
                     "ssd_chunk_scan_fwd_static: this problem needs %zu bytes of intermediates, the built-in buffer holds %u; "
@@ -806,7 +790,7 @@ extern "C" int mb200_ssd_static_status(const mb200_ssd_args *args, int *status)
     using namespace mb200;
     if (!args || !status) return fail(MB200_ERR_BAD_ARG, "ssd_static_status: NULL argument");
     if (int rc = check_ssd(*args)) return rc;
-    const SsdScratch lay = ssd_scratch_layout(*args, args->chunk_size);
+    const SsdScratch lay = ssd_scratch_layout(*args);
     if (lay.total > MB200_SSD_STATIC_SCRATCH_BYTES) return fail(MB200_ERR_BAD_ARG, "ssd_static_status: this problem does not fit the built-in buffer");
     if (int rc = enter_device(args->device)) return rc;
     // synchronises with the device: a diagnostic, not part of the hot path

@@ -15,10 +15,9 @@ bool ssd_tc_shape(const mb200_ssd_args &a);
 //   dA_cum  (batch, nheads, nchunks, Q)        inclusive cumsum of dt*A inside each chunk
 //   states  (batch, nchunks, nheads, P, N)     chunk states; the inter-chunk recurrence then
 //                                              overwrites slot c with the state ENTERING chunk c
-//   cb      (batch, nchunks, ngroups, Q, Q)    C.B^T per chunk (lower block triangle only) of the general kernels
-//   prev16  (batch, nchunks, nheads, P, N)     16-bit copy of the state entering each chunk (tensor-core path);
-//                                              [n][p] tiles of 64 columns and 64 or 128 states when the fused
-//                                              state-stream kernel wrote it
+//   cb      (batch, nchunks, ngroups, Q, Q)    C.B^T per chunk (lower block triangle only) of the general stages
+//   prev16  (batch, nchunks, nheads, P, N)     16-bit copy of the state entering each chunk (tensor-core path); [n][p]
+//                                              tiles when the fused state-stream kernel wrote it
 //   aux     sequence-split hand-over of the fused state-stream path, written by the LOCAL phase for the OUTPUT
 //           phase: prefix decay (batch, nheads, nchunks), the range's end state from a zero incoming state
 //           (batch, nheads, P, N) and the range decay (batch, nheads)
@@ -27,7 +26,6 @@ bool ssd_tc_shape(const mb200_ssd_args &a);
 //           sequence that ended the previous chunk (batch, nchunks) uint8
 //   status  one int32 in the last 256 bytes    0 after a clean run; a kernel that gave up a bounded wait
 //                                              leaves its code here (the output is then invalid)
-// The general stages work in the caller's chunks, the tensor-core stages in chunks of 256; the size asked for holds either.
 struct SsdScratch {
     size_t off_dt, off_dA, off_states, off_cb, off_prev16, off_aux, off_aux_state, off_aux_decay, off_seq_start, off_seq_carry, off_status, total;
     int nchunks;
@@ -35,37 +33,25 @@ struct SsdScratch {
 
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-inline SsdScratch ssd_scratch_regions(const mb200_ssd_args &a, int Q)
+inline SsdScratch ssd_scratch_layout(const mb200_ssd_args &a)
 {
     SsdScratch s;
+    const int Q = a.chunk_size;
     s.nchunks = (a.seqlen + Q - 1) / Q;
-    const size_t bc = (size_t)a.batch * s.nchunks, tile = (size_t)((a.headdim + 63) / 64 * 64) * ((a.dstate + 63) / 64 * 64);
+    const size_t bc = (size_t)a.batch * s.nchunks;
     const size_t per = (size_t)a.batch * a.nheads * s.nchunks * Q * sizeof(float);
     s.off_dt = 0;
     s.off_dA = align256(s.off_dt + per);
     s.off_states = align256(s.off_dA + per);
     s.off_cb = align256(s.off_states + bc * a.nheads * a.headdim * a.dstate * sizeof(float));
     s.off_prev16 = align256(s.off_cb + bc * a.ngroups * Q * Q * sizeof(float));
-    s.off_aux = align256(s.off_prev16 + (a.io_dtype == MB200_F32 ? 0 : bc * a.nheads * tile * 2));
+    s.off_aux = align256(s.off_prev16 + (ssd_tc_shape(a) ? bc * a.nheads * a.headdim * a.dstate * 2 : 0));
     s.off_aux_state = align256(s.off_aux + (size_t)a.batch * a.nheads * s.nchunks * sizeof(float));
     s.off_aux_decay = align256(s.off_aux_state + (size_t)a.batch * a.nheads * a.headdim * a.dstate * sizeof(float));
     s.off_seq_start = align256(s.off_aux_decay + (size_t)a.batch * a.nheads * sizeof(float));
     s.off_seq_carry = align256(s.off_seq_start + bc * Q);
     s.off_status = align256(s.off_seq_carry + bc);
     s.total = s.off_status + 256;
-    return s;
-}
-
-// Regions for chunks of Q steps; `total` and the place of the status word depend on the sizes of the call only.
-inline SsdScratch ssd_scratch_layout(const mb200_ssd_args &a, int Q)
-{
-    SsdScratch s = ssd_scratch_regions(a, Q);
-    s.total = ssd_scratch_regions(a, a.chunk_size).total;
-    if (a.chunk_size != kTcChunk && ssd_tc_shape(a)) {
-        const size_t t = ssd_scratch_regions(a, kTcChunk).total;
-        if (t > s.total) s.total = t;
-    }
-    s.off_status = s.total - 256;
     return s;
 }
 
@@ -77,8 +63,7 @@ inline int *ssd_status_word(const mb200_ssd_args &a, const SsdScratch &lay)
 
 // Tensor-core stages (ssd_tc.cu): whether the call qualifies, and the launches.  The LOCAL stages read
 // x, B and dt only; the OUTPUT stage adds C, z and out.  Each predicate looks at nothing else, so the two halves
-// of a sequence split agree on how the LOCAL half ran although they are handed different C / z / out.  All of them expect
-// chunk_size == kTcChunk in the arguments and in the layout.
+// of a sequence split agree on how the LOCAL half ran although they are handed different C / z / out.
 bool ssd_tc_local_eligible(const mb200_ssd_args &a);
 bool ssd_tc_output_eligible(const mb200_ssd_args &a);
 bool ssd_tc_cb_eligible(const mb200_ssd_args &a);      // C as the output kernel needs it
@@ -88,9 +73,18 @@ int ssd_tc_chunk_state(const mb200_ssd_args &a, const SsdScratch &lay, cudaStrea
 bool ssd_tc_stream_eligible(const mb200_ssd_args &a);
 int ssd_tc_state_stream(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
 int ssd_tc_output(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream);
-int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream);
+int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream);      // bf16 only
 // OUTPUT phase of a sequence split on that path: adds the incoming state's share to the entering states the LOCAL
 // phase left (H_c += prefix_decay_c * S_in) and forms the range's end state.
 int ssd_tc_apply_incoming(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
+
+// The general stages for 16-bit inputs (ssd_split.cu): chunk states, C.B^T, chunk outputs.  They read and write what the general stages
+// for fp32 do.  And the end states of packed sequences, from entering states of any form: fp32 or 16-bit in [p][n] order, or the 16-bit
+// [n][p] tiles of the state stream.
+enum class SsdStates { pn32, pn16, np16 };
+int ssd_split_states(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
+int ssd_split_cb(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
+int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
+int ssd_split_varlen(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates entering, cudaStream_t stream);
 
 }  // namespace mb200

@@ -9,7 +9,7 @@
 //   chunk_state / state_stream   S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_last - dA_k, 0)) dt_k, per chunk, and
 //               the recurrence over chunks (fused in state_stream); leave the state entering each chunk in 16 bits
 //   output      per chunk and group, over its heads: C.B^T, the decay-masked product with x, C.H, the D skip and the gate
-//   varlen      end states of packed sequences
+//   varlen      end states of packed sequences (bf16)
 //
 // Every mbarrier wait is bounded: on expiry the kernel records a code in the status word, skips the dependent work and
 // still releases its TMEM before it exits.
@@ -1106,25 +1106,25 @@ bool rows_for_tma(const void *p, const int64_t *s)
 }
 
 // ====================================================================================== end states of packed sequences
-// One CTA per (head slice, sequence): S^T[n,p] = sum over the sequence's steps in the chunk of its last token, plus the state
-// entering that chunk if the sequence began earlier.  The weighted x rows are split into a 16-bit value and a 16-bit remainder
-// (two MMAs per step of 16 rows), so the fp32 result keeps fp32-like products; B is exact as it is.  Halves of 128 rows that
-// hold no step of the sequence are skipped.  The one-thread-per-element form of this (dot products over the steps, every
-// operand re-read from L1 for each of the 8192 elements) took 2.5 ms for 23 sequences x 80 heads, twenty times the scan itself;
-// this takes 0.043 ms (0.092 when the entering state was read in the epilogue, element by element across 32 lines).
+// One CTA per (head, sequence): S^T[n,p] = sum over the sequence's steps in the chunk of its last token, plus the state entering that
+// chunk if the sequence began earlier.  bf16 inputs: the weighted x rows are cut into three bf16 values, so that the fp32 result keeps
+// fp32 products; B is exact as it is.  (Half precision would need its B cut as well: ssd_split.cu does that.)  The small products have
+// a sum of their own, which keeps the tensor core's rounding of sums out of them.  Halves of 128 rows that hold no step of the sequence are skipped.
+// 23 sequences x 80 heads, us, the wait for the launch before it included: 72; 54 with two parts and one sum, 83 with the 64-step tiles of
+// ssd_split.cu, 2500 with one thread per element.
 constexpr int kVarThreads = 288;
-template <typename T, int NH>
 __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
                                                                     const float *dtb, const float *dAb, const int32_t *cu_seqlens, float *varlen,
-                                                                    const T *prev16, int prev_np, int nchunks, int nheads, int pslices, int headdim,
-                                                                    int dstate, int heads_per_group, int seqlen, int *status)
+                                                                    const __nv_bfloat16 *prev16, int prev_np, int nchunks, int nheads, int heads_per_group,
+                                                                    int seqlen, int *status)
 {
+    using T = __nv_bfloat16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *sm = align1024(smem_raw);
-    uint8_t *Bs = sm, *xs = sm + NH * 16384, *xlo = xs + 16384;       // B boxes [128 x 64], x [128 x 64] and its remainder
-    uint64_t *bars = reinterpret_cast<uint64_t *>(xlo + 16384);
+    uint8_t *Bs = sm, *xs = sm + 2 * 16384;                    // B boxes [128 x 64]; x [128 x 64] in three parts
+    uint64_t *bars = reinterpret_cast<uint64_t *>(xs + 3 * 16384);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3);
-    const int vh = blockIdx.x, h = vh / pslices, pv = (vh % pslices) * 64, sq = blockIdx.y;
+    const int h = blockIdx.x, sq = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int start = cu_seqlens[sq], end = cu_seqlens[sq + 1];
     const bool empty = end <= start || end > seqlen || start < 0;
@@ -1136,7 +1136,7 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
         mbar_init(&bars[2], 1);      // MMAs done
         mbar_fence_init();
     }
-    if (warp == 8) tmem_alloc(tmem_slot, 64);
+    if (warp == 8) tmem_alloc(tmem_slot, 128);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -1146,8 +1146,8 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
     const float dA_end = empty ? 0.f : dAc[k1 - 1];
     // my part of the state that enters the chunk (a row of its [n][p] tile; asked for now, needed last)
     const int n = (warp & 3) * 32 + lane, p0 = ((warp >> 2) & 1) * 32;
-    const bool entering = !empty && start < t0 && warp < 8 && n < dstate;
-    const T *H = prev16 + ((int64_t)c * nheads * pslices + vh) * (prev_np ? NH * 64 * 64 : 64 * dstate);
+    const bool entering = !empty && start < t0 && warp < 8;
+    const T *H = prev16 + ((int64_t)c * nheads + h) * (kP * kN);
     uint4 hv[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) hv[q] = entering && prev_np ? reinterpret_cast<const uint4 *>(H + n * 64 + p0)[q] : make_uint4(0, 0, 0, 0);
@@ -1158,20 +1158,20 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
         if (k1 <= half * 128 || k0 >= half * 128 + 128) continue;
         if (warp == 8) {
             if (lane == 0) {
-                mbar_expect_tx(&bars[0], NH * 16384 + 16384);
-                tma_load_4d(xs, &tm_x, &bars[0], pv, h, t0 + half * 128, 0);
-                for (int kb = 0; kb < NH; ++kb) tma_load_4d(Bs + kb * 16384, &tm_B, &bars[0], kb * 64, h / heads_per_group, t0 + half * 128, 0);
+                mbar_expect_tx(&bars[0], 3 * 16384);
+                tma_load_4d(xs, &tm_x, &bars[0], 0, h, t0 + half * 128, 0);
+                for (int kb = 0; kb < 2; ++kb) tma_load_4d(Bs + kb * 16384, &tm_B, &bars[0], kb * 64, h / heads_per_group, t0 + half * 128, 0);
             }
             __syncwarp();
             ok = __all_sync(0xffffffffu, mbar_wait(&bars[1], round & 1, status, kStBarScaled) && mbar_wait(&bars[0], round & 1, status, kStBarB));
             tc_fence_after_sync();
-            const uint32_t idesc = instr_desc_f16(128, 64, Fmt<T>::v, 1, 1), tm = warp_uniform(tmem);
+            const uint32_t idesc = instr_desc_f16(128, 64, 1, 1, 1), tm = warp_uniform(tmem);
             const uint64_t dB = smem_desc_sw128(smem_u32(Bs), 16384, 1024), dx = smem_desc_sw128(smem_u32(xs), 16, 1024);
             if (elect_one()) {
                 if (ok) {
 #pragma unroll 1
-                    for (int part = 0; part < 2; ++part)
-                        mma_steps_ss(8, tm, dB, 128, dx + part * (16384 / 16), 128, idesc, round > 0 || part > 0);
+                    for (int part = 0; part < 3; ++part)
+                        mma_steps_ss(8, part ? tm + 64 : tm, dB, 128, dx + part * (16384 / 16), 128, idesc, round > 0 || part == 2);
                 }
                 mma_commit(&bars[2]);
             }
@@ -1179,25 +1179,45 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(&bars[2], round & 1, status, kStBarDone)) && ok;
         } else {
             const int r = threadIdx.x >> 1, k = half * 128 + r, cq = (threadIdx.x & 1) * 4;      // two threads per row
-            const float w = k >= k0 && k < k1 ? __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k] : 0.f;
+            const bool mine = k >= k0 && k < k1;
+            const float w = mine ? __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k] : 0.f;
             ok = mbar_wait(&bars[0], round & 1, status, kStBarX);
+            // where B is infinite the later parts of x, which may have the other sign or be zero, are made tiny and of the first one's
+            bool bad = false;
+            if (ok) {
+#pragma unroll
+                for (int ch = 0; ch < 8; ++ch) {
+                    const uint4 v = lds128(smem_u32(Bs) + (ch & 4) * 4096 + r * 128 + (((cq + (ch & 3)) ^ (r & 7)) << 4));
+                    const uint32_t m = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
+                    bad = bad || (m & 0xffffu) >= 0x7f80u || (m >> 16) >= 0x7f80u;
+                }
+            }
+            bad = __shfl_xor_sync(0xffffffffu, bad, 1) || bad;
             if (ok) {
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch) {
                     const uint32_t off = r * 128 + (((cq + ch) ^ (r & 7)) << 4);
-                    const uint4 v = lds128(smem_u32(xs) + off);
+                    if (!mine) {        // steps of other sequences count for nothing, infinite B included
+                        sts128(smem_u32(Bs) + off, make_uint4(0, 0, 0, 0));
+                        sts128(smem_u32(Bs) + 16384 + off, make_uint4(0, 0, 0, 0));
+                    }
+                    const uint4 v = mine ? lds128(smem_u32(xs) + off) : make_uint4(0, 0, 0, 0);
                     const uint32_t e[4] = {v.x, v.y, v.z, v.w};
-                    uint32_t hi[4], lo[4];
+                    uint32_t part[3][4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const float2 f = Pack2<T>::unpack(e[q]);
-                        const float a0 = w == 0.f ? 0.f : f.x * w, a1 = w == 0.f ? 0.f : f.y * w;
-                        hi[q] = Pack2<T>::pack(a0, a1);
-                        const float2 g = Pack2<T>::unpack(hi[q]);
-                        lo[q] = Pack2<T>::pack(a0 - g.x, a1 - g.y);
+                        float a0 = f.x * w, a1 = f.y * w;
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) {
+                            part[p][q] = bad && p > 0 ? (part[0][q] & 0x80008000u) | 0x01000100u : Pack2<T>::pack(a0, a1);
+                            const float2 g = Pack2<T>::unpack(part[p][q]);
+                            a0 = isinf(g.x) ? 0.f : a0 - g.x;
+                            a1 = isinf(g.y) ? 0.f : a1 - g.y;
+                        }
                     }
-                    sts128(smem_u32(xs) + off, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-                    sts128(smem_u32(xlo) + off, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) sts128(smem_u32(xs) + p * 16384 + off, make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]));
                 }
             }
             fence_proxy_async();
@@ -1212,26 +1232,30 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = 0.f;
         tc_fence_after_sync();
-        if (round > 0 && __all_sync(0xffffffffu, ok)) tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + p0, v);   // warp-collective
-        if (n < dstate) {
-            const float carry = __expf(dA_end);
-            const uint32_t hw[16] = {hv[0].x, hv[0].y, hv[0].z, hv[0].w, hv[1].x, hv[1].y, hv[1].z, hv[1].w,
-                                     hv[2].x, hv[2].y, hv[2].z, hv[2].w, hv[3].x, hv[3].y, hv[3].z, hv[3].w};
-            float *dst = varlen + (((int64_t)sq * nheads + h) * headdim + pv + p0) * dstate + n;
+        if (round > 0 && __all_sync(0xffffffffu, ok)) {      // tcgen05.ld is warp-collective
+            const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + p0;
+            float rest[32];
+            tmem_ld32(at, v);
+            tmem_ld32(at + 64, rest);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                if (pv + p0 + j >= headdim) continue;
-                if (entering) {
-                    const float2 f = Pack2<T>::unpack(hw[j >> 1]);
-                    v[j] = fmaf(prev_np ? (j & 1 ? f.y : f.x) : to_float(H[(p0 + j) * dstate + n]), carry, v[j]);
-                }
-                dst[j * dstate] = v[j];
+            for (int j = 0; j < 32; ++j) v[j] += rest[j];
+        }
+        const float carry = __expf(dA_end);
+        const uint32_t hw[16] = {hv[0].x, hv[0].y, hv[0].z, hv[0].w, hv[1].x, hv[1].y, hv[1].z, hv[1].w,
+                                 hv[2].x, hv[2].y, hv[2].z, hv[2].w, hv[3].x, hv[3].y, hv[3].z, hv[3].w};
+        float *dst = varlen + (((int64_t)sq * nheads + h) * kP + p0) * kN + n;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            if (entering) {
+                const float2 f = Pack2<T>::unpack(hw[j >> 1]);
+                v[j] = fmaf(prev_np ? (j & 1 ? f.y : f.x) : to_float(H[(p0 + j) * kN + n]), carry, v[j]);
             }
+            dst[j * kN] = v[j];
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 8) tmem_dealloc(tmem, 64);
+    if (warp == 8) tmem_dealloc(tmem, 128);
 }
 
 // ====================================================================================== host
@@ -1373,18 +1397,16 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     return MB200_OK;
 }
 
-template <typename T, int NH>
 int run_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaStream_t stream)
 {
     const TcCall k = tc_call(a, lay);
     CUtensorMap tx, tB;
-    if (!map_rows(&tx, Fmt<T>::v, a.x, a.x_stride, a.headdim, a.nheads, a, 128) || !map_rows(&tB, Fmt<T>::v, a.B, a.B_stride, a.dstate, a.ngroups, a, 128))
+    if (!map_rows(&tx, 1, a.x, a.x_stride, a.headdim, a.nheads, a, 128) || !map_rows(&tB, 1, a.B, a.B_stride, a.dstate, a.ngroups, a, 128))
         return fail(MB200_ERR_LAUNCH, "ssd: tensor map for x or B failed");
-    constexpr int smem = (NH + 2) * 16384 + 64 + 1024;
-    ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_varlen_kernel<T, NH>), smem, a.device);
-    launch_dependent(ssd_tc_varlen_kernel<T, NH>, dim3(k.vheads, a.num_seqs), kVarThreads, smem, stream,
-        tx, tB, k.dtb, k.dAb, a.cu_seqlens, a.varlen_states, static_cast<const T *>(k.prev16), h_np ? 1 : 0, k.nc, a.nheads, k.ps, a.headdim, a.dstate,
-        a.nheads / a.ngroups, a.seqlen, k.status);
+    constexpr int smem = 5 * 16384 + 64 + 1024;
+    ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_varlen_kernel), smem, a.device);
+    launch_dependent(ssd_tc_varlen_kernel, dim3(a.nheads, a.num_seqs), kVarThreads, smem, stream, tx, tB, k.dtb, k.dAb, a.cu_seqlens, a.varlen_states,
+                     static_cast<const __nv_bfloat16 *>(k.prev16), h_np ? 1 : 0, k.nc, a.nheads, a.nheads / a.ngroups, a.seqlen, k.status);
     MB200_CHECK_LAUNCH("ssd varlen states (tensor core)");
     return MB200_OK;
 }
@@ -1403,9 +1425,7 @@ template <class F> int with_types(const mb200_ssd_args &a, F f)
 bool ssd_tc_shape(const mb200_ssd_args &a)
 {
     if (a.io_dtype != MB200_BF16 && a.io_dtype != MB200_F16) return false;
-    // the halves of a sequence split hand each other chunk-wise intermediates: one shape, chunks of 256
-    if ((a.phases & MB200_SSD_PHASE_ALL) != MB200_SSD_PHASE_ALL) return a.headdim == kP && a.dstate == kN && a.chunk_size == kTcChunk;
-    return a.headdim % 8 == 0 && a.headdim <= 256 && a.dstate % 8 == 0 && a.dstate <= kN;
+    return a.headdim == kP && a.dstate == kN && a.chunk_size == kQ;
 }
 
 bool ssd_tc_local_eligible(const mb200_ssd_args &a)
@@ -1444,10 +1464,7 @@ int ssd_tc_output(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np
     return with_types(a, [&](auto t, auto nh) { return run_output<decltype(t), decltype(nh)::value>(a, lay, states_np, stream); });
 }
 
-int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream)
-{
-    return with_types(a, [&](auto t, auto nh) { return run_varlen<decltype(t), decltype(nh)::value>(a, lay, states_np, stream); });
-}
+int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream) { return run_varlen(a, lay, states_np, stream); }
 
 template <typename T>
 int run_incoming(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)

@@ -454,9 +454,9 @@ def mamba_chunk_scan_combined(x, dt, A, B, C, chunk_size, D=None, z=None, dt_bia
     Returns ``out``, ``(out, final_states)``, ``(out, varlen_states)`` or ``(out, final_states, varlen_states)``
     like the reference; final_states fp32 (batch, nheads, headdim, dstate), varlen_states fp32
     (num_sequences, nheads, headdim, dstate).  ``state_dtype`` is accepted for signature compatibility and not
-    used: the running inter-chunk state is fp32 on chip; the copy of it that the chunk-output stage multiplies by C
-    is rounded to the input dtype on the tensor-core path (as the reference's default does) and stays fp32 on the
-    general path.
+    used: the running inter-chunk state is fp32 on chip.  16-bit calls of headdim 64, dstate 128 and chunk_size 256
+    round weights, decays and the copy of the state that is multiplied by C to the input dtype (as the reference's
+    default does); all others round nothing but the result.
     """
     res = L.host().ssd_fwd(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, seq_idx, cu_seqlens, dt_softplus, dt_limit,
                            return_final_states, return_varlen_states)

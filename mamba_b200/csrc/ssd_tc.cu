@@ -1,10 +1,7 @@
 // Tensor-core stages of the SSD chunked forward for sm_100a: tcgen05.mma with TMEM accumulators,
 // operands brought into 128-byte-swizzled shared memory by TMA (cp.async.bulk.tensor, no multicast).
 //
-// Shapes served here: 16-bit inputs (bf16 / fp16), dstate <= 128 and headdim <= 256, both multiples of 8 (one tile row of
-// TMA is 16 bytes).  States are padded to 64 or 128 by TMA's zero fill, a head is walked in slices of 64 columns that share
-// its decays.  The chunk is always 256 steps: the result does not depend on where a sequence is cut, so the caller's
-// chunk_size only sets the granularity of a sequence split.  Kernels:
+// The shape served here: 16-bit inputs (bf16 / fp16), headdim 64, dstate 128, chunks of 256 steps.  Kernels:
 //
 //   chunk_state / state_stream   S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_last - dA_k, 0)) dt_k, per chunk, and
 //               the recurrence over chunks (fused in state_stream); leave the state entering each chunk in 16 bits
@@ -34,7 +31,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int kQ = kTcChunk, kP = 64, kN = 128;  // steps per chunk; columns of a head slice; most states
+constexpr int kQ = kTcChunk, kP = 64, kN = 128;  // steps per chunk, columns of a head, states
 
 // status codes written to the scratch status word
 enum { kStBarB = 11, kStBarX, kStBarScaled, kStBarDone, kStSmemAlign };
@@ -115,25 +112,24 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v)
 }
 
 // ====================================================================================== chunk state
-// grid (head slices, nchunks, batch), 288 threads.  smem: B NH x 32 KB (n halves, [256 k x 64 n]), x 32 KB.  With NH = 1 the
-// second half of A's 128 rows is read from the x tile that follows: rows of S^T that nobody stores.
+// grid (nheads, nchunks, batch), 288 threads.  smem: B 2 x 32 KB (n halves, [256 k x 64 n]), x 32 KB.
 // TMEM: 64 columns.  S^T[n,p] = sum_k B[k,n] (w_k x[k,p]): the per-step weight w_k is applied to the x rows
 // (half as many elements as B, and x is per head anyway), one row per thread, in place, fp32 product with
 // one rounding; B is used as TMA delivered it.
 constexpr int kStateThreads = 288;
-template <typename T, int NH>
+template <typename T>
 __global__ void __launch_bounds__(kStateThreads) ssd_tc_chunk_state_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
                                                                           const float *dtb, const float *dAb, float *states, int nchunks,
-                                                                          int nheads, int pslices, int dstate, int heads_per_group, const int32_t *seq_idx, int seqlen,
+                                                                          int nheads, int heads_per_group, const int32_t *seq_idx, int seqlen,
                                                                           int *status)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *sm = align1024(smem_raw);
-    uint8_t *Bs = sm;               // NH boxes [256 x 64]
-    uint8_t *xs = sm + NH * 32768;       // [256 x 64]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + (NH + 1) * 32768);
+    uint8_t *Bs = sm;               // two boxes [256 x 64]
+    uint8_t *xs = sm + 65536;       // [256 x 64]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + 98304);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4);
-    const int vh = blockIdx.x, h = vh / pslices, c = blockIdx.y, b = blockIdx.z;
+    const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z;
     const int g = h / heads_per_group;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the row weight is requested before the set-up barrier so its latency hides behind it and the TMA loads
@@ -165,9 +161,9 @@ __global__ void __launch_bounds__(kStateThreads) ssd_tc_chunk_state_kernel(const
     if (warp == 8) {
         if (lane == 0) {
             mbar_expect_tx(&bars[1], 32768);
-            tma_load_4d(xs, &tm_x, &bars[1], (vh % pslices) * 64, h, c * kQ, b);
-            mbar_expect_tx(&bars[0], NH * 32768);
-            for (int kb = 0; kb < NH; ++kb) tma_load_4d(Bs + kb * 32768, &tm_B, &bars[0], kb * 64, g, c * kQ, b);
+            tma_load_4d(xs, &tm_x, &bars[1], 0, h, c * kQ, b);
+            mbar_expect_tx(&bars[0], 65536);
+            for (int kb = 0; kb < 2; ++kb) tma_load_4d(Bs + kb * 32768, &tm_B, &bars[0], kb * 64, g, c * kQ, b);
         }
         __syncwarp();
         const bool ok = __all_sync(0xffffffffu, mbar_wait(&bars[2], 0, status, kStBarScaled) && mbar_wait(&bars[0], 0, status, kStBarB));
@@ -204,14 +200,13 @@ __global__ void __launch_bounds__(kStateThreads) ssd_tc_chunk_state_kernel(const
         const bool done = mbar_wait(&bars[3], 0, status, kStBarDone);
         tc_fence_after_sync();
         if (__all_sync(0xffffffffu, ok && done)) {   // tcgen05.ld is warp-collective
-            float *S = states + (((int64_t)b * nchunks + c) * nheads * pslices + vh) * (int64_t)(kP * dstate);
+            float *S = states + (((int64_t)b * nchunks + c) * nheads + h) * (int64_t)(kP * kN);
             const int n = (warp & 3) * 32 + lane;     // TMEM lane = state index
             const int p0 = (warp >> 2) * 32;          // which half of the head's columns this warp stores
             float v[32];
             tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + p0, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (n < dstate) S[(p0 + j) * dstate + n] = v[j];
+            for (int j = 0; j < 32; ++j) S[(p0 + j) * kN + n] = v[j];
         }
     }
     tc_fence_before_sync();
@@ -237,23 +232,22 @@ constexpr int kStreamWarps = 16;                       // element-wise warps
 constexpr int kStreamThreads = (kStreamWarps + 2) * 32;
 // HEADS heads of one group per CTA share the B tile: one stage is half a chunk of B (2 x 16 KB) and of every head's
 // x (16 KB each).  One head: 4 stages of 48 KB; two heads: 3 stages of 64 KB; plus one 16 KB state tile per head.
-// NH = halves of 64 states; with one, rows 64.. of S^T are garbage that nobody reads.
-template <int HEADS, int NH> struct StreamCfg {
-    static constexpr uint32_t kStage = NH * 16384 + HEADS * 16384;
+template <int HEADS> struct StreamCfg {
+    static constexpr uint32_t kStage = 2 * 16384 + HEADS * 16384;
     static constexpr int kStages = HEADS == 1 ? 4 : 3;
     static constexpr uint32_t kSmem = kStages * kStage + HEADS * 16384 + 256 + 1024;
 };
 enum { kStStreamFull = 41, kStStreamWeighted, kStStreamEmpty, kStStreamAcc, kStStreamAccEmpty };
 
-template <typename T, int HEADS, int NH>
+template <typename T, int HEADS>
 __global__ void __launch_bounds__(kStreamThreads, 1)
 ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
                            const __grid_constant__ CUtensorMap tm_Hs, const float *dtb, const float *dAb, const float *initial,
                            float *final_states, float *range_decay, float *prefix_decay, float *state_copy, float *decay_copy,
-                           int store_entering, int nchunks, int vheads, int pslices, int headdim, int dstate, int heads_per_group, int unit0, const int32_t *seq_idx, int seqlen,
+                           int store_entering, int nchunks, int nheads, int heads_per_group, int unit0, const int32_t *seq_idx, int seqlen,
                            int *status)
 {
-    using Cfg = StreamCfg<HEADS, NH>;
+    using Cfg = StreamCfg<HEADS>;
     constexpr int NST = Cfg::kStages;
     constexpr uint32_t kStage = Cfg::kStage;
     extern __shared__ uint8_t smem_raw[];
@@ -262,8 +256,8 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
     uint64_t *bars = reinterpret_cast<uint64_t *>(tile + HEADS * 16384);
     uint64_t *full = bars, *weighted = bars + 4, *empty = bars + 8, *acc_full = bars + 12, *acc_empty = bars + 14;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 16);
-    // work unit = HEADS consecutive head slices of one batch row (all of one group); units are numbered batch-major
-    const int unit = unit0 + blockIdx.x, upb = vheads / HEADS, nheads = vheads / pslices;
+    // work unit = HEADS consecutive heads of one batch row (all of one group); units are numbered batch-major
+    const int unit = unit0 + blockIdx.x, upb = nheads / HEADS;
     const int h0 = (unit % upb) * HEADS, b = unit / upb;
     const int g = h0 / heads_per_group;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -300,8 +294,8 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
                 const int t0 = i * 128;
                 mbar_expect_tx(&full[st], kStage);
                 for (int hd = 0; hd < HEADS; ++hd)
-                    tma_load_4d(dst + NH * 16384 + hd * 16384, &tm_x, &full[st], (h0 + hd) % pslices * 64, (h0 + hd) / pslices, t0, b);
-                for (int kb = 0; kb < NH; ++kb) tma_load_4d(dst + kb * 16384, &tm_B, &full[st], kb * 64, g, t0, b);
+                    tma_load_4d(dst + 2 * 16384 + hd * 16384, &tm_x, &full[st], 0, h0 + hd, t0, b);
+                for (int kb = 0; kb < 2; ++kb) tma_load_4d(dst + kb * 16384, &tm_B, &full[st], kb * 64, g, t0, b);
                 ++issued;
             }
             // nothing may still be landing in this CTA's shared memory when it exits
@@ -310,7 +304,7 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
     } else if (warp == kStreamWarps + 1) {
         // ------------------------------------------------------------------ MMAs: S^T[n, (head, p)] += B[k, n] xw[k, (head, p)]
         const uint32_t idesc = instr_desc_f16(128, 64 * HEADS, Fmt<T>::v, 1, 1), tm = warp_uniform(tmem);
-        const uint64_t desc_B = smem_desc_sw128(smem_u32(sm), 16384, 1024), desc_x = smem_desc_sw128(smem_u32(sm) + NH * 16384, 16384, 1024);
+        const uint64_t desc_B = smem_desc_sw128(smem_u32(sm), 16384, 1024), desc_x = smem_desc_sw128(smem_u32(sm) + 2 * 16384, 16384, 1024);
         bool ok = true;
         int st = 0, phase = 0;           // stage, and how often the ring has gone round
 #pragma unroll 1
@@ -342,24 +336,18 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
         const int r = wt / TPR, cq = (wt % TPR) * NCH;       // my x row inside a stage and my first 16-byte chunk of it
         const int n = (warp & 3) * 32 + lane;                // TMEM lane = state index
         const int p0 = (warp >> 2) * 16;                     // my quarter of every head's columns
-        const bool n_on = n < dstate;
-        const bool tile_on = NH == 2 || n < 64;              // rows of the 16-bit tiles
-        // (batch row, head) of a slice, its first element for my n and p0 in a (batch, head, headdim, dstate) tensor, and how many of
-        // my 16 columns it has
+        // (batch row, head) of mine, and their first elements for my n and p0 in a (batch, head, headdim, dstate) tensor
         int64_t bh[HEADS], elem0[HEADS];
-        int cols[HEADS];
 #pragma unroll
         for (int hd = 0; hd < HEADS; ++hd) {
-            const int hr = (h0 + hd) / pslices, pv = (h0 + hd) % pslices * 64;
-            bh[hd] = (int64_t)b * nheads + hr;
-            elem0[hd] = (bh[hd] * headdim + pv + p0) * dstate + n;
-            cols[hd] = n_on ? headdim - pv - p0 : 0;
+            bh[hd] = (int64_t)b * nheads + h0 + hd;
+            elem0[hd] = (bh[hd] * kP + p0) * kN + n;
         }
         float H[HEADS][16];
 #pragma unroll
         for (int hd = 0; hd < HEADS; ++hd)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) H[hd][j] = initial && j < cols[hd] ? initial[elem0[hd] + j * dstate] : 0.f;
+            for (int j = 0; j < 16; ++j) H[hd][j] = initial ? initial[elem0[hd] + j * kN] : 0.f;
         // per chunk: dA and dt of my two x rows (my weighting head), and every head's dA at the end of the chunk.
         // Packed sequences: a row of another sequence than the chunk's last weighs nothing (dt = 0), and a chunk
         // whose last step belongs to another sequence than the previous chunk's carries nothing over (decay 0).
@@ -418,7 +406,7 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
                 const float w = __expf(fminf(my_last - cur[2 * half], 0.f)) * cur[2 * half + 1];
                 ok = ok && mbar_wait(&full[st], (i / NST) & 1, status, kStStreamFull);
                 if (ok) {
-                    const uint32_t base = smem_u32(sm + st * kStage + NH * 16384 + whead * 16384) + r * 128;
+                    const uint32_t base = smem_u32(sm + st * kStage + 2 * 16384 + whead * 16384) + r * 128;
 #pragma unroll
                     for (int ch = 0; ch < NCH; ++ch) {
                         const uint32_t addr = base + (((cq + ch) ^ (r & 7)) << 4);
@@ -453,7 +441,6 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
                     const uint32_t row = smem_u32(tile + hd * 16384) + n * 128;
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        if (!tile_on) break;
                         uint4 o;
                         o.x = Pack2<T>::pack(H[hd][8 * q + 0], H[hd][8 * q + 1]);
                         o.y = Pack2<T>::pack(H[hd][8 * q + 2], H[hd][8 * q + 3]);
@@ -466,7 +453,7 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
                 asm volatile("bar.sync 1, 512;" ::: "memory");
                 if (tid == 0) {
                     for (int hd = 0; hd < HEADS; ++hd)
-                        tma_store_3d(&tm_Hs, tile + hd * 16384, 0, 0, (int)((((int64_t)b * nchunks + c) * vheads) + h0 + hd));
+                        tma_store_3d(&tm_Hs, tile + hd * 16384, 0, 0, (int)((((int64_t)b * nchunks + c) * nheads) + h0 + hd));
                     tma_store_commit();
                 }
             }
@@ -476,9 +463,9 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
         for (int hd = 0; hd < HEADS; ++hd) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                if (!ok || j >= cols[hd]) continue;
-                if (final_states) final_states[elem0[hd] + j * dstate] = H[hd][j];
-                if (state_copy) state_copy[elem0[hd] + j * dstate] = H[hd][j];
+                if (!ok) continue;
+                if (final_states) final_states[elem0[hd] + j * kN] = H[hd][j];
+                if (state_copy) state_copy[elem0[hd] + j * kN] = H[hd][j];
             }
         }
         if (tid == 0) {
@@ -513,7 +500,7 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 //   Y1 = C . H (A = C from shared memory), Y2 = (CB o L) . x (A from tensor memory), out = exp(dA_m) Y1 + Y2 + D x
 // Tensor memory: rows 0-127: accumulators Y1 | Y2 [0, 128), A [128, 192); rows 128-255: [192, 320), A [320, 448).  While a unit
 // starts, C.B^T in fp32 takes the place of a row block's regions (128 and 256 columns).
-// Shared memory: C (32 KB per 64 states), two stages of x 32 KB | H 8 KB per 64 states | z 32 KB; the output tile replaces
+// Shared memory: C 64 KB, two stages of x 32 KB | H 16 KB | z 32 KB; the output tile replaces
 // z in place and leaves through a TMA store.  While a unit starts, B lies in the x parts of the two stages.
 // What the layout is chosen for: C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
 // register comes back from L2 (24 element-wise warps of 72 registers spilled 96 bytes and took 0.345 ms for the shape above).
@@ -529,33 +516,32 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // The factors are rounded to the input dtype and applied with packed 16-bit multiplies.
 constexpr float kMaxDiagSpan = 100.f;
 constexpr int kRowWarps0 = 4, kRowWarps1 = 8, kElemWarps = kRowWarps0 + kRowWarps1, kOutThreads = (kElemWarps + 4) * 32;
-template <int NH> struct OutCfg {   // NH: halves of 64 states
-    static constexpr uint32_t kC = 2 * NH * 16384, kH = NH * 8192, kStage = 32768 + kH + 32768;
+struct OutCfg {
+    static constexpr uint32_t kC = 4 * 16384, kH = 2 * 8192, kStage = 32768 + kH + 32768;
     static constexpr uint32_t kScal = 1024 + 128 + 64;  // column factors, 32 refs, then flags, D
     static constexpr uint32_t kSmem = kC + 2 * kStage + 2 * kScal + 256;
 };
-static_assert(OutCfg<2>::kSmem <= 227 * 1024, "shared memory");
+static_assert(OutCfg::kSmem <= 227 * 1024, "shared memory");
 enum { kStOutUnit = 21, kStOutCb, kStOutCbRead, kStOutStage, kStOutGate, kStOutA, kStOutAcc, kStOutAccFree, kStOutScal, kStOutScalFree, kStOutTile };
 
-// Place of a (unit, head slice) pair; advanced without divisions.  Every role of the kernel walks the same list.
+// Place of a (unit, head) pair; advanced without divisions.  Every role of the kernel walks the same list.
 struct OutWalk {
-    int b, c, g, hv, h, sl;         // batch row, chunk, group; head slice inside the group; head, slice of the head
+    int b, c, g, hv, h;             // batch row, chunk, group; head inside the group; head
     bool enter;                     // first pair of this CTA in the unit (b, c, g)
-    __device__ __forceinline__ OutWalk(int it, int ngroups, int nchunks, int hpu, int pslices)
+    __device__ __forceinline__ OutWalk(int it, int ngroups, int nchunks, int hpu)
     {
         const int u = it / hpu, bc = u / ngroups;
         hv = it - u * hpu;
         g = u - bc * ngroups;
         b = bc / nchunks;
         c = bc - b * nchunks;
-        h = (g * hpu + hv) / pslices;
-        sl = hv % pslices;          // a group holds whole heads
+        h = g * hpu + hv;
         enter = true;
     }
-    __device__ __forceinline__ void step(int ngroups, int nchunks, int hpu, int pslices)
+    __device__ __forceinline__ void step(int ngroups, int nchunks, int hpu)
     {
         enter = false;
-        if (++sl == pslices) { sl = 0; ++h; }
+        ++h;
         if (++hv == hpu) {
             hv = 0;
             enter = true;
@@ -570,14 +556,13 @@ struct OutWalk {
 };
 
 // DV: D differs over the columns of a head.
-template <typename T, int NH, bool DV>
+template <typename T, bool DV>
 __global__ void __launch_bounds__(kOutThreads, 1)
 ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_C, const __grid_constant__ CUtensorMap tm_B,
                      const __grid_constant__ CUtensorMap tm_H, const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_out,
-                     const float *dtb, const float *dAb, const float *Dp, int has_z, int nchunks, int nheads, int ngroups, int pslices,
-                     int headdim, int seqlen, int total_items, int h_np, const uint8_t *seq_start, const uint8_t *seq_carry, int *status)
+                     const float *dtb, const float *dAb, const float *Dp, int has_z, int nchunks, int nheads, int ngroups, int seqlen, int total_items, int h_np, const uint8_t *seq_start, const uint8_t *seq_carry, int *status)
 {
-    using Cfg = OutCfg<NH>;
+    using Cfg = OutCfg;
     extern __shared__ __align__(1024) uint8_t sm[];
     uint8_t *Cs = sm;                                           // [row block][state half] tiles of [128][64]
     uint8_t *stages = sm + Cfg::kC;
@@ -592,7 +577,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
              *b_scal = bars + 14, *b_scalfree = bars + 16, *b_out = bars + 18, *b_unit = bars + 22;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 23);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int vheads = nheads * pslices, hpu = vheads / ngroups;        // 64-column slices of heads; of one group
+    const int hpu = nheads / ngroups;                           // heads of a group
     const int it0 = (int)((int64_t)total_items * blockIdx.x / gridDim.x), count = (int)((int64_t)total_items * (blockIdx.x + 1) / gridDim.x) - it0;
     if (threadIdx.x == kElemWarps * 32) {
         for (int i = 0; i < 2; ++i) {
@@ -635,7 +620,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         uint32_t cb[NR][16];                                 // my ranges of C.B^T, packed, masked
         const float *dA = dAb;                               // of the current (batch row, head, chunk)
         float dA_next = 0.f;
-        int left = 0, sl = 0;                                // heads left in the unit, slice of the head
+        int left = 0;                                        // heads left in the unit
         bool carry = true, rows = true;                      // my row continues the sequence that ended the previous chunk; the chunk reaches my block
         int nunits = 0, item = 0;
         [[maybe_unused]] const float *Dv = nullptr;                           // DV: D of my columns
@@ -653,12 +638,11 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             auto range = [&](int t) { return rb ? (t >> 1) * 4 + 2 * cq + (t & 1) : t; };
             if (left == 0) {
                 // a new unit: nothing of this group is in flight; C.B^T moves from tensor memory into registers
-                const OutWalk w(it0 + seq, ngroups, nchunks, hpu, pslices);
+                const OutWalk w(it0 + seq, ngroups, nchunks, hpu);
                 left = hpu - w.hv;
-                sl = w.sl;
                 rows = rb < w.row_blocks(seqlen);
                 dA = dAb + (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ;
-                if constexpr (DV) Dv = Dp + (int64_t)w.h * headdim;
+                if constexpr (DV) Dv = Dp + (int64_t)w.h * kP;
                 if (rows) {
                     int lo = 0;                              // first column of my row's sequence inside the chunk
                     if (seq_start) {
@@ -704,8 +688,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 continue;
             }
             const float dAm = dA_next * kLog2e;
-            const bool last_slice = ++sl == pslices;
-            if (left) dA_next = dA[(last_slice ? (int64_t)nchunks * kQ : 0) + r];        // a whole head ahead of its use
+            if (left) dA_next = dA[(int64_t)nchunks * kQ + r];                           // a whole head ahead of its use
             const int flags = __float_as_int(lds32(sc + 1024 + 128));
             const float Dh = lds32(sc + 1024 + 132);
 
@@ -723,10 +706,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 }
                 tmem_st_wait();
             }
-            if (last_slice) {
-                sl = 0;
-                dA += (int64_t)nchunks * kQ;
-            }
+            dA += (int64_t)nchunks * kQ;
 #pragma unroll
             for (int t = 0; t < NR; ++t) {
                 const int j = range(t);
@@ -789,7 +769,6 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             tc_fence_after_sync();
             const int e8_end = rb ? 4 * cq + 4 : 8;
             const uint64_t rs2 = pack2(rs, rs), D2 = pack2(Dh, Dh);
-            [[maybe_unused]] const int pv = (last_slice ? pslices - 1 : sl - 1) * 64;
 #pragma unroll 1
             for (int e8 = 4 * cq; e8 < e8_end; ++e8) {
                 uint32_t y1[8], y2[8];
@@ -817,8 +796,8 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                         const float2 f = Pack2<T>::unpack(xe[i]);
                         uint64_t d2 = D2;
                         if constexpr (DV) {
-                            const int pc = pv + e8 * 8 + 2 * i;
-                            d2 = pc < headdim ? pack2(Dv[pc], Dv[pc + 1]) : pack2(0.f, 0.f);       // headdim is a multiple of 8
+                            const int pc = e8 * 8 + 2 * i;
+                            d2 = pack2(Dv[pc], Dv[pc + 1]);
                         }
                         y[i] = fma2(pack2(f.x, f.y), d2, y[i]);
                     }
@@ -847,7 +826,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 }
                 sts128(zaddr, make_uint4(o[0], o[1], o[2], o[3]));
             }
-            if constexpr (DV) Dv += last_slice ? headdim : 0;
+            if constexpr (DV) Dv += kP;
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(18 + 2 * s + rb));
@@ -855,8 +834,8 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     } else if (warp == kElemWarps + 1 || warp == kElemWarps + 2) {
         // ------------------------------------------------------------------ MMAs of one row block
         const int rb = (int)warp_uniform(warp) - (kElemWarps + 1);
-        OutWalk w(it0, ngroups, nchunks, hpu, pslices);
-        auto step = [&] { w.step(ngroups, nchunks, hpu, pslices); };
+        OutWalk w(it0, ngroups, nchunks, hpu);
+        auto step = [&] { w.step(ngroups, nchunks, hpu); };
         const uint32_t tm = warp_uniform(tmem), acc = tm + (rb ? 192 : 0), A = tm + (rb ? 320 : 128);
         auto wait = [&](uint64_t *bar, int phase, int code) { return __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, status, code)) != 0; };
         bool ok = true, rows = true;
@@ -864,7 +843,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         const uint32_t idesc_cb = instr_desc_f16(128, 128, Fmt<T>::v, 0, 0) + ((uint32_t)(rb ? 128 >> 3 : 0) << 17),      // N = 128 or 256
                        idesc_y1 = instr_desc_f16(128, 64, Fmt<T>::v, 0, h_np ? 1 : 0), idesc_y2 = instr_desc_f16(128, 64, Fmt<T>::v, 0, 1);
         const uint32_t step_H = h_np ? 128 : 2;              // states along the rows of the tile, or along its columns
-        const uint64_t desc_C = smem_desc_sw128(smem_u32(Cs) + rb * NH * 16384, 16, 1024), desc_x = smem_desc_sw128(smem_u32(st_x(0)), 16, 1024),
+        const uint64_t desc_C = smem_desc_sw128(smem_u32(Cs) + rb * 2 * 16384, 16, 1024), desc_x = smem_desc_sw128(smem_u32(st_x(0)), 16, 1024),
                        desc_H = smem_desc_sw128(smem_u32(st_H(0)), 16, 1024);
 #pragma unroll 1
         for (int seq = 0; seq < count && ok; ++seq, step()) {
@@ -879,7 +858,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     tc_fence_after_sync();
                     if (elect_one()) {
 #pragma unroll 1
-                        for (int kb = 0; kb < NH; ++kb)      // B lies in the x parts of the stages
+                        for (int kb = 0; kb < 2; ++kb)      // B lies in the x parts of the stages
                             mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_x + kb * (Cfg::kStage / 16), 2, idesc_cb, kb > 0);
                         mma_commit(&b_cb[rb]);
                     }
@@ -898,7 +877,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             tc_fence_after_sync();
             if (elect_one()) {
 #pragma unroll 1
-                for (int kb = 0; kb < NH; ++kb)
+                for (int kb = 0; kb < 2; ++kb)
                     mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_H + off + kb * (8192 / 16), step_H, idesc_y1, kb > 0);
             }
             __syncwarp();
@@ -915,11 +894,11 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     } else if (warp == kElemWarps) {
         // ------------------------------------------------------------------ TMA loads and stores
         if (lane == 0) {
-            OutWalk w(it0, ngroups, nchunks, hpu, pslices);
-            auto step = [&] { w.step(ngroups, nchunks, hpu, pslices); };
+            OutWalk w(it0, ngroups, nchunks, hpu);
+            auto step = [&] { w.step(ngroups, nchunks, hpu); };
             bool ok = true;
             uint32_t outs = 0, cbs = 0;          // parities of the next completion of each b_out, b_cb
-            struct Pending { int b, h, p, t, nrb; } pend[2] = {};
+            struct Pending { int b, h, t, nrb; } pend[2] = {};
             int nunits_requested = 0, seq = 0, done = 0;         // units requested; heads requested, finished
             // Heads leave in the order in which they came: the one in stage s has its output tiles stored as they are completed,
             // and the stage is free once they have been read.  A new unit starts when both stages are free: C goes to its place,
@@ -936,7 +915,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                         ok = mbar_wait(&b_out[k], (outs >> k) & 1, status, kStOutTile);
                         outs ^= 1u << k;
                         if (ok) {
-                            tma_store_4d(&tm_out, st_z(s) + rb * 16384, pend[s].p, pend[s].h, pend[s].t + rb * 128, pend[s].b);
+                            tma_store_4d(&tm_out, st_z(s) + rb * 16384, 0, pend[s].h, pend[s].t + rb * 128, pend[s].b);
                             tma_store_commit();
                         }
                     }
@@ -948,11 +927,11 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 const int s = seq & 1, nrb = w.row_blocks(seqlen);
                 if (w.enter) {
                     ++nunits_requested;
-                    mbar_expect_tx(b_unit, nrb * NH * 16384 + NH * 32768);
+                    mbar_expect_tx(b_unit, nrb * 2 * 16384 + 2 * 32768);
 #pragma unroll 1
-                    for (int kb = 0; kb < NH; ++kb) {
+                    for (int kb = 0; kb < 2; ++kb) {
 #pragma unroll 1
-                        for (int rb = 0; rb < nrb; ++rb) tma_load_4d(Cs + (rb * NH + kb) * 16384, &tm_C, b_unit, kb * 64, w.g, w.c * kQ + rb * 128, w.b);
+                        for (int rb = 0; rb < nrb; ++rb) tma_load_4d(Cs + (rb * 2 + kb) * 16384, &tm_C, b_unit, kb * 64, w.g, w.c * kQ + rb * 128, w.b);
                         tma_load_4d(st_x(kb), &tm_B, b_unit, kb * 64, w.g, w.c * kQ, w.b);
                     }
 #pragma unroll 1
@@ -963,17 +942,17 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     if (!ok) break;
                 }
                 mbar_expect_tx(&b_xh[s], 32768 + Cfg::kH);
-                tma_load_4d(st_x(s), &tm_x, &b_xh[s], w.sl * 64, w.h, w.c * kQ, w.b);
-                const int uh = (w.b * nchunks + w.c) * vheads + w.g * hpu + w.hv;
+                tma_load_4d(st_x(s), &tm_x, &b_xh[s], 0, w.h, w.c * kQ, w.b);
+                const int uh = (w.b * nchunks + w.c) * nheads + w.h;
                 if (h_np) tma_load_3d(st_H(s), &tm_H, &b_xh[s], 0, 0, uh);                     // [n][p] tile
                 else
 #pragma unroll 1
-                    for (int kb = 0; kb < NH; ++kb) tma_load_3d(st_H(s) + kb * 8192, &tm_H, &b_xh[s], kb * 64, 0, uh);   // columns n of the [p][n] state
+                    for (int kb = 0; kb < 2; ++kb) tma_load_3d(st_H(s) + kb * 8192, &tm_H, &b_xh[s], kb * 64, 0, uh);   // columns n of the [p][n] state
                 if (has_z) {
                     mbar_expect_tx(&b_z[s], 32768);
-                    tma_load_4d(st_z(s), &tm_z, &b_z[s], w.sl * 64, w.h, w.c * kQ, w.b);
+                    tma_load_4d(st_z(s), &tm_z, &b_z[s], 0, w.h, w.c * kQ, w.b);
                 }
-                pend[s] = {w.b, w.h, w.sl * 64, w.c * kQ, nrb};
+                pend[s] = {w.b, w.h, w.c * kQ, nrb};
                 ++seq;
                 step();
             }
@@ -990,8 +969,8 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         }
     } else {
         // ------------------------------------------------------------------ per-head scalars
-        OutWalk w(it0, ngroups, nchunks, hpu, pslices);
-        auto step = [&] { w.step(ngroups, nchunks, hpu, pslices); };
+        OutWalk w(it0, ngroups, nchunks, hpu);
+        auto step = [&] { w.step(ngroups, nchunks, hpu); };
         bool ok = true;
         float dA[8], dt[8];                      // step 32 j + lane
         auto request = [&]() {
@@ -1259,9 +1238,6 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
 }
 
 // ====================================================================================== host
-// Head slices of 64 columns of a call.
-int slices(const mb200_ssd_args &a) { return (a.headdim + kP - 1) / kP; }
-
 // (rank-4) map of a (batch, seqlen, rows, inner) tensor with boxes of 64 inner elements x `steps` steps
 bool map_rows(CUtensorMap *m, int fmt, const void *p, const int64_t *st, int inner, int rows, const mb200_ssd_args &a, uint32_t steps)
 {
@@ -1273,7 +1249,7 @@ bool map_rows(CUtensorMap *m, int fmt, const void *p, const int64_t *st, int inn
 
 // The stages of a call follow one another at once: each starts, sets up its barriers, tensor memory and first loads while the one before
 // drains, and waits for it (pdl_wait) before it reads what that wrote.  Every stage waits, so the last has waited for all.  Only where
-// the output stage has at most kEarlyItems (chunk, head slice) pairs per SM: what an early start saves is a few us of any call, and
+// the output stage has at most kEarlyItems (chunk, head) pairs per SM: what an early start saves is a few us of any call, and
 // the longest ran slower with it (262144 steps of 128 heads, 886 pairs per SM: 5.33 -> 5.47 ms; 69 per SM: no difference).
 constexpr int kEarlyItems = 128;
 struct TcCall {
@@ -1281,7 +1257,7 @@ struct TcCall {
     float *dtb, *dAb;
     void *prev16;
     int *status;
-    int nc, ps, vheads, vhpg;
+    int nc, hpg;
     bool early;
 };
 TcCall tc_call(const mb200_ssd_args &a, const SsdScratch &lay)
@@ -1293,45 +1269,43 @@ TcCall tc_call(const mb200_ssd_args &a, const SsdScratch &lay)
     k.prev16 = k.base + lay.off_prev16;
     k.status = ssd_status_word(a, lay);
     k.nc = lay.nchunks;
-    k.ps = slices(a);
-    k.vheads = a.nheads * k.ps;
-    k.vhpg = k.vheads / a.ngroups;
-    k.early = (int64_t)a.batch * k.nc * k.vheads <= (int64_t)kEarlyItems * sm_count(a.device);
+    k.hpg = a.nheads / a.ngroups;
+    k.early = (int64_t)a.batch * k.nc * a.nheads <= (int64_t)kEarlyItems * sm_count(a.device);
     return k;
 }
 
-// The entering states as the state-stream kernel stores them: [n][p] tiles of (64 NH) x 64.
-template <int NH> bool map_states_np(CUtensorMap *m, int fmt, const TcCall &k, const mb200_ssd_args &a)
+// The entering states as the state-stream kernel stores them: [n][p] tiles of 128 x 64.
+bool map_states_np(CUtensorMap *m, int fmt, const TcCall &k, const mb200_ssd_args &a)
 {
-    const uint64_t d[3] = {64, 64 * NH, (uint64_t)a.batch * k.nc * k.vheads};
-    const uint64_t s[2] = {128, 64 * NH * 128};
-    const uint32_t bx[3] = {64, 64 * NH, 1};
+    const uint64_t d[3] = {kP, kN, (uint64_t)a.batch * k.nc * a.nheads};
+    const uint64_t s[2] = {2 * kP, 2 * kP * kN};
+    const uint32_t bx[3] = {kP, kN, 1};
     return encode_16bit(m, fmt, k.prev16, 3, d, s, bx);
 }
 
-template <typename T, int NH>
+template <typename T>
 int run_chunk_state(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {
     const TcCall k = tc_call(a, lay);
     CUtensorMap tx, tB;
     if (!map_rows(&tx, Fmt<T>::v, a.x, a.x_stride, a.headdim, a.nheads, a, 256) || !map_rows(&tB, Fmt<T>::v, a.B, a.B_stride, a.dstate, a.ngroups, a, 256))
         return fail(MB200_ERR_LAUNCH, "ssd: tensor map for x or B failed");
-    constexpr int smem = (NH + 1) * 32768 + 256 + 1024;
-    ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_chunk_state_kernel<T, NH>), smem, a.device);
-    ssd_tc_chunk_state_kernel<T, NH><<<dim3(k.vheads, k.nc, a.batch), kStateThreads, smem, stream>>>(
-        tx, tB, k.dtb, k.dAb, reinterpret_cast<float *>(k.base + lay.off_states), k.nc, a.nheads, k.ps, a.dstate, a.nheads / a.ngroups, a.seq_idx, a.seqlen,
+    constexpr int smem = 3 * 32768 + 256 + 1024;
+    ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_chunk_state_kernel<T>), smem, a.device);
+    ssd_tc_chunk_state_kernel<T><<<dim3(a.nheads, k.nc, a.batch), kStateThreads, smem, stream>>>(
+        tx, tB, k.dtb, k.dAb, reinterpret_cast<float *>(k.base + lay.off_states), k.nc, a.nheads, k.hpg, a.seq_idx, a.seqlen,
         k.status);
     MB200_CHECK_LAUNCH("ssd chunk_state (tensor core)");
     return MB200_OK;
 }
 
-template <typename T, int NH>
+template <typename T>
 int run_state_stream(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {
     const TcCall k = tc_call(a, lay);
     CUtensorMap tx, tB, tHs;
     if (!map_rows(&tx, Fmt<T>::v, a.x, a.x_stride, a.headdim, a.nheads, a, 128) || !map_rows(&tB, Fmt<T>::v, a.B, a.B_stride, a.dstate, a.ngroups, a, 128) ||
-        !map_states_np<NH>(&tHs, Fmt<T>::v, k, a))
+        !map_states_np(&tHs, Fmt<T>::v, k, a))
         return fail(MB200_ERR_LAUNCH, "ssd: tensor map for x, B or the states failed");
     // whole operator: from initial_states, entering states stored.  LOCAL half of a sequence split: from a zero
     // state, entering states stored as they are without the incoming state, plus what the OUTPUT half needs to
@@ -1345,24 +1319,24 @@ int run_state_stream(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_
     // CTA then runs 1.6x as long, so only whole waves of such CTAs pay; what is left over runs as pairs if that is
     // more than half a wave and as single heads otherwise.
     const int sms = sm_count(a.device);
-    const int64_t pairs = k.vhpg % 2 == 0 ? (int64_t)a.batch * (k.vheads / 2) : 0;
+    const int64_t pairs = k.hpg % 2 == 0 ? (int64_t)a.batch * (a.nheads / 2) : 0;
     int64_t paired = pairs / sms * sms;
     if (pairs - paired > sms / 2) paired = pairs;
     auto go = [&](auto heads_tag, int64_t units, int64_t unit0) {
         constexpr int HEADS = decltype(heads_tag)::value;
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_state_stream_kernel<T, HEADS, NH>), (int)StreamCfg<HEADS, NH>::kSmem, a.device);
-        launch_dependent_if(k.early, ssd_tc_state_stream_kernel<T, HEADS, NH>, dim3((unsigned)units), kStreamThreads, StreamCfg<HEADS, NH>::kSmem, stream,
-            tx, tB, tHs, k.dtb, k.dAb, init, a.final_states, a.range_decay, aux_prefix, aux_state, aux_decay, 1, k.nc, k.vheads, k.ps, a.headdim, a.dstate,
-            k.vhpg, (int)unit0, a.seq_idx, a.seqlen, k.status);
+        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_state_stream_kernel<T, HEADS>), (int)StreamCfg<HEADS>::kSmem, a.device);
+        launch_dependent_if(k.early, ssd_tc_state_stream_kernel<T, HEADS>, dim3((unsigned)units), kStreamThreads, StreamCfg<HEADS>::kSmem, stream,
+            tx, tB, tHs, k.dtb, k.dAb, init, a.final_states, a.range_decay, aux_prefix, aux_state, aux_decay, 1, k.nc, a.nheads, k.hpg,
+            (int)unit0, a.seq_idx, a.seqlen, k.status);
     };
     if (paired > 0) go(std::integral_constant<int, 2>{}, paired, 0);
-    const int64_t singles = (int64_t)a.batch * k.vheads - 2 * paired;
+    const int64_t singles = (int64_t)a.batch * a.nheads - 2 * paired;
     if (singles > 0) go(std::integral_constant<int, 1>{}, singles, 2 * paired);
     MB200_CHECK_LAUNCH("ssd state stream (tensor core)");
     return MB200_OK;
 }
 
-template <typename T, int NH>
+template <typename T>
 int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaStream_t stream)
 {
     const TcCall k = tc_call(a, lay);
@@ -1373,23 +1347,23 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     if (a.z) ok = ok && map_rows(&tz, fmt, a.z, a.z_stride, a.headdim, a.nheads, a, 256);
     else tz = tx;
     if (h_np) {
-        ok = ok && map_states_np<NH>(&tH, fmt, k, a);
+        ok = ok && map_states_np(&tH, fmt, k, a);
     } else {
-        const uint64_t d[3] = {(uint64_t)a.dstate, 64, (uint64_t)a.batch * k.nc * k.vheads};
-        const uint64_t s[2] = {(uint64_t)a.dstate * 2, (uint64_t)a.dstate * 128};
+        const uint64_t d[3] = {kN, kP, (uint64_t)a.batch * k.nc * a.nheads};
+        const uint64_t s[2] = {2 * kN, 2 * kN * kP};
         const uint32_t bx[3] = {64, 64, 1};
         ok = ok && encode_16bit(&tH, fmt, k.prev16, 3, d, s, bx);
     }
     if (!ok) return fail(MB200_ERR_LAUNCH, "ssd: a tensor map of the output stage failed");
-    const int64_t items = (int64_t)a.batch * k.nc * k.vheads;
+    const int64_t items = (int64_t)a.batch * k.nc * a.nheads;
     const int grid = (int)std::min<int64_t>(items, sm_count(a.device));
     const uint8_t *seq_start = a.seq_idx ? reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_start) : nullptr;
     const uint8_t *seq_carry = reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_carry);
     auto go = [&](auto dv) {
-        auto kernel = ssd_tc_output_kernel<T, NH, decltype(dv)::value>;
-        ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)OutCfg<NH>::kSmem, a.device);
-        launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg<NH>::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, a.z != nullptr, k.nc,
-                         a.nheads, a.ngroups, k.ps, a.headdim, a.seqlen, (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
+        auto kernel = ssd_tc_output_kernel<T, decltype(dv)::value>;
+        ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)OutCfg::kSmem, a.device);
+        launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, a.z != nullptr, k.nc,
+                         a.nheads, a.ngroups, a.seqlen, (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
     };
     if (a.D && a.D_has_hdim) go(std::true_type{});
     else go(std::false_type{});
@@ -1411,14 +1385,8 @@ int run_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     return MB200_OK;
 }
 
-// Calls f(element type, number of state halves) for the call's.
-template <class F> int with_types(const mb200_ssd_args &a, F f)
-{
-    const bool one = a.dstate <= 64;
-    using B16 = __nv_bfloat16;
-    if (a.io_dtype == MB200_BF16) return one ? f(B16{}, std::integral_constant<int, 1>{}) : f(B16{}, std::integral_constant<int, 2>{});
-    return one ? f(__half{}, std::integral_constant<int, 1>{}) : f(__half{}, std::integral_constant<int, 2>{});
-}
+// f(element type of the call)
+template <class F> int with_type(const mb200_ssd_args &a, F f) { return a.io_dtype == MB200_BF16 ? f(__nv_bfloat16{}) : f(__half{}); }
 
 }  // namespace
 
@@ -1433,7 +1401,7 @@ bool ssd_tc_local_eligible(const mb200_ssd_args &a)
     if (!ssd_tc_shape(a)) return false;
     if (!rows_for_tma(a.x, a.x_stride) || !rows_for_tma(a.B, a.B_stride)) return false;
     const int64_t nc = (a.seqlen + kQ - 1) / kQ;
-    if ((int64_t)a.batch * nc * a.nheads * slices(a) > INT32_MAX || nc > 65535) return false;
+    if ((int64_t)a.batch * nc * a.nheads > INT32_MAX || nc > 65535) return false;
     return encode_fn() != nullptr;
 }
 
@@ -1446,22 +1414,21 @@ bool ssd_tc_output_eligible(const mb200_ssd_args &a)
     return !a.z || rows_for_tma(a.z, a.z_stride);
 }
 
-// One head slice of one batch row per CTA: worth it once those fill half of the SMs, or when there are so few chunks that
-// walking them in order takes no longer than the launch of the separate recurrence.  A ragged slice always streams (the
-// per-chunk kernel stores whole slices).
+// One head of one batch row per CTA: worth it once those fill half of the SMs, or when there are so few chunks that walking them in
+// order takes no longer than the launch of the separate recurrence.
 bool ssd_tc_stream_eligible(const mb200_ssd_args &a)
 {
-    return (int64_t)a.batch * a.nheads * slices(a) >= kStreamMinUnits || a.seqlen <= 8 * kQ || a.headdim % kP != 0;
+    return (int64_t)a.batch * a.nheads >= kStreamMinUnits || a.seqlen <= 8 * kQ;
 }
 
 int ssd_tc_chunk_state(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {
-    return with_types(a, [&](auto t, auto nh) { return run_chunk_state<decltype(t), decltype(nh)::value>(a, lay, stream); });
+    return with_type(a, [&](auto t) { return run_chunk_state<decltype(t)>(a, lay, stream); });
 }
 
 int ssd_tc_output(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream)
 {
-    return with_types(a, [&](auto t, auto nh) { return run_output<decltype(t), decltype(nh)::value>(a, lay, states_np, stream); });
+    return with_type(a, [&](auto t) { return run_output<decltype(t)>(a, lay, states_np, stream); });
 }
 
 int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np, cudaStream_t stream) { return run_varlen(a, lay, states_np, stream); }
@@ -1495,7 +1462,7 @@ int ssd_tc_apply_incoming(const mb200_ssd_args &a, const SsdScratch &lay, cudaSt
 
 int ssd_tc_state_stream(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {
-    return with_types(a, [&](auto t, auto nh) { return run_state_stream<decltype(t), decltype(nh)::value>(a, lay, stream); });
+    return with_type(a, [&](auto t) { return run_state_stream<decltype(t)>(a, lay, stream); });
 }
 
 }  // namespace mb200

@@ -40,7 +40,7 @@ METRIC, UNIT = "scan_fwd_tokens_per_s", "tokens/s"
 # DRAM bytes (read + write) per launch group of a full single-GPU step, from the committed ncu captures
 NCU_TRAFFIC = {
     "c1": (659_956_992, "profiles/scan_stream_kernel__config1.md"),
-    "c2": (1_725_000_000, "profiles/ssd_forward__config2.md"),
+    "c2": (1_721_000_000, "profiles/ssd_forward__config2.md"),
     "c3": (19_190_000_000, "profiles/ssd_forward__config3_eighth.md (captured on an eighth of the sequence, scaled by 8: every kernel's traffic grows with the number of chunks)"),
     "c4": (1_288_700_000, "profiles/ssu_packet_kernel__config4.md"),
     "c1b": (3_002_000_000, "profiles/scan_bwd_kernels__config1_shape.md"),
@@ -149,8 +149,8 @@ class Workload:
                 g = torch.Generator().manual_seed(1001 + 7919 * rank)
                 self.d["dout"] = torch.randn(b, d, L, generator=g).to(bf).to(dev)
                 self.alg_bytes = 7 * b * d * L * esz + 2 * b * 16 * L * (esz + 4) + 2 * d * 16 * 4 + 4 * d * 4
-                self.launches_per_step = 2 if b > 0 else 0
-                self.kernels = "scan_bwd_states_kernel, scan_bwd_kernel (+ 5 memsets of the accumulators)"
+                self.launches_per_step = 3 if b > 0 else 0
+                self.kernels = "scan_bwd_clear_kernel, scan_bwd_states_kernel, scan_bwd_kernel"
         elif name == "c2":
             nb, L, Hall, P, N = batch or 8, 4096, 80, 64, 128
             lo, hi = split_even(Hall, world, rank)

@@ -563,7 +563,7 @@ int launch_rmsnorm(const mb200_rmsnorm_args &a, cudaStream_t stream)
     const int wvec = aligned16(a.weight) && (!a.bias || aligned16(a.bias)) ? 1 : 0;      // columns are multiples of VEC: parameter packets are aligned too
     auto go = [&](auto per_tag) {
         constexpr int P = decltype(per_tag)::value;
-        // (its CTAs find room beside the one CTA per SM of the scan that it usually follows)
+        // (its CTAs start as those of the launch before it leave: the SSD output kernel it usually follows fills an SM's registers)
         if (a.norm_before_gate) launch_dependent(rmsnorm_gated_kernel<T, P, true>, grid, threads, 0, stream, a, threads, wvec);
         else launch_dependent(rmsnorm_gated_kernel<T, P, false>, grid, threads, 0, stream, a, threads, wvec);
     };

@@ -1089,8 +1089,8 @@ bool rows_for_tma(const void *p, const int64_t *s)
 // chunk if the sequence began earlier.  bf16 inputs: the weighted x rows are cut into three bf16 values, so that the fp32 result keeps
 // fp32 products; B is exact as it is.  (Half precision would need its B cut as well: ssd_split.cu does that.)  The small products have
 // a sum of their own, which keeps the tensor core's rounding of sums out of them.  Halves of 128 rows that hold no step of the sequence are skipped.
-// 23 sequences x 80 heads, us, the wait for the launch before it included: 72; 54 with two parts and one sum, 83 with the 64-step tiles of
-// ssd_split.cu, 2500 with one thread per element.
+// 23 sequences x 80 heads: 63 us on its own; in place, the wait for the launch before it included, 72, against 54 with two parts and one
+// sum, 83 with the 64-step tiles of ssd_split.cu, 2500 with one thread per element.
 constexpr int kVarThreads = 288;
 __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
                                                                     const float *dtb, const float *dAb, const int32_t *cu_seqlens, float *varlen,
@@ -1249,8 +1249,9 @@ bool map_rows(CUtensorMap *m, int fmt, const void *p, const int64_t *st, int inn
 
 // The stages of a call follow one another at once: each starts, sets up its barriers, tensor memory and first loads while the one before
 // drains, and waits for it (pdl_wait) before it reads what that wrote.  Every stage waits, so the last has waited for all.  Only where
-// the output stage has at most kEarlyItems (chunk, head) pairs per SM: what an early start saves is a few us of any call, and
-// the longest ran slower with it (262144 steps of 128 heads, 886 pairs per SM: 5.33 -> 5.47 ms; 69 per SM: no difference).
+// the output stage has at most kEarlyItems (chunk, head) pairs per SM.  Early / in turn, us, bf16, by pairs per SM: 2 39.9 / 46.1, 9 87 / 93,
+// 17 143 / 150, 35 250 / 257, 69 439 / 447, 104 640 / 647, 138 834 / 840; from 208 on (1210 / 1212, 277: 1650 / 1673, 415: 2533 / 2484, 886:
+// 5155 / 5186) it is lost in runs that differ by up to 4 %.
 constexpr int kEarlyItems = 128;
 struct TcCall {
     char *base;

@@ -19,7 +19,7 @@ def test_short_rows_and_ragged_groups(dtype, tol, batch, dim, L, N, groups):
 
 
 @pytest.mark.parametrize("dtype,tol", DTYPES)
-@pytest.mark.parametrize("dim,L", [(1024, 139), (19008, 45), (30016, 43)])      # six-, four- and three-warp CTAs
+@pytest.mark.parametrize("dim,L", [(1024, 139), (19008, 45), (30016, 43)])      # the second and third: four- and three-warp CTAs in 16 bits, six in fp32
 @pytest.mark.parametrize("has_z", [True, False])
 def test_layouts_by_grid_size(dtype, tol, dim, L, has_z):
     run_both(make_inputs(dim + L, 1, dim, L, 16, 1, dtype, has_z=has_z), tol, f"unaligned d{dim} L{L}")

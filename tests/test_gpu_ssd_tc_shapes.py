@@ -1,5 +1,6 @@
-"""The tensor-core SSD stages at the edges of what they take: padded and sliced heads and states, lengths either side of a row
-block and a chunk, chunk sizes other than their own, few heads over many chunks, packed sequences on every one of them."""
+"""The SSD stages for 16-bit inputs at the edges of what they take: heads and states that do not fill a tile, lengths either side of a
+row block and a chunk, other chunk sizes, few heads over many chunks, packed sequences on every one of them.  Headdim 64, dstate 128 and
+chunk 256 run on 16-bit operands, all else on split ones (whose precision test_gpu_ssd_split.py checks)."""
 import pytest
 import torch
 

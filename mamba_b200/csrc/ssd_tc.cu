@@ -484,28 +484,30 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // ====================================================================================== chunk output
 // out[m] = exp(dA_m) C_m . H_c + sum_{k <= m} (C_m . B_k) exp(dA_m - dA_k) dt_k x_k + D x_m, gated by silu(z_m).
 //
-// What bounds it: DRAM.  Per (chunk of 256 steps, head) x, z and the entering state H come in (32 + 32 + 16 KB) and out
-// leaves (32 KB), 1.15 GB for batch 8, 4096 steps, 80 heads.  A kernel with one CTA per (chunk, head, 128 rows) fetched
-// C and C.B^T again for every head: 136 KB into shared memory per 128 rows, and each of its short CTAs paid the whole
-// latency chain (0.365 ms for that shape, 35 % of DRAM).  Here one persistent CTA per SM walks over the HEADS of a (chunk,
-// group) "unit": C stays in shared memory, C.B^T is formed once per unit on the tensor core and stays in REGISTERS (causal
-// and sequence masks already applied), so that a head costs its own x, z, H and out and nothing else.  The (unit, head)
-// pairs are split evenly over the CTAs in unit order, so a CTA meets few units and no wave is left nearly empty.
+// Per (chunk of 256 steps, head) x, z and the entering state H come in (32 + 32 + 16 KB) and out leaves (32 KB), 1.15 GB for batch 8, 4096
+// steps, 80 heads: 0.18 ms of DRAM.  A kernel with one CTA per (chunk, head, 128 rows) fetched C and C.B^T again for every head: 136 KB
+// into shared memory per 128 rows, and each of its short CTAs paid the whole latency chain (0.365 ms for that shape).  Here one persistent
+// CTA per SM walks over the HEADS of a (chunk, group) "unit": C stays in shared memory, C.B^T is formed once per unit on the tensor core
+// and stays in REGISTERS (causal and sequence masks already applied), so that a head costs its own x, z, H and out and nothing else.  The
+// (unit, head) pairs are split evenly over the CTAs in unit order, so a CTA meets few units and no wave is left nearly empty.
 //
-// 512 threads.  Two groups of element-wise warps, four for the chunk's first 128 rows and eight for its last (which have 2.6 times
-// as much of the mask), run on their own: each masks a head's A operand into tensor memory, waits for its MMAs and finishes the
-// outputs; while one waits the other computes.  A warp has rows 32 (w % 4) .. of the block -- its tensor-memory lanes -- and all
-// or half of the columns: four 32-column ranges of C.B^T in either group, which makes them one piece of code.  Then one warp for
-// TMA loads and stores, one MMA warp per row block, one warp for the per-head scalars.
+// 768 threads, in roles that hand a head on to one another.  Mask warps, four for the chunk's first 128 rows and eight for its last (which
+// have 2.6 times as much of the mask), hold C.B^T and form the A operand in tensor memory, a half of the steps at a time, so that the MMAs
+// of one half run while the other is formed; they are a head ahead of the output warps, four per row block, which finish the accumulators.
+// A warp has rows 32 (w % 4) .. of its block -- its tensor-memory lanes.  Mask warps have four 32-column ranges of C.B^T in either block,
+// which makes them one piece of code.  Then one warp for TMA loads and stores, one MMA warp per row block, one warp for the per-head scalars.
 //   Y1 = C . H (A = C from shared memory), Y2 = (CB o L) . x (A from tensor memory), out = exp(dA_m) Y1 + Y2 + D x
 // Tensor memory: rows 0-127: accumulators Y1 | Y2 [0, 128), A [128, 192); rows 128-255: [192, 320), A [320, 448).  While a unit
 // starts, C.B^T in fp32 takes the place of a row block's regions (128 and 256 columns).
 // Shared memory: C 64 KB, two stages of x 32 KB | H 16 KB | z 32 KB; the output tile replaces
 // z in place and leaves through a TMA store.  While a unit starts, B lies in the x parts of the two stages.
-// What the layout is chosen for: C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
-// register comes back from L2 (24 element-wise warps of 72 registers spilled 96 bytes and took 0.345 ms for the shape above).
-// Sixteen warps may have 128 registers each.  Instruction fetch is the other thing a kernel of five roles runs out of: loops are
-// rolled, waits short, places advanced without divisions (142 KB of code took 0.45 ms, the same work in 79 KB 0.30 ms).
+//
+// What bounds it: a head takes the output warps' pass over its accumulators (4200 cycles) plus the MMAs that wait for them (1400); the mask
+// warps have a third of the time to spare.  269 us for the shape above (321 with twelve warps that did both, one after the other), 2.7 ms
+// for 262144 steps of 128 heads (3.28).  C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
+// register comes back from L2: the roles share the block's registers out between them (setmaxnreg).  Instruction fetch is what bounds the
+// roles themselves: loops are rolled, waits short, places advanced without divisions.  The output loop unrolled twice takes 273 us, eight
+// times 320; with the next accumulators requested ahead 289.
 //
 // Decay mask, per thread one row m and ranges of 8 columns k:
 //   L[m,k] = exp(dA_m - dA_ref) * (exp(dA_ref - dA_k) dt_k), ref = last column of the range
@@ -515,14 +517,20 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // fails (a steeper decay, or dA not monotone) is done element by element: exp(min(dA_m - dA_k, 0)) dt_k.
 // The factors are rounded to the input dtype and applied with packed 16-bit multiplies.
 constexpr float kMaxDiagSpan = 100.f;
-constexpr int kRowWarps0 = 4, kRowWarps1 = 8, kElemWarps = kRowWarps0 + kRowWarps1, kOutThreads = (kElemWarps + 4) * 32;
+constexpr int kMaskWarps0 = 4, kMaskWarps1 = 8, kRowWarps = 4;      // that form the A operand, per row block; that finish the outputs of a row block
+constexpr int kOutWarp = kMaskWarps0 + kMaskWarps1, kHelperWarp = kOutWarp + 2 * kRowWarps, kOutThreads = (kHelperWarp + 4) * 32;
+constexpr int kMaskRegs = 104, kOutRegs = 64, kHelperRegs = 40, kOutLaunchRegs = 80;       // of a thread, by role; as the block is launched
+static_assert(kMaskRegs * kOutWarp + kOutRegs * 2 * kRowWarps + kHelperRegs * 4 <= kOutLaunchRegs * kOutThreads / 32, "an increase would wait for ever");
+constexpr uint32_t kAcc0 = 0, kA0 = 128, kAcc1 = 192, kA1 = 320;       // places in tensor memory
 struct OutCfg {
     static constexpr uint32_t kC = 4 * 16384, kH = 2 * 8192, kStage = 32768 + kH + 32768;
-    static constexpr uint32_t kScal = 1024 + 128 + 64;  // column factors, 32 refs, then flags, D
+    static constexpr uint32_t kScal = 1024 + 128 + 64;  // column factors, 32 refs, then flags
     static constexpr uint32_t kSmem = kC + 2 * kStage + 2 * kScal + 256;
 };
 static_assert(OutCfg::kSmem <= 227 * 1024, "shared memory");
-enum { kStOutUnit = 21, kStOutCb, kStOutCbRead, kStOutStage, kStOutGate, kStOutA, kStOutAcc, kStOutAccFree, kStOutScal, kStOutScalFree, kStOutTile };
+enum { kStOutUnit = 21, kStOutCb, kStOutCbRead, kStOutStage, kStOutGate, kStOutA, kStOutAcc, kStOutAccFree, kStOutScal, kStOutScalFree, kStOutTile, kStOutAFree };
+enum { kBarCb = 0, kBarCbRead = 2, kBarAcc = 4, kBarAccFree = 6, kBarXh = 8, kBarZ = 10, kBarScal = 12, kBarScalFree = 14, kBarOut = 16, kBarUnit = 20,
+       kBarA = 21, kBarAFree = 25, kBars = 29 };
 
 // Place of a (unit, head) pair; advanced without divisions.  Every role of the kernel walks the same list.
 struct OutWalk {
@@ -571,34 +579,38 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     auto st_z = [&](int s) { return stages + s * Cfg::kStage + 32768 + Cfg::kH; };
     uint8_t *scal = stages + 2 * Cfg::kStage;
     uint64_t *bars = reinterpret_cast<uint64_t *>(scal + 2 * Cfg::kScal);
-    // [row block]: C.B^T formed / read, A in place, accumulators complete / read; [stage]: x and H, z landed; scalars in place /
-    // read; output tile complete (stage * 2 + row block); C and B of a unit landed
-    uint64_t *b_cb = bars, *b_cbread = bars + 2, *b_A = bars + 4, *b_acc = bars + 6, *b_accfree = bars + 8, *b_xh = bars + 10, *b_z = bars + 12,
-             *b_scal = bars + 14, *b_scalfree = bars + 16, *b_out = bars + 18, *b_unit = bars + 22;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 23);
+    // Barriers.  [row block]: C.B^T formed / read, accumulators complete / read; [stage]: x and H, z landed; scalars in place / read;
+    // output tile complete (stage * 2 + row block); C and B of a unit landed; A in place / read (row block * 2 + half of the steps)
+    uint64_t *b_cb = bars + kBarCb, *b_cbread = bars + kBarCbRead, *b_acc = bars + kBarAcc, *b_accfree = bars + kBarAccFree, *b_xh = bars + kBarXh,
+             *b_z = bars + kBarZ, *b_scal = bars + kBarScal, *b_scalfree = bars + kBarScalFree, *b_out = bars + kBarOut, *b_unit = bars + kBarUnit,
+             *b_A = bars + kBarA, *b_Afree = bars + kBarAFree;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kBars);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hpu = nheads / ngroups;                           // heads of a group
     const int it0 = (int)((int64_t)total_items * blockIdx.x / gridDim.x), count = (int)((int64_t)total_items * (blockIdx.x + 1) / gridDim.x) - it0;
-    if (threadIdx.x == kElemWarps * 32) {
+    if (threadIdx.x == kHelperWarp * 32) {
         for (int i = 0; i < 2; ++i) {
-            const int warps = i ? kRowWarps1 : kRowWarps0;
+            const int warps = i ? kMaskWarps1 : kMaskWarps0;
             mbar_init(&b_cb[i], 1);
             mbar_init(&b_cbread[i], warps);
-            mbar_init(&b_A[i], warps);
             mbar_init(&b_acc[i], 1);
-            mbar_init(&b_accfree[i], warps);
+            mbar_init(&b_accfree[i], kRowWarps);
             mbar_init(&b_xh[i], 1);
             mbar_init(&b_z[i], 1);
             mbar_init(&b_scal[i], 1);
-            mbar_init(&b_scalfree[i], kElemWarps);
-            mbar_init(&b_out[2 * i], kRowWarps0);
-            mbar_init(&b_out[2 * i + 1], kRowWarps1);
+            mbar_init(&b_scalfree[i], kMaskWarps0 + kMaskWarps1);
+            mbar_init(&b_out[2 * i], kRowWarps);
+            mbar_init(&b_out[2 * i + 1], kRowWarps);
+        }
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&b_A[i], i < 2 ? kMaskWarps0 : kMaskWarps1);
+            mbar_init(&b_Afree[i], 1);
         }
         mbar_init(b_unit, 1);
         mbar_fence_init();
         if (smem_u32(sm) & 1023u) atomicCAS(status, 0, kStSmemAlign);   // the swizzled tiles assume a 1 KB aligned base
     }
-    if (warp == kElemWarps + 1) tmem_alloc(tmem_slot, 512);
+    if (warp == kHelperWarp + 1) tmem_alloc(tmem_slot, 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -607,188 +619,220 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     pdl_trigger();
     pdl_wait();
 
+    constexpr uint32_t kBarOff = Cfg::kC + 2 * Cfg::kStage + 2 * Cfg::kScal;
     if (!aligned) {
         // nothing runs (the status says so)
-    } else if (warp < kElemWarps) {
-        // ------------------------------------------------------------------ element-wise warps
+    } else if (warp < kOutWarp) {
+        // ------------------------------------------------------------------ mask: A = CB o L
+        registers_up<kMaskRegs>();
         constexpr int NR = 4;                                // 32-column ranges of the mask per thread
-        const int rb = warp < kRowWarps0 ? 0 : 1;            // my row block
-        const int rq = warp & 3, cq_ = rb ? (warp - kRowWarps0) >> 2 : 0;        // my rows of it, my half of the columns
-        const uint32_t tacc_ = tmem + ((uint32_t)(rq * 32) << 16) + (rb ? 192 : 0), smem_ = smem_u32(sm);
+        const int rb = warp < kMaskWarps0 ? 0 : 1;           // my row block
+        const int rq = warp & 3, cq_ = rb ? (warp - kMaskWarps0) >> 2 : 0;       // my rows of it, my half of the columns
+        const uint32_t tlane_ = tmem + ((uint32_t)(rq * 32) << 16), smem_ = smem_u32(sm);
         const int r = rb * 128 + rq * 32 + lane;             // my row of the chunk
         bool ok = true;
         uint32_t cb[NR][16];                                 // my ranges of C.B^T, packed, masked
         const float *dA = dAb;                               // of the current (batch row, head, chunk)
         float dA_next = 0.f;
         int left = 0;                                        // heads left in the unit
-        bool carry = true, rows = true;                      // my row continues the sequence that ended the previous chunk; the chunk reaches my block
+        bool rows = true;                                    // the chunk reaches my block
         int nunits = 0, item = 0;
-        [[maybe_unused]] const float *Dv = nullptr;                           // DV: D of my columns
-        constexpr uint32_t kBarOff = Cfg::kC + 2 * Cfg::kStage + 2 * Cfg::kScal;
 
 #pragma unroll 1
         for (int seq = 0; seq < count; ++seq) {
             // everything below is derived from these three; hidden from the compiler, which would otherwise keep dozens of addresses
             // and range numbers over the loop -- in spilled registers
-            uint32_t smb = smem_, tacc = tacc_;
+            uint32_t smb = smem_, tlane = tlane_;
             int cq = cq_;
-            asm volatile("" : "+r"(smb), "+r"(tacc), "+r"(cq));
-            auto bar = [&](int k) { return smb + kBarOff + 8 * k; };             // same numbering as the pointers above
+            asm volatile("" : "+r"(smb), "+r"(tlane), "+r"(cq));
+            auto bar = [&](int k) { return smb + kBarOff + 8 * k; };
             // range t of mine: columns 32 j .. of the chunk (one tile of 128 columns, or a half of each of two)
             auto range = [&](int t) { return rb ? (t >> 1) * 4 + 2 * cq + (t & 1) : t; };
             if (left == 0) {
-                // a new unit: nothing of this group is in flight; C.B^T moves from tensor memory into registers
+                // a new unit: C.B^T moves from tensor memory into registers
                 const OutWalk w(it0 + seq, ngroups, nchunks, hpu);
                 left = hpu - w.hv;
                 rows = rb < w.row_blocks(seqlen);
                 dA = dAb + (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ;
-                if constexpr (DV) Dv = Dp + (int64_t)w.h * kP;
                 if (rows) {
-                    int lo = 0;                              // first column of my row's sequence inside the chunk
-                    if (seq_start) {
-                        const int64_t bc = (int64_t)w.b * nchunks + w.c;
-                        lo = seq_start[bc * kQ + r];
-                        carry = lo == 0 && seq_carry[bc] != 0;
-                    }
+                    // first column of my row's sequence inside the chunk
+                    const int lo = seq_start ? seq_start[((int64_t)w.b * nchunks + w.c) * kQ + r] : 0;
                     dA_next = dA[r];
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(rb), nunits & 1, status, kStOutCb));      // tcgen05.ld is warp-collective
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCb + rb), nunits & 1, status, kStOutCb));      // tcgen05.ld is warp-collective
                     ++nunits;
                     if (!ok) break;
                     tc_fence_after_sync();
+                    const uint32_t from = tlane + (rb ? kAcc1 : kAcc0);
 #pragma unroll
                     for (int t = 0; t < NR; ++t) {
+                        // columns [lo, m] of the chunk stay
+                        const int k0 = 32 * range(t), first = lo - k0, last = r - k0;
+                        uint32_t keep = last < 0 ? 0u : last >= 31 ? ~0u : (2u << last) - 1u;
+                        if (first > 0) keep &= first > 31 ? 0u : ~0u << first;
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            float v[16];
-                            const int kc = 32 * range(t) + 16 * half;
-                            tmem_ld16(tacc + kc, v);
-                            // columns [lo, m] of the chunk stay
-                            const int first_k = lo - kc, last_k = r - kc;
+                        for (int e = 0; e < 4; ++e) {
+                            uint32_t v[8];
+                            tmem_ld8_issue(from + k0 + 8 * e, v);
+                            tmem_ld_wait(v);
 #pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                cb[t][8 * half + i] = Pack2<T>::pack(2 * i >= first_k && 2 * i <= last_k ? v[2 * i] : 0.f,
-                                                                     2 * i + 1 >= first_k && 2 * i + 1 <= last_k ? v[2 * i + 1] : 0.f);
+                            for (int i = 0; i < 8; ++i) v[i] = keep >> (8 * e + i) & 1u ? v[i] : 0u;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) cb[t][4 * e + i] = Pack2<T>::pack(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
                         }
                     }
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(2 + rb));
+                    if (lane == 0) mbar_arrive(bar(kBarCbRead + rb));
                     // the A operand of the lower row block takes the place of C.B^T: no warp may write it while another still reads
-                    if (rb) ok = __all_sync(0xffffffffu, mbar_wait(bar(2 + rb), (nunits - 1) & 1, status, kStOutCbRead));
+                    if (rb) ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCbRead + rb), (nunits - 1) & 1, status, kStOutCbRead));
                     if (!ok) break;
                 }
             }
-            const int s = seq & 1, sph = (seq >> 1) & 1;
+            const int s = seq & 1;
             const uint32_t sc = smb + Cfg::kC + 2 * Cfg::kStage + s * Cfg::kScal;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(14 + s), sph, status, kStOutScal));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarScal + s), (seq >> 1) & 1, status, kStOutScal));
             if (!ok) break;
             --left;
             if (!rows) {                                     // no rows here in this chunk
-                if (lane == 0) mbar_arrive(bar(16 + s));
+                if (lane == 0) mbar_arrive(bar(kBarScalFree + s));
                 continue;
             }
             const float dAm = dA_next * kLog2e;
             if (left) dA_next = dA[(int64_t)nchunks * kQ + r];                           // a whole head ahead of its use
-            const int flags = __float_as_int(lds32(sc + 1024 + 128));
-            const float Dh = lds32(sc + 1024 + 132);
-
-            // ---- A operand: my columns of CB o L
-            if (flags != 255) {
-                // rare: ranges that the factorised mask cannot do have their decays formed element by element and parked where their
-                // A words go (one rolled loop, so that it costs neither registers nor instruction cache)
-#pragma unroll 1
-                for (int i = 0; i < NR * 16; ++i) {
-                    const int j = range(i >> 4), kk = 32 * j + 2 * (i & 15);
-                    if ((flags >> j) & 1) continue;
-                    const float2 d = *reinterpret_cast<const float2 *>(dA + kk), t = *reinterpret_cast<const float2 *>(dtb + (dA - dAb) + kk);
-                    const float l0 = ex2(fminf(fmaf(d.x, -kLog2e, dAm), 0.f)) * t.x, l1 = ex2(fminf(fmaf(d.y, -kLog2e, dAm), 0.f)) * t.y;
-                    tmem_st1_issue(tacc + 128 + 16 * j + (i & 15), Pack2<T>::pack(l0, l1));
-                }
-                tmem_st_wait();
-            }
-            dA += (int64_t)nchunks * kQ;
+            const uint32_t flags = __float_as_uint(lds32(sc + 1024 + 128));
+            const uint32_t A = tlane + (rb ? kA1 : kA0);
 #pragma unroll
             for (int t = 0; t < NR; ++t) {
-                const int j = range(t);
-                const bool past = j - 4 * rb > rq;                               // wholly past the diagonal
-                const uint32_t dst = tacc + 128 + 16 * j;
-                uint32_t a[16];
-                if (past) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) a[i] = 0u;
-                } else {
-                    if ((flags >> j) & 1) {
-                        float rm[4];
-                        lds128f(sc + 1024 + 16 * j, rm);
-#pragma unroll
-                        for (int g = 0; g < 4; ++g) {
-                            const float f = ex2(fminf(dAm - rm[g], kMaxDiagSpan));       // (a range past the diagonal only has to stay finite)
-                            const uint64_t f2 = pack2(f, f);
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                uint64_t c0, c1;
-                                lds_pair2(sc + 128 * j + 32 * g + 16 * i, c0, c1);
-                                float l0, l1, l2, l3;
-                                unpack2(mul2(f2, c0), l0, l1);
-                                unpack2(mul2(f2, c1), l2, l3);
-                                if constexpr (Fmt<T>::v == 0) {  // half precision: a factor past the diagonal must not become infinite
-                                    l0 = fminf(l0, 65504.f); l1 = fminf(l1, 65504.f);
-                                    l2 = fminf(l2, 65504.f); l3 = fminf(l3, 65504.f);
-                                }
-                                a[4 * g + 2 * i] = Pack2<T>::pack(l0, l1);
-                                a[4 * g + 2 * i + 1] = Pack2<T>::pack(l2, l3);
-                            }
-                        }
-                    } else {
-                        float l[16];
-                        tmem_ld16(dst, l);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) a[i] = __float_as_uint(l[i]);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) a[i] = Pack2<T>::mul(cb[t][i], a[i]);
+                if ((t & 1) == 0) {      // half of the reduction: its MMAs run while the other half is formed, and before that the ones that read what is there now
+                    if (item) ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarAFree + 2 * rb + t / 2), (item - 1) & 1, status, kStOutAFree));
+                    if (!ok) break;
+                    tc_fence_after_sync();
                 }
-                __syncwarp();                                // tcgen05.st is warp-collective
-                tmem_st16_issue(dst, a);
+                const int j = range(t);
+                const uint32_t dst = A + 16 * j, ck = sc + 128 * j;
+                // (every branch goes one way for the whole warp: tcgen05.ld and .st are warp-collective)
+                if (j - 4 * rb > rq) {                       // wholly past the diagonal
+                    const uint32_t none[8] = {};
+                    tmem_st8_issue(dst, none);
+                    tmem_st8_issue(dst + 8, none);
+                } else if ((flags >> (4 * j)) & 1) {
+                    float f[4];
+                    lds128f(sc + 1024 + 16 * j, f);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) f[g] = ex2(fminf(dAm - f[g], kMaxDiagSpan));         // (a range past the diagonal only has to stay finite)
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        uint64_t c[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) lds_pair2(ck + 64 * half + 16 * i, c[2 * i], c[2 * i + 1]);
+                        uint32_t a[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const float fg = f[2 * half + i / 4];
+                            float l0, l1;
+                            unpack2(mul2(pack2(fg, fg), c[i]), l0, l1);
+                            if constexpr (Fmt<T>::v == 0) l0 = fminf(l0, 65504.f), l1 = fminf(l1, 65504.f);      // half precision: a factor past the diagonal must not become infinite
+                            a[i] = Pack2<T>::mul(cb[t][8 * half + i], Pack2<T>::pack(l0, l1));
+                        }
+                        tmem_st8_issue(dst + 8 * half, a);
+                    }
+                } else {
+                    // rare: a range that the factorised mask cannot do has its decays formed element by element, parked where its A words go
+                    // (in a rolled loop, so that it costs neither registers nor instruction cache)
+#pragma unroll 1
+                    for (int i = 0; i < 16; ++i) {
+                        const float2 d = *reinterpret_cast<const float2 *>(dA + 32 * j + 2 * i), w = *reinterpret_cast<const float2 *>(dtb + (dA - dAb) + 32 * j + 2 * i);
+                        const float l0 = ex2(fminf(fmaf(d.x, -kLog2e, dAm), 0.f)) * w.x, l1 = ex2(fminf(fmaf(d.y, -kLog2e, dAm), 0.f)) * w.y;
+                        __syncwarp();
+                        tmem_st1_issue(dst + i, Pack2<T>::pack(l0, l1));
+                    }
+                    tmem_st_wait();
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        uint32_t a[8];
+                        tmem_ld8_issue(dst + 8 * half, a);
+                        tmem_ld_wait(a);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) a[i] = Pack2<T>::mul(cb[t][8 * half + i], a[i]);
+                        tmem_st8_issue(dst + 8 * half, a);
+                    }
+                }
+                if (t & 1) {
+                    tmem_st_wait();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kBarA + 2 * rb + t / 2));
+                }
             }
-            tmem_st_wait();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(bar(4 + rb));
-                mbar_arrive(bar(16 + s));
+            if (!ok) break;
+            if (lane == 0) mbar_arrive(bar(kBarScalFree + s));
+            dA += (int64_t)nchunks * kQ;
+            ++item;
+        }
+    } else if (warp < kHelperWarp) {
+        // ------------------------------------------------------------------ outputs: out = exp(dA_m) Y1 + Y2 + D x, gated
+        registers_down<kOutRegs>();
+        const int rb = (warp - kOutWarp) >> 2, rq = warp & 3;
+        const uint32_t acc = tmem + ((uint32_t)(rq * 32) << 16) + (rb ? kAcc1 : kAcc0), smb = smem_u32(sm);
+        const int r = rb * 128 + rq * 32 + lane;             // my row of the chunk
+        auto bar = [&](int k) { return smb + kBarOff + 8 * k; };
+        const float *dA = dAb, *Dv = Dp;                     // of the current head; DV: D of its columns
+        float dA_next = 0.f, D_next = 0.f;
+        int left = 0, item = 0;
+        bool carry = true, rows = true, ok = true;           // my row continues the sequence that ended the previous chunk; the chunk reaches my block
+#pragma unroll 1
+        for (int seq = 0; seq < count; ++seq) {
+            if (left == 0) {
+                const OutWalk w(it0 + seq, ngroups, nchunks, hpu);
+                left = hpu - w.hv;
+                rows = rb < w.row_blocks(seqlen);
+                dA = dAb + (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ + r;
+                if (Dp) Dv = Dp + (int64_t)w.h * (DV ? kP : 1);
+                if (rows) {
+                    if (seq_start) {
+                        const int64_t bc = (int64_t)w.b * nchunks + w.c;
+                        carry = seq_start[bc * kQ + r] == 0 && seq_carry[bc] != 0;
+                    }
+                    dA_next = *dA;
+                    if (Dp && !DV) D_next = *Dv;
+                }
             }
-
-            // ---- outputs
-            const float rs = carry ? ex2(dAm) : 0.f;
+            --left;
+            if (!rows) continue;
+            const int s = seq & 1, sph = (seq >> 1) & 1;
+            const float rs = carry ? ex2(dA_next * kLog2e) : 0.f, Dh = D_next;
+            if (left) {                                      // a whole head ahead of their use
+                dA_next = dA[(int64_t)nchunks * kQ];
+                if (Dp && !DV) D_next = Dv[1];
+            }
+            dA += (int64_t)nchunks * kQ;
             const uint32_t row = smb + Cfg::kC + s * Cfg::kStage + r * 128;
-            if (has_z) ok = mbar_wait(bar(12 + s), sph, status, kStOutGate);
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(6 + rb), item & 1, status, kStOutAcc) && ok);     // tcgen05.ld is warp-collective
+            ok = mbar_wait(bar(kBarZ + s), sph, status, kStOutGate);         // (x is there when its product is)
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarAcc + rb), item & 1, status, kStOutAcc) && ok);     // tcgen05.ld is warp-collective
             ++item;
             if (!ok) break;
             tc_fence_after_sync();
-            const int e8_end = rb ? 4 * cq + 4 : 8;
             const uint64_t rs2 = pack2(rs, rs), D2 = pack2(Dh, Dh);
 #pragma unroll 1
-            for (int e8 = 4 * cq; e8 < e8_end; ++e8) {
+            for (int e8 = 0; e8 < 8; ++e8) {
                 uint32_t y1[8], y2[8];
-                tmem_ld8_issue(tacc + e8 * 8, y1);
-                tmem_ld8_issue(tacc + 64 + e8 * 8, y2);
+                tmem_ld8_issue(acc + e8 * 8, y1);
+                tmem_ld8_issue(acc + 64 + e8 * 8, y2);
                 const uint32_t xaddr = row + (uint32_t)((e8 ^ (r & 7)) << 4), zaddr = xaddr + 32768 + Cfg::kH;
                 uint4 xv = make_uint4(0, 0, 0, 0), zv = make_uint4(0, 0, 0, 0);
                 if (Dp) xv = lds128(xaddr);
                 if (has_z) zv = lds128(zaddr);
                 tmem_ld_wait(y1, y2);
-                if (e8 == e8_end - 1) {
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(8 + rb));
-                }
                 uint64_t y[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     y[i] = fma2(rs2, pack2(__uint_as_float(y1[2 * i]), __uint_as_float(y1[2 * i + 1])),
                                 pack2(__uint_as_float(y2[2 * i]), __uint_as_float(y2[2 * i + 1])));
+                if (e8 == 7) {
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kBarAccFree + rb));
+                }
                 if (Dp) {
                     const uint32_t xe[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
@@ -826,197 +870,205 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 }
                 sts128(zaddr, make_uint4(o[0], o[1], o[2], o[3]));
             }
-            if constexpr (DV) Dv += kP;
+            if (Dp) Dv += DV ? kP : 1;
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(18 + 2 * s + rb));
+            if (lane == 0) mbar_arrive(bar(kBarOut + 2 * s + rb));
         }
-    } else if (warp == kElemWarps + 1 || warp == kElemWarps + 2) {
-        // ------------------------------------------------------------------ MMAs of one row block
-        const int rb = (int)warp_uniform(warp) - (kElemWarps + 1);
-        OutWalk w(it0, ngroups, nchunks, hpu);
-        auto step = [&] { w.step(ngroups, nchunks, hpu); };
-        const uint32_t tm = warp_uniform(tmem), acc = tm + (rb ? 192 : 0), A = tm + (rb ? 320 : 128);
-        auto wait = [&](uint64_t *bar, int phase, int code) { return __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, status, code)) != 0; };
-        bool ok = true, rows = true;
-        int nunits = 0, item = 0, cb_done = 0;
-        const uint32_t idesc_cb = instr_desc_f16(128, 128, Fmt<T>::v, 0, 0) + ((uint32_t)(rb ? 128 >> 3 : 0) << 17),      // N = 128 or 256
-                       idesc_y1 = instr_desc_f16(128, 64, Fmt<T>::v, 0, h_np ? 1 : 0), idesc_y2 = instr_desc_f16(128, 64, Fmt<T>::v, 0, 1);
-        const uint32_t step_H = h_np ? 128 : 2;              // states along the rows of the tile, or along its columns
-        const uint64_t desc_C = smem_desc_sw128(smem_u32(Cs) + rb * 2 * 16384, 16, 1024), desc_x = smem_desc_sw128(smem_u32(st_x(0)), 16, 1024),
-                       desc_H = smem_desc_sw128(smem_u32(st_H(0)), 16, 1024);
+    } else {
+        registers_down<kHelperRegs>();
+        if (warp == kHelperWarp + 1 || warp == kHelperWarp + 2) {
+            // ------------------------------------------------------------------ MMAs of one row block
+            const int rb = (int)warp_uniform(warp) - (kHelperWarp + 1);
+            OutWalk w(it0, ngroups, nchunks, hpu);
+            auto step = [&] { w.step(ngroups, nchunks, hpu); };
+            const uint32_t tm = warp_uniform(tmem), acc = tm + (rb ? kAcc1 : kAcc0);
+            auto wait = [&](uint64_t *bar, int phase, int code) { return __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, status, code)) != 0; };
+            bool ok = true, rows = true;
+            int nunits = 0, item = 0, cb_done = 0;
+            const uint32_t idesc_cb = instr_desc_f16(128, 128, Fmt<T>::v, 0, 0) + ((uint32_t)(rb ? 128 >> 3 : 0) << 17),      // N = 128 or 256
+                           idesc_y1 = instr_desc_f16(128, 64, Fmt<T>::v, 0, h_np ? 1 : 0), idesc_y2 = instr_desc_f16(128, 64, Fmt<T>::v, 0, 1);
+            const uint32_t step_H = h_np ? 128 : 2;              // states along the rows of the tile, or along its columns
+            const uint64_t desc_C = smem_desc_sw128(smem_u32(Cs) + rb * 2 * 16384, 16, 1024), desc_x = smem_desc_sw128(smem_u32(st_x(0)), 16, 1024),
+                           desc_H = smem_desc_sw128(smem_u32(st_H(0)), 16, 1024);
 #pragma unroll 1
-        for (int seq = 0; seq < count && ok; ++seq, step()) {
-            if (w.enter) {
-                rows = rb < w.row_blocks(seqlen);
-                ok = wait(b_unit, nunits, kStOutUnit);       // every unit completes one phase, whatever its row blocks
-                ++nunits;
+            for (int seq = 0; seq < count && ok; ++seq, step()) {
+                if (w.enter) {
+                    rows = rb < w.row_blocks(seqlen);
+                    ok = wait(b_unit, nunits, kStOutUnit);       // every unit completes one phase, whatever its row blocks
+                    ++nunits;
+                    if (!ok) break;
+                    if (rows) {
+                        if (item) ok = wait(&b_accfree[rb], item - 1, kStOutAccFree);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        if (elect_one()) {
+#pragma unroll 1
+                            for (int kb = 0; kb < 2; ++kb)      // B lies in the x parts of the stages
+                                mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_x + kb * (Cfg::kStage / 16), 2, idesc_cb, kb > 0);
+                            mma_commit(&b_cb[rb]);
+                        }
+                        __syncwarp();
+                        ok = wait(&b_cbread[rb], cb_done, kStOutCbRead);
+                        ++cb_done;
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                    }
+                }
+                if (!rows) continue;
+                const int s = seq & 1;
+                const uint64_t off = s * (Cfg::kStage / 16);
+                ok = wait(&b_xh[s], seq >> 1, kStOutStage) && (item == 0 || wait(&b_accfree[rb], item - 1, kStOutAccFree));
                 if (!ok) break;
-                if (rows) {
-                    if (item) ok = wait(&b_accfree[rb], item - 1, kStOutAccFree);
+                tc_fence_after_sync();
+                if (elect_one()) {
+#pragma unroll 1
+                    for (int kb = 0; kb < 2; ++kb)
+                        mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_H + off + kb * (8192 / 16), step_H, idesc_y1, kb > 0);
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    ok = wait(&b_A[2 * rb + half], item, kStOutA);
                     if (!ok) break;
                     tc_fence_after_sync();
                     if (elect_one()) {
-#pragma unroll 1
-                        for (int kb = 0; kb < 2; ++kb)      // B lies in the x parts of the stages
-                            mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_x + kb * (Cfg::kStage / 16), 2, idesc_cb, kb > 0);
-                        mma_commit(&b_cb[rb]);
+                        const int steps = 4 * (rb + 1);
+                        mma_steps_ts(steps, acc + 64, tm + (rb ? kA1 : kA0) + half * steps * 8, desc_x + off + half * steps * 128, 128, idesc_y2, half > 0);
+                        mma_commit(&b_Afree[2 * rb + half]);
+                        if (half) mma_commit(&b_acc[rb]);
                     }
                     __syncwarp();
-                    ok = wait(&b_cbread[rb], cb_done, kStOutCbRead);
-                    ++cb_done;
-                    if (!ok) break;
-                    tc_fence_after_sync();
                 }
+                ++item;
+                if (!ok) break;
+                __syncwarp();
             }
-            if (!rows) continue;
-            const int s = seq & 1;
-            const uint64_t off = s * (Cfg::kStage / 16);
-            ok = wait(&b_xh[s], seq >> 1, kStOutStage) && (item == 0 || wait(&b_accfree[rb], item - 1, kStOutAccFree));
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (elect_one()) {
-#pragma unroll 1
-                for (int kb = 0; kb < 2; ++kb)
-                    mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_H + off + kb * (8192 / 16), step_H, idesc_y1, kb > 0);
-            }
-            __syncwarp();
-            ok = wait(&b_A[rb], item, kStOutA);
-            ++item;
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (elect_one()) {
-                mma_steps_ts(8 * (rb + 1), acc + 64, A, desc_x + off, 128, idesc_y2, false);
-                mma_commit(&b_acc[rb]);
-            }
-            __syncwarp();
-        }
-    } else if (warp == kElemWarps) {
-        // ------------------------------------------------------------------ TMA loads and stores
-        if (lane == 0) {
-            OutWalk w(it0, ngroups, nchunks, hpu);
-            auto step = [&] { w.step(ngroups, nchunks, hpu); };
-            bool ok = true;
-            uint32_t outs = 0, cbs = 0;          // parities of the next completion of each b_out, b_cb
-            struct Pending { int b, h, t, nrb; } pend[2] = {};
-            int nunits_requested = 0, seq = 0, done = 0;         // units requested; heads requested, finished
-            // Heads leave in the order in which they came: the one in stage s has its output tiles stored as they are completed,
-            // and the stage is free once they have been read.  A new unit starts when both stages are free: C goes to its place,
-            // B to the x parts of the stages.
-#pragma unroll 1
-            while (ok) {
-                const bool have = seq < count;
-                const int keep = have && !w.enter ? 1 : 0;       // heads that may stay in flight before the next request
-                if (done + keep < seq) {
-                    const int s = done & 1;
-#pragma unroll 1
-                    for (int rb = 0; rb < pend[s].nrb && ok; ++rb) {
-                        const int k = 2 * s + rb;
-                        ok = mbar_wait(&b_out[k], (outs >> k) & 1, status, kStOutTile);
-                        outs ^= 1u << k;
-                        if (ok) {
-                            tma_store_4d(&tm_out, st_z(s) + rb * 16384, 0, pend[s].h, pend[s].t + rb * 128, pend[s].b);
-                            tma_store_commit();
-                        }
-                    }
-                    tma_store_wait_read();
-                    ++done;
-                    continue;
-                }
-                if (!have) break;
-                const int s = seq & 1, nrb = w.row_blocks(seqlen);
-                if (w.enter) {
-                    ++nunits_requested;
-                    mbar_expect_tx(b_unit, nrb * 2 * 16384 + 2 * 32768);
-#pragma unroll 1
-                    for (int kb = 0; kb < 2; ++kb) {
-#pragma unroll 1
-                        for (int rb = 0; rb < nrb; ++rb) tma_load_4d(Cs + (rb * 2 + kb) * 16384, &tm_C, b_unit, kb * 64, w.g, w.c * kQ + rb * 128, w.b);
-                        tma_load_4d(st_x(kb), &tm_B, b_unit, kb * 64, w.g, w.c * kQ, w.b);
-                    }
-#pragma unroll 1
-                    for (int rb = 0; rb < nrb && ok; ++rb) {
-                        ok = mbar_wait(&b_cb[rb], (cbs >> rb) & 1, status, kStOutCb);        // B has been read
-                        cbs ^= 1u << rb;
-                    }
-                    if (!ok) break;
-                }
-                mbar_expect_tx(&b_xh[s], 32768 + Cfg::kH);
-                tma_load_4d(st_x(s), &tm_x, &b_xh[s], 0, w.h, w.c * kQ, w.b);
-                const int uh = (w.b * nchunks + w.c) * nheads + w.h;
-                if (h_np) tma_load_3d(st_H(s), &tm_H, &b_xh[s], 0, 0, uh);                     // [n][p] tile
-                else
-#pragma unroll 1
-                    for (int kb = 0; kb < 2; ++kb) tma_load_3d(st_H(s) + kb * 8192, &tm_H, &b_xh[s], kb * 64, 0, uh);   // columns n of the [p][n] state
-                if (has_z) {
-                    mbar_expect_tx(&b_z[s], 32768);
-                    tma_load_4d(st_z(s), &tm_z, &b_z[s], 0, w.h, w.c * kQ, w.b);
-                }
-                pend[s] = {w.b, w.h, w.c * kQ, nrb};
-                ++seq;
-                step();
-            }
-            if (!ok) {
-                // gave up: nothing may still be landing in this CTA's shared memory when it exits
-                tma_store_wait_read();
-                if (nunits_requested) mbar_wait(b_unit, (nunits_requested - 1) & 1, status, kStOutUnit);
-#pragma unroll 1
-                for (int k = seq > 2 ? seq - 2 : 0; k < seq; ++k) {
-                    mbar_wait(&b_xh[k & 1], (k >> 1) & 1, status, kStOutStage);
-                    if (has_z) mbar_wait(&b_z[k & 1], (k >> 1) & 1, status, kStOutGate);
-                }
-            }
-        }
-    } else {
-        // ------------------------------------------------------------------ per-head scalars
-        OutWalk w(it0, ngroups, nchunks, hpu);
-        auto step = [&] { w.step(ngroups, nchunks, hpu); };
-        bool ok = true;
-        float dA[8], dt[8];                      // step 32 j + lane
-        auto request = [&]() {
-            const int64_t o = (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ + lane;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                dA[j] = dAb[o + 32 * j];
-                dt[j] = dtb[o + 32 * j];
-            }
-            return (Dp && !DV) ? Dp[w.h] : 0.f;
-        };
-        float Dnext = count > 0 ? request() : 0.f;
-#pragma unroll 1
-        for (int seq = 0; seq < count && ok; ++seq) {
-            const int s = seq & 1;
-            float *ck = reinterpret_cast<float *>(scal + s * Cfg::kScal), *ref = ck + 256;
-            if (seq >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&b_scalfree[s], ((seq >> 1) - 1) & 1, status, kStOutScalFree));
-            if (!ok) break;
-            int flags = 0;                       // bit j: range j may use the factorised mask
-            bool mono = true;
-            float before = dA[0];                // dA of the step before the range's first
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float v = dA[j] * kLog2e, rf = __shfl_sync(0xffffffffu, v, lane | 7);
-                ck[32 * j + lane] = ex2(rf - v) * dt[j];
-                if ((lane & 7) == 7) ref[4 * j + (lane >> 3)] = v;
-                float up = __shfl_up_sync(0xffffffffu, dA[j], 1);
-                if (lane == 0) up = before;
-                mono = mono && dA[j] <= up + 2e-6f * fabsf(up);      // rounding of the sums aside
-                before = __shfl_sync(0xffffffffu, dA[j], 31);
-                if (__all_sync(0xffffffffu, v - rf <= kMaxDiagSpan)) flags |= 1 << j;
-            }
-            if (!__all_sync(0xffffffffu, mono)) flags = 0;
+        } else if (warp == kHelperWarp) {
+            // ------------------------------------------------------------------ TMA loads and stores
             if (lane == 0) {
-                reinterpret_cast<int *>(ref)[32] = flags;
-                ref[33] = Dnext;
+                OutWalk w(it0, ngroups, nchunks, hpu);
+                auto step = [&] { w.step(ngroups, nchunks, hpu); };
+                bool ok = true;
+                uint32_t outs = 0, cbs = 0;          // parities of the next completion of each b_out, b_cb
+                struct Pending { int b, h, t, nrb; } pend[2] = {};
+                int nunits_requested = 0, seq = 0, done = 0;         // units requested; heads requested, finished
+                // Heads leave in the order in which they came: the one in stage s has its output tiles stored as they are completed.  Then the
+                // next head's x and H may take the place of its own at once; z, whose place the output tiles have, when these have been read.
+                // A new unit starts when no head is in flight: C goes to its place, B to the x parts of the stages.
+#pragma unroll 1
+                while (ok) {
+                    const bool have = seq < count;
+                    const int keep = have && !w.enter ? 1 : 0;       // heads that may stay in flight before the next request
+                    if (done + keep < seq) {
+                        const int s = done & 1;
+#pragma unroll 1
+                        for (int rb = 0; rb < pend[s].nrb && ok; ++rb) {
+                            const int k = 2 * s + rb;
+                            ok = mbar_wait(&b_out[k], (outs >> k) & 1, status, kStOutTile);
+                            outs ^= 1u << k;
+                            if (ok) {
+                                tma_store_4d(&tm_out, st_z(s) + rb * 16384, 0, pend[s].h, pend[s].t + rb * 128, pend[s].b);
+                                tma_store_commit();
+                            }
+                        }
+                        ++done;
+                        continue;
+                    }
+                    if (!have) break;
+                    const int s = seq & 1, nrb = w.row_blocks(seqlen);
+                    if (w.enter) {
+                        ++nunits_requested;
+                        mbar_expect_tx(b_unit, nrb * 2 * 16384 + 2 * 32768);
+#pragma unroll 1
+                        for (int kb = 0; kb < 2; ++kb) {
+#pragma unroll 1
+                            for (int rb = 0; rb < nrb; ++rb) tma_load_4d(Cs + (rb * 2 + kb) * 16384, &tm_C, b_unit, kb * 64, w.g, w.c * kQ + rb * 128, w.b);
+                            tma_load_4d(st_x(kb), &tm_B, b_unit, kb * 64, w.g, w.c * kQ, w.b);
+                        }
+#pragma unroll 1
+                        for (int rb = 0; rb < nrb && ok; ++rb) {
+                            ok = mbar_wait(&b_cb[rb], (cbs >> rb) & 1, status, kStOutCb);        // B has been read
+                            cbs ^= 1u << rb;
+                        }
+                        if (!ok) break;
+                    }
+                    mbar_expect_tx(&b_xh[s], 32768 + Cfg::kH);
+                    tma_load_4d(st_x(s), &tm_x, &b_xh[s], 0, w.h, w.c * kQ, w.b);
+                    const int uh = (w.b * nchunks + w.c) * nheads + w.h;
+                    if (h_np) tma_load_3d(st_H(s), &tm_H, &b_xh[s], 0, 0, uh);                     // [n][p] tile
+                    else
+#pragma unroll 1
+                        for (int kb = 0; kb < 2; ++kb) tma_load_3d(st_H(s) + kb * 8192, &tm_H, &b_xh[s], kb * 64, 0, uh);   // columns n of the [p][n] state
+                    tma_store_wait_read();
+                    if (has_z) {
+                        mbar_expect_tx(&b_z[s], 32768);
+                        tma_load_4d(st_z(s), &tm_z, &b_z[s], 0, w.h, w.c * kQ, w.b);
+                    } else {
+                        mbar_arrive(&b_z[s]);                        // the place is free
+                    }
+                    pend[s] = {w.b, w.h, w.c * kQ, nrb};
+                    ++seq;
+                    step();
+                }
+                tma_store_wait_read();
+                if (!ok) {
+                    // gave up: nothing may still be landing in this CTA's shared memory when it exits
+                    if (nunits_requested) mbar_wait(b_unit, (nunits_requested - 1) & 1, status, kStOutUnit);
+#pragma unroll 1
+                    for (int k = seq > 2 ? seq - 2 : 0; k < seq; ++k) {
+                        mbar_wait(&b_xh[k & 1], (k >> 1) & 1, status, kStOutStage);
+                        if (has_z) mbar_wait(&b_z[k & 1], (k >> 1) & 1, status, kStOutGate);
+                    }
+                }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&b_scal[s]);
-            step();
-            if (seq + 1 < count) Dnext = request();
+        } else {
+            // ------------------------------------------------------------------ per-head scalars
+            OutWalk w(it0, ngroups, nchunks, hpu);
+            bool ok = true;
+            float4 dA[2], dt[2];                     // of my eight steps: one range of the factorised mask
+            auto request = [&]() {
+                const int64_t o = (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ + 8 * lane;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    dA[i] = *reinterpret_cast<const float4 *>(dAb + o + 4 * i);
+                    dt[i] = *reinterpret_cast<const float4 *>(dtb + o + 4 * i);
+                }
+            };
+            if (count > 0) request();
+#pragma unroll 1
+            for (int seq = 0; seq < count && ok; ++seq) {
+                const int s = seq & 1;
+                float *ck = reinterpret_cast<float *>(scal + s * Cfg::kScal), *ref = ck + 256;
+                if (seq >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&b_scalfree[s], ((seq >> 1) - 1) & 1, status, kStOutScalFree));
+                if (!ok) break;
+                const float a[8] = {dA[0].x, dA[0].y, dA[0].z, dA[0].w, dA[1].x, dA[1].y, dA[1].z, dA[1].w};
+                const float end = a[7] * kLog2e;
+                float before = __shfl_up_sync(0xffffffffu, a[7], 1);                 // dA of the step before mine
+                if (lane == 0) before = a[0];
+                bool mono = true;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) mono = mono && a[i] <= (i ? a[i - 1] : before) + 2e-6f * fabsf(i ? a[i - 1] : before);      // rounding of the sums aside
+                auto factor = [&](int i, float t) { return ex2(end - a[i] * kLog2e) * t; };
+                *reinterpret_cast<float4 *>(ck + 8 * lane) = make_float4(factor(0, dt[0].x), factor(1, dt[0].y), factor(2, dt[0].z), factor(3, dt[0].w));
+                *reinterpret_cast<float4 *>(ck + 8 * lane + 4) = make_float4(factor(4, dt[1].x), factor(5, dt[1].y), factor(6, dt[1].z), factor(7, dt[1].w));
+                ref[lane] = end;
+                // bit 4 j: the ranges of columns 32 j .. 32 j + 31 may use the factorised mask
+                uint32_t flags = __ballot_sync(0xffffffffu, a[0] * kLog2e - end <= kMaxDiagSpan);
+                flags &= flags >> 1;
+                flags &= flags >> 2;
+                if (!__all_sync(0xffffffffu, mono)) flags = 0;
+                if (lane == 0) reinterpret_cast<uint32_t *>(ref)[32] = flags;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&b_scal[s]);
+                w.step(ngroups, nchunks, hpu);
+                if (seq + 1 < count) request();
+            }
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kElemWarps + 1) tmem_dealloc(tmem, 512);
+    if (warp == kHelperWarp + 1) tmem_dealloc(tmem, 512);
 }
 
 // ====================================================================================== incoming state
@@ -1360,14 +1412,20 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     const int grid = (int)std::min<int64_t>(items, sm_count(a.device));
     const uint8_t *seq_start = a.seq_idx ? reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_start) : nullptr;
     const uint8_t *seq_carry = reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_carry);
-    auto go = [&](auto dv) {
+    auto go = [&](auto dv) -> bool {
         auto kernel = ssd_tc_output_kernel<T, decltype(dv)::value>;
+        // its warps would wait for ever for registers that the block was not launched with
+        static const bool enough = [&] {
+            cudaFuncAttributes at;
+            return cudaFuncGetAttributes(&at, reinterpret_cast<const void *>(kernel)) == cudaSuccess && at.numRegs >= kOutLaunchRegs;
+        }();
+        if (!enough) return false;
         ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)OutCfg::kSmem, a.device);
         launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, a.z != nullptr, k.nc,
                          a.nheads, a.ngroups, a.seqlen, (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
+        return true;
     };
-    if (a.D && a.D_has_hdim) go(std::true_type{});
-    else go(std::false_type{});
+    if (!(a.D && a.D_has_hdim ? go(std::true_type{}) : go(std::false_type{}))) return fail(MB200_ERR_LAUNCH, "ssd: output kernel built with too few registers");
     MB200_CHECK_LAUNCH("ssd output (tensor core)");
     return MB200_OK;
 }

@@ -108,6 +108,12 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map)
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// ---- registers -------------------------------------------------------------------------------------
+// Every warp of a warpgroup moves to N registers a thread.  What the warpgroups of a block hold together may never exceed what the
+// block was launched with (its threads x registers a thread): an increase waits for registers that others give back.
+template <int N> __device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---- tensor memory ---------------------------------------------------------------------------------
 // One warp allocates / frees; `cols` is a power of two >= 32.
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t cols)
@@ -174,18 +180,22 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[8], uint32_t (&b)[8])
                  :
                  : "memory");
 }
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
+                 :
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_st1_issue(uint32_t taddr, uint32_t v)
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void tmem_st16_issue(uint32_t taddr, const uint32_t (&r)[16])
+__device__ __forceinline__ void tmem_st8_issue(uint32_t taddr, const uint32_t (&r)[8])
 {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -246,16 +256,16 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         : "memory");
 }
 // `count` steps of K = 16 whose operands lie step_a / step_b units of 16 bytes apart (ss), or 8 columns and step_b units (ts); a
-// descriptor holds its address in those units.  The loops stay rolled: a step is some twenty instructions.
+// descriptor holds its address in those units.  Four steps (a tile of 64 along the reduction) per turn of a loop.
 __device__ __forceinline__ void mma_steps_ss(int count, uint32_t d_tmem, uint64_t a_desc, uint32_t step_a, uint64_t b_desc, uint32_t step_b, uint32_t idesc,
                                              bool accumulate)
 {
-#pragma unroll 1
+#pragma unroll 4
     for (int s = 0; s < count; ++s, a_desc += step_a, b_desc += step_b) mma_f16_ss(d_tmem, a_desc, b_desc, idesc, accumulate || s > 0);
 }
 __device__ __forceinline__ void mma_steps_ts(int count, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t step_b, uint32_t idesc, bool accumulate)
 {
-#pragma unroll 1
+#pragma unroll 4
     for (int s = 0; s < count; ++s, a_tmem += 8, b_desc += step_b) mma_f16_ts(d_tmem, a_tmem, b_desc, idesc, accumulate || s > 0);
 }
 // Arrives on `bar` once every MMA issued so far by this thread has finished.

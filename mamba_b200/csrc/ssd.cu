@@ -1,4 +1,4 @@
-// Mamba-2 SSD chunked forward for sm_100a: the stages, and their kernels for fp32 inputs.
+// Mamba-2 SSD chunked forward for sm_100a: the stages, their order, and the first and the third of them.
 //
 // Stages (each one launch, all on the caller's stream, handing fp32 intermediates through the
 // caller's scratch buffer):
@@ -8,123 +8,13 @@
 //   4. chunk_cb       CB[m,k] = C_m . B_k   (lower block triangle)
 //   5. chunk_scan     y_m = exp(dA_m) C_m.H_c + sum_{k<=m} CB[m,k] exp(min(dA_m - dA_k,0)) dt_k x_k + D x_m,
 //                     then y_m * silu(z_m)
-// The contractions here run on the fp32 FMA pipes through a 64x64 shared-memory tile loop (tile_gemm) and serve fp32 inputs.  For
-// bf16/fp16, ssd_tc.cu replaces stages 2 to 5 for the shape that most layers have, and ssd_split.cu stages 2, 4 and 5 for all others.
+// The contractions, stages 2, 4 and 5, are ssd_split.cu's; for bf16/fp16 of the shape that most layers have ssd_tc.cu replaces stages 2 to 5.
 #include <algorithm>
 
 #include "ssd_common.cuh"
 
 namespace mb200 {
 namespace {
-
-constexpr int kT = 128;       // threads per CTA in the tile kernels
-constexpr int kKT = 32;       // reduction step
-constexpr int kLd = 68;       // padded leading dimension of the staged tiles (keeps float4 alignment)
-struct TileSmem { __align__(16) float A[2][kKT * kLd], B[2][kKT * kLd]; };
-
-// Four consecutive elements, in one load where `vec` says that they lie on their own alignment; zeros from `n` on.
-__device__ __forceinline__ float4 load4(const float *p, bool vec, int n)
-{
-    if (vec && n >= 4) return *reinterpret_cast<const float4 *>(p);
-    return make_float4(n > 0 ? p[0] : 0.f, n > 1 ? p[1] : 0.f, n > 2 ? p[2] : 0.f, n > 3 ? p[3] : 0.f);
-}
-__device__ __forceinline__ void store4(float *p, bool vec, int n, const float (&v)[4])
-{
-    if (vec && n >= 4) {
-        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (i < n) p[i] = v[i];
-    }
-}
-// rows of a (batch, time, group or head, columns) tensor start where load4 can take four at once
-__device__ __forceinline__ bool rows_of_4(const float *p, int64_t s0, int64_t s1, int64_t s2)
-{
-    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ((s0 | s1 | s2) & 3) == 0;
-}
-
-// acc += A[64 x K] * B[K x 64] for the thread's 8x4 patch: rows ty*8.. in pairs (packed fp32 FMAs), columns tx*4...  fa and fb
-// return four bounds-checked operand elements that follow each other in memory: (row, k..k+3) where the source is contiguous
-// along k (KFAST), (k, column..column+3) otherwise; wa gives what fa loaded its final value when it is staged, a step later.  Terms
-// are added in the order of k.
-// What bounds it: with one buffer, a 4x4 patch and single elements staged, a step of 32 was a round trip to memory followed by
-// two shared-memory reads per 16 FMAs (73 us for the outputs of 2 x 2048 steps of 8 fp32 heads of 64 x 64; now 54 us).  Here the next
-// step's elements are on their way in registers while one is worked on, and three reads serve 32 FMAs.  A lane stages rows that
-// are contiguous along k as 2 packets of 16 rows, which fills whole sectors and hits 32 different banks.
-template <bool A_KFAST, bool B_KFAST, class FA, class WA, class FB>
-__device__ __forceinline__ void tile_gemm(uint64_t (&acc)[4][4], int K, FA fa, WA wa, FB fb, TileSmem &sm)
-{
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, warp = threadIdx.x / 32, lane = threadIdx.x & 31;
-    auto place = [&](bool kfast, int e, int &i, int &k) {       // of the e-th four elements of mine
-        if (kfast) {
-            const int block = warp * 4 + e;                     // 4 blocks of 16 rows x 4 pairs of packets
-            i = (block >> 2) * 16 + (lane >> 1);
-            k = ((block & 3) * 2 + (lane & 1)) * 4;
-        } else {
-            k = e * 8 + ty;
-            i = tx * 4;
-        }
-    };
-    float4 ra[4], rb[4];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int i, k;
-            place(A_KFAST, e, i, k);
-            ra[e] = A_KFAST ? fa(i, k0 + k) : fa(k0 + k, i);
-            place(B_KFAST, e, i, k);
-            rb[e] = B_KFAST ? fb(i, k0 + k) : fb(k0 + k, i);
-        }
-    };
-    auto stage = [&](float *dst, bool kfast, const float4 (&r)[4], auto final_value) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int i, k;
-            place(kfast, e, i, k);
-            const float4 v = final_value(i, k, r[e]);
-            if (kfast) {
-                dst[k * kLd + i] = v.x;
-                dst[(k + 1) * kLd + i] = v.y;
-                dst[(k + 2) * kLd + i] = v.z;
-                dst[(k + 3) * kLd + i] = v.w;
-            } else {
-                *reinterpret_cast<float4 *>(dst + k * kLd + i) = v;
-            }
-        }
-    };
-    if (K > 0) fetch(0);
-    int buf = 0;
-    __syncthreads();                // (a tile_gemm before this one may still be read)
-    for (int k0 = 0; k0 < K; k0 += kKT, buf ^= 1) {
-        stage(sm.A[buf], A_KFAST, ra, [&](int i, int k, float4 v) { return A_KFAST ? wa(i, k0 + k, v) : wa(k0 + k, i, v); });
-        stage(sm.B[buf], B_KFAST, rb, [](int, int, float4 v) { return v; });
-        __syncthreads();            // also: every warp is done with the other buffer
-        if (k0 + kKT < K) fetch(k0 + kKT);
-        const float *As = sm.A[buf] + ty * 8, *Bs = sm.B[buf] + tx * 4;
-#pragma unroll 8
-        for (int kk = 0; kk < kKT; ++kk) {
-            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(As + kk * kLd), a1 = *reinterpret_cast<const ulonglong2 *>(As + kk * kLd + 4);
-            const float4 bv = *reinterpret_cast<const float4 *>(Bs + kk * kLd);
-            const uint64_t ar[4] = {a0.x, a0.y, a1.x, a1.y}, br[4] = {pack2(bv.x, bv.x), pack2(bv.y, bv.y), pack2(bv.z, bv.z), pack2(bv.w, bv.w)};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma2(ar[i], br[j], acc[i][j]);
-        }
-    }
-}
-__device__ __forceinline__ float4 as_loaded(int, int, float4 v) { return v; }
-// the thread's patch row by row
-__device__ __forceinline__ void patch_row(const uint64_t (&acc)[4][4], int i, float (&v)[4])
-{
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float lo, hi;
-        unpack2(acc[i >> 1][j], lo, hi);
-        v[j] = i & 1 ? hi : lo;
-    }
-}
 
 // Sequence id of position t of batch row b (packed sequences), or 0 when no ids were given.
 __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t)
@@ -239,48 +129,6 @@ __global__ void __launch_bounds__(NW * 32) ssd_cumsum_kernel(const mb200_ssd_arg
     }
 }
 
-// ---- stage 2 ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kT, 4) ssd_chunk_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb,
-                                                             float *states, int nchunks)
-{
-    __shared__ TileSmem sm;
-    const int Q = a.chunk_size, P = a.headdim, N = a.dstate;
-    const int tilesN = (N + 63) / 64;
-    const int p0 = (blockIdx.x / tilesN) * 64, n0 = (blockIdx.x % tilesN) * 64;
-    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z;
-    const int g = h / (a.nheads / a.ngroups);
-    const int t0 = c * Q;
-    const int len = min(Q, a.seqlen - t0);
-    const float *dtc = dtb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
-    const float *dAc = dAb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
-    const float dA_last = dAc[Q - 1];
-    const float *x = static_cast<const float *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const float *B = static_cast<const float *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
-    const bool vx = rows_of_4(x, 0, a.x_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
-    uint64_t acc[4][4] = {};
-    const int seq_last = seq_at(a, b, t0 + len - 1);    // only steps of the chunk's last sequence reach its end state
-    tile_gemm<false, false>(
-        acc, len,
-        [&](int k, int i) {
-            const bool in = k < len && (!a.seq_idx || seq_at(a, b, t0 + k) == seq_last);
-            return load4(x + (int64_t)k * a.x_stride[1] + p0 + i, vx, in ? P - p0 - i : 0);
-        },
-        [&](int k, int, float4 v) {
-            const float w = k < len ? __expf(fminf(dA_last - dAc[k], 0.f)) * dtc[k] : 0.f;
-            return make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
-        },
-        [&](int k, int j) { return load4(B + (int64_t)k * a.B_stride[1] + n0 + j, vB, k < len ? N - n0 - j : 0); }, sm);
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, n = n0 + tx * 4;
-    float *S = states + (((int64_t)b * nchunks + c) * a.nheads + h) * (int64_t)P * N;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int p = p0 + ty * 8 + i;
-        float v[4];
-        patch_row(acc, i, v);
-        if (p < P && n < N) store4(S + (int64_t)p * N + n, (N & 3) == 0, N - n, v);
-    }
-}
-
 // ---- stage 3 ------------------------------------------------------------------------------------
 // Elementwise over P*N, serial over chunks.  Slot c of `states` receives the state entering chunk c;
 // with `prev16` the entering states go there as 16-bit values (the tensor-core chunk_scan reads them
@@ -350,176 +198,6 @@ __global__ void __launch_bounds__(256) ssd_state_passing_kernel(const mb200_ssd_
     }
 }
 
-// ---- stage 4 ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kT, 4) ssd_cb_kernel(const mb200_ssd_args a, float *cb, int nchunks)
-{
-    __shared__ TileSmem sm;
-    const int Q = a.chunk_size, N = a.dstate;
-    const int tiles = (Q + 63) / 64;
-    const int m0 = (blockIdx.x / tiles) * 64, k0 = (blockIdx.x % tiles) * 64;
-    if (k0 > m0) return;   // strictly upper blocks are never read
-    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, g = blockIdx.z;
-    const int t0 = c * Q;
-    const int len = min(Q, a.seqlen - t0);
-    const float *C = static_cast<const float *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
-    const float *B = static_cast<const float *>(a.B) + (int64_t)b * a.B_stride[0] + (int64_t)t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2];
-    const bool vC = rows_of_4(C, 0, a.C_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
-    uint64_t acc[4][4] = {};
-    tile_gemm<true, true>(
-        acc, N, [&](int i, int n) { return load4(C + (int64_t)(m0 + i) * a.C_stride[1] + n, vC, m0 + i < len ? N - n : 0); }, as_loaded,
-        [&](int j, int n) { return load4(B + (int64_t)(k0 + j) * a.B_stride[1] + n, vB, k0 + j < len ? N - n : 0); }, sm);
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, k = k0 + tx * 4;
-    float *out = cb + (((int64_t)b * nchunks + c) * a.ngroups + g) * (int64_t)Q * Q;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty * 8 + i;
-        float v[4];
-        patch_row(acc, i, v);
-        if (a.seq_idx) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (!(m < len && k + j < len && seq_at(a, b, t0 + m) == seq_at(a, b, t0 + k + j))) v[j] = 0.f;
-        }
-        if (m < Q && k < Q) store4(out + (int64_t)m * Q + k, (Q & 3) == 0, Q - k, v);
-    }
-}
-
-// ---- stage 5 ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kT, 4) ssd_chunk_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb,
-                                                            const float *states, const float *cb, int nchunks)
-{
-    __shared__ TileSmem sm;
-    const int Q = a.chunk_size, P = a.headdim, N = a.dstate;
-    const int tilesP = (P + 63) / 64;
-    const int m0 = (blockIdx.x / tilesP) * 64, p0 = (blockIdx.x % tilesP) * 64;
-    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z;
-    const int g = h / (a.nheads / a.ngroups);
-    const int t0 = c * Q;
-    const int len = min(Q, a.seqlen - t0);
-    if (m0 >= len) return;
-    const float *dtc = dtb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
-    const float *dAc = dAb + (((int64_t)b * a.nheads + h) * nchunks + c) * Q;
-    const float *x = static_cast<const float *>(a.x) + (int64_t)b * a.x_stride[0] + (int64_t)t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const float *C = static_cast<const float *>(a.C) + (int64_t)b * a.C_stride[0] + (int64_t)t0 * a.C_stride[1] + (int64_t)g * a.C_stride[2];
-    const float *prev = states + (((int64_t)b * nchunks + c) * a.nheads + h) * (int64_t)P * N;
-    const float *cbc = cb + (((int64_t)b * nchunks + c) * a.ngroups + g) * (int64_t)Q * Q;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const bool vx = rows_of_4(x, 0, a.x_stride[1], 0), vC = rows_of_4(C, 0, a.C_stride[1], 0), vN = (N & 3) == 0, vQ = (Q & 3) == 0;
-
-    uint64_t acc[4][4] = {};
-    // contribution of the state entering the chunk: exp(dA_m) * C_m . H[p,:]
-    tile_gemm<true, true>(
-        acc, N, [&](int i, int n) { return load4(C + (int64_t)(m0 + i) * a.C_stride[1] + n, vC, m0 + i < len ? N - n : 0); }, as_loaded,
-        [&](int j, int n) { return load4(prev + (int64_t)(p0 + j) * N + n, vN, p0 + j < P ? N - n : 0); }, sm);
-    float sc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty * 8 + i;
-        sc[i] = m < len ? __expf(dAc[m]) : 0.f;
-        // the entering state belongs to the sequence that ends the previous chunk
-        if (a.seq_idx && m < len && seq_at(a, b, t0 + m) != (c > 0 ? seq_at(a, b, t0 - 1) : 0)) sc[i] = 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = mul2(acc[i][j], pack2(sc[2 * i], sc[2 * i + 1]));
-    // causal intra-chunk part
-    const int kend = min(m0 + 64, len);
-    tile_gemm<true, false>(
-        acc, kend,
-        [&](int i, int k) {
-            const int m = m0 + i;                       // columns up to the diagonal
-            return load4(cbc + (int64_t)m * Q + k, vQ, m < len ? min(m + 1, kend) - k : 0);
-        },
-        [&](int i, int k, float4 v) {
-            const int n = min(m0 + i + 1, kend) - k;
-            const float4 d = load4(dAc + k, vQ, n), t = load4(dtc + k, vQ, n);
-            const float dm = dAc[min(m0 + i, len - 1)];
-            return make_float4(v.x * __expf(fminf(dm - d.x, 0.f)) * t.x, v.y * __expf(fminf(dm - d.y, 0.f)) * t.y,
-                               v.z * __expf(fminf(dm - d.z, 0.f)) * t.z, v.w * __expf(fminf(dm - d.w, 0.f)) * t.w);
-        },
-        [&](int k, int j) { return load4(x + (int64_t)k * a.x_stride[1] + p0 + j, vx, k < kend ? P - p0 - j : 0); }, sm);
-
-    const float *z = a.z ? static_cast<const float *>(a.z) + (int64_t)b * a.z_stride[0] + (int64_t)t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] : nullptr;
-    float *out = static_cast<float *>(a.out) + (int64_t)b * a.out_stride[0] + (int64_t)t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2];
-    const bool vz = z && rows_of_4(z, 0, a.z_stride[1], 0), vo = rows_of_4(out, 0, a.out_stride[1], 0);
-    const int p = p0 + tx * 4, np = P - p;
-    if (np <= 0) return;
-    float Dv[4] = {};
-    if (a.D) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) Dv[j] = a.D_has_hdim ? (j < np ? a.D[(int64_t)h * P + p + j] : 0.f) : a.D[h];
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty * 8 + i;
-        if (m >= len) continue;
-        float y[4];
-        patch_row(acc, i, y);
-        if (a.D) {
-            const float4 v = load4(x + (int64_t)m * a.x_stride[1] + p, vx, np);
-            y[0] = fmaf(v.x, Dv[0], y[0]); y[1] = fmaf(v.y, Dv[1], y[1]); y[2] = fmaf(v.z, Dv[2], y[2]); y[3] = fmaf(v.w, Dv[3], y[3]);
-        }
-        if (z) {
-            const float4 v = load4(z + (int64_t)m * a.z_stride[1] + p, vz, np);
-            y[0] *= silu(v.x); y[1] *= silu(v.y); y[2] *= silu(v.z); y[3] *= silu(v.w);
-        }
-        store4(out + (int64_t)m * a.out_stride[1] + p, vo, np, y);
-    }
-}
-
-// ---- packed sequences: state after the last token of each one ------------------------------------
-// A 64 x 64 tile of one (sequence, head): the contribution of the sequence's steps inside the chunk that holds its last
-// token, plus the state entering that chunk if the sequence began earlier.
-__global__ void __launch_bounds__(kT, 4) ssd_varlen_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, int nchunks)
-{
-    __shared__ TileSmem sm;
-    const int P = a.headdim, N = a.dstate, Q = a.chunk_size;
-    const int tilesN = (N + 63) / 64;
-    const int p0 = (blockIdx.x / tilesN) * 64, n0 = (blockIdx.x % tilesN) * 64;
-    const int s = blockIdx.y, h = blockIdx.z;
-    const int g = h / (a.nheads / a.ngroups);
-    const int start = a.cu_seqlens[s], end = a.cu_seqlens[s + 1];
-    const bool empty = end <= start || end > a.seqlen || start < 0;
-    const int c = empty ? 0 : (end - 1) / Q, t0 = c * Q;
-    const int first = empty ? 0 : max(start, t0);
-    const float *dtc = dtb + ((int64_t)h * nchunks + c) * Q + (first - t0);
-    const float *dAc = dAb + ((int64_t)h * nchunks + c) * Q + (first - t0);
-    const float dA_end = empty ? 0.f : dAc[end - 1 - first];
-    const float *x = static_cast<const float *>(a.x) + (int64_t)first * a.x_stride[1] + (int64_t)h * a.x_stride[2];
-    const float *B = static_cast<const float *>(a.B) + (int64_t)first * a.B_stride[1] + (int64_t)g * a.B_stride[2];
-    const bool vx = rows_of_4(x, 0, a.x_stride[1], 0), vB = rows_of_4(B, 0, a.B_stride[1], 0);
-    const int steps = empty ? 0 : end - first;
-    uint64_t acc[4][4] = {};
-    tile_gemm<false, false>(
-        acc, steps,
-        [&](int k, int i) {
-            return load4(x + (int64_t)k * a.x_stride[1] + p0 + i, vx, k < steps ? P - p0 - i : 0);
-        },
-        [&](int k, int, float4 v) {
-            const float w = k < steps ? __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k] : 0.f;
-            return make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
-        },
-        [&](int k, int j) { return load4(B + (int64_t)k * a.B_stride[1] + n0 + j, vB, k < steps ? N - n0 - j : 0); }, sm);
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, n = n0 + tx * 4;
-    const float *entering = !empty && start < t0 ? states + (((int64_t)c) * a.nheads + h) * (int64_t)P * N : nullptr;
-    const float decay = __expf(dA_end);
-    float *dst = a.varlen_states + ((int64_t)s * a.nheads + h) * P * N;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int p = p0 + ty * 8 + i;
-        if (p >= P || n >= N) continue;
-        const int64_t e = (int64_t)p * N + n;
-        float v[4];
-        patch_row(acc, i, v);
-        if (entering) {
-            const float4 in = load4(entering + e, (N & 3) == 0, N - n);
-            v[0] = fmaf(in.x, decay, v[0]); v[1] = fmaf(in.y, decay, v[1]); v[2] = fmaf(in.z, decay, v[2]); v[3] = fmaf(in.w, decay, v[3]);
-        }
-        store4(dst + e, (N & 3) == 0, N - n, v);
-    }
-}
-
 __global__ void ssd_fill_kernel(float *dst, float v, int64_t n)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -556,7 +234,6 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
     float *dtb = reinterpret_cast<float *>(base + lay.off_dt);
     float *dAb = reinterpret_cast<float *>(base + lay.off_dA);
     float *states = reinterpret_cast<float *>(base + lay.off_states);
-    float *cb = reinterpret_cast<float *>(base + lay.off_cb);
     int *status = ssd_status_word(a, lay);
     const int nc = lay.nchunks, Q = a.chunk_size;
     const int64_t PN = (int64_t)a.headdim * a.dstate;
@@ -584,14 +261,6 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
     // The LOCAL half took the streaming launch but this OUTPUT half cannot use its 16-bit entering states: the
     // scratch holds no fp32 chunk states, so they are formed here before the recurrence.
     const bool local_streamed = !has_local && fused_states && !tc_out;
-    const bool split = a.io_dtype != MB200_F32;       // the general stages for 16-bit inputs
-    const int tq = (Q + 63) / 64, tp = (a.headdim + 63) / 64, tn = (a.dstate + 63) / 64;
-    auto form_cb = [&]() -> int {
-        if (split) return ssd_split_cb(a, lay, stream);
-        ssd_cb_kernel<<<dim3(tq * tq, a.batch * nc, a.ngroups), kT, 0, stream>>>(a, cb, nc);
-        MB200_CHECK_LAUNCH("ssd chunk_cb");
-        return MB200_OK;
-    };
     auto state_passing = [&](const mb200_ssd_args &p, bool write_prev, void *to16) {
         if (PN % 4 == 0)
             ssd_state_passing_kernel<4><<<dim3((unsigned)((PN / 4 + 255) / 256), a.nheads, a.batch), 256, 0, stream>>>(p, dAb, states, nc, write_prev, to16);
@@ -619,16 +288,13 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
         if (ce != cudaSuccess) return fail(MB200_ERR_LAUNCH, "ssd chunk_cumsum: shared memory opt-in: %s", cudaGetErrorString(ce));
         MB200_CHECK_LAUNCH("ssd chunk_cumsum");
         if (cb_early)
-            if (int rc = form_cb()) return rc;
+            if (int rc = ssd_split_cb(a, lay, stream)) return rc;
         if (fused_states) {
             if (int rc = ssd_tc_state_stream(a, lay, stream)) return rc;
         } else if (tc_loc) {
             if (int rc = ssd_tc_chunk_state(a, lay, stream)) return rc;
-        } else if (split) {
-            if (int rc = ssd_split_states(a, lay, stream)) return rc;
         } else {
-            ssd_chunk_state_kernel<<<dim3(tp * tn, a.batch * nc, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, nc);
-            MB200_CHECK_LAUNCH("ssd chunk_state");
+            if (int rc = ssd_split_states(a, lay, stream)) return rc;
         }
         if (!fused_states && !has_out && (a.final_states || a.range_decay)) {
             // range summary only: fold the local chunk states from a zero state, leave the slots as they are
@@ -661,19 +327,10 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
                     return rc;
         } else {
             if (!cb_ready)
-                if (int rc = form_cb()) return rc;
-            if (split) {
-                if (int rc = ssd_split_scan(a, lay, stream)) return rc;
-                if (varlen)
-                    if (int rc = ssd_split_varlen(a, lay, SsdStates::pn32, stream)) return rc;
-            } else {
-                ssd_chunk_scan_kernel<<<dim3(tq * tp, a.batch * nc, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, cb, nc);
-                MB200_CHECK_LAUNCH("ssd chunk_scan");
-                if (varlen) {
-                    ssd_varlen_state_kernel<<<dim3(tp * tn, a.num_seqs, a.nheads), kT, 0, stream>>>(a, dtb, dAb, states, nc);
-                    MB200_CHECK_LAUNCH("ssd varlen states");
-                }
-            }
+                if (int rc = ssd_split_cb(a, lay, stream)) return rc;
+            if (int rc = ssd_split_scan(a, lay, stream)) return rc;
+            if (varlen)
+                if (int rc = ssd_split_varlen(a, lay, SsdStates::pn32, stream)) return rc;
         }
     }
     return MB200_OK;

@@ -1,18 +1,18 @@
-// Stages of the SSD chunked forward for 16-bit inputs of every shape, on the tensor cores with products as exact as fp32's.
+// Stages of the SSD chunked forward for every shape and type, on the tensor cores with products as exact as fp32's.
 //
 // ssd_tc.cu serves 16-bit calls of headdim 64, dstate 128 and chunk 256 with 16-bit operands throughout: weights, decays and entering
-// states are rounded to the input type.  Here nothing but the result is.  An fp32 operand -- C.B^T times its decay, a weighted x, an
-// entering state -- is cut into bf16 values that add up to it (three hold all 24 bits), and a half-precision input into two, so that
-// tcgen05.mma of bf16 operands forms the products, which it adds in fp32; terms below 2^-24 of a product are left out.  bf16 has
-// fp32's range: nothing overflows that fp32 holds, whatever the input type.  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64:
-// end states 1.6e-6 to 3.4e-6, outputs 1.66e-3 (bf16) and 2.07e-4 (fp16), which is their own rounding; the fp32 kernels of ssd.cu gave the
-// same to within 1 %, operands rounded to 16 bits 1.7e-3 / 2.1e-4 and 2.4e-3 / 3.0e-4.
+// states are rounded to the input type.  Here nothing but the result is.  An fp32 operand -- an fp32 input, C.B^T times its decay, a
+// weighted x, an entering state -- is cut into bf16 values that add up to it (three hold all 24 bits), and a half-precision input into two,
+// so that tcgen05.mma of bf16 operands forms the products, which it adds in fp32; terms below 2^-24 of a product are left out.  bf16 has
+// fp32's range: nothing overflows that fp32 holds, whatever the input type.  The tensor core cuts its sums off where fp32 arithmetic
+// rounds, so sums that leave in fp32 have the small products in a sum of their own.  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64:
+// end states 1.6e-6 to 3.4e-6, outputs 1.66e-3 (bf16) and 2.07e-4 (fp16), which is their own rounding; fp32 outputs 0.86e-6 to 2.0e-6.  Tiles
+// of fp32 FMAs gave the same to within 2 %, operands rounded to 16 bits 1.7e-3 / 2.1e-4 and 2.4e-3 / 3.0e-4.
 //
-// Every kernel is one tile loop: 256 threads fetch the next 64 steps of the reduction into registers while the tensor core works on the
-// last ones, form the operand values, cut them and store them to 128-byte-swizzled shared memory.  The tensor core is idle most of
-// the time; what bounds these kernels is that element-wise work and the latencies between it, which two to four CTAs per SM share.
-// Rows are read with plain loads, so any stride and alignment goes.
-// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states 28, C.B^T 5, outputs 69; the fp32 kernels took 318 for the call.
+// A tile loop: 256 threads fetch the next 64 steps of the reduction while the tensor core works on the last ones, form the operand values,
+// cut them and store them.  The tensor core is idle most of the time; what bounds these kernels is that element-wise work and the latencies
+// between it, which two to four CTAs per SM share.  Rows are read with plain loads, so any stride and alignment goes.
+// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states 28, C.B^T 5, outputs 69; fp32 FMAs took 318 for the call.
 #include <type_traits>
 
 #include "ssd_common.cuh"
@@ -26,7 +26,8 @@ using namespace tc;
 constexpr int kThreads = 256;
 constexpr uint32_t kTileA = 16384, kTileB = 8192;       // bytes of one part of a 128 x 64 and of a 64 x 64 operand
 constexpr int kParts = 3;                               // of an fp32 value
-template <typename T> constexpr int kInParts = std::is_same<T, __half>::value ? 2 : 1;       // of an input value
+// of an input value
+template <typename T> constexpr int kInParts = std::is_same<T, __nv_bfloat16>::value ? 1 : std::is_same<T, __half>::value ? 2 : kParts;
 
 enum { kStSplitState = 51, kStSplitCb, kStSplitScan };
 
@@ -34,114 +35,31 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, ui
 {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
-// Cuts eight values into NP bf16 parts and stores part p at addr + p * stride.  Each part is what is left rounded to bf16, so that the
-// rest is exact and three parts hold all of it.  Values that bf16 would round to infinity, and infinities, are cut by truncation
-// instead, which leaves infinities in the first part.
-template <int NP>
-__device__ __noinline__ void store_parts_large(uint32_t addr, uint32_t stride, float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7)
-{
-    float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t top = __float_as_uint(v[i]) & 0xffff0000u;
-            if (i & 1) w[i / 2] |= top;
-            else w[i / 2] = top >> 16;
-            v[i] = v[i] == __uint_as_float(top) ? 0.f : v[i] - __uint_as_float(top);
-        }
-        sts128(addr + p * stride, w[0], w[1], w[2], w[3]);
-    }
-}
-template <int NP>
-__device__ __forceinline__ void store_parts(uint32_t addr, uint32_t stride, float (&v)[8])
-{
-    uint32_t w[4];
-    auto round8 = [&] {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t *>(&h);
-        }
-    };
-    round8();
-    const auto abs2 = [](uint32_t u) { u &= 0x7fff7fffu; return *reinterpret_cast<const __nv_bfloat162 *>(&u); };
-    const __nv_bfloat162 most = __hmax2(__hmax2(abs2(w[0]), abs2(w[1])), __hmax2(abs2(w[2]), abs2(w[3])));
-    const uint32_t top = *reinterpret_cast<const uint32_t *>(&most);
-    if ((top & 0xffffu) == 0x7f80u || (top >> 16) == 0x7f80u) {          // an infinity
-        store_parts_large<NP>(addr, stride, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
-        return;
-    }
-    sts128(addr, w[0], w[1], w[2], w[3]);
-#pragma unroll
-    for (int p = 1; p < NP; ++p) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[2 * i] -= __uint_as_float(w[i] << 16);
-            v[2 * i + 1] -= __uint_as_float(w[i] & 0xffff0000u);
-        }
-        round8();
-        sts128(addr + p * stride, w[0], w[1], w[2], w[3]);
-    }
-}
-__device__ __noinline__ void store_first(uint32_t addr, uint32_t stride, float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7)
-{
-    const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-        w[i] = *reinterpret_cast<const uint32_t *>(&h);
-    }
-    sts128(addr, w[0], w[1], w[2], w[3]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = (w[i] & 0x80008000u) | 0x01000100u;
-    for (int p = 1; p < kParts; ++p) sts128(addr + p * stride, w[0], w[1], w[2], w[3]);
-}
-template <typename T> __device__ __forceinline__ void widen8(const uint4 &raw, float (&v)[8])
+
+// Eight elements of an input row, as they lie in memory.
+template <typename T> struct Raw8 { uint4 q[sizeof(T) / 2]; };
+template <typename T> __device__ __forceinline__ void widen8(const Raw8<T> &raw, float (&v)[8])
 {
     const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = to_float(e[i]);
 }
-// Eight input values as they are: bf16 unchanged, half precision in two parts.
-template <typename T> __device__ __forceinline__ void store_input(uint32_t addr, uint32_t stride, const uint4 &raw)
-{
-    if constexpr (kInParts<T> == 1) {
-        sts128(addr, raw.x, raw.y, raw.z, raw.w);
-    } else {
-        float v[8];
-        widen8<T>(raw, v);
-        store_parts<2>(addr, stride, v);
-    }
-}
-
-// An infinity (or a NaN) among eight inputs.  Times the first part of an operand it gives what it should, but the later parts may have the
-// other sign or be zero: where one turns up they are left out, or made tiny and of the first part's sign.
-template <typename T> __device__ __forceinline__ bool not_finite(const uint4 &r)
-{
-    constexpr uint32_t kInf = std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
-    const uint32_t m = __vmaxu2(__vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu), __vmaxu2(r.z & 0x7fff7fffu, r.w & 0x7fff7fffu));
-    return (m & 0xffffu) >= kInf || (m >> 16) >= kInf;
-}
-
 // Eight elements that follow each other in memory, zeros from `n` on; `vec`: they start on a 16-byte boundary.  What is not whole stays out
 // of line: a kernel has two dozen such loads.
-template <typename T> __device__ __noinline__ uint4 load8_ragged(const T *p, int n)
+template <typename T> __device__ __noinline__ Raw8<T> load8_ragged(const T *p, int n)
 {
-    uint4 r = make_uint4(0, 0, 0, 0);
+    Raw8<T> r = {};
     T *e = reinterpret_cast<T *>(&r);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         if (i < n) e[i] = p[i];
     return r;
 }
-template <typename T> __device__ __forceinline__ uint4 load8(const T *p, bool vec, int n)
+template <typename T> __device__ __forceinline__ Raw8<T> load8_whole(const T *p) { return *reinterpret_cast<const Raw8<T> *>(p); }
+template <typename T> __device__ __forceinline__ Raw8<T> load8(const T *p, bool vec, int n)
 {
-    static_assert(sizeof(T) == 2, "16-bit inputs");
-    if (n <= 0) return make_uint4(0, 0, 0, 0);
-    return vec && n >= 8 ? *reinterpret_cast<const uint4 *>(p) : load8_ragged(p, n);
+    if (n <= 0) return Raw8<T>{};
+    return vec && n >= 8 ? load8_whole(p) : load8_ragged(p, n);
 }
 __device__ __noinline__ float4 load4_ragged(const float *p, int n)
 {
@@ -152,14 +70,66 @@ __device__ __forceinline__ float4 load4(const float *p, bool vec, int n)
     if (n <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
     return vec && n >= 4 ? *reinterpret_cast<const float4 *>(p) : load4_ragged(p, n);
 }
-__device__ __forceinline__ void load8(const float *p, bool vec, int n, float4 &lo, float4 &hi)
-{
-    lo = load4(p, vec, n);
-    hi = load4(p + 4, vec, n - 4);
-}
 template <typename T> __device__ __forceinline__ bool rows16(const T *p, int64_t stride)
 {
-    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && stride % 8 == 0;
+    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && stride * (int64_t)sizeof(T) % 16 == 0;
+}
+
+// Cuts a pair of values into NP packed bf16 parts.  Each part is what is left rounded to bf16, so that the rest is exact and three parts
+// hold all of it.
+template <int NP> __device__ __forceinline__ void cut2(uint64_t v, uint32_t (&w)[NP])
+{
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        float a, b;
+        unpack2(v, a, b);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        w[p] = *reinterpret_cast<const uint32_t *>(&h);
+        if (p + 1 < NP) v = sub2(v, pack2(__uint_as_float(w[p] << 16), __uint_as_float(w[p] & 0xffff0000u)));
+    }
+}
+// Finds what the cut cannot do: infinities and NaNs, and values that bf16 rounds to infinity.  (An infinity in the first part of an operand
+// would meet the later parts of the other, which may have the other sign or be zero.)  A tile that holds one is left out by the tensor core
+// and added with fp32 FMAs at the end.  Fed with packed first parts, or packed 16-bit inputs: 0 x v is NaN for those.
+template <typename T> struct Finite {
+    using H2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+    uint32_t sum = 0;
+    __device__ __forceinline__ void feed(uint32_t w)
+    {
+        const uint32_t zero = 0;
+        const H2 r = __hfma2(*reinterpret_cast<const H2 *>(&w), *reinterpret_cast<const H2 *>(&zero), *reinterpret_cast<const H2 *>(&sum));
+        sum = *reinterpret_cast<const uint32_t *>(&r);
+    }
+    __device__ __forceinline__ bool bad() const { return (sum & 0x7fff7fffu) != 0; }
+};
+// Eight values in NP parts, part p at addr + p * stride.
+template <int NP> __device__ __forceinline__ bool store_parts(uint32_t addr, uint32_t stride, const float (&v)[8])
+{
+    uint32_t w[4][NP];
+    Finite<__nv_bfloat16> f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        cut2<NP>(pack2(v[2 * i], v[2 * i + 1]), w[i]);
+        f.feed(w[i][0]);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) sts128(addr + p * stride, w[0][p], w[1][p], w[2][p], w[3][p]);
+    return f.bad();
+}
+// Eight input values: bf16 as they are, half precision in two parts, fp32 in three.  Says whether one of them is none that can be cut.
+template <typename T> __device__ __forceinline__ bool store_input(uint32_t addr, uint32_t stride, const Raw8<T> &raw)
+{
+    if constexpr (kInParts<T> == 1) {
+        const uint4 q = raw.q[0];
+        sts128(addr, q.x, q.y, q.z, q.w);
+        Finite<T> f;
+        f.feed(q.x); f.feed(q.y); f.feed(q.z); f.feed(q.w);
+        return f.bad();
+    } else {
+        float v[8];
+        widen8<T>(raw, v);
+        return store_parts<kInParts<T>>(addr, stride, v);
+    }
 }
 // byte offset of 16-byte chunk `chunk` of row `row` in a tile of 128-byte rows
 __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); }
@@ -215,17 +185,18 @@ struct Tile {
     {
         if (issued > 0 && ok) ok = mbar_wait(bar, (issued - 1) & 1, status, code);
     }
-    // the tiles are complete: `go` issues the products, told whether any thread raised its flag
-    template <class F> __device__ __forceinline__ void step(bool flag, F go)
+    // the tiles are complete: `go` issues the products, unless a thread has found what cannot be cut (then it returns false)
+    template <class F> __device__ __forceinline__ bool step(bool bad, F go)
     {
         fence_proxy_async();
-        const bool any = __syncthreads_or(flag);
+        if (__syncthreads_or(bad)) return false;
         if (threadIdx.x < 32) {
-            go(any);
+            go();
             if (elect_one()) mma_commit(bar);
             __syncwarp();
         }
         ++issued;
+        return true;
     }
     __device__ __forceinline__ void close(int cols)
     {
@@ -244,7 +215,7 @@ __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { r
 // entering the chunk if the sequence began earlier.
 template <typename T> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kParts * kTileB + kTail;
 template <typename T, bool PACKED>
-__global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
                                                                       float *states, int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -281,12 +252,12 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
     const int n = n0 + (warp & 3) * 32 + lane, p = p0 + (warp >> 2) * 32;           // my state index and the first of my 32 columns
     const int64_t hc = (int64_t)c * a.nheads + h;
     uint4 in[4] = {};                               // my part of an [n][p] tile of entering states: asked for now, needed last
-    if (PACKED && carry && form == SsdStates::np16 && n < N) {
+    if (sizeof(T) == 2 && PACKED && carry && form == SsdStates::np16 && n < N) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) in[i] = reinterpret_cast<const uint4 *>(static_cast<const T *>(entering) + (hc * N + n) * P + p)[i];
     }
 
-    uint4 xr[2], Br[4];
+    Raw8<T> xr[2], Br[4];
     float w[2];
     const bool whole = vx && vB && P - p0 >= 64 && N - n0 >= (wide ? 128 : 64) && (PACKED || !a.seq_idx);
     auto fetch = [&](int k) {
@@ -295,9 +266,9 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
             for (int i = 0; i < 2; ++i) {
                 const int kk = k + r0 + 32 * i;
                 const T *Bk = B + (int64_t)kk * a.B_stride[1] + 8 * c8;
-                xr[i] = *reinterpret_cast<const uint4 *>(x + (int64_t)kk * a.x_stride[1] + 8 * c8);
-                Br[i] = *reinterpret_cast<const uint4 *>(Bk);
-                if (wide) Br[2 + i] = *reinterpret_cast<const uint4 *>(Bk + 64);
+                xr[i] = load8_whole(x + (int64_t)kk * a.x_stride[1] + 8 * c8);
+                Br[i] = load8_whole(Bk);
+                if (wide) Br[2 + i] = load8_whole(Bk + 64);
                 w[i] = __expf(fminf(dA_end - dAc[kk], 0.f)) * dtc[kk];
             }
             return;
@@ -316,9 +287,11 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
     };
     if (k0 < k1) fetch(k0);
     constexpr uint32_t idesc = instr_desc_f16(128, 64, 1, 1, 1);
+    uint32_t skipped = 0;                           // tiles left for the FMAs
 #pragma unroll 1
-    for (int k = k0; k < k1; k += 64) {
+    for (int k = k0, tile = 0; k < k1; k += 64, ++tile) {
         t.drain();
+        bool bad = false;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const uint32_t o = sw128(r0 + 32 * i, c8);
@@ -326,18 +299,17 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
             widen8<T>(xr[i], v);
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] *= w[i];
-            const bool bad = not_finite<T>(Br[i]) || (wide && not_finite<T>(Br[2 + i]));
-            if (__ballot_sync(0xffffffffu, bad) & 0xffu << (lane & 24)) store_first(t.b + o, kTileB, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);     // in my row
-            else store_parts<kParts>(t.b + o, kTileB, v);
-            store_input<T>(t.a + o, kTileA, Br[i]);                             // states n0 .. n0 + 63, then the other 64
-            if (wide) store_input<T>(t.a + 8192 + o, kTileA, Br[2 + i]);
+            bad = store_parts<kParts>(t.b + o, kTileB, v) || bad;
+            bad = store_input<T>(t.a + o, kTileA, Br[i]) || bad;                // states n0 .. n0 + 63, then the other 64
+            if (wide) bad = store_input<T>(t.a + 8192 + o, kTileA, Br[2 + i]) || bad;
         }
-        t.step(false, [&](bool) {
+        const bool first = t.issued == 0;
+        if (!t.step(bad, [&] {
             // the tensor core adds to a sum with less care than fp32 rounding: the small products have one of their own (with one for
             // all, end states were 8 to 15 % further from 64 bits than the fp32 kernels' in chunks of 128; with two 1 to 2 %)
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kInParts<T>, kParts, acc, acc + 64, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, 16, 1024), 128, idesc, k > k0);
-        });
+            multiply(kInParts<T>, kParts, acc, acc + 64, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, 16, 1024), 128, idesc, !first);
+        })) skipped |= 1u << tile;
         if (k + 64 < k1) fetch(k + 64);
     }
     t.drain();
@@ -352,6 +324,17 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
         tmem_ld32(at + 64, rest);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] += rest[j];
+    }
+    if (skipped && n < N) {
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k) {
+            if (!((skipped >> (k - k0) / 64) & 1)) continue;
+            if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
+            const float wk = __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (p + j < P) v[j] = fmaf(to_float(x[(int64_t)k * a.x_stride[1] + p - p0 + j]) * wk, Bn, v[j]);
+        }
     }
     if (n < N) {
         const int64_t slot = PACKED ? (int64_t)blockIdx.y * a.nheads + h : ((int64_t)b * nchunks + c) * a.nheads + h;
@@ -376,9 +359,10 @@ __global__ void __launch_bounds__(kThreads, 3) ssd_split_state_kernel(const mb20
 // ====================================================================================== C.B^T
 // CB[m,k] = C_m . B_k, fp32, in tiles of 128 x 64 that reach the diagonal or lie below it; pairs of different sequences get 0.  The
 // products of two inputs are exact in the input type.  grid (row blocks x column tiles, batch x chunks, groups)
-constexpr uint32_t kCbSmem = kTileA + kTileB + kTail;
+template <typename T> constexpr int kCbParts = sizeof(T) == 2 ? 1 : kParts;
+template <typename T> constexpr uint32_t kCbSmem = kCbParts<T> * (kTileA + kTileB) + kTail;
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 4) ssd_split_cb_kernel(const mb200_ssd_args a, float *cb, int nchunks, int *status)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 2) ssd_split_cb_kernel(const mb200_ssd_args a, float *cb, int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int Q = a.chunk_size, N = a.dstate, tilesK = (Q + 63) / 64;
@@ -386,20 +370,21 @@ __global__ void __launch_bounds__(kThreads, 4) ssd_split_cb_kernel(const mb200_s
     const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, g = blockIdx.z, len = min(Q, a.seqlen - c * Q);
     if (k0 >= m0 + 128 || m0 >= len || k0 >= len) return;
     Tile t;
-    t.open(smem, kTileA, kTileB, 64, status, kStSplitCb);
+    constexpr int kSums = sizeof(T) == 2 ? 64 : 128;     // columns of tensor memory: fp32's small products have a sum of their own, as in the chunk states
+    t.open(smem, kCbParts<T> * kTileA, kCbParts<T> * kTileB, kSums, status, kStSplitCb);
     pdl_wait();
     const int64_t t0 = (int64_t)c * Q;
     const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (t0 + m0) * a.C_stride[1] + (int64_t)g * a.C_stride[2];
     const T *B = static_cast<const T *>(a.B) + (int64_t)b * a.B_stride[0] + (t0 + k0) * a.B_stride[1] + (int64_t)g * a.B_stride[2];
     const bool vC = rows16(C, a.C_stride[1]), vB = rows16(B, a.B_stride[1]), whole = vC && vB && m0 + 128 <= len && k0 + 64 <= len;
     const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;
-    uint4 Cr[4], Br[2];
+    Raw8<T> Cr[4], Br[2];
     auto fetch = [&](int n) {
         if (whole && n + 64 <= N) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) Cr[i] = *reinterpret_cast<const uint4 *>(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8);
+            for (int i = 0; i < 4; ++i) Cr[i] = load8_whole(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) Br[i] = *reinterpret_cast<const uint4 *>(B + (int64_t)(r0 + 32 * i) * a.B_stride[1] + n + 8 * c8);
+            for (int i = 0; i < 2; ++i) Br[i] = load8_whole(B + (int64_t)(r0 + 32 * i) * a.B_stride[1] + n + 8 * c8);
             return;
         }
 #pragma unroll
@@ -409,25 +394,49 @@ __global__ void __launch_bounds__(kThreads, 4) ssd_split_cb_kernel(const mb200_s
     };
     fetch(0);
     constexpr uint32_t idesc = instr_desc_f16(128, 64, std::is_same<T, __half>::value ? 0 : 1, 0, 0);
+    bool all = true;                                // no tile left for the FMAs
 #pragma unroll 1
     for (int n = 0; n < N; n += 64) {
         t.drain();
+        bool bad = false;
+        auto store = [&](uint32_t to, uint32_t stride, const Raw8<T> &r) {
+            if constexpr (sizeof(T) == 2) sts128(to, r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w);        // one product, exact: nothing to look for
+            else bad = store_input<T>(to, stride, r) || bad;
+        };
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sts128(t.a + sw128(r0 + 32 * i, c8), Cr[i].x, Cr[i].y, Cr[i].z, Cr[i].w);
+        for (int i = 0; i < 4; ++i) store(t.a + sw128(r0 + 32 * i, c8), kTileA, Cr[i]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) sts128(t.b + sw128(r0 + 32 * i, c8), Br[i].x, Br[i].y, Br[i].z, Br[i].w);
-        t.step(false, [&](bool) {
+        for (int i = 0; i < 2; ++i) store(t.b + sw128(r0 + 32 * i, c8), kTileB, Br[i]);
+        const bool first = t.issued == 0;
+        all = t.step(bad, [&] {
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(1, 1, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc, n > 0);
-        });
+            multiply(kCbParts<T>, kCbParts<T>, acc, acc + kSums - 64, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc, !first);
+        }) && all;
         if (n + 64 < N) fetch(n + 64);
     }
     t.drain();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + (warp & 3) * 32 + lane, k = k0 + (warp >> 2) * 32;
     if (__all_sync(0xffffffffu, t.ok)) {
         float v[32];
-        tc_fence_after_sync();
-        tmem_ld32(t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32, v);
+        if (all) {
+            tc_fence_after_sync();
+            const uint32_t from = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32;
+            tmem_ld32(from, v);
+            if constexpr (sizeof(T) == 4) {
+                float rest[32];
+                tmem_ld32(from + 64, rest);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] += rest[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                v[j] = 0.f;
+#pragma unroll 1
+                for (int n = 0; n < N && m < len && k + j < len; ++n)
+                    v[j] = fmaf(to_float(C[(int64_t)(m - m0) * a.C_stride[1] + n]), to_float(B[(int64_t)(k + j - k0) * a.B_stride[1] + n]), v[j]);
+            }
+        }
         if (m < Q) {
             if (a.seq_idx) {
                 const int mine = m < len ? seq_at(a, b, c * Q + m) : 0;
@@ -447,21 +456,85 @@ __global__ void __launch_bounds__(kThreads, 4) ssd_split_cb_kernel(const mb200_s
             }
         }
     }
-    t.close(64);
+    t.close(kSums);
 }
 
 // ====================================================================================== chunk outputs
 // y[m,p] = exp(dA_m) C_m . H[p] + sum_{k <= m} CB[m,k] exp(min(dA_m - dA_k, 0)) dt_k x[k,p] + D x[m,p], then y silu(z).
-// grid (row blocks of 128, heaviest first, x 64-column tiles of P, batch x chunks, heads).  Two CTAs of 126 registers per SM: three of 80
-// spill, and took 76 us where this takes 69 (the half-precision call above); a second pair of tiles left L1 so little that C.B^T, which
-// every head reads again, came from L2 each time (72 -> 81 us in bf16); one CTA per SM that keeps C.B^T in tensor memory while the heads
-// pass took 78, with all its warps in step 85.
+// grid (row blocks of 128, heaviest first, x 64-column tiles of P, batch x chunks, heads).  One kernel for 16-bit inputs, one for fp32.
 // The result is rounded to the input type.  For bf16 two parts, 16 to 17 bits of an operand, leave its error what all three give.
-template <typename T> constexpr int kOutParts = std::is_same<T, __half>::value ? 3 : 2;
-template <typename T> constexpr uint32_t kScanA = kOutParts<T> * kTileA;
-template <typename T> constexpr uint32_t kScanB = kOutParts<T> * kTileB;
+template <typename T> constexpr int kOutParts = std::is_same<T, __nv_bfloat16>::value ? 2 : 3;
+
+// Decays of the steps a block of rows looks back on, factorised: exp(dA_m - dA_k) dt_k = exp(dA_m - ref) (exp(ref - dA_k) dt_k), ref = dA
+// of the last of 32 steps: an exponential per row and 32 columns instead of one per element.  dA does not increase (A <= 0, dt >= 0), so neither exponent is positive below the diagonal; in the
+// range that holds it the first is bounded.  A range for which that is not so has its decays formed one by one.  Differences are formed
+// before anything is rounded, as with a single exponential.
+constexpr float kMaxSpan = 100.f;                       // (in powers of two) of the decays within 32 steps
+inline uint32_t scan_decay_bytes(const mb200_ssd_args &a)
+{
+    const uint32_t steps = (a.chunk_size + 63) / 64, states = (a.dstate + 63) / 64;
+    return (2 * 64 * steps + 1 + (steps + states + 31) / 32) * 4;
+}
+struct ScanDecays {
+    float *ck, *dA;             // [step]: column factors, dA (the last one's for steps past the end)
+    uint32_t *plain;            // ranges that cannot be factorised, a bit each
+    uint32_t *skip;             // tiles left for the FMAs, a bit each: of the states, then of the steps
+    int cols;
+    __device__ __forceinline__ ScanDecays(uint8_t *at, int cols_) : ck(reinterpret_cast<float *>(at)), dA(ck + cols_), plain(reinterpret_cast<uint32_t *>(dA + cols_)), skip(plain + 1), cols(cols_) {}
+    // (all threads; a barrier after each)
+    __device__ __forceinline__ void clear(int ntiles) const
+    {
+        for (int i = threadIdx.x; i < 1 + (ntiles + 31) / 32; i += blockDim.x) plain[i] = 0;
+    }
+    __device__ __forceinline__ void form(const float *dAc, const float *dtc, int kend) const
+    {
+        for (int k = threadIdx.x; k < cols; k += blockDim.x) {              // (a warp has a range of 32)
+            const int kk = min(k, kend - 1);
+            const float v = dAc[kk], before = dAc[max(kk - 1, 0)], end = __shfl_sync(0xffffffffu, v, 31);
+            dA[k] = v;
+            ck[k] = k < kend ? ex2((end - v) * kLog2e) * dtc[kk] : 0.f;
+            const bool falls = __all_sync(0xffffffffu, v <= before + 2e-6f * fabsf(before)), fits = __all_sync(0xffffffffu, (v - end) * kLog2e <= kMaxSpan);      // (rounding of the sums aside)
+            if ((threadIdx.x & 31) == 0) {
+                if (!falls) atomicOr(plain, ~0u);                            // then min(dA_m - dA_k, 0) may be 0 anywhere
+                else if (!fits) atomicOr(plain, 1u << (k >> 5));
+            }
+        }
+    }
+};
+// Rare: what tiles with infinities or NaNs contribute to eight outputs of row m, in fp32.
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
+__device__ __noinline__ void add_skipped(float4 *lo, float4 *hi, const uint32_t *skip, int nH, const float *cbrow, const float *dAc, const float *dtc, int m, float sc, const T *x,
+                                         int64_t x_stride, const T *Crow, const float *H, int N, int left)
+{
+    auto skipped = [&](int t) { return (skip[t >> 5] >> (t & 31)) & 1; };
+    float y[8] = {}, s[8] = {};
+    for (int k = 0; k <= m; ++k) {
+        if (!skipped(nH + (k >> 6))) continue;
+        const float w = cbrow[k] * ex2(fminf(dAc[m] - dAc[k], 0.f) * kLog2e) * dtc[k];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e < left) y[e] = fmaf(w, to_float(x[k * x_stride + e]), y[e]);
+    }
+    for (int n = 0; n < N; ++n) {
+        if (!skipped(n >> 6)) continue;
+        const float w = to_float(Crow[n]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e < left) s[e] = fmaf(w, H[(int64_t)e * N + n], s[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) reinterpret_cast<float *>(e < 4 ? lo : hi)[e & 3] += fmaf(sc, s[e], y[e]);
+}
+
+// ---- 16 bits
+// Two CTAs of 126 registers per SM: three of 80 spill, and took 76 us where this took 69 (2 x 1500 steps of 48 half-precision heads of 64 x
+// 64); a second pair of tiles left L1 so little that C.B^T, which every head reads again, came from L2 each time (72 -> 81 us in bf16); one
+// CTA per SM that keeps C.B^T in tensor memory while the heads pass took 78, with all its warps in step 85.  The kernel for fp32 below,
+// which leaves the MMAs to a warp of their own, takes 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
+template <typename T> constexpr uint32_t kScan16A = kOutParts<T> * kTileA;
+template <typename T> constexpr uint32_t kScan16B = kOutParts<T> * kTileB;
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
                                                                      int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -471,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     const int len = min(Q, a.seqlen - c * Q);
     if (m0 >= len) return;
     Tile t;
-    t.open(smem, kScanA<T>, kScanB<T>, 128, status, kStSplitScan);
+    t.open(smem, kScan16A<T>, kScan16B<T>, 128, status, kStSplitScan);
     pdl_wait();
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
     const float *dAc = dAb + row, *dtc = dtb + row;
@@ -481,13 +554,10 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     const float *cbm = cb + ((((int64_t)b * nchunks + c) * a.ngroups + g) * Q + m0) * Q;
     const bool vx = rows16(x, a.x_stride[1]), vC = rows16(C, a.C_stride[1]), vN = N % 4 == 0, vQ = Q % 4 == 0;
     const int kend = min(m0 + 128, len);
-    // dA and dt of the steps my rows look back on
-    float *col = reinterpret_cast<float *>(smem + kScanA<T> + kScanB<T> + kTail);
     const int cols = (kend + 63) / 64 * 64;
-    for (int k = threadIdx.x; k < cols; k += kThreads) {
-        col[k] = k < kend ? dAc[k] : 0.f;
-        col[cols + k] = k < kend ? dtc[k] : 0.f;
-    }
+    const ScanDecays decays(smem + kScan16A<T> + kScan16B<T> + kTail, cols);
+    decays.clear((N + 63) / 64 + cols / 64);
+    __syncthreads();
     const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;      // my eight columns; rows r0 + 32 i of a tile
     float dm[4];
 #pragma unroll
@@ -495,12 +565,12 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 
     // whole tiles need no look at any edge
     const bool whole_rows = m0 + 128 <= len, whole_cols = P - p0 >= 64;
-    union { uint4 u[8]; float4 f[8]; } A;           // C rows, or CB rows in two halves
-    union { uint4 u[4]; float4 f[4]; } Bq;          // H rows in two halves, or x rows
+    union { Raw8<T> u[4]; float4 f[8]; } A;         // C rows, or CB rows in two halves
+    union { Raw8<T> u[2]; float4 f[4]; } Bq;        // H rows in two halves, or x rows
     auto fetch_states = [&](int n) {
         if (vC && vN && whole_rows && whole_cols && n + 64 <= N) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) A.u[i] = *reinterpret_cast<const uint4 *>(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8);
+            for (int i = 0; i < 4; ++i) A.u[i] = load8_whole(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8);
 #pragma unroll
             for (int i = 0; i < 4; ++i) Bq.f[i] = reinterpret_cast<const float4 *>(H + (int64_t)(r0 + 32 * (i / 2)) * N + n + 8 * c8)[i & 1];
             return;
@@ -508,20 +578,20 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 #pragma unroll
         for (int i = 0; i < 4; ++i) A.u[i] = load8(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8, vC, m0 + r0 + 32 * i < len ? N - n - 8 * c8 : 0);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            load8(H + (int64_t)(r0 + 32 * i) * N + n + 8 * c8, vN, p0 + r0 + 32 * i < P ? N - n - 8 * c8 : 0, Bq.f[2 * i], Bq.f[2 * i + 1]);
+        for (int i = 0; i < 4; ++i)
+            Bq.f[i] = load4(H + (int64_t)(r0 + 32 * (i / 2)) * N + n + 8 * c8 + 4 * (i & 1), vN, p0 + r0 + 32 * (i / 2) < P ? N - n - 8 * c8 - 4 * (i & 1) : 0);
     };
     auto fetch_steps = [&](int k) {
         if (vx && vQ && whole_rows && whole_cols) {        // (then kend is a multiple of 64 as well)
 #pragma unroll
             for (int i = 0; i < 8; ++i) A.f[i] = reinterpret_cast<const float4 *>(cbm + (int64_t)(r0 + 32 * (i / 2)) * Q + k + 8 * c8)[i & 1];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) Bq.u[i] = *reinterpret_cast<const uint4 *>(x + (int64_t)(k + r0 + 32 * i) * a.x_stride[1] + 8 * c8);
+            for (int i = 0; i < 2; ++i) Bq.u[i] = load8_whole(x + (int64_t)(k + r0 + 32 * i) * a.x_stride[1] + 8 * c8);
             return;
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            load8(cbm + (int64_t)(r0 + 32 * i) * Q + k + 8 * c8, vQ, m0 + r0 + 32 * i < len ? kend - k - 8 * c8 : 0, A.f[2 * i], A.f[2 * i + 1]);
+        for (int i = 0; i < 8; ++i)
+            A.f[i] = load4(cbm + (int64_t)(r0 + 32 * (i / 2)) * Q + k + 8 * c8 + 4 * (i & 1), vQ, m0 + r0 + 32 * (i / 2) < len ? kend - k - 8 * c8 - 4 * (i & 1) : 0);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int kk = k + r0 + 32 * i;
@@ -529,6 +599,16 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         }
     };
     fetch_states(0);
+    const float Dh = a.D && !a.D_has_hdim ? a.D[h] : 0.f;
+    decays.form(dAc, dtc, kend);
+    __syncthreads();
+    const uint32_t plains = *decays.plain;
+    const int nH = (N + 63) / 64;
+    bool left_out = false;                          // tiles have been left for the FMAs (a bit each in the skip words)
+    auto leave_out = [&](int tile) {
+        left_out = true;
+        if (threadIdx.x == 0) decays.skip[tile >> 5] |= 1u << (tile & 31);
+    };
     // contribution of the state entering the chunk: C . H, into the first 64 columns
     constexpr uint32_t idesc_h = instr_desc_f16(128, 64, 1, 0, 0), idesc_x = instr_desc_f16(128, 64, 1, 0, 1);
 #pragma unroll 1
@@ -536,33 +616,37 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         t.drain();
         bool bad = false;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            bad = bad || not_finite<T>(A.u[i]);
-            store_input<T>(t.a + sw128(r0 + 32 * i, c8), kTileA, A.u[i]);
-        }
+        for (int i = 0; i < 4; ++i) bad = store_input<T>(t.a + sw128(r0 + 32 * i, c8), kTileA, A.u[i]) || bad;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float4 lo = Bq.f[2 * i], hi = Bq.f[2 * i + 1];
-            float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            store_parts<kOutParts<T>>(t.b + sw128(r0 + 32 * i, c8), kTileB, v);
+            const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            bad = store_parts<kOutParts<T>>(t.b + sw128(r0 + 32 * i, c8), kTileB, v) || bad;
         }
-        t.step(bad, [&](bool any) {
+        const bool first = t.issued == 0;
+        if (!t.step(bad, [&] {
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kInParts<T>, any ? 1 : kOutParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc_h, n > 0);
-        });
+            multiply(kInParts<T>, kOutParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc_h, !first);
+        })) leave_out(n >> 6);
         if (n + 64 < N) fetch_states(n + 64);
         else fetch_steps(0);
     }
     // the steps of the chunk up to the diagonal, into the other 64
+    const int states_done = t.issued;
 #pragma unroll 1
     for (int k = 0; k < kend; k += 64) {
         t.drain();
-        uint64_t dk[4], tk[4];
+        uint64_t fk[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            dk[e] = *reinterpret_cast<const uint64_t *>(col + k + 8 * c8 + 2 * e);
-            tk[e] = *reinterpret_cast<const uint64_t *>(col + cols + k + 8 * c8 + 2 * e);
+        for (int q = 0; q < 2; ++q) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(decays.ck + k + 8 * c8 + 4 * q);
+            fk[2 * q] = v.x;
+            fk[2 * q + 1] = v.y;
         }
+        const int range = (k >> 5) + (c8 >> 2);
+        const float end = decays.dA[32 * range + 31];
+        const bool plain = (plains >> range) & 1;
+        bool bad = false;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t to = t.a + sw128(r0 + 32 * i, c8);
@@ -572,41 +656,48 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
                 continue;
             }
             const float4 lo = A.f[2 * i], hi = A.f[2 * i + 1];
+            uint64_t f[4] = {fk[0], fk[1], fk[2], fk[3]};
+            float fm = ex2(fminf((dm[i] - end) * kLog2e, kMaxSpan));            // (past the diagonal it only has to stay finite)
+            if (plain) {
+                fm = 1.f;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int kk = k + 8 * c8 + 2 * e;
+                    f[e] = pack2(kk < kend ? ex2(fminf(dm[i] - decays.dA[kk], 0.f) * kLog2e) * dtc[kk] : 0.f,
+                                 kk + 1 < kend ? ex2(fminf(dm[i] - decays.dA[kk + 1], 0.f) * kLog2e) * dtc[kk + 1] : 0.f);
+                }
+            }
             const uint64_t cbv[4] = {pack2(lo.x, lo.y), pack2(lo.z, lo.w), pack2(hi.x, hi.y), pack2(hi.z, hi.w)};
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float d0, d1;
-                unpack2(sub2(pack2(dm[i], dm[i]), dk[e]), d0, d1);
-                unpack2(mul2(pack2(fminf(d0, 0.f), fminf(d1, 0.f)), pack2(kLog2e, kLog2e)), d0, d1);
-                unpack2(mul2(mul2(cbv[e], pack2(ex2(d0), ex2(d1))), tk[e]), v[2 * e], v[2 * e + 1]);
-            }
+            for (int e = 0; e < 4; ++e) unpack2(mul2(mul2(cbv[e], f[e]), pack2(fm, fm)), v[2 * e], v[2 * e + 1]);
             if (k + 64 > m0) {
                 const int past = m0 + r0 + 32 * i - (k + 8 * c8);       // columns up to the diagonal
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = e <= past ? v[e] : 0.f;
             }
-            store_parts<kOutParts<T>>(to, kTileA, v);
+            bad = store_parts<kOutParts<T>>(to, kTileA, v) || bad;
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i) store_input<T>(t.b + sw128(r0 + 32 * i, c8), kTileB, Bq.u[i]);
-        t.step(not_finite<T>(Bq.u[0]) || not_finite<T>(Bq.u[1]), [&](bool any) {
+        for (int i = 0; i < 2; ++i) bad = store_input<T>(t.b + sw128(r0 + 32 * i, c8), kTileB, Bq.u[i]) || bad;
+        const bool first = t.issued == states_done;
+        if (!t.step(bad, [&] {
             const uint32_t acc = warp_uniform(t.tmem) + 64;
-            multiply(any ? 1 : kOutParts<T>, kInParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 128, idesc_x, k > 0);
-        });
+            multiply(kOutParts<T>, kInParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 128, idesc_x, !first);
+        })) leave_out(nH + (k >> 6));
         if (k + 64 < kend) fetch_steps(k + 64);
     }
     // x and z of my rows are on their way while the last products are formed
     const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
     const bool vz = z && rows16(z, a.z_stride[1]);
     const int left = P - p0 - 8 * c8;
-    uint4 xm[4], zm[4];
+    Raw8<T> xm[4], zm[4];
     if (whole_rows && whole_cols && vx && (!z || vz)) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int64_t m = m0 + r0 + 32 * i;
-            if (a.D) xm[i] = *reinterpret_cast<const uint4 *>(x + m * a.x_stride[1] + 8 * c8);
-            if (z) zm[i] = *reinterpret_cast<const uint4 *>(z + m * a.z_stride[1] + 8 * c8);
+            if (a.D) xm[i] = load8_whole(x + m * a.x_stride[1] + 8 * c8);
+            if (z) zm[i] = load8_whole(z + m * a.z_stride[1] + 8 * c8);
         }
     } else {
 #pragma unroll
@@ -621,9 +712,12 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
         tc_fence_after_sync();
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lm = (warp & 3) * 32 + lane, m = m0 + lm;
-        float sc = m < len ? __expf(dAc[m]) : 0.f;
-        // the entering state belongs to the sequence that ends the previous chunk
-        if (a.seq_idx && m < len && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0)) sc = 0.f;
+        auto scale = [&](int m) {                   // the entering state belongs to the sequence that ends the previous chunk
+            if (m >= len || (a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0))) return 0.f;
+            return __expf(decays.dA[m]);
+        };
+        const float sc = scale(m);
+        const bool any1 = states_done > 0, any2 = t.issued > states_done;        // sums that the tensor core has formed
         auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + r * 256 + ((chunk ^ (r & 7)) << 4)); };
 #pragma unroll
         for (int j = (warp >> 2) * 32; j < (warp >> 2) * 32 + 32; j += 8) {
@@ -634,16 +728,20 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
             tmem_ld_wait(y1, y2);
             float y[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = fmaf(sc, __uint_as_float(y1[e]), __uint_as_float(y2[e]));
+            for (int e = 0; e < 8; ++e) y[e] = fmaf(sc, any1 ? __uint_as_float(y1[e]) : 0.f, any2 ? __uint_as_float(y2[e]) : 0.f);
             *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
             *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
         }
         __syncthreads();
         T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
         const bool vo = rows16(out, a.out_stride[1]);
-        float Dv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) Dv[e] = !a.D ? 0.f : !a.D_has_hdim ? a.D[h] : e < left ? a.D[(int64_t)h * P + p0 + 8 * c8 + e] : 0.f;
+        if (left_out) {
+#pragma unroll 1
+            for (int r = r0; r < 128; r += 32)
+                if (m0 + r < len && left > 0)
+                    add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), decays.skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
+                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int r = r0 + 32 * i;
@@ -653,20 +751,20 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
             if (a.D) {
                 widen8<T>(xm[i], f);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dv[e], y[e]);
+                for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], !a.D_has_hdim ? Dh : e < left ? a.D[(int64_t)h * P + p0 + 8 * c8 + e] : 0.f, y[e]);
             }
             if (z) {
                 widen8<T>(zm[i], f);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) y[e] *= fast_silu(f[e]);
             }
-            uint4 o;
+            Raw8<T> o;
             T *oe = reinterpret_cast<T *>(&o);
 #pragma unroll
             for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
             T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
             if (vo && left >= 8) {
-                *reinterpret_cast<uint4 *>(om) = o;
+                *reinterpret_cast<Raw8<T> *>(om) = o;
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
@@ -675,6 +773,465 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         }
     }
     t.close(128);
+}
+
+
+// ---- fp32
+// Eight warps form the operands of a tile of 64 along the reduction -- first the states, then the steps of the chunk up to the diagonal --
+// and a ninth issues its MMAs: the A operand (C, then CB with its decays) goes to tensor memory, B (H, then x) to shared memory.  A warp
+// has rows 32 (w % 4) .. and one half of the 64 columns; tcgen05.st.16x128b gives a lane four of these rows, and four lanes a row's 16
+// bytes, so that the loads fill whole sectors.  The order within a tile is free: a lane's four consecutive elements go to where its words
+// are, and B's rows (or H's columns) follow.  The small products have a sum of their own, as in the chunk states.
+// What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
+// middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us,
+// 2 x 3000 steps of 32 heads of 64 x 128 149; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
+constexpr int kScanThreads = kThreads + 32;
+// Shared memory: B, then two stages of C.B^T, 4 KB a warp.  The sums leave through the first of them.
+constexpr uint32_t kScanB = kParts * kTileB, kScanTiles = kScanB + 65536;
+constexpr uint32_t kScanTail = 48;                      // barriers and tensor-memory slot behind the tiles
+constexpr uint32_t kScanA = 128;                        // tensor memory: the sums of large and of small products, then A
+
+// where step `k` of a tile lies along the reduction: a lane's elements 4 j .. 4 j + 3 of 16 are words j and 4 + j
+__device__ __forceinline__ int place4(int k) { return (k & ~15) + ((k >> 1) & 1) * 8 + ((k >> 2) & 3) * 2 + (k & 1); }
+__device__ __forceinline__ void tmem_st_16x128b(uint32_t taddr, uint32_t a, uint32_t b)
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x1.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in)      // zeros where not `in`
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
+                                                                         int nchunks, int *status)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    using T = float;
+    constexpr int NP = kParts;
+    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesP = (P + 63) / 64;
+    const int m0 = ((Q + 127) / 128 - 1 - blockIdx.x / tilesP) * 128, p0 = (blockIdx.x % tilesP) * 64;
+    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z, g = h / (a.nheads / a.ngroups);
+    const int len = min(Q, a.seqlen - c * Q);
+    if (m0 >= len) return;
+    const int kend = min(m0 + 128, len), ksteps = (kend + 63) / 64, cols = ksteps * 64, nH = (N + 63) / 64, ntiles = nH + ksteps;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool mma_warp = warp == kThreads / 32;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + kScanTiles), *done = full + 2;      // [tile & 1]: operands in place; their products added
+    uint32_t *slot = reinterpret_cast<uint32_t *>(done + 2);
+    const ScanDecays decays(smem + kScanTiles + kScanTail, cols);
+    float *const ck = decays.ck, *const dAs = decays.dA;
+    uint32_t *const skip = decays.skip;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&full[i], kThreads / 32);
+            mbar_init(&done[i], 1);
+        }
+        mbar_fence_init();
+        if (smem_u32(smem) & 1023u) atomicCAS(status, 0, kStSplitScan);             // the swizzled tiles assume a 1 KB aligned base
+    }
+    if (mma_warp) tmem_alloc(slot, 256);
+    decays.clear(ntiles);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    pdl_wait();
+    const uint32_t tmem = *slot, tiles = smem_u32(smem);
+    const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
+    const float *dAc = dAb + row, *dtc = dtb + row;
+    const T *x = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2] + p0;
+    const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (t0 + m0) * a.C_stride[1] + (int64_t)g * a.C_stride[2];
+    const float *H = states + (((int64_t)b * nchunks + c) * a.nheads + h) * (int64_t)P * N + (int64_t)p0 * N;
+    const float *cbm = cb + ((((int64_t)b * nchunks + c) * a.ngroups + g) * Q + m0) * Q;
+    const bool vx = rows16(x, a.x_stride[1]), vC = rows16(C, a.C_stride[1]), vN = N % 2 == 0, vQ = Q % 4 == 0;
+    const bool whole_rows = m0 + 128 <= len, whole_cols = P - p0 >= 64;
+    const int j4 = lane & 3, rw = (warp & 3) * 32, ra = rw + (lane >> 2), ch = (warp >> 2) * 32;       // A: rows ra + 8 i, columns of half ch
+    const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;                                             // B: rows r0 + 32 i, chunk c8
+
+    Raw8<T> Cr[4];
+    float2 Hr[2][4];
+    auto fetch_states = [&](int n) {
+        // a lane's elements of a row of C: 16 q + 4 j .. + 3; H's columns lie as they do
+        const T *pC = C + (int64_t)ra * a.C_stride[1] + n + ch + 4 * j4;
+        const float *pH = H + (int64_t)r0 * N + n + 16 * (c8 >> 1) + 2 * (c8 & 1);
+        if (vC && vN && whole_rows && whole_cols && n + 64 <= N) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) Cr[r].q[q] = *reinterpret_cast<const uint4 *>(pC + (int64_t)(8 * r) * a.C_stride[1] + 16 * q);
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) Hr[r][j] = *reinterpret_cast<const float2 *>(pH + (int64_t)(32 * r) * N + 4 * j);
+            return;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const T *p = pC + (int64_t)(8 * r) * a.C_stride[1];
+            const int left = m0 + ra + 8 * r < len ? N - (int)(p - (C + (int64_t)(ra + 8 * r) * a.C_stride[1])) : 0;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float4 v = load4(p + 16 * q, vC, left - 16 * q);
+                Cr[r].q[q] = *reinterpret_cast<const uint4 *>(&v);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float *p = pH + (int64_t)(32 * r) * N + 4 * j;
+                const int left = p0 + r0 + 32 * r < P ? N - (int)(p - (H + (int64_t)(r0 + 32 * r) * N)) : 0;
+                Hr[r][j] = make_float2(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f);
+            }
+    };
+    Raw8<T> xr[2];
+    auto fetch_x = [&](int k) {
+        if (vx && whole_rows && whole_cols) {                // no edge, nothing to look at (kend is a multiple of 64 as well)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) xr[i] = load8_whole(x + (int64_t)(k + r0 + 32 * i) * a.x_stride[1] + 8 * c8);
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int kk = k + r0 + 32 * i;
+            xr[i] = load8(x + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, kk < kend ? P - p0 - 8 * c8 : 0);
+        }
+    };
+    // my warp's 32 x 32 of C.B^T: packets of a row, halves of odd rows swapped, so that a lane's reads below meet no conflict
+    constexpr int kAhead = 2;                                // stages
+    const uint32_t ring = tiles + kScanB + warp * 4096;
+    auto request_cb = [&](int k) {
+        const uint32_t to = ring + ((k >> 6) & 1) * 32768 + (lane >> 3) * 128;
+        const uint32_t to0 = to + (((lane & 7) ^ ((lane >> 1) & 4)) << 4);                 // rows lane / 8 + 4 i: odd where lane / 8 is
+        if (k < kend && m0 + rw + 31 >= k + ch) {            // (else my rows are above the diagonal)
+            const int col = k + ch + 4 * (lane & 7), r = rw + (lane >> 3);
+            const float *p = cbm + (int64_t)r * Q + col;
+            if (vQ && whole_rows) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) cp_async16(to0 + 512 * i, p + (int64_t)(4 * i) * Q, true);
+            } else {
+#pragma unroll 1
+                for (int i = 0; i < 8; ++i) {
+                    const bool in = m0 + r + 4 * i < len && col < Q;
+                    if (vQ) {
+                        cp_async16(to0 + 512 * i, in ? p + (int64_t)(4 * i) * Q : cbm, in);
+                    } else {
+                        const float4 v = load4(p + (int64_t)(4 * i) * Q, false, in ? Q - col : 0);
+                        sts128(to0 + 512 * i, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+                    }
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (!mma_warp) {
+        fetch_states(0);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) request_cb(64 * i);
+    }
+    const float Dh = a.D && !a.D_has_hdim ? a.D[h] : 0.f;
+    decays.form(dAc, dtc, kend);
+    __syncthreads();
+    bool ok = true;
+    if (mma_warp) {
+        // ------------------------------------------------------------------ MMAs
+        constexpr uint32_t idesc_h = instr_desc_f16(128, 64, 1, 0, 0), idesc_x = instr_desc_f16(128, 64, 1, 0, 1);
+        const uint32_t tm = warp_uniform(tmem);
+        const uint64_t desc = smem_desc_sw128(tiles, 16, 1024);
+        bool begun = false;                                  // the sums hold something
+#pragma unroll 1
+        for (int i = 0; i < ntiles && ok; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[i & 1], (i >> 1) & 1, status, kStSplitScan));
+            if (!ok) break;
+            tc_fence_after_sync();
+            const bool steps = i >= nH, on = !((reinterpret_cast<volatile uint32_t *>(skip)[i >> 5] >> (i & 31)) & 1);
+            const uint32_t A = tm + kScanA;
+            begun = begun || steps;                          // (scaled, they do)
+            const uint32_t step_b = steps ? 128 : 2, idesc = steps ? idesc_x : idesc_h;
+            if (elect_one()) {
+                if (on) {
+                    mma_steps_ts(4, tm, A, desc, step_b, idesc, begun);
+                    bool more = begun;
+#pragma unroll 1
+                    for (int pa = 0; pa < NP; ++pa)
+#pragma unroll 1
+                        for (int pb = pa ? 0 : 1; pa + pb < NP; ++pb) {
+                            mma_steps_ts(4, tm + 64, A + 32 * pa, desc + pb * (kTileB / 16), step_b, idesc, more);
+                            more = true;
+                        }
+                }
+                mma_commit(&done[i & 1]);
+            }
+            __syncwarp();
+            begun = begun || on;
+        }
+    } else {
+        // ------------------------------------------------------------------ operands
+        const uint32_t at = tmem + ((uint32_t)rw << 16) + kScanA + ch / 2;
+        const uint32_t plains = *decays.plain;
+        float dm[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dm[i] = dAs[min(m0 + ra + 8 * i, cols - 1)];
+        const int lm = rw + lane, m = m0 + lm;               // my row of the sums, whose columns ch .. ch + 31 I have
+        auto scale = [&](int m) {                            // the entering state belongs to the sequence that ends the previous chunk
+            if (m >= len || (a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0))) return 0.f;
+            return __expf(dAs[m]);
+        };
+        const float sc = scale(m);
+        auto skipped = [&](int t) { return (reinterpret_cast<volatile uint32_t *>(skip)[t >> 5] >> (t & 31)) & 1; };
+        auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + kScanB + r * 256 + ((chunk ^ (r & 7)) << 4)); };
+        auto wait_done = [&](int i) {
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1, status, kStSplitScan));
+            if (ok) tc_fence_after_sync();
+            return ok;
+        };
+        auto finish = [&](int i, bool bad) {                 // my part of tile i is in place
+            tmem_st_wait();
+            fence_proxy_async();
+            tc_fence_before_sync();
+            if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&skip[i >> 5], 1u << (i & 31));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[i & 1]);
+        };
+        // columns j .. j + 7 of my row's sums
+        const uint32_t sums = tmem + ((uint32_t)rw << 16);
+        auto load_sums = [&](int j, float (&y)[8]) {
+            uint32_t u[8], w[8];
+            tmem_ld8_issue(sums + j, u);
+            tmem_ld8_issue(sums + 64 + j, w);
+            tmem_ld_wait(u, w);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(u[e]) + __uint_as_float(w[e]);
+        };
+
+        // ---- the state entering the chunk: C . H
+        int i = 0;
+#pragma unroll 1
+        for (int n = 0; n < N; n += 64, ++i) {
+            if (i > 0 && !wait_done(i - 1)) break;
+            bool bad = false;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float v[8] = {Hr[r][0].x, Hr[r][0].y, Hr[r][1].x, Hr[r][1].y, Hr[r][2].x, Hr[r][2].y, Hr[r][3].x, Hr[r][3].y};
+                bad = store_parts<NP>(tiles + sw128(r0 + 32 * r, c8), kTileB, v) || bad;
+            }
+            Finite<__nv_bfloat16> f;
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                uint32_t w[NP][8];
+#pragma unroll
+                for (int hr = 0; hr < 2; ++hr) {
+                    float v[8];
+                    widen8<T>(Cr[2 * hh + hr], v);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t parts[NP];
+                        cut2<NP>(pack2(v[2 * q], v[2 * q + 1]), parts);
+                        f.feed(parts[0]);
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
+            }
+            if (n + 64 < N) fetch_states(n + 64);
+            else fetch_x(0);
+            finish(i, bad || f.bad());
+        }
+
+        // ---- steps of the chunk up to the diagonal
+#pragma unroll 1
+        for (int k = 0; k < kend && ok; k += 64, ++i) {
+            if (!wait_done(i - 1)) break;
+            if (k == 0) {
+                // the sums over the states, times exp(dA_m), are where those over the steps begin
+                bool any = false;
+                for (int t = 0; t < nH; ++t) any = any || !skipped(t);
+#pragma unroll 1
+                for (int j = ch; j < ch + 32; j += 8) {
+                    float y[8];
+                    uint32_t u[8];
+                    load_sums(j, y);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) u[e] = any ? __float_as_uint(sc * y[e]) : 0u;
+                    tmem_st8_issue(sums + j, u);
+                    const uint32_t none[8] = {};
+                    tmem_st8_issue(sums + 64 + j, none);
+                }
+            }
+            bool bad = false;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) bad = store_input<T>(tiles + sw128(place4(r0 + 32 * r), c8), kTileB, xr[r]) || bad;
+            if (k + 64 < kend) fetch_x(k + 64);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            if (m0 + rw + 31 < k + ch) {
+                const uint32_t none[8] = {};
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    tmem_st_16x128b_x4(at + 32 * p, none);
+                    tmem_st_16x128b_x4(at + 32 * p + (16u << 16), none);
+                }
+            } else {
+                Finite<__nv_bfloat16> f;
+                if (!((plains >> ((k + ch) >> 5)) & 1)) {
+                    uint64_t fk[4];                          // of my columns 16 q + 4 j .. + 3
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(ck + k + ch + 4 * j4 + 16 * q);
+                        fk[2 * q] = v.x;
+                        fk[2 * q + 1] = v.y;
+                    }
+                    const float end = dAs[k + ch + 31];
+                    const uint32_t from = ring + ((k >> 6) & 1) * 32768 + (lane >> 2) * 128 + j4 * 16, flip = (lane & 4) << 4;       // (row & 1 = lane / 4 & 1)
+                    const bool diagonal = k + ch + 31 > m0 + rw;
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        uint32_t w[NP][8];
+#pragma unroll
+                        for (int hr = 0; hr < 2; ++hr) {
+                            const int r = 2 * hh + hr;
+                            uint64_t cbv[4];
+#pragma unroll
+                            for (int q = 0; q < 2; ++q)
+                                asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
+                            const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
+                            const float fm = ex2(fminf((dm[r] - end) * kLog2e, kMaxSpan));             // (past the diagonal it only has to stay finite)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                uint64_t v = mul2(mul2(cbv[q], fk[q]), pack2(fm, fm));
+                                if (diagonal) {
+                                    float v0, v1;
+                                    unpack2(v, v0, v1);
+                                    const int e = 16 * (q >> 1) + 2 * (q & 1);
+                                    v = pack2(e <= past ? v0 : 0.f, e + 1 <= past ? v1 : 0.f);
+                                }
+                                uint32_t parts[NP];
+                                cut2<NP>(v, parts);
+                                f.feed(parts[0]);
+#pragma unroll
+                                for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
+                            }
+                        }
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
+                    }
+                } else {
+                    // rare, and kept short: one word of two rows at a time
+#pragma unroll 1
+                    for (int e = 0; e < 8; ++e) {
+                        const int q = e & 3, hh = e >> 2, kk = k + ch + 4 * j4 + 16 * (q >> 1) + 2 * (q & 1);
+                        uint32_t w[2][NP];
+#pragma unroll
+                        for (int hr = 0; hr < 2; ++hr) {
+                            const int rr = ra + 8 * (2 * hh + hr), m = m0 + rr;
+                            auto one = [&](int kk) { return m < len && kk <= m ? cbm[(int64_t)rr * Q + kk] * ex2(fminf(dAc[m] - dAc[kk], 0.f) * kLog2e) * dtc[kk] : 0.f; };
+                            cut2<NP>(pack2(one(kk), one(kk + 1)), w[hr]);
+                            f.feed(w[hr][0]);
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) tmem_st_16x128b(at + 32 * p + 4 * q + ((16u * hh) << 16), w[0][p], w[1][p]);
+                    }
+                }
+                bad = f.bad() || bad;
+            }
+            __syncwarp();
+            request_cb(k + 64 * kAhead);
+            finish(i, bad);
+        }
+
+        // ---- x and z of my rows are on their way while the last products are formed
+        const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
+        const bool vz = z && rows16(z, a.z_stride[1]);
+        const int left = P - p0 - 8 * c8;
+        Raw8<T> xm[4], zm[4];
+        if (whole_rows && whole_cols && vx && (!z || vz)) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int64_t m = m0 + r0 + 32 * r;
+                if (a.D) xm[r] = load8_whole(x + m * a.x_stride[1] + 8 * c8);
+                if (z) zm[r] = load8_whole(z + m * a.z_stride[1] + 8 * c8);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int64_t m = m0 + r0 + 32 * r;
+                if (a.D) xm[r] = load8(x + m * a.x_stride[1] + 8 * c8, vx, m < len ? left : 0);
+                if (z) zm[r] = load8(z + m * a.z_stride[1] + 8 * c8, vz, m < len ? left : 0);
+            }
+        }
+        wait_done(ntiles - 1);
+        uint32_t every;                                      // (also: everyone's writes to the skip words are there, and C.B^T is not needed any more)
+        asm volatile("{\n\t.reg .pred q, o;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred o, 1, 256, q;\n\tselp.u32 %0, 1, 0, o;\n\t}" : "=r"(every) : "r"((uint32_t)ok) : "memory");
+        if (every) {
+            bool fma = false;                                // something is left
+            for (int t = 0; t < ntiles; ++t) fma = fma || skipped(t);
+            // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
+            tc_fence_after_sync();
+#pragma unroll
+            for (int j = ch; j < ch + 32; j += 8) {
+                float y[8];
+                load_sums(j, y);
+                *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
+                *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
+            const bool vo = rows16(out, a.out_stride[1]);
+            if (fma) {
+#pragma unroll 1
+                for (int r = r0; r < 128; r += 32)
+                    if (m0 + r < len && left > 0)
+                        add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
+                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + 32 * q;
+                if (m0 + r >= len || left <= 0) continue;
+                const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
+                float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
+                if (a.D) {
+                    widen8<T>(xm[q], f);
+                    if (!a.D_has_hdim) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dh, y[e]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (e < left) y[e] = fmaf(f[e], a.D[(int64_t)h * P + p0 + 8 * c8 + e], y[e]);
+                    }
+                }
+                if (z) {
+                    widen8<T>(zm[q], f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[e] *= silu(f[e]);
+                }
+                Raw8<T> o;
+                T *oe = reinterpret_cast<T *>(&o);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
+                T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
+                if (vo && left >= 8) {
+                    *reinterpret_cast<Raw8<T> *>(om) = o;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (e < left) om[e] = oe[e];
+                }
+            }
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (mma_warp) tmem_dealloc(tmem, 256);
 }
 
 struct Buffers {
@@ -691,7 +1248,7 @@ struct Buffers {
     }
 };
 // f(element type of the call)
-template <class F> int with_type(const mb200_ssd_args &a, F f) { return a.io_dtype == MB200_BF16 ? f(__nv_bfloat16{}) : f(__half{}); }
+template <class F> int with_type(const mb200_ssd_args &a, F f) { return a.io_dtype == MB200_BF16 ? f(__nv_bfloat16{}) : a.io_dtype == MB200_F16 ? f(__half{}) : f(float{}); }
 
 template <bool PACKED> int run_states(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates form, cudaStream_t stream)
 {
@@ -718,9 +1275,9 @@ int ssd_split_cb(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t st
     return with_type(a, [&](auto tag) -> int {
         using T = decltype(tag);
         const Buffers s(a, lay);
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_cb_kernel<T>), (int)kCbSmem, a.device);
+        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_cb_kernel<T>), (int)kCbSmem<T>, a.device);
         const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.chunk_size + 63) / 64));
-        launch_dependent(ssd_split_cb_kernel<T>, dim3(tiles, a.batch * lay.nchunks, a.ngroups), kThreads, kCbSmem, stream, a, s.cb, lay.nchunks, s.status);
+        launch_dependent(ssd_split_cb_kernel<T>, dim3(tiles, a.batch * lay.nchunks, a.ngroups), kThreads, kCbSmem<T>, stream, a, s.cb, lay.nchunks, s.status);
         MB200_CHECK_LAUNCH("ssd C.B^T (split products)");
         return MB200_OK;
     });
@@ -731,10 +1288,14 @@ int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t 
     return with_type(a, [&](auto tag) -> int {
         using T = decltype(tag);
         const Buffers s(a, lay);
-        const uint32_t smem = kScanA<T> + kScanB<T> + kTail + 2 * ((a.chunk_size + 63) / 64 * 64) * (uint32_t)sizeof(float);
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_scan_kernel<T>), (int)smem, a.device);
-        const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.headdim + 63) / 64));
-        launch_dependent(ssd_split_scan_kernel<T>, dim3(tiles, a.batch * lay.nchunks, a.nheads), kThreads, smem, stream, a, s.dt, s.dA, s.states, s.cb, lay.nchunks, s.status);
+        auto go = [&](auto kernel, int threads, uint32_t smem) {
+            smem += scan_decay_bytes(a);
+            ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem, a.device);
+            const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.headdim + 63) / 64));
+            launch_dependent(kernel, dim3(tiles, a.batch * lay.nchunks, a.nheads), threads, smem, stream, a, s.dt, s.dA, s.states, s.cb, lay.nchunks, s.status);
+        };
+        if constexpr (sizeof(T) == 2) go(ssd_split_scan16_kernel<T>, kThreads, kScan16A<T> + kScan16B<T> + kTail);
+        else go(ssd_split_scan_kernel, kScanThreads, kScanTiles + kScanTail);
         MB200_CHECK_LAUNCH("ssd outputs (split products)");
         return MB200_OK;
     });

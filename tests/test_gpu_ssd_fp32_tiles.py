@@ -1,5 +1,5 @@
-"""The fp32 tile kernels of the chunked scan where their tiles end: chunk, head and state sizes off 64, off 32 and off 4 (element
-loads), packed sequences, and 16-bit shapes that take the same kernels."""
+"""The chunked scan in fp32 where its tiles end: chunk, head and state sizes off 64, off 32 and off 4 (element
+loads), packed sequences, and 16-bit calls of the same shapes."""
 import pytest
 import torch
 

@@ -1,0 +1,66 @@
+"""The split-product stages where their short cuts end: decays that cannot be factorised over 32 steps (steeper than 2^100, or rising),
+fp32 inputs at the edges of tiles, and fp32 infinities and NaNs, which the tensor core leaves to fp32 FMAs."""
+import pytest
+import torch
+
+import oracle
+from test_gpu_ssd import DEV, _c, _fn, make
+from test_gpu_ssd_split import F32, rel, run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("A", [-400.0, -40.0])
+def test_decays_formed_one_by_one(dtype, A):
+    """One head with decays of that kind among ordinary ones; 32 steps of the steepest take it past the smallest fp32."""
+    inp = make(900, 2, 300, 3, 64, 1, 64, dtype, init=True)
+    inp["A"][1] = A
+    run(inp, 256, f"A {A}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_rising_sums(dtype):
+    """A > 0: differences of the running sums are cut off at 0, as documented, so that no decay exceeds 1."""
+    inp = make(905, 1, 200, 2, 64, 1, 64, dtype, has_z=False, init=True)
+    inp["A"][1] = 0.02
+    d = {k: v.double() for k, v in inp.items() if v is not None}
+    dt = torch.nn.functional.softplus(d["dt"] + d["dt_bias"])[0]                          # (L, H)
+    sums = torch.cumsum(dt * d["A"], 0).T                                                 # (H, L)
+    decay = torch.exp((sums[:, :, None] - sums[:, None, :]).clamp(max=0)).tril() * dt.T[:, None, :]
+    want = torch.einsum("mn,kn,hmk,khp->mhp", d["C"][0, :, 0], d["B"][0, :, 0], decay, d["x"][0])
+    want += torch.einsum("mn,hm,hpn->mhp", d["C"][0, :, 0], torch.exp(sums), d["initial_states"][0]) + d["x"][0] * (d["D"] if d["D"].dim() == 2 else d["D"][:, None])
+    wfin = torch.exp(sums[:, -1])[:, None, None] * d["initial_states"][0] + torch.einsum("kn,hk,khp->hpn", d["B"][0, :, 0], decay[:, -1], d["x"][0])
+    run(inp, 256, "rising", (want[None].float(), wfin[None].float()))
+
+
+@pytest.mark.parametrize("P,N,H,Q,L", [(64, 64, 2, 256, 129), (128, 128, 1, 128, 257), (65, 66, 2, 64, 65), (7, 130, 1, 100, 101), (64, 64, 1, 1024, 1100), (1, 1, 1, 1, 3)])
+def test_fp32_shapes(P, N, H, Q, L):
+    run(make(910 + P + N, 2, L, H, P, 1, N, torch.float32, has_z=L % 2 == 0, D_hdim=P % 2 == 0, init=True), Q, f"P{P} N{N} Q{Q} L{L}")
+
+
+@pytest.mark.parametrize("name", ["x", "B", "C"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_fp32_values_that_cannot_be_cut(name, value):
+    """They reach what they reach through nonzero factors, as infinities or NaNs, and leave everything else as exact as it was."""
+    t, e = 140, 9
+    inp = make(920, 1, 300, 2, 64, 1, 64, torch.float32, has_z=False, init=True)
+    kw = dict(dt_softplus=True)
+    want, wfin = oracle.ssd_chunk_scan(inp["x"], inp["dt"], inp["A"], inp["B"], inp["C"], 256, inp["D"], None, inp["dt_bias"], inp["initial_states"], **kw)
+    inp[name][0, t, 0, e] = value
+    c = {k: _c(v) for k, v in inp.items()}
+    out, fin = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 256, D=c["D"], dt_bias=c["dt_bias"], initial_states=c["initial_states"], return_final_states=True, **kw)
+    out, fin = out.cpu(), fin.cpu()
+    assert rel(out[0, :t], want[0, :t]) <= F32                               # nothing goes back in time
+    if name == "x":                                                          # one column of one head
+        assert torch.isfinite(out[0, :, 1]).all() and rel(out[0, :, 1], want[0, :, 1]) <= F32
+        keep = torch.arange(64) != e
+        assert rel(out[0, :, 0, keep], want[0, :, 0, keep]) <= F32 and rel(fin[0, 0, keep], wfin[0, 0, keep]) <= F32
+        if value != 3.4e38:
+            assert not torch.isfinite(out[0, t, 0, e])
+    if name == "B":                                                          # one state of every head
+        keep = torch.arange(64) != e
+        assert rel(fin[..., keep], wfin[..., keep]) <= F32
+    if name == "C":                                                          # one step
+        later = torch.arange(300) != t
+        assert rel(out[0, later], want[0, later]) <= F32 and rel(fin, wfin) <= F32

@@ -144,6 +144,8 @@ __global__ void __launch_bounds__(256) ssd_state_passing_kernel(const mb200_ssd_
     const int h = blockIdx.y, b = blockIdx.z;
     const int Q = a.chunk_size;
     const float *dA_last = dAb + ((int64_t)b * a.nheads + h) * nchunks * Q + (Q - 1);
+    pdl_trigger();
+    pdl_wait();
     if (e < PN) {
         float run[VEC];
 #pragma unroll
@@ -248,6 +250,7 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
     // rules that kernel out (which both halves can tell: they are handed the same C) does it.
     const bool tc_cb = ssd_tc_local_eligible(a) && ssd_tc_cb_eligible(a);
     const bool cb_early = has_local && !has_out && (a.phases & MB200_SSD_PHASE_CB) && a.C && !tc_cb;
+    const bool cb_first = cb_early || (has_local && has_out && !tc_out);       // formed beside the chunk states
     const bool cb_ready = !has_local && has_out && (a.phases & MB200_SSD_PHASE_CB_READY) && !tc_cb;
     void *prev16 = tc_out ? static_cast<void *>(base + lay.off_prev16) : nullptr;
     if (!has_local) {      // the cumsum kernel of the LOCAL stages clears the word otherwise
@@ -263,9 +266,9 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
     const bool local_streamed = !has_local && fused_states && !tc_out;
     auto state_passing = [&](const mb200_ssd_args &p, bool write_prev, void *to16) {
         if (PN % 4 == 0)
-            ssd_state_passing_kernel<4><<<dim3((unsigned)((PN / 4 + 255) / 256), a.nheads, a.batch), 256, 0, stream>>>(p, dAb, states, nc, write_prev, to16);
+            launch_dependent(ssd_state_passing_kernel<4>, dim3((unsigned)((PN / 4 + 255) / 256), a.nheads, a.batch), 256, 0, stream, p, dAb, states, nc, write_prev, to16);
         else
-            ssd_state_passing_kernel<1><<<dim3((unsigned)((PN + 255) / 256), a.nheads, a.batch), 256, 0, stream>>>(p, dAb, states, nc, write_prev, to16);
+            launch_dependent(ssd_state_passing_kernel<1>, dim3((unsigned)((PN + 255) / 256), a.nheads, a.batch), 256, 0, stream, p, dAb, states, nc, write_prev, to16);
     };
     if (has_local) {
         const size_t cs_smem = sizeof(float) * Q * 33;
@@ -287,14 +290,12 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
         const cudaError_t ce = a.dt_dtype == MB200_F32 ? cumsum(float{}) : a.dt_dtype == MB200_BF16 ? cumsum(__nv_bfloat16{}) : cumsum(__half{});
         if (ce != cudaSuccess) return fail(MB200_ERR_LAUNCH, "ssd chunk_cumsum: shared memory opt-in: %s", cudaGetErrorString(ce));
         MB200_CHECK_LAUNCH("ssd chunk_cumsum");
-        if (cb_early)
-            if (int rc = ssd_split_cb(a, lay, stream)) return rc;
+        if (!tc_loc || cb_first)
+            if (int rc = ssd_split_first(a, lay, !tc_loc, cb_first, stream)) return rc;
         if (fused_states) {
             if (int rc = ssd_tc_state_stream(a, lay, stream)) return rc;
         } else if (tc_loc) {
             if (int rc = ssd_tc_chunk_state(a, lay, stream)) return rc;
-        } else {
-            if (int rc = ssd_split_states(a, lay, stream)) return rc;
         }
         if (!fused_states && !has_out && (a.final_states || a.range_decay)) {
             // range summary only: fold the local chunk states from a zero state, leave the slots as they are
@@ -326,8 +327,8 @@ int run_ssd(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
                                                       : ssd_split_varlen(a, lay, fused_states ? SsdStates::np16 : SsdStates::pn16, stream))
                     return rc;
         } else {
-            if (!cb_ready)
-                if (int rc = ssd_split_cb(a, lay, stream)) return rc;
+            if (!cb_ready && !cb_first)
+                if (int rc = ssd_split_first(a, lay, false, true, stream)) return rc;
             if (int rc = ssd_split_scan(a, lay, stream)) return rc;
             if (varlen)
                 if (int rc = ssd_split_varlen(a, lay, SsdStates::pn32, stream)) return rc;

@@ -78,12 +78,10 @@ int ssd_tc_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool states_np
 // phase left (H_c += prefix_decay_c * S_in) and forms the range's end state.
 int ssd_tc_apply_incoming(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
 
-// The general stages for 16-bit inputs (ssd_split.cu): chunk states, C.B^T, chunk outputs.  They read and write what the general stages
-// for fp32 do.  And the end states of packed sequences, from entering states of any form: fp32 or 16-bit in [p][n] order, or the 16-bit
-// [n][p] tiles of the state stream.
+// The general stages (ssd_split.cu): chunk states and C.B^T, either or both; chunk outputs.  And the end states of packed sequences, from
+// entering states of any form: fp32 or 16-bit in [p][n] order, or the 16-bit [n][p] tiles of the state stream.
 enum class SsdStates { pn32, pn16, np16 };
-int ssd_split_states(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
-int ssd_split_cb(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
+int ssd_split_first(const mb200_ssd_args &a, const SsdScratch &lay, bool with_states, bool with_cb, cudaStream_t stream);
 int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream);
 int ssd_split_varlen(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates entering, cudaStream_t stream);
 

@@ -210,24 +210,24 @@ constexpr uint32_t kTail = 16;                          // barrier and tensor-me
 __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { return a.seq_idx ? a.seq_idx[(int64_t)b * a.seqlen + t] : 0; }
 
 // ====================================================================================== chunk states
-// S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_end - dA_k, 0)) dt_k; grid (64-column tiles of P x 128-state tiles, (batch, chunk)
-// or sequence, heads).  PACKED: the state after the last token of a packed sequence -- its steps in the chunk of that token, plus the state
+// S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_end - dA_k, 0)) dt_k; a CTA has a tile of 64 columns of P x 128 states of a (batch, chunk) or
+// sequence and a head.  PACKED: the state after the last token of a packed sequence -- its steps in the chunk of that token, plus the state
 // entering the chunk if the sequence began earlier.
 template <typename T> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kParts * kTileB + kTail;
 template <typename T, bool PACKED>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_state_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
-                                                                      float *states, int nchunks, int *status)
+__device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_or_seq, int h, const mb200_ssd_args &a, const float *dtb, const float *dAb, const void *entering,
+                                            SsdStates form, float *states, int nchunks, int *status)
 {
-    extern __shared__ __align__(1024) uint8_t smem[];
     const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesN = (N + 127) / 128;
-    const int p0 = (blockIdx.x / tilesN) * 64, n0 = (blockIdx.x % tilesN) * 128, h = blockIdx.z, g = h / (a.nheads / a.ngroups);
+    const int p0 = (tile / tilesN) * 64, n0 = (tile % tilesN) * 128, g = h / (a.nheads / a.ngroups);
     Tile t;
     t.open(smem, kInParts<T> * kTileA, kParts * kTileB, 128, status, kStSplitState);
+    pdl_trigger();
     pdl_wait();
     int b, c, k0, k1;                               // my steps of the chunk: [k0, k1)
     bool carry = false;
     if constexpr (PACKED) {
-        const int start = a.cu_seqlens[blockIdx.y], end = a.cu_seqlens[blockIdx.y + 1];
+        const int start = a.cu_seqlens[chunk_or_seq], end = a.cu_seqlens[chunk_or_seq + 1];
         const bool empty = end <= start || end > a.seqlen || start < 0;
         b = 0;
         c = empty ? 0 : (end - 1) / Q;
@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_st
         k1 = empty ? 0 : end - c * Q;
         carry = !empty && start < c * Q;
     } else {
-        b = blockIdx.y / nchunks;
-        c = blockIdx.y % nchunks;
+        b = chunk_or_seq / nchunks;
+        c = chunk_or_seq % nchunks;
         k0 = 0;
         k1 = min(Q, a.seqlen - c * Q);
     }
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_st
     constexpr uint32_t idesc = instr_desc_f16(128, 64, 1, 1, 1);
     uint32_t skipped = 0;                           // tiles left for the FMAs
 #pragma unroll 1
-    for (int k = k0, tile = 0; k < k1; k += 64, ++tile) {
+    for (int k = k0, i64 = 0; k < k1; k += 64, ++i64) {
         t.drain();
         bool bad = false;
 #pragma unroll
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_st
             // all, end states were 8 to 15 % further from 64 bits than the fp32 kernels' in chunks of 128; with two 1 to 2 %)
             const uint32_t acc = warp_uniform(t.tmem);
             multiply(kInParts<T>, kParts, acc, acc + 64, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, 16, 1024), 128, idesc, !first);
-        })) skipped |= 1u << tile;
+        })) skipped |= 1u << i64;
         if (k + 64 < k1) fetch(k + 64);
     }
     t.drain();
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_st
         }
     }
     if (n < N) {
-        const int64_t slot = PACKED ? (int64_t)blockIdx.y * a.nheads + h : ((int64_t)b * nchunks + c) * a.nheads + h;
+        const int64_t slot = PACKED ? (int64_t)chunk_or_seq * a.nheads + h : ((int64_t)b * nchunks + c) * a.nheads + h;
         float *S = states + slot * P * N + n;
         const float decay = carry ? __expf(dA_end) : 0.f;
         const T *tile = reinterpret_cast<const T *>(in);
@@ -358,20 +358,20 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_st
 
 // ====================================================================================== C.B^T
 // CB[m,k] = C_m . B_k, fp32, in tiles of 128 x 64 that reach the diagonal or lie below it; pairs of different sequences get 0.  The
-// products of two inputs are exact in the input type.  grid (row blocks x column tiles, batch x chunks, groups)
+// products of two inputs are exact in the input type.  A CTA has one tile of a (batch, chunk) and a group.
 template <typename T> constexpr int kCbParts = sizeof(T) == 2 ? 1 : kParts;
 template <typename T> constexpr uint32_t kCbSmem = kCbParts<T> * (kTileA + kTileB) + kTail;
 template <typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 2) ssd_split_cb_kernel(const mb200_ssd_args a, float *cb, int nchunks, int *status)
+__device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int g, const mb200_ssd_args &a, float *cb, int nchunks, int *status)
 {
-    extern __shared__ __align__(1024) uint8_t smem[];
     const int Q = a.chunk_size, N = a.dstate, tilesK = (Q + 63) / 64;
-    const int m0 = (blockIdx.x / tilesK) * 128, k0 = (blockIdx.x % tilesK) * 64;
-    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, g = blockIdx.z, len = min(Q, a.seqlen - c * Q);
+    const int m0 = (tile / tilesK) * 128, k0 = (tile % tilesK) * 64;
+    const int b = chunk / nchunks, c = chunk % nchunks, len = min(Q, a.seqlen - c * Q);
     if (k0 >= m0 + 128 || m0 >= len || k0 >= len) return;
     Tile t;
     constexpr int kSums = sizeof(T) == 2 ? 64 : 128;     // columns of tensor memory: fp32's small products have a sum of their own, as in the chunk states
     t.open(smem, kCbParts<T> * kTileA, kCbParts<T> * kTileB, kSums, status, kStSplitCb);
+    pdl_trigger();
     pdl_wait();
     const int64_t t0 = (int64_t)c * Q;
     const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (t0 + m0) * a.C_stride[1] + (int64_t)g * a.C_stride[2];
@@ -457,6 +457,26 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 2) ssd_split_cb
         }
     }
     t.close(kSums);
+}
+
+// Both in one launch: the chunk states need what the launch before formed, C.B^T nothing, and its short CTAs fill the last wave of the other's.
+// (states of PACKED sequences have a launch of their own, after the recurrence)
+template <typename T, bool PACKED>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_first_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
+                                                                                           float *states, float *cb, int state_ctas, int state_tiles, int cb_tiles, int nchunks, int *status)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    int i = blockIdx.x;
+    if (i < state_ctas) {
+        const int rows = PACKED ? a.num_seqs : a.batch * nchunks, tile = i % state_tiles;
+        i /= state_tiles;
+        split_state<T, PACKED>(smem, tile, i % rows, i / rows, a, dtb, dAb, entering, form, states, nchunks, status);
+    } else if constexpr (!PACKED) {
+        i -= state_ctas;
+        const int rows = a.batch * nchunks, tile = i % cb_tiles;
+        i /= cb_tiles;
+        split_cb<T>(smem, tile, i % rows, i / rows, a, cb, nchunks, status);
+    }
 }
 
 // ====================================================================================== chunk outputs
@@ -545,6 +565,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     if (m0 >= len) return;
     Tile t;
     t.open(smem, kScan16A<T>, kScan16B<T>, 128, status, kStSplitScan);
+    pdl_trigger();
     pdl_wait();
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
     const float *dAc = dAb + row, *dtc = dtb + row;
@@ -840,6 +861,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    pdl_trigger();
     pdl_wait();
     const uint32_t tmem = *slot, tiles = smem_u32(smem);
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
@@ -1250,38 +1272,33 @@ struct Buffers {
 // f(element type of the call)
 template <class F> int with_type(const mb200_ssd_args &a, F f) { return a.io_dtype == MB200_BF16 ? f(__nv_bfloat16{}) : a.io_dtype == MB200_F16 ? f(__half{}) : f(float{}); }
 
-template <bool PACKED> int run_states(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates form, cudaStream_t stream)
+template <bool PACKED> int run_first(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates form, bool with_states, bool with_cb, cudaStream_t stream)
 {
     return with_type(a, [&](auto tag) -> int {
         using T = decltype(tag);
         const Buffers s(a, lay);
         const void *entering = static_cast<const char *>(a.scratch) + (form == SsdStates::pn32 ? lay.off_states : lay.off_prev16);
-        const unsigned tiles = (unsigned)((a.headdim + 63) / 64 * ((a.dstate + 127) / 128));
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_state_kernel<T, PACKED>), (int)kStateSmem<T>, a.device);
-        launch_dependent(ssd_split_state_kernel<T, PACKED>, dim3(tiles, PACKED ? a.num_seqs : a.batch * lay.nchunks, a.nheads), kThreads, kStateSmem<T>, stream, a, s.dt, s.dA,
-                         entering, form, PACKED ? a.varlen_states : s.states, lay.nchunks, s.status);
-        MB200_CHECK_LAUNCH("ssd states (split products)");
+        const int state_tiles = (a.headdim + 63) / 64 * ((a.dstate + 127) / 128), cb_tiles = (a.chunk_size + 127) / 128 * ((a.chunk_size + 63) / 64);
+        const int64_t rows = PACKED ? a.num_seqs : (int64_t)a.batch * lay.nchunks, state_ctas = with_states ? rows * state_tiles * a.nheads : 0,
+                      ctas = state_ctas + (with_cb ? rows * cb_tiles * a.ngroups : 0);
+        if (ctas == 0) return MB200_OK;
+        if (ctas > INT32_MAX) return fail(MB200_ERR_BAD_ARG, "ssd: too many chunks and heads");
+        constexpr uint32_t smem = kStateSmem<T> > kCbSmem<T> ? kStateSmem<T> : kCbSmem<T>;
+        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_first_kernel<T, PACKED>), (int)smem, a.device);
+        launch_dependent(ssd_split_first_kernel<T, PACKED>, dim3((unsigned)ctas), kThreads, smem, stream, a, s.dt, s.dA, entering, form, PACKED ? a.varlen_states : s.states, s.cb,
+                         (int)state_ctas, state_tiles, cb_tiles, lay.nchunks, s.status);
+        MB200_CHECK_LAUNCH("ssd states and C.B^T (split products)");
         return MB200_OK;
     });
 }
 
 }  // namespace
 
-int ssd_split_states(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream) { return run_states<false>(a, lay, SsdStates::pn32, stream); }
-int ssd_split_varlen(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates entering, cudaStream_t stream) { return run_states<true>(a, lay, entering, stream); }
-
-int ssd_split_cb(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
+int ssd_split_first(const mb200_ssd_args &a, const SsdScratch &lay, bool with_states, bool with_cb, cudaStream_t stream)
 {
-    return with_type(a, [&](auto tag) -> int {
-        using T = decltype(tag);
-        const Buffers s(a, lay);
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_cb_kernel<T>), (int)kCbSmem<T>, a.device);
-        const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.chunk_size + 63) / 64));
-        launch_dependent(ssd_split_cb_kernel<T>, dim3(tiles, a.batch * lay.nchunks, a.ngroups), kThreads, kCbSmem<T>, stream, a, s.cb, lay.nchunks, s.status);
-        MB200_CHECK_LAUNCH("ssd C.B^T (split products)");
-        return MB200_OK;
-    });
+    return run_first<false>(a, lay, SsdStates::pn32, with_states, with_cb, stream);
 }
+int ssd_split_varlen(const mb200_ssd_args &a, const SsdScratch &lay, SsdStates entering, cudaStream_t stream) { return run_first<true>(a, lay, entering, true, false, stream); }
 
 int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t stream)
 {

@@ -57,7 +57,11 @@ template <> __device__ __forceinline__ float from_float<float>(float v) { return
 template <> __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// Programmatic dependent launch: lets the next launch of the stream start its set-up / waits for the launches before this one.
+// Programmatic dependent launch: lets the next launch of the stream start its set-up / waits for the launches before this one.  A kernel
+// that takes a caller's tensors waits first and triggers then: what runs after its trigger, even before it has waited itself, finds
+// everything that the caller queued before the call complete.  Not for a grid of long CTAs that fills the GPU once (the scan of many
+// channels and its gradients): CTAs that come as the last launch's leave are spread unevenly (gradients of 5 x 5120 channels of 8 states,
+// 1212 steps: 2.53 for 2.29 ms).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A launch that may start before the one ahead of it in the stream has ended; the kernel calls pdl_wait before it reads what that wrote,

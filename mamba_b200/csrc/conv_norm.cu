@@ -108,6 +108,7 @@ constexpr int kConvSteps = 16;      // output steps per thread of the channels-c
 template <typename T, int W, bool SID, bool ACT>
 __global__ void __launch_bounds__(128, 3) conv1d_cl_kernel(const mb200_conv1d_args a)
 {
+    pdl_wait();
     pdl_trigger();
     constexpr int PB = 16, VEC = PB / sizeof(T), NP = VEC / 2;
     constexpr int TT = kConvSteps, H = W - 1;       // H rows of history before the first output step
@@ -250,6 +251,8 @@ __global__ void __launch_bounds__(128, 3) conv1d_cl_kernel(const mb200_conv1d_ar
 template <typename T, int W, bool ACT>
 __global__ void __launch_bounds__(256) conv1d_rows_kernel(const mb200_conv1d_args a, const int warps_per_row)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int VEC = 16 / sizeof(T), H = W - 1, NI = VEC + H;       // inputs of a granule of outputs
     const int64_t wid = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int c = (int)(wid / warps_per_row), lane = threadIdx.x & 31, b = blockIdx.y;
@@ -323,6 +326,8 @@ constexpr int kRun = 8;
 template <typename T>
 __global__ void __launch_bounds__(256) conv1d_any_kernel(const mb200_conv1d_args a)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int K = kMaxWidth;
     const int runs = (a.seqlen + kRun - 1) / kRun;
     const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -373,6 +378,8 @@ __global__ void __launch_bounds__(256) conv1d_any_kernel(const mb200_conv1d_args
 template <typename T>
 __global__ void __launch_bounds__(256) conv1d_update_kernel(const mb200_conv1d_update_args a)
 {
+    pdl_wait();
+    pdl_trigger();
     const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (idx >= (int64_t)a.batch * a.dim) return;
     const int b = (int)(idx / a.dim), c = (int)(idx % a.dim);
@@ -399,6 +406,7 @@ __global__ void __launch_bounds__(256, 3) rmsnorm_gated_kernel(const mb200_rmsno
     constexpr int VEC = 16 / sizeof(T);
     __shared__ float red[8];
     pdl_wait();
+    pdl_trigger();
     const int64_t rowi = blockIdx.x;
     const int g = blockIdx.y;
     const int G = a.group_size;
@@ -469,6 +477,8 @@ __global__ void __launch_bounds__(256, 3) rmsnorm_gated_kernel(const mb200_rmsno
 template <typename T>
 __global__ void __launch_bounds__(32) rmsnorm_gated_any_kernel(const mb200_rmsnorm_args a)
 {
+    pdl_wait();
+    pdl_trigger();
     const int64_t rowi = blockIdx.x;
     const int g = blockIdx.y, G = a.group_size, lane = threadIdx.x;
     const T *x = static_cast<const T *>(a.x) + rowi * a.x_stride + (int64_t)g * G;
@@ -516,11 +526,11 @@ int launch_conv1d(const mb200_conv1d_args &a, cudaStream_t stream)
         auto go = [&](auto w_tag) {
             constexpr int W = decltype(w_tag)::value;
             if (a.seq_idx) {
-                if (a.activation) conv1d_cl_kernel<T, W, true, true><<<grid, 128, 0, stream>>>(a);
-                else conv1d_cl_kernel<T, W, true, false><<<grid, 128, 0, stream>>>(a);
+                if (a.activation) launch_dependent(conv1d_cl_kernel<T, W, true, true>, grid, 128, 0, stream, a);
+                else launch_dependent(conv1d_cl_kernel<T, W, true, false>, grid, 128, 0, stream, a);
             } else {
-                if (a.activation) conv1d_cl_kernel<T, W, false, true><<<grid, 128, 0, stream>>>(a);
-                else conv1d_cl_kernel<T, W, false, false><<<grid, 128, 0, stream>>>(a);
+                if (a.activation) launch_dependent(conv1d_cl_kernel<T, W, false, true>, grid, 128, 0, stream, a);
+                else launch_dependent(conv1d_cl_kernel<T, W, false, false>, grid, 128, 0, stream, a);
             }
         };
         if (a.width == 4) go(std::integral_constant<int, 4>{});
@@ -531,15 +541,15 @@ int launch_conv1d(const mb200_conv1d_args &a, cudaStream_t stream)
         const dim3 grid((unsigned)(((int64_t)a.dim * per_row + 7) / 8), a.batch);
         auto go = [&](auto w_tag) {
             constexpr int W = decltype(w_tag)::value;
-            if (a.activation) conv1d_rows_kernel<T, W, true><<<grid, 256, 0, stream>>>(a, per_row);
-            else conv1d_rows_kernel<T, W, false><<<grid, 256, 0, stream>>>(a, per_row);
+            if (a.activation) launch_dependent(conv1d_rows_kernel<T, W, true>, grid, 256, 0, stream, a, per_row);
+            else launch_dependent(conv1d_rows_kernel<T, W, false>, grid, 256, 0, stream, a, per_row);
         };
         if (a.width == 4) go(std::integral_constant<int, 4>{});
         else if (a.width == 3) go(std::integral_constant<int, 3>{});
         else go(std::integral_constant<int, 2>{});
     } else {
         const int64_t work = (int64_t)a.dim * ((a.seqlen + kRun - 1) / kRun);
-        conv1d_any_kernel<T><<<dim3((unsigned)((work + 255) / 256), a.batch), 256, 0, stream>>>(a);
+        launch_dependent(conv1d_any_kernel<T>, dim3((unsigned)((work + 255) / 256), a.batch), 256, 0, stream, a);
     }
     return MB200_OK;
 }
@@ -553,7 +563,7 @@ int launch_rmsnorm(const mb200_rmsnorm_args &a, cudaStream_t stream)
                         a.out_stride % VEC == 0 && (!a.z || a.z_stride % VEC == 0) && G <= 256 * 4 * VEC;
     dim3 grid((unsigned)a.nrows, ngroups);
     if (!vec_ok) {
-        rmsnorm_gated_any_kernel<T><<<grid, 32, 0, stream>>>(a);
+        launch_dependent(rmsnorm_gated_any_kernel<T>, grid, 32, 0, stream, a);
         return MB200_OK;
     }
     const int packets = G / VEC;
@@ -613,9 +623,9 @@ extern "C" int mb200_causal_conv1d_update(const mb200_conv1d_update_args *args, 
     if (int rc = enter_device(a.device)) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     const unsigned blocks = (unsigned)(((int64_t)a.batch * a.dim + 255) / 256);
-    if (a.io_dtype == MB200_F32) conv1d_update_kernel<float><<<blocks, 256, 0, stream>>>(a);
-    else if (a.io_dtype == MB200_BF16) conv1d_update_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(a);
-    else conv1d_update_kernel<__half><<<blocks, 256, 0, stream>>>(a);
+    if (a.io_dtype == MB200_F32) launch_dependent(conv1d_update_kernel<float>, blocks, 256, 0, stream, a);
+    else if (a.io_dtype == MB200_BF16) launch_dependent(conv1d_update_kernel<__nv_bfloat16>, blocks, 256, 0, stream, a);
+    else launch_dependent(conv1d_update_kernel<__half>, blocks, 256, 0, stream, a);
     MB200_CHECK_LAUNCH("causal_conv1d_update");
     return MB200_OK;
 }

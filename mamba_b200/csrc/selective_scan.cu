@@ -308,6 +308,8 @@ template <int CH> struct FewSmem {
 template <typename T, int CH>
 __global__ void __launch_bounds__(CH * 128) scan_few_kernel(const mb200_scan_args a, const int vec_flags)
 {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ __align__(16) uint8_t few_raw[];
     FewSmem<CH> &sm = *reinterpret_cast<FewSmem<CH> *>(few_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cl = warp >> 2, q = warp & 3;
@@ -1185,8 +1187,7 @@ int launch_stream(const mb200_scan_args &a, cudaStream_t stream)
                 constexpr int threads = 32 * (SW + (SPLIT ? 2 : 1));
                 constexpr size_t smem = sizeof(StreamSmem<T, NS, SW, SPLIT, TMA>);
                 auto kernel = scan_stream_kernel<T, NS, SUM, SW, SPLIT, TMA>;
-                if (split.h0) launch_dependent(kernel, grid, threads, smem, stream, a, maps, split);        // after the fold
-                else kernel<<<grid, threads, smem, stream>>>(a, maps, split);
+                launch_dependent_if(split.h0 != nullptr, kernel, grid, threads, smem, stream, a, maps, split);        // (after the fold)
             };
             // fp32 rows fetched by the lanes take two granules per hand-off, of which shared memory holds three: a single scalar warp would
             // wait for the last it asked for.  Rows off their 16-byte boundaries need twice the sectors, and the six-warp layout whatever
@@ -1252,7 +1253,7 @@ int launch_scan(const mb200_scan_args &a, cudaStream_t stream)
             constexpr int CH = decltype(ch_c)::value;
             const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void *>(&scan_few_kernel<T, CH>), (int)sizeof(FewSmem<CH>), a.device);
             if (e != cudaSuccess) return fail(MB200_ERR_LAUNCH, "selective_scan: shared memory opt-in (%zu B): %s", sizeof(FewSmem<CH>), cudaGetErrorString(e));
-            scan_few_kernel<T, CH><<<dim3(a.ngroups * ((per_group + CH - 1) / CH), a.batch), CH * 128, sizeof(FewSmem<CH>), stream>>>(a, vec_flags);
+            launch_dependent(scan_few_kernel<T, CH>, dim3(a.ngroups * ((per_group + CH - 1) / CH), a.batch), CH * 128, sizeof(FewSmem<CH>), stream, a, vec_flags);
             return (int)MB200_OK;
         };
         return (int64_t)a.batch * a.dim > 2 * 148 ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 2>{});

@@ -1066,6 +1066,8 @@ struct ClearList {
 };
 __global__ void __launch_bounds__(256) scan_bwd_clear_kernel(const ClearList l)
 {
+    pdl_wait();
+    pdl_trigger();
     float *p = l.p[blockIdx.y];
     const size_t n = l.n[blockIdx.y], first = (size_t)blockIdx.x * 256 + threadIdx.x, step = (size_t)gridDim.x * 256;
     const size_t packets = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? n / 4 : 0;
@@ -1250,7 +1252,7 @@ extern "C" int mb200_selective_scan_bwd(const mb200_scan_bwd_args *args, void *s
     } else {
         const size_t pn = sizeof(float) * (size_t)a.dim;
         const ClearList list = {{a.dA, a.dB, a.dC, a.dD, a.ddelta_bias}, {wn / 4, a.dB ? bn / 4 : 0, a.dC ? cn / 4 : 0, a.dD ? pn / 4 : 0, a.ddelta_bias ? pn / 4 : 0}};
-        scan_bwd_clear_kernel<<<dim3(148, 5), 256, 0, stream>>>(list);
+        launch_dependent(scan_bwd_clear_kernel, dim3(148, 5), 256, 0, stream, list);
         MB200_CHECK_LAUNCH("selective_scan_bwd: clearing the accumulators");
     }
     if (a.batch == 0 || a.seqlen == 0) return MB200_OK;

@@ -65,6 +65,8 @@ __device__ __forceinline__ void load_row(const void *p, int dtype, int64_t i, in
 template <typename StateT, int LPR, int NC, bool TIED>
 __global__ void __launch_bounds__(kThreads) ssu_packet_kernel(const mb200_ssu_args a, const int row_tile)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int VEC = 16 / sizeof(StateT);
     constexpr int GROUPS = kThreads / LPR;
     const int b = blockIdx.y, h = blockIdx.z;
@@ -231,6 +233,8 @@ __global__ void __launch_bounds__(kThreads) ssu_packet_kernel(const mb200_ssu_ar
 // One warp per state row, every access scalar and fully strided.
 __global__ void __launch_bounds__(128) ssu_general_kernel(const mb200_ssu_args a)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.y, h = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = blockIdx.x * 4 + warp;
@@ -280,9 +284,9 @@ int launch_packet(const mb200_ssu_args &a, bool tied, cudaStream_t stream)
     if (row_tile > a.dim) row_tile = a.dim;
     dim3 grid((a.dim + row_tile - 1) / row_tile, a.batch, a.nheads);
     if (tied)
-        ssu_packet_kernel<StateT, LPR, NC, true><<<grid, kThreads, 0, stream>>>(a, row_tile);
+        launch_dependent(ssu_packet_kernel<StateT, LPR, NC, true>, grid, kThreads, 0, stream, a, row_tile);
     else
-        ssu_packet_kernel<StateT, LPR, NC, false><<<grid, kThreads, 0, stream>>>(a, row_tile);
+        launch_dependent(ssu_packet_kernel<StateT, LPR, NC, false>, grid, kThreads, 0, stream, a, row_tile);
     return MB200_OK;
 }
 
@@ -338,7 +342,7 @@ extern "C" int mb200_selective_state_update(const mb200_ssu_args *args, void *st
     }
     if (!done) {
         dim3 grid((a.dim + 3) / 4, a.batch, a.nheads);
-        ssu_general_kernel<<<grid, 128, 0, stream>>>(a);
+        launch_dependent(ssu_general_kernel, grid, 128, 0, stream, a);
     }
     MB200_CHECK_LAUNCH("selective_state_update");
     return MB200_OK;

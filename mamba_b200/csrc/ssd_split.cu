@@ -222,7 +222,6 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
     const int p0 = (tile / tilesN) * 64, n0 = (tile % tilesN) * 128, g = h / (a.nheads / a.ngroups);
     Tile t;
     t.open(smem, kInParts<T> * kTileA, kParts * kTileB, 128, status, kStSplitState);
-    pdl_trigger();
     pdl_wait();
     int b, c, k0, k1;                               // my steps of the chunk: [k0, k1)
     bool carry = false;
@@ -371,7 +370,6 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
     Tile t;
     constexpr int kSums = sizeof(T) == 2 ? 64 : 128;     // columns of tensor memory: fp32's small products have a sum of their own, as in the chunk states
     t.open(smem, kCbParts<T> * kTileA, kCbParts<T> * kTileB, kSums, status, kStSplitCb);
-    pdl_trigger();
     pdl_wait();
     const int64_t t0 = (int64_t)c * Q;
     const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (t0 + m0) * a.C_stride[1] + (int64_t)g * a.C_stride[2];
@@ -461,6 +459,8 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
 
 // Both in one launch: the chunk states need what the launch before formed, C.B^T nothing, and its short CTAs fill the last wave of the other's.
 // (states of PACKED sequences have a launch of their own, after the recurrence)
+// None of these kernels lets the next one in early: 45 us for 48, 102 for 106 where they do not (2 x 2048 steps of 8 fp32 heads, 2 x 1500
+// of 48 half-precision heads of 64 x 64).
 template <typename T, bool PACKED>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_first_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
                                                                                            float *states, float *cb, int state_ctas, int state_tiles, int cb_tiles, int nchunks, int *status)
@@ -565,7 +565,6 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     if (m0 >= len) return;
     Tile t;
     t.open(smem, kScan16A<T>, kScan16B<T>, 128, status, kStSplitScan);
-    pdl_trigger();
     pdl_wait();
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
     const float *dAc = dAb + row, *dtc = dtb + row;
@@ -861,7 +860,6 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    pdl_trigger();
     pdl_wait();
     const uint32_t tmem = *slot, tiles = smem_u32(smem);
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;

@@ -13,6 +13,7 @@
 // cut them and store them.  The tensor core is idle most of the time; what bounds these kernels is that element-wise work and the latencies
 // between it, which two to four CTAs per SM share.  Rows are read with plain loads, so any stride and alignment goes.
 // 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states 28, C.B^T 5, outputs 69; fp32 FMAs took 318 for the call.
+#include <algorithm>
 #include <type_traits>
 
 #include "ssd_common.cuh"
@@ -137,7 +138,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int chunk) { return row * 128
 // The products of one 64-step tile, parts against parts: D += A B, those of the first parts to `d`, the others to `rest`; of `na` parts of A
 // and `nb` of B, without those below 2^-24.  Called by a whole warp.
 __device__ __forceinline__ void multiply(int na, int nb, uint32_t d, uint32_t rest, uint64_t a, uint32_t step_a, uint64_t b, uint32_t step_b, uint32_t idesc,
-                                         bool accumulate)
+                                         bool accumulate, uint32_t part_b = kTileB)
 {
     if (elect_one()) {
         mma_steps_ss(4, d, a, step_a, b, step_b, idesc, accumulate);
@@ -146,7 +147,7 @@ __device__ __forceinline__ void multiply(int na, int nb, uint32_t d, uint32_t re
         for (int i = 0; i < na; ++i)
 #pragma unroll 1
             for (int j = i == 0 ? 1 : 0; j < nb && i + j < max(na, nb); ++j) {
-                mma_steps_ss(4, rest, a + i * (kTileA / 16), step_a, b + j * (kTileB / 16), step_b, idesc, more);
+                mma_steps_ss(4, rest, a + i * (kTileA / 16), step_a, b + j * (part_b / 16), step_b, idesc, more);
                 more = true;
             }
     }
@@ -210,18 +211,23 @@ constexpr uint32_t kTail = 16;                          // barrier and tensor-me
 __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { return a.seq_idx ? a.seq_idx[(int64_t)b * a.seqlen + t] : 0; }
 
 // ====================================================================================== chunk states
-// S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_end - dA_k, 0)) dt_k; a CTA has a tile of 64 columns of P x 128 states of a (batch, chunk) or
-// sequence and a head.  PACKED: the state after the last token of a packed sequence -- its steps in the chunk of that token, plus the state
-// entering the chunk if the sequence began earlier.
-template <typename T> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kParts * kTileB + kTail;
-template <typename T, bool PACKED>
-__device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_or_seq, int h, const mb200_ssd_args &a, const float *dtb, const float *dAb, const void *entering,
+// S^T[n,p] = sum_k B[k,n] (w_k x[k,p]), w_k = exp(min(dA_end - dA_k, 0)) dt_k.  A unit is 64 columns of a head; a CTA has U units that follow
+// each other in a group, and 128 states, of a (batch, chunk) or sequence.  PACKED: the state after the last token of a packed sequence -- its
+// steps in the chunk of that token, plus the state entering the chunk if the sequence began earlier.
+// Two units share B: fetched, cut, stored and read by the tensor core once.  That pays where B is cut, as soon as single units would not all
+// fit the GPU at once (2 x 1500 steps of 48 half-precision heads of 64 x 64: 29 us with one, 23 with two; 2 x 3000 of 32 fp32 heads of 64 x
+// 128: 48 / 45, C.B^T included); in bf16, whose B is stored as it is, two CTAs per SM lose what it saves (2 x 3000 of 32 heads of 128 x 128:
+// 52 / 57), and so do the short sums of packed sequences (46 / 54).
+template <typename T, int U> constexpr uint32_t kStateB = kParts * U * kTileB;
+template <typename T, int U> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kStateB<T, U> + kTail;
+template <typename T, bool PACKED, int U>
+__device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_or_seq, int g, const mb200_ssd_args &a, const float *dtb, const float *dAb, const void *entering,
                                             SsdStates form, float *states, int nchunks, int *status)
 {
-    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesN = (N + 127) / 128;
-    const int p0 = (tile / tilesN) * 64, n0 = (tile % tilesN) * 128, g = h / (a.nheads / a.ngroups);
+    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesN = (N + 127) / 128, tilesP = (P + 63) / 64, hpg = a.nheads / a.ngroups;
+    const int unit0 = (tile / tilesN) * U, n0 = (tile % tilesN) * 128;
     Tile t;
-    t.open(smem, kInParts<T> * kTileA, kParts * kTileB, 128, status, kStSplitState);
+    t.open(smem, kInParts<T> * kTileA, kStateB<T, U>, 128 * U, status, kStSplitState);
     pdl_wait();
     int b, c, k0, k1;                               // my steps of the chunk: [k0, k1)
     bool carry = false;
@@ -239,36 +245,57 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
         k0 = 0;
         k1 = min(Q, a.seqlen - c * Q);
     }
-    const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
-    const float *dtc = dtb + row, *dAc = dAb + row;
-    const float dA_end = PACKED ? (k1 > 0 ? dAc[k1 - 1] : 0.f) : dAc[Q - 1];
-    const T *x = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2] + p0;
+    const int64_t t0 = (int64_t)c * Q;
+    // of each unit (one past the group's last is the last again, and stores nothing)
+    int h[U], p0[U];
+    const float *dtc[U], *dAc[U];
+    float dA_end[U];
+    const T *x[U];
+    bool vx = true, whole_p = true;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int unit = min(unit0 + u, hpg * tilesP - 1);
+        h[u] = g * hpg + unit / tilesP;
+        p0[u] = unit % tilesP * 64;
+        const int64_t row = (((int64_t)b * a.nheads + h[u]) * nchunks + c) * Q;
+        dtc[u] = dtb + row;
+        dAc[u] = dAb + row;
+        dA_end[u] = PACKED ? (k1 > 0 ? dAc[u][k1 - 1] : 0.f) : dAc[u][Q - 1];
+        x[u] = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + t0 * a.x_stride[1] + (int64_t)h[u] * a.x_stride[2] + p0[u];
+        vx = vx && rows16(x[u], a.x_stride[1]);
+        whole_p = whole_p && P - p0[u] >= 64;
+    }
     const T *B = static_cast<const T *>(a.B) + (int64_t)b * a.B_stride[0] + t0 * a.B_stride[1] + (int64_t)g * a.B_stride[2] + n0;
-    const bool vx = rows16(x, a.x_stride[1]), vB = rows16(B, a.B_stride[1]), wide = N - n0 > 64;
+    const bool vB = rows16(B, a.B_stride[1]), wide = N - n0 > 64;
     const int seq_last = PACKED || k1 == 0 ? 0 : seq_at(a, b, c * Q + k1 - 1);      // only steps of the chunk's last sequence reach its end state
     const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;      // my eight columns; rows r0 and r0 + 32 of a tile
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = n0 + (warp & 3) * 32 + lane, p = p0 + (warp >> 2) * 32;           // my state index and the first of my 32 columns
-    const int64_t hc = (int64_t)c * a.nheads + h;
-    uint4 in[4] = {};                               // my part of an [n][p] tile of entering states: asked for now, needed last
+    // results: my state index; one unit: half of its columns, two: all of one's
+    const int n = n0 + (warp & 3) * 32 + lane, mine = U == 2 ? warp >> 2 : 0;
+    const int my_h = U == 2 && mine ? h[U - 1] : h[0], p = (U == 2 && mine ? p0[U - 1] : p0[0]) + (U == 2 ? 0 : (warp >> 2) * 32);
+    const int64_t hc = (int64_t)c * a.nheads + my_h;
+    uint4 in[4 * U] = {};                           // my part of an [n][p] tile of entering states: asked for now, needed last
     if (sizeof(T) == 2 && PACKED && carry && form == SsdStates::np16 && n < N) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) in[i] = reinterpret_cast<const uint4 *>(static_cast<const T *>(entering) + (hc * N + n) * P + p)[i];
+        for (int i = 0; i < 4 * U; ++i) in[i] = reinterpret_cast<const uint4 *>(static_cast<const T *>(entering) + (hc * N + n) * P + p)[i];
     }
 
-    Raw8<T> xr[2], Br[4];
-    float w[2];
-    const bool whole = vx && vB && P - p0 >= 64 && N - n0 >= (wide ? 128 : 64) && (PACKED || !a.seq_idx);
+    Raw8<T> xr[U][2], Br[4];
+    float w[U][2];
+    const bool whole = vx && vB && whole_p && N - n0 >= (wide ? 128 : 64) && (PACKED || !a.seq_idx);
     auto fetch = [&](int k) {
         if (whole && k + 64 <= k1) {                // no edge, nothing to look at
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int kk = k + r0 + 32 * i;
                 const T *Bk = B + (int64_t)kk * a.B_stride[1] + 8 * c8;
-                xr[i] = load8_whole(x + (int64_t)kk * a.x_stride[1] + 8 * c8);
                 Br[i] = load8_whole(Bk);
                 if (wide) Br[2 + i] = load8_whole(Bk + 64);
-                w[i] = __expf(fminf(dA_end - dAc[kk], 0.f)) * dtc[kk];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    xr[u][i] = load8_whole(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8);
+                    w[u][i] = __expf(fminf(dA_end[u] - dAc[u][kk], 0.f)) * dtc[u][kk];
+                }
             }
             return;
         }
@@ -277,15 +304,18 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             const int kk = k + r0 + 32 * i;
             bool on = kk < k1;
             if (!PACKED && a.seq_idx) on = on && seq_at(a, b, c * Q + kk) == seq_last;
-            xr[i] = load8(x + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, on ? P - p0 - 8 * c8 : 0);
-            w[i] = on ? __expf(fminf(dA_end - dAc[kk], 0.f)) * dtc[kk] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                xr[u][i] = load8(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, on ? P - p0[u] - 8 * c8 : 0);
+                w[u][i] = on ? __expf(fminf(dA_end[u] - dAc[u][kk], 0.f)) * dtc[u][kk] : 0.f;
+            }
             const T *Bk = B + (int64_t)kk * a.B_stride[1] + 8 * c8;
             Br[i] = load8(Bk, vB, kk < k1 ? N - n0 - 8 * c8 : 0);
             if (wide) Br[2 + i] = load8(Bk + 64, vB, kk < k1 ? N - n0 - 64 - 8 * c8 : 0);
         }
     };
     if (k0 < k1) fetch(k0);
-    constexpr uint32_t idesc = instr_desc_f16(128, 64, 1, 1, 1);
+    constexpr uint32_t idesc = instr_desc_f16(128, 64 * U, 1, 1, 1);
     uint32_t skipped = 0;                           // tiles left for the FMAs
 #pragma unroll 1
     for (int k = k0, i64 = 0; k < k1; k += 64, ++i64) {
@@ -294,11 +324,14 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const uint32_t o = sw128(r0 + 32 * i, c8);
-            float v[8];
-            widen8<T>(xr[i], v);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] *= w[i];
-            bad = store_parts<kParts>(t.b + o, kTileB, v) || bad;
+            for (int u = 0; u < U; ++u) {
+                float v[8];
+                widen8<T>(xr[u][i], v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] *= w[u][i];
+                bad = store_parts<kParts>(t.b + u * kTileB + o, U * kTileB, v) || bad;
+            }
             bad = store_input<T>(t.a + o, kTileA, Br[i]) || bad;                // states n0 .. n0 + 63, then the other 64
             if (wide) bad = store_input<T>(t.a + 8192 + o, kTileA, Br[2 + i]) || bad;
         }
@@ -307,52 +340,60 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             // the tensor core adds to a sum with less care than fp32 rounding: the small products have one of their own (with one for
             // all, end states were 8 to 15 % further from 64 bits than the fp32 kernels' in chunks of 128; with two 1 to 2 %)
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kInParts<T>, kParts, acc, acc + 64, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, 16, 1024), 128, idesc, !first);
+            multiply(kInParts<T>, kParts, acc, acc + 64 * U, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, kTileB, 1024), 128, idesc, !first, U * kTileB);
         })) skipped |= 1u << i64;
         if (k + 64 < k1) fetch(k + 64);
     }
     t.drain();
-    float v[32];
+    const bool formed = __all_sync(0xffffffffu, t.ok && t.issued > 0);
+    const bool live = n < N && unit0 + mine < hpg * tilesP;
+    const float *my_dAc = U == 2 && mine ? dAc[U - 1] : dAc[0], *my_dtc = U == 2 && mine ? dtc[U - 1] : dtc[0];
+    const float my_end = U == 2 && mine ? dA_end[U - 1] : dA_end[0], decay = carry ? __expf(my_end) : 0.f;
+    const T *my_x = U == 2 && mine ? x[U - 1] : x[0];
+    const int my_p0 = U == 2 && mine ? p0[U - 1] : p0[0];
+    const int64_t slot = PACKED ? (int64_t)chunk_or_seq * a.nheads + my_h : ((int64_t)b * nchunks + c) * a.nheads + my_h;
+    tc_fence_after_sync();
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = 0.f;
-    if (__all_sync(0xffffffffu, t.ok && t.issued > 0)) {        // tcgen05.ld is warp-collective
-        tc_fence_after_sync();
-        const uint32_t at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32;
-        float rest[32];
-        tmem_ld32(at, v);
-        tmem_ld32(at + 64, rest);
+    for (int half = 0; half < U; ++half) {          // 32 columns each
+        const int pc = p + 32 * half;
+        float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += rest[j];
-    }
-    if (skipped && n < N) {
-#pragma unroll 1
-        for (int k = k0; k < k1; ++k) {
-            if (!((skipped >> (k - k0) / 64) & 1)) continue;
-            if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
-            const float wk = __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
+        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        if (formed) {                               // tcgen05.ld is warp-collective
+            const uint32_t at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + mine * 64 + pc - my_p0;
+            float rest[32];
+            tmem_ld32(at, v);
+            tmem_ld32(at + 64 * U, rest);
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (p + j < P) v[j] = fmaf(to_float(x[(int64_t)k * a.x_stride[1] + p - p0 + j]) * wk, Bn, v[j]);
+            for (int j = 0; j < 32; ++j) v[j] += rest[j];
         }
-    }
-    if (n < N) {
-        const int64_t slot = PACKED ? (int64_t)chunk_or_seq * a.nheads + h : ((int64_t)b * nchunks + c) * a.nheads + h;
+        if (!live) continue;
+        if (skipped) {
+#pragma unroll 1
+            for (int k = k0; k < k1; ++k) {
+                if (!((skipped >> (k - k0) / 64) & 1)) continue;
+                if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
+                const float wk = __expf(fminf(my_end - my_dAc[k], 0.f)) * my_dtc[k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (pc + j < P) v[j] = fmaf(to_float(my_x[(int64_t)k * a.x_stride[1] + pc - my_p0 + j]) * wk, Bn, v[j]);
+            }
+        }
         float *S = states + slot * P * N + n;
-        const float decay = carry ? __expf(dA_end) : 0.f;
-        const T *tile = reinterpret_cast<const T *>(in);
+        const T *tile_in = reinterpret_cast<const T *>(in) + 32 * half;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-            if (p + j >= P) continue;
+            if (pc + j >= P) continue;
             if (PACKED && carry) {
-                const int64_t e = (hc * P + p + j) * N + n;
-                const float was = form == SsdStates::np16 ? to_float(tile[j]) : form == SsdStates::pn16 ? to_float(static_cast<const T *>(entering)[e])
-                                                                                                        : static_cast<const float *>(entering)[e];
+                const int64_t e = (hc * P + pc + j) * N + n;
+                const float was = form == SsdStates::np16 ? to_float(tile_in[j]) : form == SsdStates::pn16 ? to_float(static_cast<const T *>(entering)[e])
+                                                                                                           : static_cast<const float *>(entering)[e];
                 v[j] = fmaf(was, decay, v[j]);
             }
-            S[(int64_t)(p + j) * N] = v[j];
+            S[(int64_t)(pc + j) * N] = v[j];
         }
     }
-    t.close(128);
+    t.close(128 * U);
 }
 
 // ====================================================================================== C.B^T
@@ -461,8 +502,8 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
 // (states of PACKED sequences have a launch of their own, after the recurrence)
 // None of these kernels lets the next one in early: 45 us for 48, 102 for 106 where they do not (2 x 2048 steps of 8 fp32 heads, 2 x 1500
 // of 48 half-precision heads of 64 x 64).
-template <typename T, bool PACKED>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_first_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
+template <typename T, bool PACKED, int U>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 && U == 1 ? 3 : 2) ssd_split_first_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const void *entering, SsdStates form,
                                                                                            float *states, float *cb, int state_ctas, int state_tiles, int cb_tiles, int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -470,7 +511,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 3 : 2) ssd_split_fi
     if (i < state_ctas) {
         const int rows = PACKED ? a.num_seqs : a.batch * nchunks, tile = i % state_tiles;
         i /= state_tiles;
-        split_state<T, PACKED>(smem, tile, i % rows, i / rows, a, dtb, dAb, entering, form, states, nchunks, status);
+        split_state<T, PACKED, U>(smem, tile, i % rows, i / rows, a, dtb, dAb, entering, form, states, nchunks, status);
     } else if constexpr (!PACKED) {
         i -= state_ctas;
         const int rows = a.batch * nchunks, tile = i % cb_tiles;
@@ -1276,17 +1317,27 @@ template <bool PACKED> int run_first(const mb200_ssd_args &a, const SsdScratch &
         using T = decltype(tag);
         const Buffers s(a, lay);
         const void *entering = static_cast<const char *>(a.scratch) + (form == SsdStates::pn32 ? lay.off_states : lay.off_prev16);
-        const int state_tiles = (a.headdim + 63) / 64 * ((a.dstate + 127) / 128), cb_tiles = (a.chunk_size + 127) / 128 * ((a.chunk_size + 63) / 64);
-        const int64_t rows = PACKED ? a.num_seqs : (int64_t)a.batch * lay.nchunks, state_ctas = with_states ? rows * state_tiles * a.nheads : 0,
-                      ctas = state_ctas + (with_cb ? rows * cb_tiles * a.ngroups : 0);
-        if (ctas == 0) return MB200_OK;
-        if (ctas > INT32_MAX) return fail(MB200_ERR_BAD_ARG, "ssd: too many chunks and heads");
-        constexpr uint32_t smem = kStateSmem<T> > kCbSmem<T> ? kStateSmem<T> : kCbSmem<T>;
-        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_first_kernel<T, PACKED>), (int)smem, a.device);
-        launch_dependent(ssd_split_first_kernel<T, PACKED>, dim3((unsigned)ctas), kThreads, smem, stream, a, s.dt, s.dA, entering, form, PACKED ? a.varlen_states : s.states, s.cb,
-                         (int)state_ctas, state_tiles, cb_tiles, lay.nchunks, s.status);
-        MB200_CHECK_LAUNCH("ssd states and C.B^T (split products)");
-        return MB200_OK;
+        const int units = (a.headdim + 63) / 64 * (a.nheads / a.ngroups), tilesN = (a.dstate + 127) / 128;
+        const int cb_tiles = (a.chunk_size + 127) / 128 * ((a.chunk_size + 63) / 64);
+        const int64_t rows = PACKED ? a.num_seqs : (int64_t)a.batch * lay.nchunks, cb_ctas = with_cb ? rows * cb_tiles * a.ngroups : 0;
+        auto go = [&](auto u_c) -> int {
+            constexpr int U = decltype(u_c)::value;
+            const int state_tiles = (units + U - 1) / U * tilesN;
+            const int64_t state_ctas = with_states ? rows * state_tiles * a.ngroups : 0, ctas = state_ctas + cb_ctas;
+            if (ctas == 0) return MB200_OK;
+            if (ctas > INT32_MAX) return fail(MB200_ERR_BAD_ARG, "ssd: too many chunks and heads");
+            const uint32_t smem = state_ctas == 0 ? kCbSmem<T> : std::max(kStateSmem<T, U>, kCbSmem<T>);
+            ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_first_kernel<T, PACKED, U>), (int)std::max(kStateSmem<T, U>, kCbSmem<T>), a.device);
+            launch_dependent(ssd_split_first_kernel<T, PACKED, U>, dim3((unsigned)ctas), kThreads, smem, stream, a, s.dt, s.dA, entering, form, PACKED ? a.varlen_states : s.states,
+                             s.cb, (int)state_ctas, state_tiles, cb_tiles, lay.nchunks, s.status);
+            MB200_CHECK_LAUNCH("ssd states and C.B^T (split products)");
+            return MB200_OK;
+        };
+        if constexpr (kInParts<T> > 1 && !PACKED) {
+            const bool pairs = with_states && units > 1 && rows * units * tilesN * a.ngroups > (int64_t)(sizeof(T) == 2 ? 3 : 2) * sm_count(a.device);
+            if (pairs) return go(std::integral_constant<int, 2>{});
+        }
+        return go(std::integral_constant<int, 1>{});
     });
 }
 

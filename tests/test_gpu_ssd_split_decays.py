@@ -64,3 +64,10 @@ def test_fp32_values_that_cannot_be_cut(name, value):
     if name == "C":                                                          # one step
         later = torch.arange(300) != t
         assert rel(out[0, later], want[0, later]) <= F32 and rel(fin, wfin) <= F32
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("P,N,G,H", [(64, 64, 1, 15), (72, 40, 3, 15), (64, 136, 1, 9)])
+def test_two_heads_share_their_b(dtype, P, N, G, H):
+    """Enough chunks and heads for the chunk states to go by pairs, an odd head or column tile out among them."""
+    run(make(930 + P + N, 2, 1000, H, P, G, N, dtype, has_z=False, init=True), 64, f"P{P} N{N} G{G} H{H}")

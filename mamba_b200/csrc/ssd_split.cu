@@ -593,19 +593,21 @@ __device__ __noinline__ void add_skipped(float4 *lo, float4 *hi, const uint32_t 
 // CTA per SM that keeps C.B^T in tensor memory while the heads pass took 78, with all its warps in step 85.  The kernel for fp32 below,
 // which leaves the MMAs to a warp of their own, takes 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
 template <typename T> constexpr uint32_t kScan16A = kOutParts<T> * kTileA;
-template <typename T> constexpr uint32_t kScan16B = kOutParts<T> * kTileB;
-template <typename T>
+template <typename T, int W> constexpr uint32_t kScan16B = kOutParts<T> * W * kTileB;
+// W: tiles of 64 columns that share A, whose forming is most of the work: two of a head that has them, where single ones would not all fit the
+// GPU at once (2 x 3000 steps of 32 bf16 heads of 128 x 128: 154 us with one, 122 with two).
+template <typename T, int W>
 __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
                                                                      int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesP = (P + 63) / 64;
-    const int m0 = ((Q + 127) / 128 - 1 - blockIdx.x / tilesP) * 128, p0 = (blockIdx.x % tilesP) * 64;
+    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesP = (P + 64 * W - 1) / (64 * W);
+    const int m0 = ((Q + 127) / 128 - 1 - blockIdx.x / tilesP) * 128, p0 = (blockIdx.x % tilesP) * 64 * W;
     const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z, g = h / (a.nheads / a.ngroups);
     const int len = min(Q, a.seqlen - c * Q);
     if (m0 >= len) return;
     Tile t;
-    t.open(smem, kScan16A<T>, kScan16B<T>, 128, status, kStSplitScan);
+    t.open(smem, kScan16A<T>, kScan16B<T, W>, 128 * W, status, kStSplitScan);
     pdl_wait();
     const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
     const float *dAc = dAb + row, *dtc = dtb + row;
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     const bool vx = rows16(x, a.x_stride[1]), vC = rows16(C, a.C_stride[1]), vN = N % 4 == 0, vQ = Q % 4 == 0;
     const int kend = min(m0 + 128, len);
     const int cols = (kend + 63) / 64 * 64;
-    const ScanDecays decays(smem + kScan16A<T> + kScan16B<T> + kTail, cols);
+    const ScanDecays decays(smem + kScan16A<T> + kScan16B<T, W> + kTail, cols);
     decays.clear((N + 63) / 64 + cols / 64);
     __syncthreads();
     const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;      // my eight columns; rows r0 + 32 i of a tile
@@ -625,21 +627,21 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     for (int i = 0; i < 4; ++i) dm[i] = m0 + r0 + 32 * i < len ? dAc[m0 + r0 + 32 * i] : 0.f;
 
     // whole tiles need no look at any edge
-    const bool whole_rows = m0 + 128 <= len, whole_cols = P - p0 >= 64;
+    const bool whole_rows = m0 + 128 <= len, whole_cols = P - p0 >= 64 * W;
     union { Raw8<T> u[4]; float4 f[8]; } A;         // C rows, or CB rows in two halves
-    union { Raw8<T> u[2]; float4 f[4]; } Bq;        // H rows in two halves, or x rows
+    union { Raw8<T> u[2 * W]; float4 f[4 * W]; } Bq;        // H rows in two halves, or x rows
     auto fetch_states = [&](int n) {
         if (vC && vN && whole_rows && whole_cols && n + 64 <= N) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) A.u[i] = load8_whole(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) Bq.f[i] = reinterpret_cast<const float4 *>(H + (int64_t)(r0 + 32 * (i / 2)) * N + n + 8 * c8)[i & 1];
+            for (int i = 0; i < 4 * W; ++i) Bq.f[i] = reinterpret_cast<const float4 *>(H + (int64_t)(r0 + 32 * (i / 2)) * N + n + 8 * c8)[i & 1];
             return;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) A.u[i] = load8(C + (int64_t)(r0 + 32 * i) * a.C_stride[1] + n + 8 * c8, vC, m0 + r0 + 32 * i < len ? N - n - 8 * c8 : 0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4 * W; ++i)
             Bq.f[i] = load4(H + (int64_t)(r0 + 32 * (i / 2)) * N + n + 8 * c8 + 4 * (i & 1), vN, p0 + r0 + 32 * (i / 2) < P ? N - n - 8 * c8 - 4 * (i & 1) : 0);
     };
     auto fetch_steps = [&](int k) {
@@ -647,16 +649,16 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 #pragma unroll
             for (int i = 0; i < 8; ++i) A.f[i] = reinterpret_cast<const float4 *>(cbm + (int64_t)(r0 + 32 * (i / 2)) * Q + k + 8 * c8)[i & 1];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) Bq.u[i] = load8_whole(x + (int64_t)(k + r0 + 32 * i) * a.x_stride[1] + 8 * c8);
+            for (int i = 0; i < 2 * W; ++i) Bq.u[i] = load8_whole(x + (int64_t)(k + r0 + 32 * (i & 1)) * a.x_stride[1] + 64 * (i >> 1) + 8 * c8);
             return;
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             A.f[i] = load4(cbm + (int64_t)(r0 + 32 * (i / 2)) * Q + k + 8 * c8 + 4 * (i & 1), vQ, m0 + r0 + 32 * (i / 2) < len ? kend - k - 8 * c8 - 4 * (i & 1) : 0);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int kk = k + r0 + 32 * i;
-            Bq.u[i] = load8(x + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, kk < kend ? P - p0 - 8 * c8 : 0);
+        for (int i = 0; i < 2 * W; ++i) {
+            const int kk = k + r0 + 32 * (i & 1), col = 64 * (i >> 1) + 8 * c8;
+            Bq.u[i] = load8(x + (int64_t)kk * a.x_stride[1] + col, vx, kk < kend ? P - p0 - col : 0);
         }
     };
     fetch_states(0);
@@ -670,8 +672,8 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
         left_out = true;
         if (threadIdx.x == 0) decays.skip[tile >> 5] |= 1u << (tile & 31);
     };
-    // contribution of the state entering the chunk: C . H, into the first 64 columns
-    constexpr uint32_t idesc_h = instr_desc_f16(128, 64, 1, 0, 0), idesc_x = instr_desc_f16(128, 64, 1, 0, 1);
+    // contribution of the state entering the chunk: C . H, into the first columns
+    constexpr uint32_t idesc_h = instr_desc_f16(128, 64 * W, 1, 0, 0), idesc_x = instr_desc_f16(128, 64 * W, 1, 0, 1);
 #pragma unroll 1
     for (int n = 0; n < N; n += 64) {
         t.drain();
@@ -679,20 +681,20 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 #pragma unroll
         for (int i = 0; i < 4; ++i) bad = store_input<T>(t.a + sw128(r0 + 32 * i, c8), kTileA, A.u[i]) || bad;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 2 * W; ++i) {
             const float4 lo = Bq.f[2 * i], hi = Bq.f[2 * i + 1];
             const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            bad = store_parts<kOutParts<T>>(t.b + sw128(r0 + 32 * i, c8), kTileB, v) || bad;
+            bad = store_parts<kOutParts<T>>(t.b + sw128(r0 + 32 * i, c8), W * kTileB, v) || bad;
         }
         const bool first = t.issued == 0;
         if (!t.step(bad, [&] {
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kInParts<T>, kOutParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc_h, !first);
+            multiply(kInParts<T>, kOutParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc_h, !first, W * kTileB);
         })) leave_out(n >> 6);
         if (n + 64 < N) fetch_states(n + 64);
         else fetch_steps(0);
     }
-    // the steps of the chunk up to the diagonal, into the other 64
+    // the steps of the chunk up to the diagonal, into the others
     const int states_done = t.issued;
 #pragma unroll 1
     for (int k = 0; k < kend; k += 64) {
@@ -740,34 +742,37 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
             bad = store_parts<kOutParts<T>>(to, kTileA, v) || bad;
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i) bad = store_input<T>(t.b + sw128(r0 + 32 * i, c8), kTileB, Bq.u[i]) || bad;
+        for (int i = 0; i < 2 * W; ++i) bad = store_input<T>(t.b + (i >> 1) * kTileB + sw128(r0 + 32 * (i & 1), c8), W * kTileB, Bq.u[i]) || bad;
         const bool first = t.issued == states_done;
         if (!t.step(bad, [&] {
-            const uint32_t acc = warp_uniform(t.tmem) + 64;
-            multiply(kOutParts<T>, kInParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 128, idesc_x, !first);
+            const uint32_t acc = warp_uniform(t.tmem) + 64 * W;
+            multiply(kOutParts<T>, kInParts<T>, acc, acc, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, kTileB, 1024), 128, idesc_x, !first, W * kTileB);
         })) leave_out(nH + (k >> 6));
         if (k + 64 < kend) fetch_steps(k + 64);
     }
     // x and z of my rows are on their way while the last products are formed
     const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
     const bool vz = z && rows16(z, a.z_stride[1]);
-    const int left = P - p0 - 8 * c8;
     Raw8<T> xm[4], zm[4];
-    if (whole_rows && whole_cols && vx && (!z || vz)) {
+    auto request = [&](int w) {                     // of column tile w
+        const int col = 64 * w + 8 * c8, left = P - p0 - col;
+        if (whole_rows && whole_cols && vx && (!z || vz)) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int64_t m = m0 + r0 + 32 * i;
-            if (a.D) xm[i] = load8_whole(x + m * a.x_stride[1] + 8 * c8);
-            if (z) zm[i] = load8_whole(z + m * a.z_stride[1] + 8 * c8);
-        }
-    } else {
+            for (int i = 0; i < 4; ++i) {
+                const int64_t m = m0 + r0 + 32 * i;
+                if (a.D) xm[i] = load8_whole(x + m * a.x_stride[1] + col);
+                if (z) zm[i] = load8_whole(z + m * a.z_stride[1] + col);
+            }
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int64_t m = m0 + r0 + 32 * i;
-            if (a.D) xm[i] = load8(x + m * a.x_stride[1] + 8 * c8, vx, m < len ? left : 0);
-            if (z) zm[i] = load8(z + m * a.z_stride[1] + 8 * c8, vz, m < len ? left : 0);
+            for (int i = 0; i < 4; ++i) {
+                const int64_t m = m0 + r0 + 32 * i;
+                if (a.D) xm[i] = load8(x + m * a.x_stride[1] + col, vx, m < len ? left : 0);
+                if (z) zm[i] = load8(z + m * a.z_stride[1] + col, vz, m < len ? left : 0);
+            }
         }
-    }
+    };
+    request(0);
     t.drain();
     if (__syncthreads_and(t.ok)) {
         // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
@@ -780,60 +785,68 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
         const float sc = scale(m);
         const bool any1 = states_done > 0, any2 = t.issued > states_done;        // sums that the tensor core has formed
         auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + r * 256 + ((chunk ^ (r & 7)) << 4)); };
-#pragma unroll
-        for (int j = (warp >> 2) * 32; j < (warp >> 2) * 32 + 32; j += 8) {
-            uint32_t y1[8], y2[8];
-            const uint32_t at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + j;
-            tmem_ld8_issue(at, y1);
-            tmem_ld8_issue(at + 64, y2);
-            tmem_ld_wait(y1, y2);
-            float y[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = fmaf(sc, any1 ? __uint_as_float(y1[e]) : 0.f, any2 ? __uint_as_float(y2[e]) : 0.f);
-            *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
-            *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
-        }
-        __syncthreads();
-        T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
-        const bool vo = rows16(out, a.out_stride[1]);
-        if (left_out) {
 #pragma unroll 1
-            for (int r = r0; r < 128; r += 32)
-                if (m0 + r < len && left > 0)
-                    add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), decays.skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
-                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = r0 + 32 * i;
-            if (m0 + r >= len || left <= 0) continue;
-            const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
-            float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
-            if (a.D) {
-                widen8<T>(xm[i], f);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], !a.D_has_hdim ? Dh : e < left ? a.D[(int64_t)h * P + p0 + 8 * c8 + e] : 0.f, y[e]);
+        for (int w = 0; w < W; ++w) {
+            const int col = 64 * w + 8 * c8, left = P - p0 - col;
+            if (w > 0) {
+                __syncthreads();
+                request(w);
             }
-            if (z) {
-                widen8<T>(zm[i], f);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) y[e] *= fast_silu(f[e]);
+            for (int j = (warp >> 2) * 32; j < (warp >> 2) * 32 + 32; j += 8) {
+                uint32_t y1[8], y2[8];
+                const uint32_t at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 * w + j;
+                tmem_ld8_issue(at, y1);
+                tmem_ld8_issue(at + 64 * W, y2);
+                tmem_ld_wait(y1, y2);
+                float y[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) y[e] = fmaf(sc, any1 ? __uint_as_float(y1[e]) : 0.f, any2 ? __uint_as_float(y2[e]) : 0.f);
+                *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
+                *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
             }
-            Raw8<T> o;
-            T *oe = reinterpret_cast<T *>(&o);
+            __syncthreads();
+            T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + col;
+            const bool vo = rows16(out, a.out_stride[1]);
+            if (left_out) {
+#pragma unroll 1
+                for (int r = r0; r < 128; r += 32)
+                    if (m0 + r < len && left > 0)
+                        add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), decays.skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + col, a.x_stride[1],
+                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)col * N, N, left);
+            }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
-            T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
-            if (vo && left >= 8) {
-                *reinterpret_cast<Raw8<T> *>(om) = o;
-            } else {
+            for (int i = 0; i < 4; ++i) {
+                const int r = r0 + 32 * i;
+                if (m0 + r >= len || left <= 0) continue;
+                const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
+                float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
+                if (a.D) {
+                    widen8<T>(xm[i], f);
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (e < left) om[e] = oe[e];
+                    for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], !a.D_has_hdim ? Dh : e < left ? a.D[(int64_t)h * P + p0 + col + e] : 0.f, y[e]);
+                }
+                if (z) {
+                    widen8<T>(zm[i], f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[e] *= fast_silu(f[e]);
+                }
+                Raw8<T> o;
+                T *oe = reinterpret_cast<T *>(&o);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
+                T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
+                if (vo && left >= 8) {
+                    *reinterpret_cast<Raw8<T> *>(om) = o;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (e < left) om[e] = oe[e];
+                }
             }
         }
     }
-    t.close(128);
+    t.close(128 * W);
 }
 
 
@@ -1354,14 +1367,19 @@ int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t 
     return with_type(a, [&](auto tag) -> int {
         using T = decltype(tag);
         const Buffers s(a, lay);
-        auto go = [&](auto kernel, int threads, uint32_t smem) {
+        auto go = [&](auto kernel, int threads, uint32_t smem, int width) {
             smem += scan_decay_bytes(a);
             ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem, a.device);
-            const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.headdim + 63) / 64));
+            const unsigned tiles = (unsigned)((a.chunk_size + 127) / 128 * ((a.headdim + width - 1) / width));
             launch_dependent(kernel, dim3(tiles, a.batch * lay.nchunks, a.nheads), threads, smem, stream, a, s.dt, s.dA, s.states, s.cb, lay.nchunks, s.status);
         };
-        if constexpr (sizeof(T) == 2) go(ssd_split_scan16_kernel<T>, kThreads, kScan16A<T> + kScan16B<T> + kTail);
-        else go(ssd_split_scan_kernel, kScanThreads, kScanTiles + kScanTail);
+        if constexpr (sizeof(T) == 2) {
+            const int64_t singles = (int64_t)((a.chunk_size + 127) / 128) * ((a.headdim + 63) / 64) * a.batch * lay.nchunks * a.nheads;
+            if (a.headdim > 64 && singles > 2 * sm_count(a.device)) go(ssd_split_scan16_kernel<T, 2>, kThreads, kScan16A<T> + kScan16B<T, 2> + kTail, 128);
+            else go(ssd_split_scan16_kernel<T, 1>, kThreads, kScan16A<T> + kScan16B<T, 1> + kTail, 64);
+        } else {
+            go(ssd_split_scan_kernel, kScanThreads, kScanTiles + kScanTail, 64);
+        }
         MB200_CHECK_LAUNCH("ssd outputs (split products)");
         return MB200_OK;
     });

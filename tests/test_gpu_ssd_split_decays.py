@@ -71,3 +71,10 @@ def test_fp32_values_that_cannot_be_cut(name, value):
 def test_two_heads_share_their_b(dtype, P, N, G, H):
     """Enough chunks and heads for the chunk states to go by pairs, an odd head or column tile out among them."""
     run(make(930 + P + N, 2, 1000, H, P, G, N, dtype, has_z=False, init=True), 64, f"P{P} N{N} G{G} H{H}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("P,N,H,L", [(128, 64, 8, 1000), (72, 40, 9, 999), (200, 130, 5, 1000)])
+def test_two_column_tiles_share_their_a(dtype, P, N, H, L):
+    """Enough chunks and heads for the outputs to go by two column tiles of a head, the second (third) of them ragged."""
+    run(make(940 + P + N, 2, L, H, P, 1, N, dtype, has_z=P == 72, D_hdim=P == 200, init=True), 64, f"P{P} N{N} H{H}")

@@ -1140,11 +1140,15 @@ bool rows_for_tma(const void *p, const int64_t *s)
 // One CTA per (head, sequence): S^T[n,p] = sum over the sequence's steps in the chunk of its last token, plus the state entering that
 // chunk if the sequence began earlier.  bf16 inputs: the weighted x rows are cut into three bf16 values, so that the fp32 result keeps
 // fp32 products; B is exact as it is.  (Half precision would need its B cut as well: ssd_split.cu does that.)  The small products have
-// a sum of their own, which keeps the tensor core's rounding of sums out of them.  Halves of 128 rows that hold no step of the sequence are skipped.
-// 23 sequences x 80 heads: 63 us on its own; in place, the wait for the launch before it included, 72, against 54 with two parts and one
-// sum, 83 with the 64-step tiles of ssd_split.cu, 2500 with one thread per element.
+// a sum of their own, which keeps the tensor core's rounding of sums out of them.  Tiles of ROWS rows that hold no step of the sequence are
+// skipped.  A CTA is a chain of copy, cut and MMAs per tile between two ends: tiles of 64 rows let four CTAs share an SM, which pays where
+// there are that many (40 sequences x 48 heads: 130 us a call with 128 rows, 113 with 64; x 128 heads 318 / 292; 20 x 64 407 / 370; 23 x 80 185 / 184),
+// tiles of 128 make the chain shorter (3 x 24: 44 / 48; 5 x 32: 284 / 293; 8 x 80 336 / 338).  2500 us with one thread per element (23 x 80).
 constexpr int kVarThreads = 288;
-__global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
+template <int ROWS> constexpr uint32_t kVarTile = ROWS * 128;                            // [rows][64]
+template <int ROWS> constexpr uint32_t kVarSmem = 5 * kVarTile<ROWS> + 64 + 1024;        // of B two, of x three parts
+template <int ROWS>
+__global__ void __launch_bounds__(kVarThreads, ROWS == 64 ? 4 : 2) ssd_tc_varlen_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_B,
                                                                     const float *dtb, const float *dAb, const int32_t *cu_seqlens, float *varlen,
                                                                     const __nv_bfloat16 *prev16, int prev_np, int nchunks, int nheads, int heads_per_group,
                                                                     int seqlen, int *status)
@@ -1152,8 +1156,8 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
     using T = __nv_bfloat16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *sm = align1024(smem_raw);
-    uint8_t *Bs = sm, *xs = sm + 2 * 16384;                    // B boxes [128 x 64]; x [128 x 64] in three parts
-    uint64_t *bars = reinterpret_cast<uint64_t *>(xs + 3 * 16384);
+    uint8_t *Bs = sm, *xs = sm + 2 * kVarTile<ROWS>;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(xs + 3 * kVarTile<ROWS>);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3);
     const int h = blockIdx.x, sq = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1185,31 +1189,32 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
     bool ok = true;
     int round = 0;
 #pragma unroll 1
-    for (int half = 0; half < 2 && ok; ++half) {
-        if (k1 <= half * 128 || k0 >= half * 128 + 128) continue;
+    for (int r_first = 0; r_first < kQ && ok; r_first += ROWS) {
+        if (k1 <= r_first || k0 >= r_first + ROWS) continue;
         if (warp == 8) {
             if (lane == 0) {
-                mbar_expect_tx(&bars[0], 3 * 16384);
-                tma_load_4d(xs, &tm_x, &bars[0], 0, h, t0 + half * 128, 0);
-                for (int kb = 0; kb < 2; ++kb) tma_load_4d(Bs + kb * 16384, &tm_B, &bars[0], kb * 64, h / heads_per_group, t0 + half * 128, 0);
+                mbar_expect_tx(&bars[0], 3 * kVarTile<ROWS>);
+                tma_load_4d(xs, &tm_x, &bars[0], 0, h, t0 + r_first, 0);
+                for (int kb = 0; kb < 2; ++kb) tma_load_4d(Bs + kb * kVarTile<ROWS>, &tm_B, &bars[0], kb * 64, h / heads_per_group, t0 + r_first, 0);
             }
             __syncwarp();
             ok = __all_sync(0xffffffffu, mbar_wait(&bars[1], round & 1, status, kStBarScaled) && mbar_wait(&bars[0], round & 1, status, kStBarB));
             tc_fence_after_sync();
             const uint32_t idesc = instr_desc_f16(128, 64, 1, 1, 1), tm = warp_uniform(tmem);
-            const uint64_t dB = smem_desc_sw128(smem_u32(Bs), 16384, 1024), dx = smem_desc_sw128(smem_u32(xs), 16, 1024);
+            const uint64_t dB = smem_desc_sw128(smem_u32(Bs), kVarTile<ROWS>, 1024), dx = smem_desc_sw128(smem_u32(xs), 16, 1024);
             if (elect_one()) {
                 if (ok) {
 #pragma unroll 1
                     for (int part = 0; part < 3; ++part)
-                        mma_steps_ss(8, part ? tm + 64 : tm, dB, 128, dx + part * (16384 / 16), 128, idesc, round > 0 || part == 2);
+                        mma_steps_ss(ROWS / 16, part ? tm + 64 : tm, dB, 128, dx + part * (kVarTile<ROWS> / 16), 128, idesc, round > 0 || part == 2);
                 }
                 mma_commit(&bars[2]);
             }
             __syncwarp();
             ok = __all_sync(0xffffffffu, mbar_wait(&bars[2], round & 1, status, kStBarDone)) && ok;
         } else {
-            const int r = threadIdx.x >> 1, k = half * 128 + r, cq = (threadIdx.x & 1) * 4;      // two threads per row
+            constexpr int TPR = 256 / ROWS, NC = 8 / TPR;       // threads per row, and 16-byte chunks of each
+            const int r = threadIdx.x / TPR, k = r_first + r, cq = (threadIdx.x % TPR) * NC;
             const bool mine = k >= k0 && k < k1;
             const float w = mine ? __expf(fminf(dA_end - dAc[k], 0.f)) * dtc[k] : 0.f;
             ok = mbar_wait(&bars[0], round & 1, status, kStBarX);
@@ -1217,20 +1222,21 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
             bool bad = false;
             if (ok) {
 #pragma unroll
-                for (int ch = 0; ch < 8; ++ch) {
-                    const uint4 v = lds128(smem_u32(Bs) + (ch & 4) * 4096 + r * 128 + (((cq + (ch & 3)) ^ (r & 7)) << 4));
+                for (int ch = 0; ch < 2 * NC; ++ch) {
+                    const uint4 v = lds128(smem_u32(Bs) + (ch / NC) * kVarTile<ROWS> + r * 128 + (((cq + ch % NC) ^ (r & 7)) << 4));
                     const uint32_t m = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
                     bad = bad || (m & 0xffffu) >= 0x7f80u || (m >> 16) >= 0x7f80u;
                 }
             }
             bad = __shfl_xor_sync(0xffffffffu, bad, 1) || bad;
+            if (TPR == 4) bad = __shfl_xor_sync(0xffffffffu, bad, 2) || bad;
             if (ok) {
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
+                for (int ch = 0; ch < NC; ++ch) {
                     const uint32_t off = r * 128 + (((cq + ch) ^ (r & 7)) << 4);
                     if (!mine) {        // steps of other sequences count for nothing, infinite B included
                         sts128(smem_u32(Bs) + off, make_uint4(0, 0, 0, 0));
-                        sts128(smem_u32(Bs) + 16384 + off, make_uint4(0, 0, 0, 0));
+                        sts128(smem_u32(Bs) + kVarTile<ROWS> + off, make_uint4(0, 0, 0, 0));
                     }
                     const uint4 v = mine ? lds128(smem_u32(xs) + off) : make_uint4(0, 0, 0, 0);
                     const uint32_t e[4] = {v.x, v.y, v.z, v.w};
@@ -1248,7 +1254,7 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
                         }
                     }
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) sts128(smem_u32(xs) + p * 16384 + off, make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]));
+                    for (int p = 0; p < 3; ++p) sts128(smem_u32(xs) + p * kVarTile<ROWS> + off, make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]));
                 }
             }
             fence_proxy_async();
@@ -1259,29 +1265,32 @@ __global__ void __launch_bounds__(kVarThreads) ssd_tc_varlen_kernel(const __grid
         ++round;
     }
     if (warp < 8) {
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
         tc_fence_after_sync();
-        if (round > 0 && __all_sync(0xffffffffu, ok)) {      // tcgen05.ld is warp-collective
-            const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + p0;
-            float rest[32];
-            tmem_ld32(at, v);
-            tmem_ld32(at + 64, rest);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += rest[j];
-        }
+        const bool formed = round > 0 && __all_sync(0xffffffffu, ok);        // tcgen05.ld is warp-collective
         const float carry = __expf(dA_end);
-        const uint32_t hw[16] = {hv[0].x, hv[0].y, hv[0].z, hv[0].w, hv[1].x, hv[1].y, hv[1].z, hv[1].w,
-                                 hv[2].x, hv[2].y, hv[2].z, hv[2].w, hv[3].x, hv[3].y, hv[3].z, hv[3].w};
         float *dst = varlen + (((int64_t)sq * nheads + h) * kP + p0) * kN + n;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            if (entering) {
-                const float2 f = Pack2<T>::unpack(hw[j >> 1]);
-                v[j] = fmaf(prev_np ? (j & 1 ? f.y : f.x) : to_float(H[(p0 + j) * kN + n]), carry, v[j]);
+        for (int q = 0; q < 2; ++q) {
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+            if (formed) {
+                const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + p0 + 16 * q;
+                float rest[16];
+                tmem_ld16(at, v);
+                tmem_ld16(at + 64, rest);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] += rest[j];
             }
-            dst[j * kN] = v[j];
+            const uint32_t hw[8] = {hv[2 * q].x, hv[2 * q].y, hv[2 * q].z, hv[2 * q].w, hv[2 * q + 1].x, hv[2 * q + 1].y, hv[2 * q + 1].z, hv[2 * q + 1].w};
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (entering) {
+                    const float2 f = Pack2<T>::unpack(hw[j >> 1]);
+                    v[j] = fmaf(prev_np ? (j & 1 ? f.y : f.x) : to_float(H[(p0 + 16 * q + j) * kN + n]), carry, v[j]);
+                }
+                dst[(16 * q + j) * kN] = v[j];
+            }
         }
     }
     tc_fence_before_sync();
@@ -1433,15 +1442,18 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
 int run_varlen(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaStream_t stream)
 {
     const TcCall k = tc_call(a, lay);
-    CUtensorMap tx, tB;
-    if (!map_rows(&tx, 1, a.x, a.x_stride, a.headdim, a.nheads, a, 128) || !map_rows(&tB, 1, a.B, a.B_stride, a.dstate, a.ngroups, a, 128))
-        return fail(MB200_ERR_LAUNCH, "ssd: tensor map for x or B failed");
-    constexpr int smem = 5 * 16384 + 64 + 1024;
-    ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_varlen_kernel), smem, a.device);
-    launch_dependent(ssd_tc_varlen_kernel, dim3(a.nheads, a.num_seqs), kVarThreads, smem, stream, tx, tB, k.dtb, k.dAb, a.cu_seqlens, a.varlen_states,
-                     static_cast<const __nv_bfloat16 *>(k.prev16), h_np ? 1 : 0, k.nc, a.nheads, a.nheads / a.ngroups, a.seqlen, k.status);
-    MB200_CHECK_LAUNCH("ssd varlen states (tensor core)");
-    return MB200_OK;
+    auto go = [&](auto rows_c) -> int {
+        constexpr int ROWS = decltype(rows_c)::value;
+        CUtensorMap tx, tB;
+        if (!map_rows(&tx, 1, a.x, a.x_stride, a.headdim, a.nheads, a, ROWS) || !map_rows(&tB, 1, a.B, a.B_stride, a.dstate, a.ngroups, a, ROWS))
+            return fail(MB200_ERR_LAUNCH, "ssd: tensor map for x or B failed");
+        ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_tc_varlen_kernel<ROWS>), (int)kVarSmem<ROWS>, a.device);
+        launch_dependent(ssd_tc_varlen_kernel<ROWS>, dim3(a.nheads, a.num_seqs), kVarThreads, kVarSmem<ROWS>, stream, tx, tB, k.dtb, k.dAb, a.cu_seqlens, a.varlen_states,
+                         static_cast<const __nv_bfloat16 *>(k.prev16), h_np ? 1 : 0, k.nc, a.nheads, a.nheads / a.ngroups, a.seqlen, k.status);
+        MB200_CHECK_LAUNCH("ssd varlen states (tensor core)");
+        return MB200_OK;
+    };
+    return (int64_t)a.nheads * a.num_seqs > 8 * sm_count(a.device) ? go(std::integral_constant<int, 64>{}) : go(std::integral_constant<int, 128>{});
 }
 
 // f(element type of the call)

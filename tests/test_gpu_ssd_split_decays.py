@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import oracle
-from test_gpu_ssd import DEV, _c, _fn, make
+from test_gpu_ssd import DEV, _c, _fn, _packed, make
 from test_gpu_ssd_split import F32, rel, run
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +78,18 @@ def test_two_heads_share_their_b(dtype, P, N, G, H):
 def test_two_column_tiles_share_their_a(dtype, P, N, H, L):
     """Enough chunks and heads for the outputs to go by two column tiles of a head, the second (third) of them ragged."""
     run(make(940 + P + N, 2, L, H, P, 1, N, dtype, has_z=P == 72, D_hdim=P == 200, init=True), 64, f"P{P} N{N} H{H}")
+
+
+def test_end_states_of_many_short_sequences():
+    """Enough sequences and heads for the 64-row tiles of the end states; lengths around 64, 128 and 256, one across two chunks."""
+    lens = [1, 63, 64, 65, 127, 128, 129, 255, 256, 257, 300] + [5] * 39
+    inp, seq_idx, cu = _packed(950, lens, 24, 64, 1, 128, torch.bfloat16)
+    c = {k: _c(v) for k, v in inp.items()}
+    _, _, var = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 256, D=c["D"], dt_bias=c["dt_bias"], seq_idx=seq_idx.to(DEV), cu_seqlens=cu.to(DEV),
+                      dt_softplus=True, return_final_states=True, return_varlen_states=True)
+    for i in range(len(lens)):
+        sl = slice(int(cu[i]), int(cu[i + 1]))
+        _, wfin = oracle.ssd_chunk_scan(inp["x"][:, sl].float(), inp["dt"][:, sl].float(), inp["A"], inp["B"][:, sl].float(), inp["C"][:, sl].float(), 256, inp["D"], None,
+                                        inp["dt_bias"], None, dt_softplus=True)
+        inside = int(cu[i]) // 256 == (int(cu[i + 1]) - 1) // 256        # nothing of it went through a 16-bit state
+        assert rel(var[i:i + 1], wfin) <= (F32 if inside else 3e-3), f"end state of sequence {i}: {rel(var[i:i + 1], wfin):.3e}"

@@ -563,12 +563,13 @@ struct OutWalk {
     __device__ __forceinline__ int row_blocks(int seqlen) const { return seqlen - c * kQ > 128 ? 2 : 1; }     // that hold steps of the sequence
 };
 
-// DV: D differs over the columns of a head.
-template <typename T, bool DV>
+// DM: no D, one per head, one per column of a head.  Z: with a gate.
+enum { kNoD, kHeadD, kColumnD };
+template <typename T, int DM, bool Z>
 __global__ void __launch_bounds__(kOutThreads, 1)
 ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_C, const __grid_constant__ CUtensorMap tm_B,
                      const __grid_constant__ CUtensorMap tm_H, const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_out,
-                     const float *dtb, const float *dAb, const float *Dp, int has_z, int nchunks, int nheads, int ngroups, int seqlen, int total_items, int h_np, const uint8_t *seq_start, const uint8_t *seq_carry, int *status)
+                     const float *dtb, const float *dAb, const float *Dp, int nchunks, int nheads, int ngroups, int seqlen, int total_items, int h_np, const uint8_t *seq_start, const uint8_t *seq_carry, int *status)
 {
     using Cfg = OutCfg;
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -776,7 +777,8 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         const uint32_t acc = tmem + ((uint32_t)(rq * 32) << 16) + (rb ? kAcc1 : kAcc0), smb = smem_u32(sm);
         const int r = rb * 128 + rq * 32 + lane;             // my row of the chunk
         auto bar = [&](int k) { return smb + kBarOff + 8 * k; };
-        const float *dA = dAb, *Dv = Dp;                     // of the current head; DV: D of its columns
+        const float *dA = dAb;                               // of the current head
+        [[maybe_unused]] const float *Dv = Dp;
         float dA_next = 0.f, D_next = 0.f;
         int left = 0, item = 0;
         bool carry = true, rows = true, ok = true;           // my row continues the sequence that ended the previous chunk; the chunk reaches my block
@@ -787,14 +789,14 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 left = hpu - w.hv;
                 rows = rb < w.row_blocks(seqlen);
                 dA = dAb + (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ + r;
-                if (Dp) Dv = Dp + (int64_t)w.h * (DV ? kP : 1);
+                if constexpr (DM != kNoD) Dv = Dp + (int64_t)w.h * (DM == kColumnD ? kP : 1);
                 if (rows) {
                     if (seq_start) {
                         const int64_t bc = (int64_t)w.b * nchunks + w.c;
                         carry = seq_start[bc * kQ + r] == 0 && seq_carry[bc] != 0;
                     }
                     dA_next = *dA;
-                    if (Dp && !DV) D_next = *Dv;
+                    if constexpr (DM == kHeadD) D_next = *Dv;
                 }
             }
             --left;
@@ -803,7 +805,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             const float rs = carry ? ex2(dA_next * kLog2e) : 0.f, Dh = D_next;
             if (left) {                                      // a whole head ahead of their use
                 dA_next = dA[(int64_t)nchunks * kQ];
-                if (Dp && !DV) D_next = Dv[1];
+                if constexpr (DM == kHeadD) D_next = Dv[1];
             }
             dA += (int64_t)nchunks * kQ;
             const uint32_t row = smb + Cfg::kC + s * Cfg::kStage + r * 128;
@@ -820,8 +822,8 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 tmem_ld8_issue(acc + 64 + e8 * 8, y2);
                 const uint32_t xaddr = row + (uint32_t)((e8 ^ (r & 7)) << 4), zaddr = xaddr + 32768 + Cfg::kH;
                 uint4 xv = make_uint4(0, 0, 0, 0), zv = make_uint4(0, 0, 0, 0);
-                if (Dp) xv = lds128(xaddr);
-                if (has_z) zv = lds128(zaddr);
+                if constexpr (DM != kNoD) xv = lds128(xaddr);
+                if constexpr (Z) zv = lds128(zaddr);
                 tmem_ld_wait(y1, y2);
                 uint64_t y[4];
 #pragma unroll
@@ -833,20 +835,20 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar(kBarAccFree + rb));
                 }
-                if (Dp) {
+                if constexpr (DM != kNoD) {
                     const uint32_t xe[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float2 f = Pack2<T>::unpack(xe[i]);
                         uint64_t d2 = D2;
-                        if constexpr (DV) {
+                        if constexpr (DM == kColumnD) {
                             const int pc = e8 * 8 + 2 * i;
                             d2 = pack2(Dv[pc], Dv[pc + 1]);
                         }
                         y[i] = fma2(pack2(f.x, f.y), d2, y[i]);
                     }
                 }
-                if (has_z) {
+                if constexpr (Z) {
                     const uint32_t ze[4] = {zv.x, zv.y, zv.z, zv.w};
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -870,7 +872,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 }
                 sts128(zaddr, make_uint4(o[0], o[1], o[2], o[3]));
             }
-            if (Dp) Dv += DV ? kP : 1;
+            if constexpr (DM != kNoD) Dv += DM == kColumnD ? kP : 1;
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(kBarOut + 2 * s + rb));
@@ -1001,7 +1003,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
 #pragma unroll 1
                         for (int kb = 0; kb < 2; ++kb) tma_load_3d(st_H(s) + kb * 8192, &tm_H, &b_xh[s], kb * 64, 0, uh);   // columns n of the [p][n] state
                     tma_store_wait_read();
-                    if (has_z) {
+                    if (Z) {
                         mbar_expect_tx(&b_z[s], 32768);
                         tma_load_4d(st_z(s), &tm_z, &b_z[s], 0, w.h, w.c * kQ, w.b);
                     } else {
@@ -1018,7 +1020,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
 #pragma unroll 1
                     for (int k = seq > 2 ? seq - 2 : 0; k < seq; ++k) {
                         mbar_wait(&b_xh[k & 1], (k >> 1) & 1, status, kStOutStage);
-                        if (has_z) mbar_wait(&b_z[k & 1], (k >> 1) & 1, status, kStOutGate);
+                        if (Z) mbar_wait(&b_z[k & 1], (k >> 1) & 1, status, kStOutGate);
                     }
                 }
             }
@@ -1421,8 +1423,8 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     const int grid = (int)std::min<int64_t>(items, sm_count(a.device));
     const uint8_t *seq_start = a.seq_idx ? reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_start) : nullptr;
     const uint8_t *seq_carry = reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_carry);
-    auto go = [&](auto dv) -> bool {
-        auto kernel = ssd_tc_output_kernel<T, decltype(dv)::value>;
+    auto go = [&](auto dm, auto with_z) -> bool {
+        auto kernel = ssd_tc_output_kernel<T, decltype(dm)::value, decltype(with_z)::value>;
         // its warps would wait for ever for registers that the block was not launched with
         static const bool enough = [&] {
             cudaFuncAttributes at;
@@ -1430,11 +1432,13 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
         }();
         if (!enough) return false;
         ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)OutCfg::kSmem, a.device);
-        launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, a.z != nullptr, k.nc,
-                         a.nheads, a.ngroups, a.seqlen, (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
+        launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, k.nc, a.nheads, a.ngroups, a.seqlen,
+                            (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
         return true;
     };
-    if (!(a.D && a.D_has_hdim ? go(std::true_type{}) : go(std::false_type{}))) return fail(MB200_ERR_LAUNCH, "ssd: output kernel built with too few registers");
+    auto with_d = [&](auto dm) { return a.z ? go(dm, std::true_type{}) : go(dm, std::false_type{}); };
+    const bool launched = !a.D ? with_d(std::integral_constant<int, kNoD>{}) : a.D_has_hdim ? with_d(std::integral_constant<int, kColumnD>{}) : with_d(std::integral_constant<int, kHeadD>{});
+    if (!launched) return fail(MB200_ERR_LAUNCH, "ssd: output kernel built with too few registers");
     MB200_CHECK_LAUNCH("ssd output (tensor core)");
     return MB200_OK;
 }

@@ -12,7 +12,7 @@
 // A tile loop: 256 threads fetch the next 64 steps of the reduction while the tensor core works on the last ones, form the operand values,
 // cut them and store them.  The tensor core is idle most of the time; what bounds these kernels is that element-wise work and the latencies
 // between it, which two to four CTAs per SM share.  Rows are read with plain loads, so any stride and alignment goes.
-// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states 28, C.B^T 5, outputs 69; fp32 FMAs took 318 for the call.
+// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states and C.B^T 23, outputs 68; fp32 FMAs took 318 for the call.
 #include <algorithm>
 #include <type_traits>
 
@@ -869,8 +869,8 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 // bytes, so that the loads fill whole sectors.  The order within a tile is free: a lane's four consecutive elements go to where its words
 // are, and B's rows (or H's columns) follow.  The small products have a sum of their own, as in the chunk states.
 // What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
-// middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us,
-// 2 x 3000 steps of 32 heads of 64 x 128 149; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
+// middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its start, which overlaps the recurrence, included),
+// 2 x 3000 steps of 32 heads of 64 x 128 142; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
 constexpr int kScanThreads = kThreads + 32;
 // Shared memory: B, then two stages of C.B^T, 4 KB a warp.  The sums leave through the first of them.
 constexpr uint32_t kScanB = kParts * kTileB, kScanTiles = kScanB + 65536;

@@ -14,6 +14,7 @@
 // between it, which two to four CTAs per SM share.  Rows are read with plain loads, so any stride and alignment goes.
 // 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states and C.B^T 23, outputs 68; fp32 FMAs took 318 for the call.
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 #include "ssd_common.cuh"
@@ -535,8 +536,9 @@ template <typename T> constexpr int kOutParts = std::is_same<T, __nv_bfloat16>::
 
 // Decays of the steps a block of rows looks back on, factorised: exp(dA_m - dA_k) dt_k = exp(dA_m - ref) (exp(ref - dA_k) dt_k), ref = dA
 // of the last of 32 steps: an exponential per row and 32 columns instead of one per element.  dA does not increase (A <= 0, dt >= 0), so neither exponent is positive below the diagonal; in the
-// range that holds it the first is bounded.  A range for which that is not so has its decays formed one by one.  Differences are formed
-// before anything is rounded, as with a single exponential.
+// range that holds it the first is bounded.  The two are multiplied with each other before CB, whose product with a column factor of 2^-100
+// may be subnormal; a column factor that is so itself (a step of almost no length) would lose bits as well.  A range for which one of these
+// is not so has its decays formed one by one.
 constexpr float kMaxSpan = 100.f;                       // (in powers of two) of the decays within 32 steps
 inline uint32_t scan_decay_bytes(const mb200_ssd_args &a)
 {
@@ -560,8 +562,10 @@ struct ScanDecays {
             const int kk = min(k, kend - 1);
             const float v = dAc[kk], before = dAc[max(kk - 1, 0)], end = __shfl_sync(0xffffffffu, v, 31);
             dA[k] = v;
-            ck[k] = k < kend ? ex2((end - v) * kLog2e) * dtc[kk] : 0.f;
-            const bool falls = __all_sync(0xffffffffu, v <= before + 2e-6f * fabsf(before)), fits = __all_sync(0xffffffffu, (v - end) * kLog2e <= kMaxSpan);      // (rounding of the sums aside)
+            const float step = dtc[kk], w = ex2((end - v) * kLog2e) * step;
+            ck[k] = k < kend ? w : 0.f;
+            const bool falls = __all_sync(0xffffffffu, v <= before + 2e-6f * fabsf(before));      // (rounding of the sums aside)
+            const bool fits = __all_sync(0xffffffffu, (v - end) * kLog2e <= kMaxSpan && (w >= FLT_MIN || step == 0.f));
             if ((threadIdx.x & 31) == 0) {
                 if (!falls) atomicOr(plain, ~0u);                            // then min(dA_m - dA_k, 0) may be 0 anywhere
                 else if (!fits) atomicOr(plain, 1u << (k >> 5));
@@ -744,7 +748,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
             const uint64_t cbv[4] = {pack2(lo.x, lo.y), pack2(lo.z, lo.w), pack2(hi.x, hi.y), pack2(hi.z, hi.w)};
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) unpack2(mul2(mul2(cbv[e], f[e]), pack2(fm, fm)), v[2 * e], v[2 * e + 1]);
+            for (int e = 0; e < 4; ++e) unpack2(mul2(cbv[e], mul2(f[e], pack2(fm, fm))), v[2 * e], v[2 * e + 1]);
             if (k + 64 > m0) {
                 const int past = m0 + r0 + 32 * i - (k + 8 * c8);       // columns up to the diagonal
 #pragma unroll
@@ -1191,7 +1195,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
                             const float fm = ex2(fminf((dm[r] - end) * kLog2e, kMaxSpan));             // (past the diagonal it only has to stay finite)
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
-                                uint64_t v = mul2(mul2(cbv[q], fk[q]), pack2(fm, fm));
+                                uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));
                                 if (diagonal) {
                                     float v0, v1;
                                     unpack2(v, v0, v1);

@@ -1,5 +1,7 @@
 """The split-product stages where their short cuts end: decays that cannot be factorised over 32 steps (steeper than 2^100, or rising),
 fp32 inputs at the edges of tiles, and fp32 infinities and NaNs, which the tensor core leaves to fp32 FMAs."""
+import math
+
 import pytest
 import torch
 
@@ -32,6 +34,32 @@ def test_rising_sums(dtype):
     want += torch.einsum("mn,hm,hpn->mhp", d["C"][0, :, 0], torch.exp(sums), d["initial_states"][0]) + d["x"][0] * (d["D"] if d["D"].dim() == 2 else d["D"][:, None])
     wfin = torch.exp(sums[:, -1])[:, None, None] * d["initial_states"][0] + torch.einsum("kn,hk,khp->hpn", d["B"][0, :, 0], decay[:, -1], d["x"][0])
     run(inp, 256, "rising", (want[None].float(), wfin[None].float()))
+
+
+def _steady(inp, step):
+    """Every step has length 0.1375 and decays its head by `step` nats, with no skip that would cover the sums."""
+    inp["A"][:], inp["dt"][:], inp["D"] = -step / 0.1375, 0.0, None
+    inp["dt_bias"][:] = math.log(math.expm1(0.1375))
+    return inp
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("P", [64, 128])
+def test_steep_decays_and_small_products(dtype, P):
+    """98 powers of two within 32 steps, the steepest that is factorised: C.B of 1e-15 meets column factors of 2^-98, whose product would be subnormal."""
+    inp = _steady(make(960 + P, 2, 300, 3, P, 1, 64, dtype, has_z=False), 2.2)
+    inp["B"], inp["C"] = inp["B"] * 1e-8, inp["C"] * 1e-8
+    run(inp, 256, f"small products P{P}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_steep_decays_and_a_step_of_almost_no_length(dtype):
+    """The only step with an input has dt of 1e-15 and 30 of the steepest steps behind it in its range: the column factor would be subnormal."""
+    inp = _steady(make(962, 1, 200, 2, 64, 1, 64, dtype, has_z=False), 2.2)
+    inp["dt"][:, 33] = -34.5 - inp["dt_bias"]
+    keep = torch.arange(200) == 33
+    inp["x"][:, ~keep] = 0
+    run(inp, 256, "short step")
 
 
 @pytest.mark.parametrize("P,N,H,Q,L", [(64, 64, 2, 256, 129), (128, 128, 1, 128, 257), (65, 66, 2, 64, 65), (7, 130, 1, 100, 101), (64, 64, 1, 1024, 1100), (1, 1, 1, 1, 3)])

@@ -67,6 +67,18 @@ def test_fp32_shapes(P, N, H, Q, L):
     run(make(910 + P + N, 2, L, H, P, 1, N, torch.float32, has_z=L % 2 == 0, D_hdim=P % 2 == 0, init=True), Q, f"P{P} N{N} Q{Q} L{L}")
 
 
+def test_fp32_gate_far_below_zero():
+    """silu(z) for z below -87.3, where 1 + exp(-z) exceeds 2^126: -1e-36 and not zero (below -88.7 exp(-z) is infinite, as in silu itself)."""
+    inp = make(966, 1, 130, 2, 64, 1, 64, torch.float32)
+    inp["z"] = torch.linspace(-88.7, -80.0, inp["z"].numel()).reshape(inp["z"].shape)
+    c = {k: _c(v) for k, v in inp.items()}
+    out = lambda z: _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 128, D=c["D"], z=z, dt_bias=c["dt_bias"], dt_softplus=True).cpu().double()
+    z = inp["z"].double()
+    want = out(None) * z * torch.sigmoid(z)
+    keep = want.abs() > 1.2e-38                                              # (what is subnormal has fewer bits)
+    assert (keep & (z < -87.4)).any() and ((out(c["z"]) - want).abs()[keep] / want.abs()[keep]).max() <= 1e-6       # five roundings and expf's
+
+
 @pytest.mark.parametrize("name", ["x", "B", "C"])
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
 def test_fp32_values_that_cannot_be_cut(name, value):

@@ -539,39 +539,54 @@ template <typename T> constexpr int kOutParts = std::is_same<T, __nv_bfloat16>::
 // range that holds it the first is bounded.  The two are multiplied with each other before CB, whose product with a column factor of 2^-100
 // may be subnormal; a column factor that is so itself (a step of almost no length) would lose bits as well.  A range for which one of these
 // is not so has its decays formed one by one.
+// In that range two exponents of up to 100 replace one that is small where the weight is large, so neither may lose what the other does not
+// give back: the distance of a step from the range's last is summed within the range, not taken from the chunk's sums, which are rounded to
+// 2^-24 of their size, and its rows use the same rounded distances as its columns, so that the exponents of a step's weight on itself cancel.
 constexpr float kMaxSpan = 100.f;                       // (in powers of two) of the decays within 32 steps
 inline uint32_t scan_decay_bytes(const mb200_ssd_args &a)
 {
-    const uint32_t steps = (a.chunk_size + 63) / 64, states = (a.dstate + 63) / 64;
-    return (2 * 64 * steps + 1 + (steps + states + 31) / 32) * 4;
+    const uint32_t blocks = (a.chunk_size + 127) / 128, states = (a.dstate + 63) / 64;
+    return (3 * 128 * blocks + 1 + (2 * blocks + states + 31) / 32) * 4;
 }
 struct ScanDecays {
-    float *ck, *dA;             // [step]: column factors, dA (the last one's for steps past the end)
+    float *ck, *dA, *rel;       // [step], to the end of the row block: column factors; dA (steps past the end have the last one's); powers of two that
+                                // the step's state decays by to the last of its range
     uint32_t *plain;            // ranges that cannot be factorised, a bit each
     uint32_t *skip;             // tiles left for the FMAs, a bit each: of the states, then of the steps
     int cols;
-    __device__ __forceinline__ ScanDecays(uint8_t *at, int cols_) : ck(reinterpret_cast<float *>(at)), dA(ck + cols_), plain(reinterpret_cast<uint32_t *>(dA + cols_)), skip(plain + 1), cols(cols_) {}
+    __device__ __forceinline__ ScanDecays(uint8_t *at, int cols_)
+        : ck(reinterpret_cast<float *>(at)), dA(ck + cols_), rel(dA + cols_), plain(reinterpret_cast<uint32_t *>(rel + cols_)), skip(plain + 1), cols(cols_) {}
     // (all threads; a barrier after each)
     __device__ __forceinline__ void clear(int ntiles) const
     {
         for (int i = threadIdx.x; i < 1 + (ntiles + 31) / 32; i += blockDim.x) plain[i] = 0;
     }
-    __device__ __forceinline__ void form(const float *dAc, const float *dtc, int kend) const
+    __device__ __forceinline__ void form(const float *dAc, const float *dtc, float A, int kend) const
     {
+        const int lane = threadIdx.x & 31;
         for (int k = threadIdx.x; k < cols; k += blockDim.x) {              // (a warp has a range of 32)
-            const int kk = min(k, kend - 1);
-            const float v = dAc[kk], before = dAc[max(kk - 1, 0)], end = __shfl_sync(0xffffffffu, v, 31);
+            const float v = dAc[min(k, kend - 1)], dt = k < kend ? dtc[k] : 0.f, step = dt * A;
+            float after = step;                         // the steps behind mine
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float far = __shfl_down_sync(0xffffffffu, after, o);
+                if (lane + o < 32) after += far;
+            }
+            after = __shfl_down_sync(0xffffffffu, after, 1);
+            const float down = lane < 31 ? after * kLog2e : 0.f, w = ex2(down) * dt;
             dA[k] = v;
-            const float step = dtc[kk], w = ex2((end - v) * kLog2e) * step;
-            ck[k] = k < kend ? w : 0.f;
-            const bool falls = __all_sync(0xffffffffu, v <= before + 2e-6f * fabsf(before));      // (rounding of the sums aside)
-            const bool fits = __all_sync(0xffffffffu, (v - end) * kLog2e <= kMaxSpan && (w >= FLT_MIN || step == 0.f));
-            if ((threadIdx.x & 31) == 0) {
+            rel[k] = -down;
+            ck[k] = w;
+            const bool falls = __all_sync(0xffffffffu, step <= 0.f && v >= -FLT_MAX);
+            const bool fits = __all_sync(0xffffffffu, down >= -kMaxSpan && (w >= FLT_MIN || dt == 0.f));
+            if (lane == 0) {
                 if (!falls) atomicOr(plain, ~0u);                            // then min(dA_m - dA_k, 0) may be 0 anywhere
                 else if (!fits) atomicOr(plain, 1u << (k >> 5));
             }
         }
     }
+    // exp(dA_m - ref), ref = dA of the last of range `range`; before that range it only has to stay finite
+    __device__ __forceinline__ float row(int m, int range) const { return ex2(fminf(fmaf(dA[m | 31] - dA[32 * range + 31], kLog2e, rel[m]), kMaxSpan)); }
 };
 // Rare: what tiles with infinities or NaNs contribute to eight outputs of row m, in fp32.
 template <typename T>
@@ -628,15 +643,10 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     const float *cbm = cb + ((((int64_t)b * nchunks + c) * a.ngroups + g) * Q + m0) * Q;
     const bool vx = rows16(x, a.x_stride[1]), vC = rows16(C, a.C_stride[1]), vN = N % 4 == 0, vQ = Q % 4 == 0;
     const int kend = min(m0 + 128, len);
-    const int cols = (kend + 63) / 64 * 64;
-    const ScanDecays decays(smem + kScan16A<T> + kScan16B<T, W> + kTail, cols);
-    decays.clear((N + 63) / 64 + cols / 64);
+    const ScanDecays decays(smem + kScan16A<T> + kScan16B<T, W> + kTail, m0 + 128);
+    decays.clear((N + 63) / 64 + (kend + 63) / 64);
     __syncthreads();
     const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3;      // my eight columns; rows r0 + 32 i of a tile
-    float dm[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dm[i] = m0 + r0 + 32 * i < len ? dAc[m0 + r0 + 32 * i] : 0.f;
-
     // whole tiles need no look at any edge
     const bool whole_rows = m0 + 128 <= len, whole_cols = P - p0 >= 64 * W;
     union { Raw8<T> u[4]; float4 f[8]; } A;         // C rows, or CB rows in two halves
@@ -674,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     };
     fetch_states(0);
     const float Dh = a.D && !a.D_has_hdim ? a.D[h] : 0.f;
-    decays.form(dAc, dtc, kend);
+    decays.form(dAc, dtc, a.A[h], kend);
     __syncthreads();
     const uint32_t plains = *decays.plain;
     const int nH = (N + 63) / 64;
@@ -722,7 +732,6 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
             fk[2 * q + 1] = v.y;
         }
         const int range = (k >> 5) + (c8 >> 2);
-        const float end = decays.dA[32 * range + 31];
         const bool plain = (plains >> range) & 1;
         bool bad = false;
 #pragma unroll
@@ -735,14 +744,15 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
             }
             const float4 lo = A.f[2 * i], hi = A.f[2 * i + 1];
             uint64_t f[4] = {fk[0], fk[1], fk[2], fk[3]};
-            float fm = ex2(fminf((dm[i] - end) * kLog2e, kMaxSpan));            // (past the diagonal it only has to stay finite)
+            float fm = decays.row(m0 + r0 + 32 * i, range);
             if (plain) {
+                const float dm = decays.dA[m0 + r0 + 32 * i];
                 fm = 1.f;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int kk = k + 8 * c8 + 2 * e;
-                    f[e] = pack2(kk < kend ? ex2(fminf(dm[i] - decays.dA[kk], 0.f) * kLog2e) * dtc[kk] : 0.f,
-                                 kk + 1 < kend ? ex2(fminf(dm[i] - decays.dA[kk + 1], 0.f) * kLog2e) * dtc[kk + 1] : 0.f);
+                    f[e] = pack2(kk < kend ? ex2(fminf(dm - decays.dA[kk], 0.f) * kLog2e) * dtc[kk] : 0.f,
+                                 kk + 1 < kend ? ex2(fminf(dm - decays.dA[kk + 1], 0.f) * kLog2e) * dtc[kk + 1] : 0.f);
                 }
             }
             const uint64_t cbv[4] = {pack2(lo.x, lo.y), pack2(lo.z, lo.w), pack2(hi.x, hi.y), pack2(hi.z, hi.w)};
@@ -909,13 +919,12 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
     const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z, g = h / (a.nheads / a.ngroups);
     const int len = min(Q, a.seqlen - c * Q);
     if (m0 >= len) return;
-    const int kend = min(m0 + 128, len), ksteps = (kend + 63) / 64, cols = ksteps * 64, nH = (N + 63) / 64, ntiles = nH + ksteps;
+    const int kend = min(m0 + 128, len), ksteps = (kend + 63) / 64, nH = (N + 63) / 64, ntiles = nH + ksteps;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool mma_warp = warp == kThreads / 32;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kScanTiles), *done = full + 2;      // [tile & 1]: operands in place; their products added
     uint32_t *slot = reinterpret_cast<uint32_t *>(done + 2);
-    const ScanDecays decays(smem + kScanTiles + kScanTail, cols);
-    float *const ck = decays.ck, *const dAs = decays.dA;
+    const ScanDecays decays(smem + kScanTiles + kScanTail, m0 + 128);
     uint32_t *const skip = decays.skip;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
@@ -1025,7 +1034,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
         for (int i = 0; i < kAhead; ++i) request_cb(64 * i);
     }
     const float Dh = a.D && !a.D_has_hdim ? a.D[h] : 0.f;
-    decays.form(dAc, dtc, kend);
+    decays.form(dAc, dtc, a.A[h], kend);
     __syncthreads();
     bool ok = true;
     if (mma_warp) {
@@ -1064,13 +1073,10 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
         // ------------------------------------------------------------------ operands
         const uint32_t at = tmem + ((uint32_t)rw << 16) + kScanA + ch / 2;
         const uint32_t plains = *decays.plain;
-        float dm[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) dm[i] = dAs[min(m0 + ra + 8 * i, cols - 1)];
         const int lm = rw + lane, m = m0 + lm;               // my row of the sums, whose columns ch .. ch + 31 I have
         auto scale = [&](int m) {                            // the entering state belongs to the sequence that ends the previous chunk
             if (m >= len || (a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0))) return 0.f;
-            return __expf(dAs[m]);
+            return __expf(decays.dA[m]);
         };
         const float sc = scale(m);
         auto skipped = [&](int t) { return (reinterpret_cast<volatile uint32_t *>(skip)[t >> 5] >> (t & 31)) & 1; };
@@ -1174,11 +1180,10 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
                     uint64_t fk[4];                          // of my columns 16 q + 4 j .. + 3
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(ck + k + ch + 4 * j4 + 16 * q);
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(decays.ck + k + ch + 4 * j4 + 16 * q);
                         fk[2 * q] = v.x;
                         fk[2 * q + 1] = v.y;
                     }
-                    const float end = dAs[k + ch + 31];
                     const uint32_t from = ring + ((k >> 6) & 1) * 32768 + (lane >> 2) * 128 + j4 * 16, flip = (lane & 4) << 4;       // (row & 1 = lane / 4 & 1)
                     const bool diagonal = k + ch + 31 > m0 + rw;
 #pragma unroll
@@ -1192,7 +1197,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
                             for (int q = 0; q < 2; ++q)
                                 asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
                             const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
-                            const float fm = ex2(fminf((dm[r] - end) * kLog2e, kMaxSpan));             // (past the diagonal it only has to stay finite)
+                            const float fm = decays.row(m0 + ra + 8 * r, (k + ch) >> 5);
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
                                 uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));

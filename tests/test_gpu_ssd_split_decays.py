@@ -62,6 +62,25 @@ def test_steep_decays_and_a_step_of_almost_no_length(dtype):
     run(inp, 256, "short step")
 
 
+def test_weights_within_32_steps():
+    """dt and dt exp(-1.4) for the step itself and the next, though the chunk's sums reach 358, where they are rounded to 3e-5.  Inputs 65 steps
+    apart, so that what came before has decayed to nothing."""
+    L, decay = 65 * 128, 1.4
+    inp = _steady(make(964, 1, L, 2, 64, 1, 64, torch.float32, has_z=False), decay)
+    inp["B"][:], inp["C"][:], inp["x"][:] = 0.0, 0.0, 0.0
+    inp["B"][..., 0], inp["C"][..., 0] = 1.0, 1.0
+    at = torch.arange(0, L, 65)
+    inp["x"][:, at] = 1.0
+    dt = torch.full_like(inp["dt"], 0.1375)
+    out = _fn()(*(_c(t) for t in (inp["x"], dt, inp["A"], inp["B"], inp["C"])), 256).cpu().double()
+    dt = dt.double()[0, 0, :, None]
+    rounding = 4 * 2.0 ** -23 + 4 * 2.0 ** -24                                   # two exponentials of at most 2 ulp, four roundings
+    assert (out[:, at] / dt - 1).abs().max() <= rounding
+    at = at[at % 32 != 31]                                                       # (the next step belongs to the same 32)
+    # two distances of up to 31 steps, summed in five rounds of 2, 4, 8, 16 and 31, then times log2 e: each rounds by at most 2^-24 of its size
+    assert (out[:, at + 1] / (dt * torch.exp(dt * inp["A"].double()[:, None])) - 1).abs().max() <= rounding + 2 * 2.0 ** -24 * (61 + 31) * decay
+
+
 @pytest.mark.parametrize("P,N,H,Q,L", [(64, 64, 2, 256, 129), (128, 128, 1, 128, 257), (65, 66, 2, 64, 65), (7, 130, 1, 100, 101), (64, 64, 1, 1024, 1100), (1, 1, 1, 1, 3)])
 def test_fp32_shapes(P, N, H, Q, L):
     run(make(910 + P + N, 2, L, H, P, 1, N, torch.float32, has_z=L % 2 == 0, D_hdim=P % 2 == 0, init=True), Q, f"P{P} N{N} Q{Q} L{L}")

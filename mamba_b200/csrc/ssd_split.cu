@@ -878,14 +878,14 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 
 // ---- fp32
 // Eight warps form the operands of a tile of 64 along the reduction -- first the states, then the steps of the chunk up to the diagonal --
-// and a ninth issues its MMAs: the A operand (C, then CB with its decays) goes to tensor memory, B (H, then x) to shared memory.  A warp
+// and the first issues its MMAs: the A operand (C, then CB with its decays) goes to tensor memory, B (H, then x) to shared memory.  A warp
 // has rows 32 (w % 4) .. and one half of the 64 columns; tcgen05.st.16x128b gives a lane four of these rows, and four lanes a row's 16
 // bytes, so that the loads fill whole sectors.  The order within a tile is free: a lane's four consecutive elements go to where its words
-// are, and B's rows (or H's columns) follow.  The small products have a sum of their own, as in the chunk states.
+// are, and B's rows (or H's columns) follow.  The small products have a sum of their own, as in the chunk states.  (A ninth warp for the MMAs
+// alone leaves a thread 96 registers for 128, because a quarter of the SM then has five warps: 600 bytes of spills for 84, 28.0 us for 26.2.)
 // What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
 // middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its start, which overlaps the recurrence, included),
 // 2 x 3000 steps of 32 heads of 64 x 128 142; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
-constexpr int kScanThreads = kThreads + 32;
 // Shared memory: B, then two stages of C.B^T, 4 KB a warp.  The sums leave through the first of them.
 constexpr uint32_t kScanB = kParts * kTileB, kScanTiles = kScanB + 65536;
 constexpr uint32_t kScanTail = 48;                      // barriers and tensor-memory slot behind the tiles
@@ -908,7 +908,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool i
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
+__global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
                                                                          int nchunks, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -921,7 +921,6 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
     if (m0 >= len) return;
     const int kend = min(m0 + 128, len), ksteps = (kend + 63) / 64, nH = (N + 63) / 64, ntiles = nH + ksteps;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool mma_warp = warp == kThreads / 32;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kScanTiles), *done = full + 2;      // [tile & 1]: operands in place; their products added
     uint32_t *slot = reinterpret_cast<uint32_t *>(done + 2);
     const ScanDecays decays(smem + kScanTiles + kScanTail, m0 + 128);
@@ -934,7 +933,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
         mbar_fence_init();
         if (smem_u32(smem) & 1023u) atomicCAS(status, 0, kStSplitScan);             // the swizzled tiles assume a 1 KB aligned base
     }
-    if (mma_warp) tmem_alloc(slot, 256);
+    if (warp == 0) tmem_alloc(slot, 256);
     decays.clear(ntiles);
     tc_fence_before_sync();
     __syncthreads();
@@ -1028,305 +1027,297 @@ __global__ void __launch_bounds__(kScanThreads, 2) ssd_split_scan_kernel(const m
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (!mma_warp) {
-        fetch_states(0);
+    fetch_states(0);
 #pragma unroll
-        for (int i = 0; i < kAhead; ++i) request_cb(64 * i);
-    }
+    for (int i = 0; i < kAhead; ++i) request_cb(64 * i);
     const float Dh = a.D && !a.D_has_hdim ? a.D[h] : 0.f;
     decays.form(dAc, dtc, a.A[h], kend);
     __syncthreads();
     bool ok = true;
-    if (mma_warp) {
-        // ------------------------------------------------------------------ MMAs
-        constexpr uint32_t idesc_h = instr_desc_f16(128, 64, 1, 0, 0), idesc_x = instr_desc_f16(128, 64, 1, 0, 1);
-        const uint32_t tm = warp_uniform(tmem);
+    // the operands of tile i are in place: the first warp issues its MMAs
+    bool begun = false;                                      // (its own) the sums hold something
+    auto issue = [&](int i) {
+        if (warp != 0) return;
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(&full[i & 1], (i >> 1) & 1, status, kStSplitScan));
+        if (!ok) return;
+        tc_fence_after_sync();
+        const uint32_t tm = warp_uniform(tmem), A = tm + kScanA;
         const uint64_t desc = smem_desc_sw128(tiles, 16, 1024);
-        bool begun = false;                                  // the sums hold something
+        const bool steps = i >= nH, on = !((reinterpret_cast<volatile uint32_t *>(skip)[i >> 5] >> (i & 31)) & 1);
+        const uint32_t step_b = steps ? 128 : 2, idesc = instr_desc_f16(128, 64, 1, 0, 0) | (steps ? instr_desc_f16(128, 64, 1, 0, 1) : 0);
+        begun = begun || steps;                              // (scaled, they do)
+        if (elect_one()) {
+            if (on) {
+                mma_steps_ts(4, tm, A, desc, step_b, idesc, begun);
+                bool more = begun;
 #pragma unroll 1
-        for (int i = 0; i < ntiles && ok; ++i) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&full[i & 1], (i >> 1) & 1, status, kStSplitScan));
-            if (!ok) break;
-            tc_fence_after_sync();
-            const bool steps = i >= nH, on = !((reinterpret_cast<volatile uint32_t *>(skip)[i >> 5] >> (i & 31)) & 1);
-            const uint32_t A = tm + kScanA;
-            begun = begun || steps;                          // (scaled, they do)
-            const uint32_t step_b = steps ? 128 : 2, idesc = steps ? idesc_x : idesc_h;
-            if (elect_one()) {
-                if (on) {
-                    mma_steps_ts(4, tm, A, desc, step_b, idesc, begun);
-                    bool more = begun;
+                for (int pa = 0; pa < NP; ++pa)
 #pragma unroll 1
-                    for (int pa = 0; pa < NP; ++pa)
-#pragma unroll 1
-                        for (int pb = pa ? 0 : 1; pa + pb < NP; ++pb) {
-                            mma_steps_ts(4, tm + 64, A + 32 * pa, desc + pb * (kTileB / 16), step_b, idesc, more);
-                            more = true;
-                        }
-                }
-                mma_commit(&done[i & 1]);
+                    for (int pb = pa ? 0 : 1; pa + pb < NP; ++pb) {
+                        mma_steps_ts(4, tm + 64, A + 32 * pa, desc + pb * (kTileB / 16), step_b, idesc, more);
+                        more = true;
+                    }
             }
-            __syncwarp();
-            begun = begun || on;
+            mma_commit(&done[i & 1]);
         }
-    } else {
-        // ------------------------------------------------------------------ operands
-        const uint32_t at = tmem + ((uint32_t)rw << 16) + kScanA + ch / 2;
-        const uint32_t plains = *decays.plain;
-        const int lm = rw + lane, m = m0 + lm;               // my row of the sums, whose columns ch .. ch + 31 I have
-        auto scale = [&](int m) {                            // the entering state belongs to the sequence that ends the previous chunk
-            if (m >= len || (a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0))) return 0.f;
-            return __expf(decays.dA[m]);
-        };
-        const float sc = scale(m);
-        auto skipped = [&](int t) { return (reinterpret_cast<volatile uint32_t *>(skip)[t >> 5] >> (t & 31)) & 1; };
-        auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + kScanB + r * 256 + ((chunk ^ (r & 7)) << 4)); };
-        auto wait_done = [&](int i) {
-            ok = ok && __all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1, status, kStSplitScan));
-            if (ok) tc_fence_after_sync();
-            return ok;
-        };
-        auto finish = [&](int i, bool bad) {                 // my part of tile i is in place
-            tmem_st_wait();
-            fence_proxy_async();
-            tc_fence_before_sync();
-            if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&skip[i >> 5], 1u << (i & 31));
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[i & 1]);
-        };
-        // columns j .. j + 7 of my row's sums
-        const uint32_t sums = tmem + ((uint32_t)rw << 16);
-        auto load_sums = [&](int j, float (&y)[8]) {
-            uint32_t u[8], w[8];
-            tmem_ld8_issue(sums + j, u);
-            tmem_ld8_issue(sums + 64 + j, w);
-            tmem_ld_wait(u, w);
+        __syncwarp();
+        begun = begun || on;
+    };
+    const uint32_t at = tmem + ((uint32_t)rw << 16) + kScanA + ch / 2;
+    const uint32_t plains = *decays.plain;
+    const int lm = rw + lane, m = m0 + lm;               // my row of the sums, whose columns ch .. ch + 31 I have
+    auto scale = [&](int m) {                            // the entering state belongs to the sequence that ends the previous chunk
+        if (m >= len || (a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0))) return 0.f;
+        return __expf(decays.dA[m]);
+    };
+    const float sc = scale(m);
+    auto skipped = [&](int t) { return (reinterpret_cast<volatile uint32_t *>(skip)[t >> 5] >> (t & 31)) & 1; };
+    auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + kScanB + r * 256 + ((chunk ^ (r & 7)) << 4)); };
+    auto wait_done = [&](int i) {
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1, status, kStSplitScan));
+        if (ok) tc_fence_after_sync();
+        return ok;
+    };
+    auto finish = [&](int i, bool bad) {                 // my part of tile i is in place
+        tmem_st_wait();
+        fence_proxy_async();
+        tc_fence_before_sync();
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&skip[i >> 5], 1u << (i & 31));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[i & 1]);
+    };
+    // columns j .. j + 7 of my row's sums
+    const uint32_t sums = tmem + ((uint32_t)rw << 16);
+    auto load_sums = [&](int j, float (&y)[8]) {
+        uint32_t u[8], w[8];
+        tmem_ld8_issue(sums + j, u);
+        tmem_ld8_issue(sums + 64 + j, w);
+        tmem_ld_wait(u, w);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(u[e]) + __uint_as_float(w[e]);
-        };
+        for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(u[e]) + __uint_as_float(w[e]);
+    };
 
-        // ---- the state entering the chunk: C . H
-        int i = 0;
+    // ---- the state entering the chunk: C . H
+    int i = 0;
 #pragma unroll 1
-        for (int n = 0; n < N; n += 64, ++i) {
-            if (i > 0 && !wait_done(i - 1)) break;
-            bool bad = false;
+    for (int n = 0; n < N; n += 64, ++i) {
+        if (i > 0 && !wait_done(i - 1)) break;
+        bool bad = false;
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const float v[8] = {Hr[r][0].x, Hr[r][0].y, Hr[r][1].x, Hr[r][1].y, Hr[r][2].x, Hr[r][2].y, Hr[r][3].x, Hr[r][3].y};
-                bad = store_parts<NP>(tiles + sw128(r0 + 32 * r, c8), kTileB, v) || bad;
-            }
-            Finite<__nv_bfloat16> f;
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                uint32_t w[NP][8];
-#pragma unroll
-                for (int hr = 0; hr < 2; ++hr) {
-                    float v[8];
-                    widen8<T>(Cr[2 * hh + hr], v);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t parts[NP];
-                        cut2<NP>(pack2(v[2 * q], v[2 * q + 1]), parts);
-                        f.feed(parts[0]);
-#pragma unroll
-                        for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
-                    }
-                }
-#pragma unroll
-                for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
-            }
-            if (n + 64 < N) fetch_states(n + 64);
-            else fetch_x(0);
-            finish(i, bad || f.bad());
+        for (int r = 0; r < 2; ++r) {
+            const float v[8] = {Hr[r][0].x, Hr[r][0].y, Hr[r][1].x, Hr[r][1].y, Hr[r][2].x, Hr[r][2].y, Hr[r][3].x, Hr[r][3].y};
+            bad = store_parts<NP>(tiles + sw128(r0 + 32 * r, c8), kTileB, v) || bad;
         }
+        Finite<__nv_bfloat16> f;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            uint32_t w[NP][8];
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                float v[8];
+                widen8<T>(Cr[2 * hh + hr], v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t parts[NP];
+                    cut2<NP>(pack2(v[2 * q], v[2 * q + 1]), parts);
+                    f.feed(parts[0]);
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
+        }
+        if (n + 64 < N) fetch_states(n + 64);
+        else fetch_x(0);
+        finish(i, bad || f.bad());
+        issue(i);
+    }
 
-        // ---- steps of the chunk up to the diagonal
+    // ---- steps of the chunk up to the diagonal
 #pragma unroll 1
-        for (int k = 0; k < kend && ok; k += 64, ++i) {
-            if (!wait_done(i - 1)) break;
-            if (k == 0) {
-                // the sums over the states, times exp(dA_m), are where those over the steps begin
-                bool any = false;
-                for (int t = 0; t < nH; ++t) any = any || !skipped(t);
+    for (int k = 0; k < kend && ok; k += 64, ++i) {
+        if (!wait_done(i - 1)) break;
+        if (k == 0) {
+            // the sums over the states, times exp(dA_m), are where those over the steps begin
+            bool any = false;
+            for (int t = 0; t < nH; ++t) any = any || !skipped(t);
 #pragma unroll 1
-                for (int j = ch; j < ch + 32; j += 8) {
-                    float y[8];
-                    uint32_t u[8];
-                    load_sums(j, y);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) u[e] = any ? __float_as_uint(sc * y[e]) : 0u;
-                    tmem_st8_issue(sums + j, u);
-                    const uint32_t none[8] = {};
-                    tmem_st8_issue(sums + 64 + j, none);
-                }
-            }
-            bool bad = false;
-#pragma unroll
-            for (int r = 0; r < 2; ++r) bad = store_input<T>(tiles + sw128(place4(r0 + 32 * r), c8), kTileB, xr[r]) || bad;
-            if (k + 64 < kend) fetch_x(k + 64);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncwarp();
-            if (m0 + rw + 31 < k + ch) {
-                const uint32_t none[8] = {};
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    tmem_st_16x128b_x4(at + 32 * p, none);
-                    tmem_st_16x128b_x4(at + 32 * p + (16u << 16), none);
-                }
-            } else {
-                Finite<__nv_bfloat16> f;
-                if (!((plains >> ((k + ch) >> 5)) & 1)) {
-                    uint64_t fk[4];                          // of my columns 16 q + 4 j .. + 3
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(decays.ck + k + ch + 4 * j4 + 16 * q);
-                        fk[2 * q] = v.x;
-                        fk[2 * q + 1] = v.y;
-                    }
-                    const uint32_t from = ring + ((k >> 6) & 1) * 32768 + (lane >> 2) * 128 + j4 * 16, flip = (lane & 4) << 4;       // (row & 1 = lane / 4 & 1)
-                    const bool diagonal = k + ch + 31 > m0 + rw;
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        uint32_t w[NP][8];
-#pragma unroll
-                        for (int hr = 0; hr < 2; ++hr) {
-                            const int r = 2 * hh + hr;
-                            uint64_t cbv[4];
-#pragma unroll
-                            for (int q = 0; q < 2; ++q)
-                                asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
-                            const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
-                            const float fm = decays.row(m0 + ra + 8 * r, (k + ch) >> 5);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));
-                                if (diagonal) {
-                                    float v0, v1;
-                                    unpack2(v, v0, v1);
-                                    const int e = 16 * (q >> 1) + 2 * (q & 1);
-                                    v = pack2(e <= past ? v0 : 0.f, e + 1 <= past ? v1 : 0.f);
-                                }
-                                uint32_t parts[NP];
-                                cut2<NP>(v, parts);
-                                f.feed(parts[0]);
-#pragma unroll
-                                for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
-                            }
-                        }
-#pragma unroll
-                        for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
-                    }
-                } else {
-                    // rare, and kept short: one word of two rows at a time
-#pragma unroll 1
-                    for (int e = 0; e < 8; ++e) {
-                        const int q = e & 3, hh = e >> 2, kk = k + ch + 4 * j4 + 16 * (q >> 1) + 2 * (q & 1);
-                        uint32_t w[2][NP];
-#pragma unroll
-                        for (int hr = 0; hr < 2; ++hr) {
-                            const int rr = ra + 8 * (2 * hh + hr), m = m0 + rr;
-                            auto one = [&](int kk) { return m < len && kk <= m ? cbm[(int64_t)rr * Q + kk] * ex2(fminf(dAc[m] - dAc[kk], 0.f) * kLog2e) * dtc[kk] : 0.f; };
-                            cut2<NP>(pack2(one(kk), one(kk + 1)), w[hr]);
-                            f.feed(w[hr][0]);
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int p = 0; p < NP; ++p) tmem_st_16x128b(at + 32 * p + 4 * q + ((16u * hh) << 16), w[0][p], w[1][p]);
-                    }
-                }
-                bad = f.bad() || bad;
-            }
-            __syncwarp();
-            request_cb(k + 64 * kAhead);
-            finish(i, bad);
-        }
-
-        // ---- x and z of my rows are on their way while the last products are formed
-        const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
-        const bool vz = z && rows16(z, a.z_stride[1]);
-        const int left = P - p0 - 8 * c8;
-        Raw8<T> xm[4], zm[4];
-        if (whole_rows && whole_cols && vx && (!z || vz)) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int64_t m = m0 + r0 + 32 * r;
-                if (a.D) xm[r] = load8_whole(x + m * a.x_stride[1] + 8 * c8);
-                if (z) zm[r] = load8_whole(z + m * a.z_stride[1] + 8 * c8);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int64_t m = m0 + r0 + 32 * r;
-                if (a.D) xm[r] = load8(x + m * a.x_stride[1] + 8 * c8, vx, m < len ? left : 0);
-                if (z) zm[r] = load8(z + m * a.z_stride[1] + 8 * c8, vz, m < len ? left : 0);
-            }
-        }
-        wait_done(ntiles - 1);
-        uint32_t every;                                      // (also: everyone's writes to the skip words are there, and C.B^T is not needed any more)
-        asm volatile("{\n\t.reg .pred q, o;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred o, 1, 256, q;\n\tselp.u32 %0, 1, 0, o;\n\t}" : "=r"(every) : "r"((uint32_t)ok) : "memory");
-        if (every) {
-            bool fma = false;                                // something is left
-            for (int t = 0; t < ntiles; ++t) fma = fma || skipped(t);
-            // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
-            tc_fence_after_sync();
-#pragma unroll
             for (int j = ch; j < ch + 32; j += 8) {
                 float y[8];
+                uint32_t u[8];
                 load_sums(j, y);
-                *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
-                *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) u[e] = any ? __float_as_uint(sc * y[e]) : 0u;
+                tmem_st8_issue(sums + j, u);
+                const uint32_t none[8] = {};
+                tmem_st8_issue(sums + 64 + j, none);
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
-            const bool vo = rows16(out, a.out_stride[1]);
-            if (fma) {
-#pragma unroll 1
-                for (int r = r0; r < 128; r += 32)
-                    if (m0 + r < len && left > 0)
-                        add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
-                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
+        }
+        bool bad = false;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) bad = store_input<T>(tiles + sw128(place4(r0 + 32 * r), c8), kTileB, xr[r]) || bad;
+        if (k + 64 < kend) fetch_x(k + 64);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        if (m0 + rw + 31 < k + ch) {
+            const uint32_t none[8] = {};
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                tmem_st_16x128b_x4(at + 32 * p, none);
+                tmem_st_16x128b_x4(at + 32 * p + (16u << 16), none);
             }
+        } else {
+            Finite<__nv_bfloat16> f;
+            if (!((plains >> ((k + ch) >> 5)) & 1)) {
+                uint64_t fk[4];                          // of my columns 16 q + 4 j .. + 3
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = r0 + 32 * q;
-                if (m0 + r >= len || left <= 0) continue;
-                const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
-                float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
-                if (a.D) {
-                    widen8<T>(xm[q], f);
-                    if (!a.D_has_hdim) {
+                for (int q = 0; q < 2; ++q) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(decays.ck + k + ch + 4 * j4 + 16 * q);
+                    fk[2 * q] = v.x;
+                    fk[2 * q + 1] = v.y;
+                }
+                const uint32_t from = ring + ((k >> 6) & 1) * 32768 + (lane >> 2) * 128 + j4 * 16, flip = (lane & 4) << 4;       // (row & 1 = lane / 4 & 1)
+                const bool diagonal = k + ch + 31 > m0 + rw;
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dh, y[e]);
-                    } else {
+                for (int hh = 0; hh < 2; ++hh) {
+                    uint32_t w[NP][8];
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (e < left) y[e] = fmaf(f[e], a.D[(int64_t)h * P + p0 + 8 * c8 + e], y[e]);
+                    for (int hr = 0; hr < 2; ++hr) {
+                        const int r = 2 * hh + hr;
+                        uint64_t cbv[4];
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
+                        const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
+                        const float fm = decays.row(m0 + ra + 8 * r, (k + ch) >> 5);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));
+                            if (diagonal) {
+                                float v0, v1;
+                                unpack2(v, v0, v1);
+                                const int e = 16 * (q >> 1) + 2 * (q & 1);
+                                v = pack2(e <= past ? v0 : 0.f, e + 1 <= past ? v1 : 0.f);
+                            }
+                            uint32_t parts[NP];
+                            cut2<NP>(v, parts);
+                            f.feed(parts[0]);
+#pragma unroll
+                            for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
+                        }
                     }
-                }
-                if (z) {
-                    widen8<T>(zm[q], f);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) y[e] *= silu(f[e]);
+                    for (int p = 0; p < NP; ++p) tmem_st_16x128b_x4(at + 32 * p + ((16u * hh) << 16), w[p]);
                 }
-                Raw8<T> o;
-                T *oe = reinterpret_cast<T *>(&o);
+            } else {
+                // rare, and kept short: one word of two rows at a time
+#pragma unroll 1
+                for (int e = 0; e < 8; ++e) {
+                    const int q = e & 3, hh = e >> 2, kk = k + ch + 4 * j4 + 16 * (q >> 1) + 2 * (q & 1);
+                    uint32_t w[2][NP];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
-                T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
-                if (vo && left >= 8) {
-                    *reinterpret_cast<Raw8<T> *>(om) = o;
+                    for (int hr = 0; hr < 2; ++hr) {
+                        const int rr = ra + 8 * (2 * hh + hr), m = m0 + rr;
+                        auto one = [&](int kk) { return m < len && kk <= m ? cbm[(int64_t)rr * Q + kk] * ex2(fminf(dAc[m] - dAc[kk], 0.f) * kLog2e) * dtc[kk] : 0.f; };
+                        cut2<NP>(pack2(one(kk), one(kk + 1)), w[hr]);
+                        f.feed(w[hr][0]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) tmem_st_16x128b(at + 32 * p + 4 * q + ((16u * hh) << 16), w[0][p], w[1][p]);
+                }
+            }
+            bad = f.bad() || bad;
+        }
+        __syncwarp();
+        finish(i, bad);
+        issue(i);
+        request_cb(k + 64 * kAhead);
+    }
+
+    // ---- x and z of my rows are on their way while the last products are formed
+    const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
+    const bool vz = z && rows16(z, a.z_stride[1]);
+    const int left = P - p0 - 8 * c8;
+    Raw8<T> xm[4], zm[4];
+    if (whole_rows && whole_cols && vx && (!z || vz)) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int64_t m = m0 + r0 + 32 * r;
+            if (a.D) xm[r] = load8_whole(x + m * a.x_stride[1] + 8 * c8);
+            if (z) zm[r] = load8_whole(z + m * a.z_stride[1] + 8 * c8);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int64_t m = m0 + r0 + 32 * r;
+            if (a.D) xm[r] = load8(x + m * a.x_stride[1] + 8 * c8, vx, m < len ? left : 0);
+            if (z) zm[r] = load8(z + m * a.z_stride[1] + 8 * c8, vz, m < len ? left : 0);
+        }
+    }
+    wait_done(ntiles - 1);
+    if (__syncthreads_and(ok)) {                         // (also: everyone's writes to the skip words are there, and C.B^T is not needed any more)
+        bool fma = false;                                // something is left
+        for (int t = 0; t < ntiles; ++t) fma = fma || skipped(t);
+        // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
+        tc_fence_after_sync();
+#pragma unroll
+        for (int j = ch; j < ch + 32; j += 8) {
+            float y[8];
+            load_sums(j, y);
+            *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
+            *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
+        }
+        __syncthreads();
+        T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
+        const bool vo = rows16(out, a.out_stride[1]);
+        if (fma) {
+#pragma unroll 1
+            for (int r = r0; r < 128; r += 32)
+                if (m0 + r < len && left > 0)
+                    add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
+                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + 32 * q;
+            if (m0 + r >= len || left <= 0) continue;
+            const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
+            float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
+            if (a.D) {
+                widen8<T>(xm[q], f);
+                if (!a.D_has_hdim) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dh, y[e]);
                 } else {
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        if (e < left) om[e] = oe[e];
+                        if (e < left) y[e] = fmaf(f[e], a.D[(int64_t)h * P + p0 + 8 * c8 + e], y[e]);
                 }
+            }
+            if (z) {
+                widen8<T>(zm[q], f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) y[e] *= silu(f[e]);
+            }
+            Raw8<T> o;
+            T *oe = reinterpret_cast<T *>(&o);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
+            T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
+            if (vo && left >= 8) {
+                *reinterpret_cast<Raw8<T> *>(om) = o;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (e < left) om[e] = oe[e];
             }
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (mma_warp) tmem_dealloc(tmem, 256);
+    if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
 struct Buffers {
@@ -1399,7 +1390,7 @@ int ssd_split_scan(const mb200_ssd_args &a, const SsdScratch &lay, cudaStream_t 
             if (a.headdim > 64 && singles > 2 * sm_count(a.device)) go(ssd_split_scan16_kernel<T, 2>, kThreads, kScan16A<T> + kScan16B<T, 2> + kTail, 128);
             else go(ssd_split_scan16_kernel<T, 1>, kThreads, kScan16A<T> + kScan16B<T, 1> + kTail, 64);
         } else {
-            go(ssd_split_scan_kernel, kScanThreads, kScanTiles + kScanTail, 64);
+            go(ssd_split_scan_kernel, kThreads, kScanTiles + kScanTail, 64);
         }
         MB200_CHECK_LAUNCH("ssd outputs (split products)");
         return MB200_OK;

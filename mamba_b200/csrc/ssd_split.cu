@@ -5,7 +5,10 @@
 // weighted x, an entering state -- is cut into bf16 values that add up to it (three hold all 24 bits), and a half-precision input into two,
 // so that tcgen05.mma of bf16 operands forms the products, which it adds in fp32; terms below 2^-24 of a product are left out.  bf16 has
 // fp32's range: nothing overflows that fp32 holds, whatever the input type.  The tensor core cuts its sums off where fp32 arithmetic
-// rounds, so sums that leave in fp32 have the small products in a sum of their own.  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64:
+// rounds.  Sums that leave a 16-bit call in fp32 have the small products in a sum of their own; in fp32 calls the tensor core adds the products
+// of 64 steps only, the small ones first, and fp32 additions do the rest: without decays, where the sums are the whole error, states of 256
+// steps are 2.3e-7 from 64 bits, outputs 2.6e-7 (4.0e-7 and 6.4e-7 with two sums over all steps, 3.3e-7 and 4.3e-7 with tiles of fp32 FMAs;
+// 2 x 2048 steps of 8 heads of 64 x 64: 44.4 us for 43.6).  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64:
 // end states 1.6e-6 to 3.4e-6, outputs 1.66e-3 (bf16) and 2.07e-4 (fp16), which is their own rounding; fp32 outputs 0.86e-6 to 2.0e-6.  Tiles
 // of fp32 FMAs gave the same to within 2 %, operands rounded to 16 bits 1.7e-3 / 2.1e-4 and 2.4e-3 / 3.0e-4.
 //
@@ -158,6 +161,45 @@ __device__ __forceinline__ void multiply(int na, int nb, uint32_t d, uint32_t re
             }
     }
     __syncwarp();
+}
+
+// The same of fp32 operands, into a sum of the tile's own.  The small products come first, so that only the last ones meet a large sum.
+__device__ __forceinline__ void multiply_tile(uint32_t d, uint64_t a, uint32_t step_a, uint64_t b, uint32_t step_b, uint32_t idesc, uint32_t part_b = kTileB)
+{
+    if (elect_one()) {
+        bool more = false;
+#pragma unroll 1
+        for (int s = kParts - 1; s >= 0; --s)
+#pragma unroll 1
+            for (int i = 0; i <= s; ++i) {
+                mma_steps_ss(4, d, a + i * (kTileA / 16), step_a, b + (s - i) * (part_b / 16), step_b, idesc, more);
+                more = true;
+            }
+    }
+    __syncwarp();
+}
+// Tensor memory: a tile's products join the sum over the tiles (`first`: begin it), times `scale`; `cols` columns of my row.  The next MMAs may
+// follow a barrier.
+__device__ __forceinline__ void fold(uint32_t tile, uint32_t sum, int cols, bool on, bool first, float scale = 1.f)
+{
+#pragma unroll 1
+    for (int j = 0; j < cols; j += 16) {
+        uint32_t x[2][8], y[2][8];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            tmem_ld8_issue(tile + j + 8 * i, x[i]);
+            tmem_ld8_issue(sum + j + 8 * i, y[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            tmem_ld_wait(x[i], y[i]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[i][e] = __float_as_uint(((on ? __uint_as_float(x[i][e]) : 0.f) + (first ? 0.f : __uint_as_float(y[i][e]))) * scale);
+            tmem_st8_issue(sum + j + 8 * i, y[i]);
+        }
+    }
+    tmem_st_wait();
+    tc_fence_before_sync();
 }
 
 // What the kernels share: a pair of operand tiles, the barrier that the MMAs of a step arrive on, and tensor memory.
@@ -323,9 +365,18 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
     if (k0 < k1) fetch(k0);
     constexpr uint32_t idesc = instr_desc_f16(128, 64 * U, 1, 1, 1);
     uint32_t skipped = 0;                           // tiles left for the FMAs
+    const uint32_t mine_at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (U == 2 ? mine * 64 : (warp >> 2) * 32);       // my columns of the sums
+    int folded = 0;                                 // fp32: tiles whose products have joined the sum
+    auto fold_last = [&] {
+        if (sizeof(T) == 2 || t.issued == folded) return;
+        tc_fence_after_sync();
+        fold(mine_at, mine_at + 64 * U, 32 * U, true, folded == 0);
+        folded = t.issued;
+    };
 #pragma unroll 1
     for (int k = k0, i64 = 0; k < k1; k += 64, ++i64) {
         t.drain();
+        fold_last();
         bool bad = false;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -344,10 +395,16 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
         if (kEarly<T> && k + 64 < k1) fetch(k + 64);
         const bool first = t.issued == 0;
         if (!t.step(bad, [&] {
-            // the tensor core adds to a sum with less care than fp32 rounding: the small products have one of their own (with one for
-            // all, end states were 8 to 15 % further from 64 bits than the fp32 kernels' in chunks of 128; with two 1 to 2 %)
+            // (16 bits: with one sum for large and small products end states were 8 to 15 % further from 64 bits than tiles of fp32 FMAs in chunks
+            // of 128; with two 1 to 2 %)
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kInParts<T>, kParts, acc, acc + 64 * U, smem_desc_sw128(t.a, 8192, 1024), 128, smem_desc_sw128(t.b, kTileB, 1024), 128, idesc, !first, U * kTileB);
+            const uint64_t da = smem_desc_sw128(t.a, 8192, 1024), db = smem_desc_sw128(t.b, kTileB, 1024);
+            if constexpr (sizeof(T) == 4) {
+                tc_fence_after_sync();
+                multiply_tile(acc, da, 128, db, 128, idesc, U * kTileB);
+            } else {
+                multiply(kInParts<T>, kParts, acc, acc + 64 * U, da, 128, db, 128, idesc, !first, U * kTileB);
+            }
         })) skipped |= 1u << i64;
         if (!kEarly<T> && k + 64 < k1) fetch(k + 64);
     }
@@ -367,12 +424,11 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = 0.f;
         if (formed) {                               // tcgen05.ld is warp-collective
-            const uint32_t at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + mine * 64 + pc - my_p0;
             float rest[32];
-            tmem_ld32(at, v);
-            tmem_ld32(at + 64 * U, rest);
+            tmem_ld32(mine_at + 32 * half, v);
+            tmem_ld32(mine_at + 32 * half + 64 * U, rest);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += rest[j];
+            for (int j = 0; j < 32; ++j) v[j] = sizeof(T) == 2 ? v[j] + rest[j] : (t.issued > folded ? v[j] : 0.f) + (folded > 0 ? rest[j] : 0.f);
         }
         if (!live) continue;
         if (skipped) {
@@ -416,7 +472,7 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
     const int b = chunk / nchunks, c = chunk % nchunks, len = min(Q, a.seqlen - c * Q);
     if (k0 >= m0 + 128 || m0 >= len || k0 >= len) return;
     Tile t;
-    constexpr int kSums = sizeof(T) == 2 ? 64 : 128;     // columns of tensor memory: fp32's small products have a sum of their own, as in the chunk states
+    constexpr int kSums = sizeof(T) == 2 ? 64 : 128;     // columns of tensor memory: in fp32 the products of a tile, and the sum over the tiles
     t.open(smem, kCbParts<T> * kTileA, kCbParts<T> * kTileB, kSums, status, kStSplitCb);
     pdl_wait();
     const int64_t t0 = (int64_t)c * Q;
@@ -441,9 +497,15 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
     fetch(0);
     constexpr uint32_t idesc = instr_desc_f16(128, 64, std::is_same<T, __half>::value ? 0 : 1, 0, 0);
     bool all = true;                                // no tile left for the FMAs
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + (warp & 3) * 32 + lane, k = k0 + (warp >> 2) * 32;
+    const uint32_t mine_at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32;                // my columns of the sums
 #pragma unroll 1
     for (int n = 0; n < N; n += 64) {
         t.drain();
+        if (sizeof(T) == 4 && n > 0 && all) {
+            tc_fence_after_sync();
+            fold(mine_at, mine_at + 64, 32, true, n == 64);
+        }
         bool bad = false;
         auto store = [&](uint32_t to, uint32_t stride, const Raw8<T> &r) {
             if constexpr (sizeof(T) == 2) sts128(to, r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w);        // one product, exact: nothing to look for
@@ -457,23 +519,27 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
         const bool first = t.issued == 0;
         all = t.step(bad, [&] {
             const uint32_t acc = warp_uniform(t.tmem);
-            multiply(kCbParts<T>, kCbParts<T>, acc, acc + kSums - 64, smem_desc_sw128(t.a, 16, 1024), 2, smem_desc_sw128(t.b, 16, 1024), 2, idesc, !first);
+            const uint64_t da = smem_desc_sw128(t.a, 16, 1024), db = smem_desc_sw128(t.b, 16, 1024);
+            if constexpr (sizeof(T) == 4) {
+                tc_fence_after_sync();
+                multiply_tile(acc, da, 2, db, 2, idesc);
+            } else {
+                multiply(1, 1, acc, acc, da, 2, db, 2, idesc, !first);
+            }
         }) && all;
         if (!kEarly<T> && n + 64 < N) fetch(n + 64);
     }
     t.drain();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + (warp & 3) * 32 + lane, k = k0 + (warp >> 2) * 32;
     if (__all_sync(0xffffffffu, t.ok)) {
         float v[32];
         if (all) {
             tc_fence_after_sync();
-            const uint32_t from = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * 32;
-            tmem_ld32(from, v);
-            if constexpr (sizeof(T) == 4) {
-                float rest[32];
-                tmem_ld32(from + 64, rest);
+            tmem_ld32(mine_at, v);
+            if (sizeof(T) == 4 && N > 64) {
+                float sum[32];
+                tmem_ld32(mine_at + 64, sum);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += rest[j];
+                for (int j = 0; j < 32; ++j) v[j] += sum[j];
             }
         } else {
 #pragma unroll
@@ -881,8 +947,8 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 // and the first issues its MMAs: the A operand (C, then CB with its decays) goes to tensor memory, B (H, then x) to shared memory.  A warp
 // has rows 32 (w % 4) .. and one half of the 64 columns; tcgen05.st.16x128b gives a lane four of these rows, and four lanes a row's 16
 // bytes, so that the loads fill whole sectors.  The order within a tile is free: a lane's four consecutive elements go to where its words
-// are, and B's rows (or H's columns) follow.  The small products have a sum of their own, as in the chunk states.  (A ninth warp for the MMAs
-// alone leaves a thread 96 registers for 128, because a quarter of the SM then has five warps: 600 bytes of spills for 84, 28.0 us for 26.2.)
+// are, and B's rows (or H's columns) follow.  (A ninth warp for the MMAs alone leaves a thread 96 registers for 128, because a quarter of the
+// SM then has five warps: 600 bytes of spills for 84, 28.0 us for 26.2.)
 // What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
 // middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its start, which overlaps the recurrence, included),
 // 2 x 3000 steps of 32 heads of 64 x 128 142; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
@@ -1035,7 +1101,6 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     __syncthreads();
     bool ok = true;
     // the operands of tile i are in place: the first warp issues its MMAs
-    bool begun = false;                                      // (its own) the sums hold something
     auto issue = [&](int i) {
         if (warp != 0) return;
         ok = ok && __all_sync(0xffffffffu, mbar_wait(&full[i & 1], (i >> 1) & 1, status, kStSplitScan));
@@ -1045,23 +1110,18 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         const uint64_t desc = smem_desc_sw128(tiles, 16, 1024);
         const bool steps = i >= nH, on = !((reinterpret_cast<volatile uint32_t *>(skip)[i >> 5] >> (i & 31)) & 1);
         const uint32_t step_b = steps ? 128 : 2, idesc = instr_desc_f16(128, 64, 1, 0, 0) | (steps ? instr_desc_f16(128, 64, 1, 0, 1) : 0);
-        begun = begun || steps;                              // (scaled, they do)
         if (elect_one()) {
-            if (on) {
-                mma_steps_ts(4, tm, A, desc, step_b, idesc, begun);
-                bool more = begun;
+            bool more = false;                               // (as in multiply_tile)
 #pragma unroll 1
-                for (int pa = 0; pa < NP; ++pa)
+            for (int s = NP - 1; s >= 0 && on; --s)
 #pragma unroll 1
-                    for (int pb = pa ? 0 : 1; pa + pb < NP; ++pb) {
-                        mma_steps_ts(4, tm + 64, A + 32 * pa, desc + pb * (kTileB / 16), step_b, idesc, more);
-                        more = true;
-                    }
-            }
+                for (int pa = 0; pa <= s; ++pa) {
+                    mma_steps_ts(4, tm, A + 32 * pa, desc + (s - pa) * (kTileB / 16), step_b, idesc, more);
+                    more = true;
+                }
             mma_commit(&done[i & 1]);
         }
         __syncwarp();
-        begun = begun || on;
     };
     const uint32_t at = tmem + ((uint32_t)rw << 16) + kScanA + ch / 2;
     const uint32_t plains = *decays.plain;
@@ -1086,22 +1146,22 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[i & 1]);
     };
-    // columns j .. j + 7 of my row's sums
-    const uint32_t sums = tmem + ((uint32_t)rw << 16);
-    auto load_sums = [&](int j, float (&y)[8]) {
-        uint32_t u[8], w[8];
-        tmem_ld8_issue(sums + j, u);
-        tmem_ld8_issue(sums + 64 + j, w);
-        tmem_ld_wait(u, w);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(u[e]) + __uint_as_float(w[e]);
+    const uint32_t tile_at = tmem + ((uint32_t)rw << 16) + ch, sum_at = tile_at + 64;        // my row's columns: a tile's products, the sum over the tiles
+    bool begun = false;                                  // that sum holds something
+    auto join = [&](int i, bool scaled) {                // the products of tile i join it; then times exp(dA_m)
+        const bool on = !skipped(i);
+        if (on || (begun && scaled)) fold(tile_at, sum_at, 32, on, !begun, scaled ? sc : 1.f);
+        begun = begun || on;
     };
 
     // ---- the state entering the chunk: C . H
     int i = 0;
 #pragma unroll 1
     for (int n = 0; n < N; n += 64, ++i) {
-        if (i > 0 && !wait_done(i - 1)) break;
+        if (i > 0) {
+            if (!wait_done(i - 1)) break;
+            join(i - 1, false);
+        }
         bool bad = false;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -1138,22 +1198,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 #pragma unroll 1
     for (int k = 0; k < kend && ok; k += 64, ++i) {
         if (!wait_done(i - 1)) break;
-        if (k == 0) {
-            // the sums over the states, times exp(dA_m), are where those over the steps begin
-            bool any = false;
-            for (int t = 0; t < nH; ++t) any = any || !skipped(t);
-#pragma unroll 1
-            for (int j = ch; j < ch + 32; j += 8) {
-                float y[8];
-                uint32_t u[8];
-                load_sums(j, y);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) u[e] = any ? __float_as_uint(sc * y[e]) : 0u;
-                tmem_st8_issue(sums + j, u);
-                const uint32_t none[8] = {};
-                tmem_st8_issue(sums + 64 + j, none);
-            }
-        }
+        join(i - 1, k == 0);
         bool bad = false;
 #pragma unroll
         for (int r = 0; r < 2; ++r) bad = store_input<T>(tiles + sw128(place4(r0 + 32 * r), c8), kTileB, xr[r]) || bad;
@@ -1260,12 +1305,18 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     if (__syncthreads_and(ok)) {                         // (also: everyone's writes to the skip words are there, and C.B^T is not needed any more)
         bool fma = false;                                // something is left
         for (int t = 0; t < ntiles; ++t) fma = fma || skipped(t);
+        const bool on = !skipped(ntiles - 1);
         // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
         tc_fence_after_sync();
 #pragma unroll
         for (int j = ch; j < ch + 32; j += 8) {
+            uint32_t u[8], w[8];
+            tmem_ld8_issue(tile_at + j - ch, u);
+            tmem_ld8_issue(sum_at + j - ch, w);
+            tmem_ld_wait(u, w);
             float y[8];
-            load_sums(j, y);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = (on ? __uint_as_float(u[e]) : 0.f) + (begun ? __uint_as_float(w[e]) : 0.f);
             *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
             *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
         }

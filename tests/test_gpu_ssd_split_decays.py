@@ -81,6 +81,19 @@ def test_weights_within_32_steps():
     assert (out[:, at + 1] / (dt * torch.exp(dt * inp["A"].double()[:, None])) - 1).abs().max() <= rounding + 2 * 2.0 ** -24 * (61 + 31) * decay
 
 
+@pytest.mark.parametrize("seed", [970, 971, 972])
+def test_fp32_sums_without_decay(seed):
+    """Next to no decay, so that the sums over 256 steps and over the states are the whole error.  FMAs one after the other round each of n sums
+    that grow as their square root by 0.29 ulp: 0.29 2^-23 sqrt(256 / 2) = 3.9e-7 for the states, of which 3.3e-7 was measured, and 4.3e-7 for
+    the outputs.  Sums left to the tensor core, which cuts off where FMAs round, were at 4.0e-7 and 6.4e-7."""
+    inp = make(seed, 2, 1500, 8, 64, 1, 64, torch.float32, has_z=False)
+    inp["A"] *= 1e-4
+    want, wfin = oracle.ssd_chunk_scan(inp["x"], inp["dt"], inp["A"], inp["B"], inp["C"], 256, inp["D"], None, inp["dt_bias"], None, dt_softplus=True)
+    c = {k: _c(v) for k, v in inp.items()}
+    got, fin = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 256, D=c["D"], dt_bias=c["dt_bias"], dt_softplus=True, return_final_states=True)
+    assert rel(fin, wfin) <= 3.3e-7 and rel(got, want) <= 4.3e-7, (rel(fin, wfin), rel(got, want))
+
+
 @pytest.mark.parametrize("P,N,H,Q,L", [(64, 64, 2, 256, 129), (128, 128, 1, 128, 257), (65, 66, 2, 64, 65), (7, 130, 1, 100, 101), (64, 64, 1, 1024, 1100), (1, 1, 1, 1, 3)])
 def test_fp32_shapes(P, N, H, Q, L):
     run(make(910 + P + N, 2, L, H, P, 1, N, torch.float32, has_z=L % 2 == 0, D_hdim=P % 2 == 0, init=True), Q, f"P{P} N{N} Q{Q} L{L}")

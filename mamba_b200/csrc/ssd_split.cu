@@ -267,7 +267,8 @@ __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { r
 // 128: 48 / 45, C.B^T included); in bf16, whose B is stored as it is, two CTAs per SM lose what it saves (2 x 3000 of 32 heads of 128 x 128:
 // 52 / 57), and so do the short sums of packed sequences (46 / 54).
 template <typename T, int U> constexpr uint32_t kStateB = kParts * U * kTileB;
-template <typename T, int U> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kStateB<T, U> + kTail;
+template <typename T, int U> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kStateB<T, U> + kTail;      // and the weights of the chunk's steps:
+template <int U> inline uint32_t state_weight_bytes(const mb200_ssd_args &a) { return U * ((a.chunk_size + 31) / 32 * 32) * 4; }
 template <typename T, bool PACKED, int U>
 __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_or_seq, int g, const mb200_ssd_args &a, const float *dtb, const float *dAb, const void *entering,
                                             SsdStates form, float *states, int nchunks, int *status)
@@ -328,8 +329,28 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
         for (int i = 0; i < 4 * U; ++i) in[i] = reinterpret_cast<const uint4 *>(static_cast<const T *>(entering) + (hc * N + n) * P + p)[i];
     }
 
+    // The weights: the distance of a step from the last of its 32 is summed within them and not taken from the chunk's sums, which are
+    // rounded to 2^-24 of their size (end states of 2 x 1500 steps of 16 heads of 64 x 64 were 2.9e-6 from 64 bits with those, and are 0.2e-6 to
+    // 1.0e-6).
+    float *const weights = reinterpret_cast<float *>(smem + kInParts<T> * kTileA + kStateB<T, U> + kTail);
+    const int ranges = (Q + 31) / 32 * 32;
+    auto form_weights = [&] {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            for (int k = (k0 & ~31) + (int)threadIdx.x; k < ((k1 + 31) & ~31); k += kThreads) {         // (a warp has a range of 32)
+                const float end = k1 > 0 ? dAc[u][min(k | 31, k1 - 1)] : 0.f, dt = k >= k0 && k < k1 ? dtc[u][k] : 0.f;
+                float after = dt * a.A[h[u]];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const float far = __shfl_down_sync(0xffffffffu, after, o);
+                    if (lane + o < 32) after += far;
+                }
+                after = __shfl_down_sync(0xffffffffu, after, 1);
+                const bool on = PACKED || !a.seq_idx || (k < k1 && seq_at(a, b, c * Q + k) == seq_last);
+                weights[u * ranges + k] = on ? __expf(fminf(dA_end[u] - end + (lane < 31 ? after : 0.f), 0.f)) * dt : 0.f;
+            }
+    };
     Raw8<T> xr[U][2], Br[4];
-    float w[U][2];
     const bool whole = vx && vB && whole_p && N - n0 >= (wide ? 128 : 64) && (PACKED || !a.seq_idx);
     auto fetch = [&](int k) {
         if (whole && k + 64 <= k1) {                // no edge, nothing to look at
@@ -340,10 +361,7 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
                 Br[i] = load8_whole(Bk);
                 if (wide) Br[2 + i] = load8_whole(Bk + 64);
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    xr[u][i] = load8_whole(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8);
-                    w[u][i] = __expf(fminf(dA_end[u] - dAc[u][kk], 0.f)) * dtc[u][kk];
-                }
+                for (int u = 0; u < U; ++u) xr[u][i] = load8_whole(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8);
             }
             return;
         }
@@ -353,16 +371,15 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             bool on = kk < k1;
             if (!PACKED && a.seq_idx) on = on && seq_at(a, b, c * Q + kk) == seq_last;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                xr[u][i] = load8(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, on ? P - p0[u] - 8 * c8 : 0);
-                w[u][i] = on ? __expf(fminf(dA_end[u] - dAc[u][kk], 0.f)) * dtc[u][kk] : 0.f;
-            }
+            for (int u = 0; u < U; ++u) xr[u][i] = load8(x[u] + (int64_t)kk * a.x_stride[1] + 8 * c8, vx, on ? P - p0[u] - 8 * c8 : 0);
             const T *Bk = B + (int64_t)kk * a.B_stride[1] + 8 * c8;
             Br[i] = load8(Bk, vB, kk < k1 ? N - n0 - 8 * c8 : 0);
             if (wide) Br[2 + i] = load8(Bk + 64, vB, kk < k1 ? N - n0 - 64 - 8 * c8 : 0);
         }
     };
     if (k0 < k1) fetch(k0);
+    form_weights();
+    __syncthreads();
     constexpr uint32_t idesc = instr_desc_f16(128, 64 * U, 1, 1, 1);
     uint32_t skipped = 0;                           // tiles left for the FMAs
     const uint32_t mine_at = t.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (U == 2 ? mine * 64 : (warp >> 2) * 32);       // my columns of the sums
@@ -385,8 +402,10 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             for (int u = 0; u < U; ++u) {
                 float v[8];
                 widen8<T>(xr[u][i], v);
+                const int kk = k + r0 + 32 * i;
+                const float w = kk < k1 ? weights[u * ranges + kk] : 0.f;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] *= w[u][i];
+                for (int e = 0; e < 8; ++e) v[e] *= w;
                 bad = store_parts<kParts>(t.b + u * kTileB + o, U * kTileB, v) || bad;
             }
             bad = store_input<T>(t.a + o, kTileA, Br[i]) || bad;                // states n0 .. n0 + 63, then the other 64
@@ -411,7 +430,6 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
     t.drain();
     const bool formed = __all_sync(0xffffffffu, t.ok && t.issued > 0);
     const bool live = n < N && unit0 + mine < hpg * tilesP;
-    const float *my_dAc = U == 2 && mine ? dAc[U - 1] : dAc[0], *my_dtc = U == 2 && mine ? dtc[U - 1] : dtc[0];
     const float my_end = U == 2 && mine ? dA_end[U - 1] : dA_end[0], decay = carry ? __expf(my_end) : 0.f;
     const T *my_x = U == 2 && mine ? x[U - 1] : x[0];
     const int my_p0 = U == 2 && mine ? p0[U - 1] : p0[0];
@@ -436,7 +454,7 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             for (int k = k0; k < k1; ++k) {
                 if (!((skipped >> (k - k0) / 64) & 1)) continue;
                 if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
-                const float wk = __expf(fminf(my_end - my_dAc[k], 0.f)) * my_dtc[k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
+                const float wk = weights[mine * ranges + k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
                     if (pc + j < P) v[j] = fmaf(to_float(my_x[(int64_t)k * a.x_stride[1] + pc - my_p0 + j]) * wk, Bn, v[j]);
@@ -1402,8 +1420,8 @@ template <bool PACKED> int run_first(const mb200_ssd_args &a, const SsdScratch &
             const int64_t state_ctas = with_states ? rows * state_tiles * a.ngroups : 0, ctas = state_ctas + cb_ctas;
             if (ctas == 0) return MB200_OK;
             if (ctas > INT32_MAX) return fail(MB200_ERR_BAD_ARG, "ssd: too many chunks and heads");
-            const uint32_t smem = state_ctas == 0 ? kCbSmem<T> : std::max(kStateSmem<T, U>, kCbSmem<T>);
-            ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_first_kernel<T, PACKED, U>), (int)std::max(kStateSmem<T, U>, kCbSmem<T>), a.device);
+            const uint32_t both = std::max(kStateSmem<T, U> + state_weight_bytes<U>(a), kCbSmem<T>), smem = state_ctas == 0 ? kCbSmem<T> : both;
+            ensure_dynamic_smem(reinterpret_cast<const void *>(&ssd_split_first_kernel<T, PACKED, U>), (int)both, a.device);
             launch_dependent(ssd_split_first_kernel<T, PACKED, U>, dim3((unsigned)ctas), kThreads, smem, stream, a, s.dt, s.dA, entering, form, PACKED ? a.varlen_states : s.states,
                              s.cb, (int)state_ctas, state_tiles, cb_tiles, lay.nchunks, s.status);
             MB200_CHECK_LAUNCH("ssd states and C.B^T (split products)");

@@ -81,6 +81,30 @@ def test_weights_within_32_steps():
     assert (out[:, at + 1] / (dt * torch.exp(dt * inp["A"].double()[:, None])) - 1).abs().max() <= rounding + 2 * 2.0 ** -24 * (61 + 31) * decay
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("packed", [False, True])
+def test_weights_of_end_states(dtype, packed):
+    """The only input of a sequence is the last but one: its end state is dt exp(-1.4) x B, though the chunk's sums reach 350, where they are rounded to 3e-5."""
+    lens = [67, 130, 250, 256, 40, 31, 301, 93] if packed else [245]
+    inp = _steady(make(974, 1, sum(lens), 2, 64, 1, 64, dtype, has_z=False), 1.4)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    dt, A = torch.full_like(inp["dt"], 0.125), torch.full_like(inp["A"], -11.2)
+    at = cu[1:].long() - 2
+    keep = torch.zeros(sum(lens), dtype=torch.bool).index_fill(0, at, True)
+    inp["x"][:, ~keep] = 0
+    kw = dict(return_final_states=True)
+    if packed:
+        seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens))[None].to(torch.int32)
+        kw.update(seq_idx=seq.to(DEV), cu_seqlens=cu.to(DEV), return_varlen_states=True)
+    got = _fn()(*(_c(t) for t in (inp["x"], dt, A, inp["B"], inp["C"])), 256, **kw)[-1].cpu().double()
+    step = dt.double()[0, 0, 0] * A.double()[0]
+    want = dt.double()[0, 0, 0] * torch.exp(step) * torch.einsum("shp,sn->shpn", inp["x"][0, at].double(), inp["B"][0, at, 0].double())
+    same = (at % 256) % 32 != 31                                    # (in the 32 steps of the last one)
+    # the exponential: 2 ulp and 2^-24 of its argument; the weight, the weighted x, their cut and the sum: a rounding each; truncation: 2^-23
+    bound = (2 * 2 + 1.4 + 4 + 2) * 2.0 ** -24
+    assert same.any() and ((got - want).abs() <= bound * want.abs())[same].all()
+
+
 @pytest.mark.parametrize("seed", [970, 971, 972])
 def test_fp32_sums_without_decay(seed):
     """Next to no decay, so that the sums over 256 steps and over the states are the whole error.  FMAs one after the other round each of n sums

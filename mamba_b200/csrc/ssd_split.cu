@@ -669,8 +669,9 @@ struct ScanDecays {
             }
         }
     }
-    // exp(dA_m - ref), ref = dA of the last of range `range`; before that range it only has to stay finite
-    __device__ __forceinline__ float row(int m, int range) const { return ex2(fminf(fmaf(dA[m | 31] - dA[32 * range + 31], kLog2e, rel[m]), kMaxSpan)); }
+    // exp(dA_m - ref) for a row `rel_m` before the last of its own range, ref = dA of the last of range `range`; rows before that range's only have
+    // to stay finite
+    __device__ __forceinline__ float row(float rel_m, float own_end, int range) const { return ex2(fminf(fmaf(own_end - dA[32 * range + 31], kLog2e, rel_m), kMaxSpan)); }
 };
 // Rare: what tiles with infinities or NaNs contribute to eight outputs of row m, in fp32.
 template <typename T>
@@ -771,6 +772,12 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
     decays.form(dAc, dtc, a.A[h], kend);
     __syncthreads();
     const uint32_t plains = *decays.plain;
+    float rel[4], own_end[4];                       // of my rows
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        rel[i] = decays.rel[m0 + r0 + 32 * i];
+        own_end[i] = decays.dA[m0 + 32 * i + 31];
+    }
     const int nH = (N + 63) / 64;
     bool left_out = false;                          // tiles have been left for the FMAs (a bit each in the skip words)
     auto leave_out = [&](int tile) {
@@ -828,7 +835,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
             }
             const float4 lo = A.f[2 * i], hi = A.f[2 * i + 1];
             uint64_t f[4] = {fk[0], fk[1], fk[2], fk[3]};
-            float fm = decays.row(m0 + r0 + 32 * i, range);
+            float fm = decays.row(rel[i], own_end[i], range);
             if (plain) {
                 const float dm = decays.dA[m0 + r0 + 32 * i];
                 fm = 1.f;
@@ -1253,7 +1260,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
                         for (int q = 0; q < 2; ++q)
                             asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
                         const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
-                        const float fm = decays.row(m0 + ra + 8 * r, (k + ch) >> 5);
+                        const float fm = decays.row(decays.rel[m0 + ra + 8 * r], decays.dA[m0 + rw + 31], (k + ch) >> 5);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));

@@ -515,6 +515,8 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // non-increasing (A <= 0, dt >= 0), so both exponents are <= 0 below the diagonal; in the range that holds the diagonal the row
 // factor is at most 2^kMaxDiagSpan and the columns past the diagonal meet a zero of C.B^T.  A 32-column range in which that
 // fails (a steeper decay, or dA not monotone) is done element by element: exp(min(dA_m - dA_k, 0)) dt_k.
+// Both exponents are differences of the same rounded products dA log2 e, so that those of a step's weight on itself cancel exactly: the
+// products are kept from being contracted into the differences, which would leave a residue of half an ulp of dA.
 // The factors are rounded to the input dtype and applied with packed 16-bit multiplies.
 constexpr float kMaxDiagSpan = 100.f;
 constexpr int kMaskWarps0 = 4, kMaskWarps1 = 8, kRowWarps = 4;      // that form the A operand, per row block; that finish the outputs of a row block
@@ -698,7 +700,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 if (lane == 0) mbar_arrive(bar(kBarScalFree + s));
                 continue;
             }
-            const float dAm = dA_next * kLog2e;
+            const float dAm = __fmul_rn(dA_next, kLog2e);
             if (left) dA_next = dA[(int64_t)nchunks * kQ + r];                           // a whole head ahead of its use
             const uint32_t flags = __float_as_uint(lds32(sc + 1024 + 128));
             const uint32_t A = tlane + (rb ? kA1 : kA0);
@@ -720,7 +722,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                     float f[4];
                     lds128f(sc + 1024 + 16 * j, f);
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) f[g] = ex2(fminf(dAm - f[g], kMaxDiagSpan));         // (a range past the diagonal only has to stay finite)
+                    for (int g = 0; g < 4; ++g) f[g] = ex2(fminf(__fsub_rn(dAm, f[g]), kMaxDiagSpan));         // (a range past the diagonal only has to stay finite)
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         uint64_t c[8];
@@ -1045,13 +1047,13 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 if (seq >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&b_scalfree[s], ((seq >> 1) - 1) & 1, status, kStOutScalFree));
                 if (!ok) break;
                 const float a[8] = {dA[0].x, dA[0].y, dA[0].z, dA[0].w, dA[1].x, dA[1].y, dA[1].z, dA[1].w};
-                const float end = a[7] * kLog2e;
+                const float end = __fmul_rn(a[7], kLog2e);
                 float before = __shfl_up_sync(0xffffffffu, a[7], 1);                 // dA of the step before mine
                 if (lane == 0) before = a[0];
                 bool mono = true;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) mono = mono && a[i] <= (i ? a[i - 1] : before) + 2e-6f * fabsf(i ? a[i - 1] : before);      // rounding of the sums aside
-                auto factor = [&](int i, float t) { return ex2(end - a[i] * kLog2e) * t; };
+                auto factor = [&](int i, float t) { return ex2(__fsub_rn(end, __fmul_rn(a[i], kLog2e))) * t; };
                 *reinterpret_cast<float4 *>(ck + 8 * lane) = make_float4(factor(0, dt[0].x), factor(1, dt[0].y), factor(2, dt[0].z), factor(3, dt[0].w));
                 *reinterpret_cast<float4 *>(ck + 8 * lane + 4) = make_float4(factor(4, dt[1].x), factor(5, dt[1].y), factor(6, dt[1].z), factor(7, dt[1].w));
                 ref[lane] = end;

@@ -43,6 +43,20 @@ def test_decays_steeper_than_the_factorised_mask(dtype, A):
     run_both(inp, 256, TOL_BF16, f"A {A}")
 
 
+@pytest.mark.parametrize("dtype,tie", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+def test_weight_of_a_step_on_itself(dtype, tie):
+    """On 16-bit operands: dt, though it is formed with two exponents from sums of up to 500.  Here it lies 1e-6 below the middle between 1 and the
+    next number of the input type and has to be rounded to 1; two exponentials of 2^-22 do not reach that middle, half an ulp of the sums does.
+    Inputs 73 steps apart, at every place of eight, so that what came before has decayed to nothing."""
+    L, H = 73 * 64, 2
+    x, B = torch.zeros(1, L, H, 64, dtype=dtype), torch.zeros(1, L, 1, 128, dtype=dtype)
+    x[:, ::73] = 1.0
+    B[..., 0] = 1.0
+    dt, A = torch.full((1, L, H), (1.0 + tie) * (1 - 1e-6)), torch.tensor([-0.7, -1.3])
+    out = _fn()(*(_c(t) for t in (x, dt, A, B, B)), 256).cpu()
+    assert _status() == 0 and torch.equal(out[:, ::73], x[:, ::73])
+
+
 @pytest.mark.parametrize("P,N,H,lens", [(64, 64, 4, [100, 156, 1, 300, 40]), (128, 128, 2, [257, 255, 130]), (40, 24, 2, [3, 128, 200]),
                                         (64, 128, 2, [1000, 1, 1400, 128])])
 def test_packed_sequences_and_their_end_states(P, N, H, lens):

@@ -7,7 +7,7 @@ import torch
 
 import oracle
 from test_gpu_ssd import DEV, _c, _fn, _packed, make
-from test_gpu_ssd_split import F32, rel, run
+from test_gpu_ssd_split import F32, check_out, rel, run
 
 pytestmark = pytest.mark.gpu
 
@@ -174,6 +174,61 @@ def test_two_heads_share_their_b(dtype, P, N, G, H):
 def test_two_column_tiles_share_their_a(dtype, P, N, H, L):
     """Enough chunks and heads for the outputs to go by two column tiles of a head, the second (third) of them ragged."""
     run(make(940 + P + N, 2, L, H, P, 1, N, dtype, has_z=P == 72, D_hdim=P == 200, init=True), 64, f"P{P} N{N} H{H}")
+
+
+# two heads of a group share B (U2: 64 columns, enough heads and chunks), or two column tiles of a head share A (W2: more columns)
+U2 = [(torch.float32, 64, 64, 15), (torch.float16, 64, 64, 15), (torch.float16, 72, 40, 9)]
+W2 = [(torch.bfloat16, 128, 64, 8), (torch.float16, 128, 64, 8), (torch.float16, 200, 130, 5)]
+
+
+@pytest.mark.parametrize("dtype,P,N,H", U2 + W2)
+def test_shared_operands_in_packed_sequences(dtype, P, N, H):
+    lens = [100, 156, 1, 300, 43, 64, 640, 63, 65, 568]
+    inp, seq_idx, cu = _packed(980 + P + N, lens, H, P, 1, N, dtype)
+    c = {k: _c(v) for k, v in inp.items()}
+    out, fin, var = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 64, D=c["D"], z=c["z"], dt_bias=c["dt_bias"], seq_idx=seq_idx.to(DEV), cu_seqlens=cu.to(DEV),
+                          dt_softplus=True, return_final_states=True, return_varlen_states=True)
+    f = lambda t: t.float()
+    for i in range(len(lens)):
+        sl = slice(int(cu[i]), int(cu[i + 1]))
+        want, wfin = oracle.ssd_chunk_scan(f(inp["x"][:, sl]), f(inp["dt"][:, sl]), inp["A"], f(inp["B"][:, sl]), f(inp["C"][:, sl]), 64, inp["D"], f(inp["z"][:, sl]),
+                                           inp["dt_bias"], None, dt_softplus=True)
+        check_out(out[:, sl], want, f"packed out seq {i}")
+        assert rel(var[i:i + 1], wfin) <= F32, f"end state of sequence {i}: {rel(var[i:i + 1], wfin):.3e}"
+    assert rel(fin, wfin) <= F32
+
+
+@pytest.mark.parametrize("dtype,P,N,H", U2 + W2)
+@pytest.mark.parametrize("name", ["x", "B"])
+def test_shared_operands_with_an_infinity(dtype, P, N, H, name):
+    """In the second of two heads, and in the second column tile where there is one: it stays in what it reaches."""
+    t, e = 140, P - 1 if name == "x" else 9
+    inp = make(990 + P + N, 2, 1000, H, P, 1, N, dtype, has_z=False, init=True)
+    f = lambda v: v.float()
+    want, wfin = oracle.ssd_chunk_scan(f(inp["x"]), f(inp["dt"]), inp["A"], f(inp["B"]), f(inp["C"]), 64, inp["D"], None, inp["dt_bias"], inp["initial_states"], dt_softplus=True)
+    inp[name][0, t, 1 if name == "x" else 0, e] = float("inf")
+    c = {k: _c(v) for k, v in inp.items()}
+    out, fin = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 64, D=c["D"], dt_bias=c["dt_bias"], initial_states=c["initial_states"], dt_softplus=True,
+                     return_final_states=True)
+    out, fin = out.cpu(), fin.cpu()
+    check_out(out[1], want[1], "other row")
+    check_out(out[0, :t], want[0, :t], "earlier steps")
+    assert rel(fin[1], wfin[1]) <= F32
+    if name == "x":
+        others, keep = torch.arange(H) != 1, torch.arange(P) != e
+        check_out(out[0, :, others], want[0, :, others], "other heads")
+        check_out(out[0, :, 1, keep], want[0, :, 1, keep], "other columns")
+        assert torch.isinf(out[0, t, 1, e]) and rel(fin[0, others], wfin[0, others]) <= F32 and rel(fin[0, 1, keep], wfin[0, 1, keep]) <= F32
+    else:
+        keep = torch.arange(N) != e
+        assert not torch.isfinite(out[0, t]).any() and rel(fin[0][..., keep], wfin[0][..., keep]) <= F32
+
+
+@pytest.mark.parametrize("dtype,P,N,H", U2 + W2)
+def test_shared_operands_and_decays_formed_one_by_one(dtype, P, N, H):
+    inp = make(1000 + P + N, 2, 1000, H, P, 1, N, dtype, has_z=False, init=True)
+    inp["A"][1], inp["A"][3] = -400.0, -40.0
+    run(inp, 64, f"steep P{P} N{N}")
 
 
 def test_end_states_of_many_short_sequences():

@@ -34,6 +34,11 @@ constexpr int kParts = 3;                               // of an fp32 value
 // of an input value
 template <typename T> constexpr int kInParts = std::is_same<T, __nv_bfloat16>::value ? 1 : std::is_same<T, __half>::value ? 2 : kParts;
 
+// fp32 operands are cut times 2^17: a value down to the smallest normal number then has all its parts among bf16's numbers, whose smallest is
+// 2^-133 (as they are, one of 1e-36 kept 10 bits).  Sums come out times 2^34.  What becomes too large for that, an operand or a sum, is left
+// to fp32 FMAs like what cannot be cut at all.
+constexpr float kLift = 0x1p17f, kDrop = 0x1p-34f;
+
 // The next tile is requested before the barrier that completes this one, whose cutting takes no time in bf16, or behind it (2 x 3000 steps of
 // 32 heads of 128 x 128 in bf16 187 us behind, 183 before; 2 x 1500 of 48 half-precision heads of 64 x 64 93 / 94.4, 2 x 2048 of 8 fp32
 // heads 44.2 / 45.3).
@@ -112,14 +117,15 @@ template <typename T> struct Finite {
     }
     __device__ __forceinline__ bool bad() const { return (sum & 0x7fff7fffu) != 0; }
 };
+__device__ __forceinline__ uint64_t lift2(float a, float b) { return mul2(pack2(a, b), pack2(kLift, kLift)); }
 // Eight values in NP parts, part p at addr + p * stride.
-template <int NP> __device__ __forceinline__ bool store_parts(uint32_t addr, uint32_t stride, const float (&v)[8])
+template <int NP, bool LIFT = false> __device__ __forceinline__ bool store_parts(uint32_t addr, uint32_t stride, const float (&v)[8])
 {
     uint32_t w[4][NP];
     Finite<__nv_bfloat16> f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        cut2<NP>(pack2(v[2 * i], v[2 * i + 1]), w[i]);
+        cut2<NP>(LIFT ? lift2(v[2 * i], v[2 * i + 1]) : pack2(v[2 * i], v[2 * i + 1]), w[i]);
         f.feed(w[i][0]);
     }
 #pragma unroll
@@ -138,7 +144,7 @@ template <typename T> __device__ __forceinline__ bool store_input(uint32_t addr,
     } else {
         float v[8];
         widen8<T>(raw, v);
-        return store_parts<kInParts<T>>(addr, stride, v);
+        return store_parts<kInParts<T>, sizeof(T) == 4>(addr, stride, v);
     }
 }
 // byte offset of 16-byte chunk `chunk` of row `row` in a tile of 128-byte rows
@@ -178,8 +184,8 @@ __device__ __forceinline__ void multiply_tile(uint32_t d, uint64_t a, uint32_t s
     }
     __syncwarp();
 }
-// Tensor memory: a tile's products join the sum over the tiles (`first`: begin it), times `scale`; `cols` columns of my row.  The next MMAs may
-// follow a barrier.
+// Tensor memory: a tile's (lifted) products join the sum over the tiles (`first`: begin it), times `scale`; `cols` columns of my row.  The next
+// MMAs may follow a barrier.
 __device__ __forceinline__ void fold(uint32_t tile, uint32_t sum, int cols, bool on, bool first, float scale = 1.f)
 {
 #pragma unroll 1
@@ -194,13 +200,15 @@ __device__ __forceinline__ void fold(uint32_t tile, uint32_t sum, int cols, bool
         for (int i = 0; i < 2; ++i) {
             tmem_ld_wait(x[i], y[i]);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[i][e] = __float_as_uint(((on ? __uint_as_float(x[i][e]) : 0.f) + (first ? 0.f : __uint_as_float(y[i][e]))) * scale);
+            for (int e = 0; e < 8; ++e) y[i][e] = __float_as_uint(fmaf(on ? __uint_as_float(x[i][e]) : 0.f, kDrop, first ? 0.f : __uint_as_float(y[i][e])) * scale);
             tmem_st8_issue(sum + j + 8 * i, y[i]);
         }
     }
     tmem_st_wait();
     tc_fence_before_sync();
 }
+
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= FLT_MAX; }
 
 // What the kernels share: a pair of operand tiles, the barrier that the MMAs of a step arrive on, and tensor memory.
 struct Tile {
@@ -403,7 +411,8 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
                 float v[8];
                 widen8<T>(xr[u][i], v);
                 const int kk = k + r0 + 32 * i;
-                const float w = kk < k1 ? weights[u * ranges + kk] : 0.f;
+                float w = kk < k1 ? weights[u * ranges + kk] : 0.f;
+                if (sizeof(T) == 4) w *= kLift;
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] *= w;
                 bad = store_parts<kParts>(t.b + u * kTileB + o, U * kTileB, v) || bad;
@@ -446,13 +455,24 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             tmem_ld32(mine_at + 32 * half, v);
             tmem_ld32(mine_at + 32 * half + 64 * U, rest);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = sizeof(T) == 2 ? v[j] + rest[j] : (t.issued > folded ? v[j] : 0.f) + (folded > 0 ? rest[j] : 0.f);
+            for (int j = 0; j < 32; ++j) v[j] = sizeof(T) == 2 ? v[j] + rest[j] : fmaf(t.issued > folded ? v[j] : 0.f, kDrop, folded > 0 ? rest[j] : 0.f);
         }
         if (!live) continue;
-        if (skipped) {
+        uint32_t fma_tiles = skipped;
+        if constexpr (sizeof(T) == 4) {
+            bool fits = true;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) fits = fits && finite(v[j]);
+            if (!fits) {                            // the lifted sums did not: all of it by FMAs
+                fma_tiles = ~0u;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = 0.f;
+            }
+        }
+        if (fma_tiles) {
 #pragma unroll 1
             for (int k = k0; k < k1; ++k) {
-                if (!((skipped >> (k - k0) / 64) & 1)) continue;
+                if (!((fma_tiles >> (k - k0) / 64) & 1)) continue;
                 if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
                 const float wk = weights[mine * ranges + k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
 #pragma unroll
@@ -553,15 +573,17 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
         if (all) {
             tc_fence_after_sync();
             tmem_ld32(mine_at, v);
-            if (sizeof(T) == 4 && N > 64) {
+            if constexpr (sizeof(T) == 4) {
                 float sum[32];
                 tmem_ld32(mine_at + 64, sum);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += sum[j];
+                for (int j = 0; j < 32; ++j) v[j] = fmaf(v[j], kDrop, N > 64 ? sum[j] : 0.f);
             }
-        } else {
+        }
+        if constexpr (sizeof(T) == 4) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
+                if (all && finite(v[j])) continue;      // (else the lifted sums did not fit, or a tile could not be cut)
                 v[j] = 0.f;
 #pragma unroll 1
                 for (int n = 0; n < N && m < len && k + j < len; ++n)
@@ -676,13 +698,17 @@ struct ScanDecays {
 // Rare: what tiles with infinities or NaNs contribute to eight outputs of row m, in fp32.
 template <typename T>
 __device__ __noinline__ void add_skipped(float4 *lo, float4 *hi, const uint32_t *skip, int nH, const float *cbrow, const float *dAc, const float *dtc, int m, float sc, const T *x,
-                                         int64_t x_stride, const T *Crow, const float *H, int N, int left)
+                                         int64_t x_stride, const T *Crow, const float *H, int N, int left, bool lifted)
 {
-    auto skipped = [&](int t) { return (skip[t >> 5] >> (t & 31)) & 1; };
+    bool every = false;                                 // sums of lifted operands that did not fit: all of it
+    if (lifted)
+        for (int e = 0; e < 8; ++e) every = every || !finite(reinterpret_cast<const float *>(e < 4 ? lo : hi)[e & 3]);
+    if (every) *lo = *hi = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto skipped = [&](int t) { return every || ((skip[t >> 5] >> (t & 31)) & 1); };
     float y[8] = {}, s[8] = {};
     for (int k = 0; k <= m; ++k) {
         if (!skipped(nH + (k >> 6))) continue;
-        const float w = cbrow[k] * ex2(fminf(dAc[m] - dAc[k], 0.f) * kLog2e) * dtc[k];
+        const float w = cbrow[k] * (__expf(fminf(dAc[m] - dAc[k], 0.f)) * dtc[k]);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
             if (e < left) y[e] = fmaf(w, to_float(x[k * x_stride + e]), y[e]);
@@ -930,7 +956,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
                 for (int r = r0; r < 128; r += 32)
                     if (m0 + r < len && left > 0)
                         add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), decays.skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + col, a.x_stride[1],
-                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)col * N, N, left);
+                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)col * N, N, left, false);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -1191,7 +1217,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float v[8] = {Hr[r][0].x, Hr[r][0].y, Hr[r][1].x, Hr[r][1].y, Hr[r][2].x, Hr[r][2].y, Hr[r][3].x, Hr[r][3].y};
-            bad = store_parts<NP>(tiles + sw128(r0 + 32 * r, c8), kTileB, v) || bad;
+            bad = store_parts<NP, true>(tiles + sw128(r0 + 32 * r, c8), kTileB, v) || bad;
         }
         Finite<__nv_bfloat16> f;
 #pragma unroll
@@ -1204,7 +1230,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     uint32_t parts[NP];
-                    cut2<NP>(pack2(v[2 * q], v[2 * q + 1]), parts);
+                    cut2<NP>(lift2(v[2 * q], v[2 * q + 1]), parts);
                     f.feed(parts[0]);
 #pragma unroll
                     for (int p = 0; p < NP; ++p) w[p][2 * q + hr] = parts[p];
@@ -1260,7 +1286,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
                         for (int q = 0; q < 2; ++q)
                             asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(cbv[2 * q]), "=l"(cbv[2 * q + 1]) : "r"(from + r * 1024 + ((q << 6) ^ flip)));
                         const int past = m0 + ra + 8 * r - (k + ch + 4 * j4);           // columns up to the diagonal
-                        const float fm = decays.row(decays.rel[m0 + ra + 8 * r], decays.dA[m0 + rw + 31], (k + ch) >> 5);
+                        const float fm = decays.row(decays.rel[m0 + ra + 8 * r], decays.dA[m0 + rw + 31], (k + ch) >> 5) * kLift;
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint64_t v = mul2(cbv[q], mul2(fk[q], pack2(fm, fm)));
@@ -1289,7 +1315,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
 #pragma unroll
                     for (int hr = 0; hr < 2; ++hr) {
                         const int rr = ra + 8 * (2 * hh + hr), m = m0 + rr;
-                        auto one = [&](int kk) { return m < len && kk <= m ? cbm[(int64_t)rr * Q + kk] * ex2(fminf(dAc[m] - dAc[kk], 0.f) * kLog2e) * dtc[kk] : 0.f; };
+                        auto one = [&](int kk) { return m < len && kk <= m ? cbm[(int64_t)rr * Q + kk] * (__expf(fminf(dAc[m] - dAc[kk], 0.f)) * dtc[kk] * kLift) : 0.f; };
                         cut2<NP>(pack2(one(kk), one(kk + 1)), w[hr]);
                         f.feed(w[hr][0]);
                     }
@@ -1328,7 +1354,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     }
     wait_done(ntiles - 1);
     if (__syncthreads_and(ok)) {                         // (also: everyone's writes to the skip words are there, and C.B^T is not needed any more)
-        bool fma = false;                                // something is left
+        bool fma = false, fits = true;                   // something is left; the lifted sums of my row did
         for (int t = 0; t < ntiles; ++t) fma = fma || skipped(t);
         const bool on = !skipped(ntiles - 1);
         // from tensor memory, where a thread has a row, to shared memory, so that eight lanes store a row's 64 columns together
@@ -1341,11 +1367,13 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
             tmem_ld_wait(u, w);
             float y[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = (on ? __uint_as_float(u[e]) : 0.f) + (begun ? __uint_as_float(w[e]) : 0.f);
+            for (int e = 0; e < 8; ++e) y[e] = fmaf(on ? __uint_as_float(u[e]) : 0.f, kDrop, begun ? __uint_as_float(w[e]) : 0.f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) fits = fits && finite(y[e]);
             *place(lm, j / 4) = make_float4(y[0], y[1], y[2], y[3]);
             *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
         }
-        __syncthreads();
+        fma = __syncthreads_or(!fits) || fma;
         T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
         const bool vo = rows16(out, a.out_stride[1]);
         if (fma) {
@@ -1353,7 +1381,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
             for (int r = r0; r < 128; r += 32)
                 if (m0 + r < len && left > 0)
                     add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
-                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left);
+                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left, true);
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

@@ -105,6 +105,17 @@ def test_weights_of_end_states(dtype, packed):
     assert same.any() and ((got - want).abs() <= bound * want.abs())[same].all()
 
 
+@pytest.mark.parametrize("x,B,C", [(1e-36, 1, 1), (1, 1e-36, 1), (1, 1, 1e-36), (1e20, 1e12, 1e-3), (1e-20, 1e15, 1e15), (1e37, 1e-10, 1e-20)])
+def test_fp32_keeps_its_range(x, B, C):
+    """Operands near the smallest normal number have all their bits, and operands and sums too large for the tensor core's are what fp32 holds."""
+    inp = make(976, 2, 300, 3, 64, 1, 64, torch.float32, has_z=False, init=True)
+    want, wfin = oracle.ssd_chunk_scan(inp["x"], inp["dt"], inp["A"], inp["B"], inp["C"], 256, None, None, inp["dt_bias"], inp["initial_states"], dt_softplus=True)
+    inp["x"], inp["B"], inp["C"], inp["initial_states"] = inp["x"] * x, inp["B"] * B, inp["C"] * C, inp["initial_states"] * (x * B)
+    c = {k: _c(v) for k, v in inp.items()}
+    out, fin = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 256, dt_bias=c["dt_bias"], initial_states=c["initial_states"], dt_softplus=True, return_final_states=True)
+    assert rel(out.double() / (x * B * C), want) <= F32 and rel(fin.double() / (x * B), wfin) <= F32
+
+
 @pytest.mark.parametrize("seed", [970, 971, 972])
 def test_fp32_sums_without_decay(seed):
     """Next to no decay, so that the sums over 256 steps and over the states are the whole error.  FMAs one after the other round each of n sums

@@ -811,8 +811,10 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             }
             dA += (int64_t)nchunks * kQ;
             const uint32_t row = smb + Cfg::kC + s * Cfg::kStage + r * 128;
-            ok = mbar_wait(bar(kBarZ + s), sph, status, kStOutGate);         // (x is there when its product is)
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarAcc + rb), item & 1, status, kStOutAcc) && ok);     // tcgen05.ld is warp-collective
+            // The product first: x is there when it is, and so are the gates of all heads before.  A warp that came past the heads of a chunk
+            // without rows of its block may be many phases ahead of the gate's barrier, whose parity alone does not tell it that.
+            ok = mbar_wait(bar(kBarAcc + rb), item & 1, status, kStOutAcc) && mbar_wait(bar(kBarZ + s), sph, status, kStOutGate);
+            ok = __all_sync(0xffffffffu, ok);                // tcgen05.ld is warp-collective
             ++item;
             if (!ok) break;
             tc_fence_after_sync();

@@ -105,7 +105,7 @@ def test_weights_of_end_states(dtype, packed):
     assert same.any() and ((got - want).abs() <= bound * want.abs())[same].all()
 
 
-@pytest.mark.parametrize("x,B,C", [(1e-36, 1, 1), (1, 1e-36, 1), (1, 1, 1e-36), (1e20, 1e12, 1e-3), (1e-20, 1e15, 1e15), (1e37, 1e-10, 1e-20)])
+@pytest.mark.parametrize("x,B,C", [(1e-36, 1, 1), (1, 1e-36, 1), (1, 1, 1e-36), (1e20, 1e12, 1e-3), (1e-20, 1e15, 1e15), (1e37, 1e-10, 1e-20), (1e-20, 1e37, 1e-10), (1e-10, 1e-20, 1e37)])
 def test_fp32_keeps_its_range(x, B, C):
     """Operands near the smallest normal number have all their bits, and operands and sums too large for the tensor core's are what fp32 holds."""
     inp = make(976, 2, 300, 3, 64, 1, 64, torch.float32, has_z=False, init=True)
@@ -168,9 +168,13 @@ def test_fp32_values_that_cannot_be_cut(name, value):
     if name == "B":                                                          # one state of every head
         keep = torch.arange(64) != e
         assert rel(fin[..., keep], wfin[..., keep]) <= F32
+        if value != 3.4e38:                                                  # (times a decay of 0 a NaN)
+            assert not torch.isfinite(fin[..., e]).any() and not torch.isfinite(out[0, t]).any()
     if name == "C":                                                          # one step
         later = torch.arange(300) != t
         assert rel(out[0, later], want[0, later]) <= F32 and rel(fin, wfin) <= F32
+        if value != 3.4e38:
+            assert not torch.isfinite(out[0, t]).any()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])

@@ -11,6 +11,7 @@
 // Every mbarrier wait is bounded: on expiry the kernel records a code in the status word, skips the dependent work and
 // still releases its TMEM before it exits.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "ssd_common.cuh"
@@ -1427,22 +1428,28 @@ int run_output(const mb200_ssd_args &a, const SsdScratch &lay, bool h_np, cudaSt
     const int grid = (int)std::min<int64_t>(items, sm_count(a.device));
     const uint8_t *seq_start = a.seq_idx ? reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_start) : nullptr;
     const uint8_t *seq_carry = reinterpret_cast<const uint8_t *>(k.base + lay.off_seq_carry);
-    auto go = [&](auto dm, auto with_z) -> bool {
+    auto go = [&](auto dm, auto with_z) -> int {
         auto kernel = ssd_tc_output_kernel<T, decltype(dm)::value, decltype(with_z)::value>;
         // its warps would wait for ever for registers that the block was not launched with
-        static const bool enough = [&] {
+        static std::atomic<bool> enough{false};              // (a query that failed is made again by the next call)
+        if (!enough.load(std::memory_order_relaxed)) {
             cudaFuncAttributes at;
-            return cudaFuncGetAttributes(&at, reinterpret_cast<const void *>(kernel)) == cudaSuccess && at.numRegs >= kOutLaunchRegs;
-        }();
-        if (!enough) return false;
+            const cudaError_t e = cudaFuncGetAttributes(&at, reinterpret_cast<const void *>(kernel));
+            if (e != cudaSuccess) {
+                cudaGetLastError();                          // (it is not the next launch's)
+                return fail(MB200_ERR_LAUNCH, "ssd: attributes of the output kernel: %s", cudaGetErrorString(e));
+            }
+            if (at.numRegs < kOutLaunchRegs) return fail(MB200_ERR_LAUNCH, "ssd: output kernel built with too few registers (%d)", at.numRegs);
+            enough.store(true, std::memory_order_relaxed);
+        }
         ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)OutCfg::kSmem, a.device);
         launch_dependent_if(k.early, kernel, dim3(grid), kOutThreads, OutCfg::kSmem, stream, tx, tC, tB, tH, tz, tout, k.dtb, k.dAb, a.D, k.nc, a.nheads, a.ngroups, a.seqlen,
                             (int)items, h_np ? 1 : 0, seq_start, seq_carry, k.status);
-        return true;
+        return MB200_OK;
     };
     auto with_d = [&](auto dm) { return a.z ? go(dm, std::true_type{}) : go(dm, std::false_type{}); };
-    const bool launched = !a.D ? with_d(std::integral_constant<int, kNoD>{}) : a.D_has_hdim ? with_d(std::integral_constant<int, kColumnD>{}) : with_d(std::integral_constant<int, kHeadD>{});
-    if (!launched) return fail(MB200_ERR_LAUNCH, "ssd: output kernel built with too few registers");
+    if (int rc = !a.D ? with_d(std::integral_constant<int, kNoD>{}) : a.D_has_hdim ? with_d(std::integral_constant<int, kColumnD>{}) : with_d(std::integral_constant<int, kHeadD>{}))
+        return rc;
     MB200_CHECK_LAUNCH("ssd output (tensor core)");
     return MB200_OK;
 }

@@ -262,6 +262,7 @@ struct Tile {
         if (threadIdx.x < 32) tmem_dealloc(tmem, cols);
     }
 };
+constexpr int kSlice = 16;                              // of what is left to the FMAs, along the reduction
 constexpr uint32_t kTail = 16;                          // barrier and tensor-memory slot behind the tiles
 
 __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { return a.seq_idx ? a.seq_idx[(int64_t)b * a.seqlen + t] : 0; }
@@ -277,6 +278,93 @@ __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { r
 template <typename T, int U> constexpr uint32_t kStateB = kParts * U * kTileB;
 template <typename T, int U> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kStateB<T, U> + kTail;      // and the weights of the chunk's steps:
 template <int U> inline uint32_t state_weight_bytes(const mb200_ssd_args &a) { return U * ((a.chunk_size + 31) / 32 * 32) * 4; }
+// Rare: the states of a CTA some of whose tiles the tensor core has left out: those are added with fp32 FMAs, 16 steps at a time in the place
+// of the operands.  (It finds everything by itself and ends the work on these states, so that the kernel keeps nothing for it.)
+template <typename T, bool PACKED, int U>
+__device__ __noinline__ void finish_left_out_states(const mb200_ssd_args a, const float *dAb, const void *entering, SsdStates form, float *states, int nchunks, int tile, int chunk_or_seq,
+                                                    int g, uint8_t *smem, uint32_t tmem, uint32_t skipped, bool formed)
+{
+    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, tilesN = (N + 127) / 128, tilesP = (P + 63) / 64, units = a.nheads / a.ngroups * tilesP;
+    const int unit0 = (tile / tilesN) * U, n0 = (tile % tilesN) * 128;
+    const int start = PACKED ? a.cu_seqlens[chunk_or_seq] : 0, end = PACKED ? a.cu_seqlens[chunk_or_seq + 1] : 0;
+    const int b = PACKED ? 0 : chunk_or_seq / nchunks, c = PACKED ? (end - 1) / Q : chunk_or_seq % nchunks;
+    const int k0 = PACKED ? max(start - c * Q, 0) : 0, k1 = PACKED ? end - c * Q : min(Q, a.seqlen - c * Q);
+    const bool carry = PACKED && start < c * Q;
+    const int64_t t0 = (int64_t)c * Q;
+    const float *const weights = reinterpret_cast<const float *>(smem + kInParts<T> * kTileA + kStateB<T, U> + kTail);
+    const int ranges = (Q + 31) / 32 * 32, seq_last = PACKED ? 0 : seq_at(a, b, c * Q + k1 - 1);
+    auto head = [&](int u) { return g * (a.nheads / a.ngroups) + min(unit0 + u, units - 1) / tilesP; };
+    auto first_col = [&](int u) { return min(unit0 + u, units - 1) % tilesP * 64; };
+    auto x_at = [&](int u, int k, int p) {
+        return to_float(static_cast<const T *>(a.x)[(int64_t)b * a.x_stride[0] + (t0 + k) * a.x_stride[1] + (int64_t)head(u) * a.x_stride[2] + p]);
+    };
+    auto B_at = [&](int k, int n) { return to_float(static_cast<const T *>(a.B)[(int64_t)b * a.B_stride[0] + (t0 + k) * a.B_stride[1] + (int64_t)g * a.B_stride[2] + n]); };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = n0 + (warp & 3) * 32 + lane, mine = U == 2 ? warp >> 2 : 0;
+    const int h = head(mine), col0 = U == 2 ? mine * 64 : (warp >> 2) * 32;             // my columns of the sums
+    const bool live = n < N && unit0 + mine < units;
+    float *const Bs = reinterpret_cast<float *>(smem), *const xs = Bs + kSlice * 128;
+    tc_fence_after_sync();
+#pragma unroll 1
+    for (int half = 0; half < U; ++half) {          // 32 columns each
+        const int p = first_col(mine) + col0 - mine * 64 + 32 * half;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        if (formed) {                               // (of fp32 operands the sum over the tiles)
+            const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col0 + 32 * half;
+            float rest[32];
+            tmem_ld32(at, v);
+            tmem_ld32(at + 64 * U, rest);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = sizeof(T) == 2 ? v[j] + rest[j] : rest[j];
+        }
+        bool fits = true;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) fits = fits && finite(v[j]);
+        const bool again = sizeof(T) == 4 && live && !fits;  // the lifted sums did not: all of it by FMAs
+        if (again) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        }
+        const bool every = __syncthreads_or(again);
+#pragma unroll 1
+        for (int k = k0; k < k1; k += kSlice) {
+            const bool out = skipped >> (k - k0) / 64 & 1;
+            if (!out && !every) continue;
+            __syncthreads();
+            const int s = threadIdx.x >> 4, kk = k + s, col = threadIdx.x & 15;
+#pragma unroll
+            for (int e = 0; e < 128; e += 16) Bs[s * 128 + e + col] = kk < k1 && n0 + e + col < N ? B_at(kk, n0 + e + col) : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int pu = first_col(u) + col;
+#pragma unroll
+                for (int e = 0; e < 64; e += 16) xs[(s * U + u) * 64 + e + col] = kk < k1 && pu + e < P ? x_at(u, kk, pu + e) * weights[u * ranges + kk] : 0.f;
+            }
+            __syncthreads();
+            if (!out && !again) continue;
+#pragma unroll 1
+            for (int i = 0; i < kSlice && k + i < k1; ++i) {
+                if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k + i) != seq_last) continue;
+                const float Bn = Bs[i * 128 + n - n0], *xk = xs + i * 64 * U + col0 + 32 * half;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = fmaf(xk[j], Bn, v[j]);
+            }
+        }
+        if (!live) continue;
+        const float decay = carry ? __expf(dAb[(((int64_t)b * a.nheads + h) * nchunks + c) * Q + k1 - 1]) : 0.f;
+        const int64_t slot = PACKED ? (int64_t)chunk_or_seq * a.nheads + h : ((int64_t)b * nchunks + c) * a.nheads + h, hc = (int64_t)c * a.nheads + h;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            if (p + j >= P) continue;
+            if (carry) {
+                const int64_t e = form == SsdStates::np16 ? (hc * N + n) * P + p + j : (hc * P + p + j) * N + n;
+                v[j] = fmaf(form == SsdStates::pn32 ? static_cast<const float *>(entering)[e] : to_float(static_cast<const T *>(entering)[e]), decay, v[j]);
+            }
+            states[(slot * P + p + j) * N + n] = v[j];
+        }
+    }
+}
 template <typename T, bool PACKED, int U>
 __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_or_seq, int g, const mb200_ssd_args &a, const float *dtb, const float *dAb, const void *entering,
                                             SsdStates form, float *states, int nchunks, int *status)
@@ -443,6 +531,12 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
     const T *my_x = U == 2 && mine ? x[U - 1] : x[0];
     const int my_p0 = U == 2 && mine ? p0[U - 1] : p0[0];
     const int64_t slot = PACKED ? (int64_t)chunk_or_seq * a.nheads + my_h : ((int64_t)b * nchunks + c) * a.nheads + my_h;
+    if (skipped) {
+        fold_last();
+        finish_left_out_states<T, PACKED, U>(a, dAb, entering, form, states, nchunks, tile, chunk_or_seq, g, smem, t.tmem, skipped, formed);
+        t.close(128 * U);
+        return;
+    }
     tc_fence_after_sync();
 #pragma unroll
     for (int half = 0; half < U; ++half) {          // 32 columns each
@@ -458,26 +552,21 @@ __device__ __forceinline__ void split_state(uint8_t *smem, int tile, int chunk_o
             for (int j = 0; j < 32; ++j) v[j] = sizeof(T) == 2 ? v[j] + rest[j] : fmaf(t.issued > folded ? v[j] : 0.f, kDrop, folded > 0 ? rest[j] : 0.f);
         }
         if (!live) continue;
-        uint32_t fma_tiles = skipped;
         if constexpr (sizeof(T) == 4) {
             bool fits = true;
 #pragma unroll
             for (int j = 0; j < 32; ++j) fits = fits && finite(v[j]);
             if (!fits) {                            // the lifted sums did not: all of it by FMAs
-                fma_tiles = ~0u;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = 0.f;
-            }
-        }
-        if (fma_tiles) {
 #pragma unroll 1
-            for (int k = k0; k < k1; ++k) {
-                if (!((fma_tiles >> (k - k0) / 64) & 1)) continue;
-                if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
-                const float wk = weights[mine * ranges + k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
+                for (int k = k0; k < k1; ++k) {
+                    if (!PACKED && a.seq_idx && seq_at(a, b, c * Q + k) != seq_last) continue;
+                    const float wk = weights[mine * ranges + k], Bn = to_float(B[(int64_t)k * a.B_stride[1] + n - n0]);
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (pc + j < P) v[j] = fmaf(to_float(my_x[(int64_t)k * a.x_stride[1] + pc - my_p0 + j]) * wk, Bn, v[j]);
+                    for (int j = 0; j < 32; ++j)
+                        if (pc + j < P) v[j] = fmaf(to_float(my_x[(int64_t)k * a.x_stride[1] + pc - my_p0 + j]) * wk, Bn, v[j]);
+                }
             }
         }
         float *S = states + slot * P * N + n;
@@ -568,22 +657,40 @@ __device__ __forceinline__ void split_cb(uint8_t *smem, int tile, int chunk, int
         if (!kEarly<T> && n + 64 < N) fetch(n + 64);
     }
     t.drain();
-    if (__all_sync(0xffffffffu, t.ok)) {
-        float v[32];
-        if (all) {
-            tc_fence_after_sync();
-            tmem_ld32(mine_at, v);
-            if constexpr (sizeof(T) == 4) {
-                float sum[32];
-                tmem_ld32(mine_at + 64, sum);
+    float v[32];
+    if (sizeof(T) == 4 && !all) {                   // a tile could not be cut: fp32 FMAs, 16 states at a time in the place of the operands
+        float *const Cs = reinterpret_cast<float *>(smem), *const Bs = Cs + kSlice * 132;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = fmaf(v[j], kDrop, N > 64 ? sum[j] : 0.f);
+        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+#pragma unroll 1
+        for (int n = 0; n < N; n += kSlice) {
+            const int s = threadIdx.x & 15, row = threadIdx.x >> 4;
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < 8; ++e) Cs[s * 132 + row + 16 * e] = n + s < N && m0 + row + 16 * e < len ? to_float(C[(int64_t)(row + 16 * e) * a.C_stride[1] + n + s]) : 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) Bs[s * 68 + row + 16 * e] = n + s < N && k0 + row + 16 * e < len ? to_float(B[(int64_t)(row + 16 * e) * a.B_stride[1] + n + s]) : 0.f;
+            __syncthreads();
+#pragma unroll 1
+            for (int i = 0; i < kSlice && n + i < N; ++i) {
+                const float Cn = Cs[i * 132 + m - m0];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = fmaf(Cn, Bs[i * 68 + k - k0 + j], v[j]);
             }
         }
-        if constexpr (sizeof(T) == 4) {
+    }
+    if (__all_sync(0xffffffffu, t.ok)) {
+        if (sizeof(T) == 2 || all) {
+            tc_fence_after_sync();
+            tmem_ld32(mine_at, v);
+        }
+        if (sizeof(T) == 4 && all) {
+            float sum[32];
+            tmem_ld32(mine_at + 64, sum);
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-                if (all && finite(v[j])) continue;      // (else the lifted sums did not fit, or a tile could not be cut)
+                v[j] = fmaf(v[j], kDrop, N > 64 ? sum[j] : 0.f);
+                if (finite(v[j])) continue;             // (else the lifted sum did not fit)
                 v[j] = 0.f;
 #pragma unroll 1
                 for (int n = 0; n < N && m < len && k + j < len; ++n)
@@ -695,33 +802,108 @@ struct ScanDecays {
     // to stay finite
     __device__ __forceinline__ float row(float rel_m, float own_end, int range) const { return ex2(fminf(fmaf(own_end - dA[32 * range + 31], kLog2e, rel_m), kMaxSpan)); }
 };
-// Rare: what tiles with infinities or NaNs contribute to eight outputs of row m, in fp32.
+// Rare: the outputs of a CTA some of whose tiles the tensor core has left out.  The sums of 128 x 64 of them lie in shared memory; what those
+// tiles contribute is added with fp32 FMAs, 16 states or steps at a time.  A thread has eight columns of rows r0 + 32 i.
+constexpr uint32_t kLeftOutBytes = kSlice * (132 + 64) * 4;
+__device__ __forceinline__ float4 *sum_chunk(uint8_t *sums, int r, int chunk) { return reinterpret_cast<float4 *>(sums + r * 256 + ((chunk ^ (r & 7)) << 4)); }
+// (It finds everything by itself and ends the work on these outputs, so that the kernels keep nothing for it.  `lifted`: sums of lifted operands; eight that did not all fit are
+// formed again from all tiles.)
 template <typename T>
-__device__ __noinline__ void add_skipped(float4 *lo, float4 *hi, const uint32_t *skip, int nH, const float *cbrow, const float *dAc, const float *dtc, int m, float sc, const T *x,
-                                         int64_t x_stride, const T *Crow, const float *H, int N, int left, bool lifted)
+__device__ __noinline__ void finish_left_out(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb, int nchunks, int tile_cols, int p0,
+                                          float *stage, uint8_t *sums, const uint32_t *skip, bool lifted)
 {
-    bool every = false;                                 // sums of lifted operands that did not fit: all of it
-    if (lifted)
-        for (int e = 0; e < 8; ++e) every = every || !finite(reinterpret_cast<const float *>(e < 4 ? lo : hi)[e & 3]);
-    if (every) *lo = *hi = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto skipped = [&](int t) { return every || ((skip[t >> 5] >> (t & 31)) & 1); };
-    float y[8] = {}, s[8] = {};
-    for (int k = 0; k <= m; ++k) {
-        if (!skipped(nH + (k >> 6))) continue;
-        const float w = cbrow[k] * (__expf(fminf(dAc[m] - dAc[k], 0.f)) * dtc[k]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (e < left) y[e] = fmaf(w, to_float(x[k * x_stride + e]), y[e]);
+    const int Q = a.chunk_size, P = a.headdim, N = a.dstate, m0 = ((Q + 127) / 128 - 1 - blockIdx.x / ((P + tile_cols - 1) / tile_cols)) * 128;
+    const int b = blockIdx.y / nchunks, c = blockIdx.y % nchunks, h = blockIdx.z, g = h / (a.nheads / a.ngroups);
+    const int len = min(Q, a.seqlen - c * Q), kend = min(m0 + 128, len), left = P - p0;
+    const int64_t row = (((int64_t)b * a.nheads + h) * nchunks + c) * Q, t0 = (int64_t)c * Q;
+    const float *dAc = dAb + row, *dtc = dtb + row;
+    const T *x = static_cast<const T *>(a.x) + (int64_t)b * a.x_stride[0] + t0 * a.x_stride[1] + (int64_t)h * a.x_stride[2] + p0;
+    const T *C = static_cast<const T *>(a.C) + (int64_t)b * a.C_stride[0] + (t0 + m0) * a.C_stride[1] + (int64_t)g * a.C_stride[2];
+    const float *H = states + (((int64_t)b * nchunks + c) * a.nheads + h) * (int64_t)P * N + (int64_t)p0 * N;
+    const float *cbm = cb + ((((int64_t)b * nchunks + c) * a.ngroups + g) * Q + m0) * Q;
+    const int c8 = threadIdx.x & 7, r0 = threadIdx.x >> 3, nH = (N + 63) / 64, ntiles = nH + (kend + 63) / 64;
+    float *const As = stage, *const Bs = As + kSlice * 132;
+    uint32_t again = 0;                 // rows of mine whose sums did not fit
+    for (int i = 0; i < 4 && lifted; ++i) {
+        float4 *lo = sum_chunk(sums, r0 + 32 * i, 2 * c8), *hi = sum_chunk(sums, r0 + 32 * i, 2 * c8 + 1);
+        if (finite(lo->x) && finite(lo->y) && finite(lo->z) && finite(lo->w) && finite(hi->x) && finite(hi->y) && finite(hi->z) && finite(hi->w)) continue;
+        *lo = *hi = make_float4(0.f, 0.f, 0.f, 0.f);
+        again |= 1u << i;
     }
-    for (int n = 0; n < N; ++n) {
-        if (!skipped(n >> 6)) continue;
-        const float w = to_float(Crow[n]);
+    const bool every = __syncthreads_or(again);
+    float acc[4][8] = {};
+    bool scaled = false;
+    auto scale = [&] {                  // the states' part is complete
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (e < left) s[e] = fmaf(w, H[(int64_t)e * N + n], s[e]);
+        for (int i = 0; i < 4; ++i) {
+            const int m = m0 + r0 + 32 * i;
+            const bool on = m < len && !(a.seq_idx && seq_at(a, b, c * Q + m) != (c > 0 ? seq_at(a, b, c * Q - 1) : 0));
+            const float sc = on ? __expf(dAc[m]) : 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[i][e] *= sc;
+        }
+        scaled = true;
+    };
+#pragma unroll 1
+    for (int t = 0; t < ntiles; ++t) {
+        const bool out = (skip[t >> 5] >> (t & 31)) & 1, steps = t >= nH;
+        if (!out && !every) continue;
+        if (steps && !scaled) scale();
+        const uint32_t rows = out ? 15u : again;
+        const int first = (steps ? t - nH : t) * 64, end = min(first + 64, steps ? kend : N);
+#pragma unroll 1
+        for (int k = first; k < end; k += kSlice) {
+            __syncthreads();
+            const int s = threadIdx.x & 15, kk = k + s, row = threadIdx.x >> 4;
+#pragma unroll 1
+            for (int r = row; r < 128; r += 16) {
+                const int m = m0 + r;
+                float v = 0.f;
+                if (m < len && kk < end && (!steps || kk <= m))
+                    v = steps ? cbm[(int64_t)r * Q + kk] * (__expf(fminf(dAc[m] - dAc[kk], 0.f)) * dtc[kk]) : to_float(C[r * a.C_stride[1] + kk]);
+                As[s * 132 + r] = v;
+            }
+            if (steps) {
+                const int ks = k + row;
+#pragma unroll 1
+                for (int p = s; p < 64; p += 16) Bs[row * 64 + p] = ks < end && p < left ? to_float(x[ks * a.x_stride[1] + p]) : 0.f;
+            } else {
+#pragma unroll 1
+                for (int p = row; p < 64; p += 16) Bs[s * 64 + p] = kk < end && p < left ? H[(int64_t)p * N + kk] : 0.f;
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int i = 0; i < kSlice && k + i < end; ++i) {
+                const float4 lo = *reinterpret_cast<const float4 *>(Bs + i * 64 + 8 * c8), hi = *reinterpret_cast<const float4 *>(Bs + i * 64 + 8 * c8 + 4);
+                const float b[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!(rows >> q & 1) || (steps && k + i > m0 + r0 + 32 * q)) continue;     // (nothing goes back in time, not as 0 x inf either)
+                    const float w = As[i * 132 + r0 + 32 * q];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[q][e] = fmaf(w, b[e], acc[q][e]);
+                }
+            }
+        }
     }
+    if (!scaled) scale();
+    const T *z = a.z ? static_cast<const T *>(a.z) + (int64_t)b * a.z_stride[0] + t0 * a.z_stride[1] + (int64_t)h * a.z_stride[2] + p0 : nullptr;
+    T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) reinterpret_cast<float *>(e < 4 ? lo : hi)[e & 3] += fmaf(sc, s[e], y[e]);
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 32 * i;
+        const int64_t m = m0 + r;
+        const float *sum[2] = {&sum_chunk(sums, r, 2 * c8)->x, &sum_chunk(sums, r, 2 * c8 + 1)->x};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int col = 8 * c8 + e;
+            if (m >= len || col >= left) continue;
+            float y = sum[e >> 2][e & 3] + acc[i][e];
+            if (a.D) y = fmaf(to_float(x[m * a.x_stride[1] + col]), a.D[a.D_has_hdim ? (int64_t)h * P + p0 + col : h], y);
+            if (z) y *= sizeof(T) == 2 ? fast_silu(to_float(z[m * a.z_stride[1] + col])) : silu(to_float(z[m * a.z_stride[1] + col]));
+            out[m * a.out_stride[1] + col] = from_float<T>(y);
+        }
+    }
 }
 
 // ---- 16 bits
@@ -731,6 +913,7 @@ __device__ __noinline__ void add_skipped(float4 *lo, float4 *hi, const uint32_t 
 // which leaves the MMAs to a warp of their own, takes 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
 template <typename T> constexpr uint32_t kScan16A = kOutParts<T> * kTileA;
 template <typename T, int W> constexpr uint32_t kScan16B = kOutParts<T> * W * kTileB;
+static_assert(32768 + kLeftOutBytes <= kScan16A<__nv_bfloat16> + kScan16B<__nv_bfloat16, 1>, "sums and what is added to them");
 // W: tiles of 64 columns that share A, whose forming is most of the work: two of a head that has them, where single ones would not all fit the
 // GPU at once (2 x 3000 steps of 32 bf16 heads of 128 x 128: 154 us with one, 122 with two).
 template <typename T, int W>
@@ -927,14 +1110,8 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
         };
         const float sc = scale(m);
         const bool any1 = states_done > 0, any2 = t.issued > states_done;        // sums that the tensor core has formed
-        auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + r * 256 + ((chunk ^ (r & 7)) << 4)); };
-#pragma unroll 1
-        for (int w = 0; w < W; ++w) {
-            const int col = 64 * w + 8 * c8, left = P - p0 - col;
-            if (w > 0) {
-                __syncthreads();
-                request(w);
-            }
+        auto place = [&](int r, int chunk) { return sum_chunk(smem, r, chunk); };
+        auto collect = [&](int w) {
 #pragma unroll
             for (int j = (warp >> 2) * 32; j < (warp >> 2) * 32 + 32; j += 8) {
                 uint32_t y1[8], y2[8];
@@ -949,15 +1126,25 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
                 *place(lm, j / 4 + 1) = make_float4(y[4], y[5], y[6], y[7]);
             }
             __syncthreads();
+        };
+        if (left_out) {
+#pragma unroll 1
+            for (int w = 0; w < W; ++w) {
+                if (w > 0) __syncthreads();
+                collect(w);
+                finish_left_out<T>(a, dtb, dAb, states, cb, nchunks, 64 * W, p0 + 64 * w, reinterpret_cast<float *>(smem + 32768), smem, decays.skip, false);
+            }
+        }
+#pragma unroll 1
+        for (int w = 0; w < W && !left_out; ++w) {
+            const int col = 64 * w + 8 * c8, left = P - p0 - col;
+            if (w > 0) {
+                __syncthreads();
+                request(w);
+            }
+            collect(w);
             T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + col;
             const bool vo = rows16(out, a.out_stride[1]);
-            if (left_out) {
-#pragma unroll 1
-                for (int r = r0; r < 128; r += 32)
-                    if (m0 + r < len && left > 0)
-                        add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), decays.skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + col, a.x_stride[1],
-                                    C + (int64_t)r * a.C_stride[1], H + (int64_t)col * N, N, left, false);
-            }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = r0 + 32 * i;
@@ -1183,7 +1370,7 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
     };
     const float sc = scale(m);
     auto skipped = [&](int t) { return (reinterpret_cast<volatile uint32_t *>(skip)[t >> 5] >> (t & 31)) & 1; };
-    auto place = [&](int r, int chunk) { return reinterpret_cast<float4 *>(smem + kScanB + r * 256 + ((chunk ^ (r & 7)) << 4)); };
+    auto place = [&](int r, int chunk) { return sum_chunk(smem + kScanB, r, chunk); };
     auto wait_done = [&](int i) {
         ok = ok && __all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1, status, kStSplitScan));
         if (ok) tc_fence_after_sync();
@@ -1377,45 +1564,42 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan_kernel(const mb200
         T *out = static_cast<T *>(a.out) + (int64_t)b * a.out_stride[0] + t0 * a.out_stride[1] + (int64_t)h * a.out_stride[2] + p0 + 8 * c8;
         const bool vo = rows16(out, a.out_stride[1]);
         if (fma) {
-#pragma unroll 1
-            for (int r = r0; r < 128; r += 32)
-                if (m0 + r < len && left > 0)
-                    add_skipped(place(r, 2 * c8), place(r, 2 * c8 + 1), skip, nH, cbm + (int64_t)r * Q, dAc, dtc, m0 + r, scale(m0 + r), x + 8 * c8, a.x_stride[1],
-                                C + (int64_t)r * a.C_stride[1], H + (int64_t)(8 * c8) * N, N, left, true);
-        }
+            finish_left_out<T>(a, dtb, dAb, states, cb, nchunks, 64, p0, reinterpret_cast<float *>(smem), smem + kScanB, skip, true);
+        } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = r0 + 32 * q;
-            if (m0 + r >= len || left <= 0) continue;
-            const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
-            float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
-            if (a.D) {
-                widen8<T>(xm[q], f);
-                if (!a.D_has_hdim) {
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + 32 * q;
+                if (m0 + r >= len || left <= 0) continue;
+                const float4 lo = *place(r, 2 * c8), hi = *place(r, 2 * c8 + 1);
+                float y[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, f[8];
+                if (a.D) {
+                    widen8<T>(xm[q], f);
+                    if (!a.D_has_hdim) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dh, y[e]);
+                        for (int e = 0; e < 8; ++e) y[e] = fmaf(f[e], Dh, y[e]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (e < left) y[e] = fmaf(f[e], a.D[(int64_t)h * P + p0 + 8 * c8 + e], y[e]);
+                    }
+                }
+                if (z) {
+                    widen8<T>(zm[q], f);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[e] *= silu(f[e]);
+                }
+                Raw8<T> o;
+                T *oe = reinterpret_cast<T *>(&o);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
+                T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
+                if (vo && left >= 8) {
+                    *reinterpret_cast<Raw8<T> *>(om) = o;
                 } else {
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        if (e < left) y[e] = fmaf(f[e], a.D[(int64_t)h * P + p0 + 8 * c8 + e], y[e]);
+                        if (e < left) om[e] = oe[e];
                 }
-            }
-            if (z) {
-                widen8<T>(zm[q], f);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) y[e] *= silu(f[e]);
-            }
-            Raw8<T> o;
-            T *oe = reinterpret_cast<T *>(&o);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) oe[e] = from_float<T>(y[e]);
-            T *om = out + (int64_t)(m0 + r) * a.out_stride[1];
-            if (vo && left >= 8) {
-                *reinterpret_cast<Raw8<T> *>(om) = o;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (e < left) om[e] = oe[e];
             }
         }
     }

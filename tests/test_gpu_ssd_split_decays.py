@@ -177,6 +177,40 @@ def test_fp32_values_that_cannot_be_cut(name, value):
             assert not torch.isfinite(out[0, t]).any()
 
 
+@pytest.mark.parametrize("name", ["x", "B", "C"])
+@pytest.mark.parametrize("P,N,lens", [(64, 64, [100, 200]), (72, 40, [100, 199]), (136, 130, [3, 250])])
+def test_fp32_values_too_large_to_be_cut(name, P, N, lens):
+    """The tiles that hold one are added with fp32 FMAs: gated, with D per column, packed and ragged, all is what the oracle gives."""
+    t, e = sum(lens) - 160, 9
+    inp, seq_idx, cu = _packed(925 + P, lens, 3, P, 1, N, torch.float32)
+    inp["D"] = torch.randn(3, P, generator=torch.Generator().manual_seed(P))
+    inp[name][0, t, 0, e] = 3e36
+    c = {k: _c(v) for k, v in inp.items()}
+    out, _, var = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 128, D=c["D"], z=c["z"], dt_bias=c["dt_bias"], seq_idx=seq_idx.to(DEV), cu_seqlens=cu.to(DEV),
+                        dt_softplus=True, return_final_states=True, return_varlen_states=True)
+    out, var = out.cpu(), var.cpu()
+    for i in range(2):
+        sl = slice(int(cu[i]), int(cu[i + 1]))
+        want, wfin = oracle.ssd_chunk_scan(inp["x"][:, sl], inp["dt"][:, sl], inp["A"], inp["B"][:, sl], inp["C"][:, sl], 128, inp["D"], inp["z"][:, sl], inp["dt_bias"], None,
+                                           dt_softplus=True)
+        got, state, at = out[:, sl], var[i:i + 1], max(t - sl.start, 0) if i == 1 else sl.stop
+        assert rel(got[:, :at], want[:, :at]) <= F32 or at == 0
+        if i == 0 or name == "C":
+            assert rel(state, wfin) <= F32
+        if i == 0:
+            continue
+        assert rel(got[:, at], want[:, at]) <= F32
+        if name == "x":                                                      # one column of one head
+            cols = torch.arange(P) != e
+            assert rel(got[:, :, 0, cols], want[:, :, 0, cols]) <= F32 and rel(got[:, :, 1:], want[:, :, 1:]) <= F32
+            assert rel(state[:, 0, cols], wfin[:, 0, cols]) <= F32 and rel(state[:, 1:], wfin[:, 1:]) <= F32 and rel(state[:, 0, e], wfin[:, 0, e]) <= F32
+        if name == "B":                                                      # one state of every head
+            keep = torch.arange(N) != e
+            assert rel(state[..., keep], wfin[..., keep]) <= F32 and rel(state[..., e], wfin[..., e]) <= F32
+        if name == "C":                                                      # one step
+            assert rel(got[:, at + 1:], want[:, at + 1:]) <= F32
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("P,N,G,H", [(64, 64, 1, 15), (72, 40, 3, 15), (64, 136, 1, 9)])
 def test_two_heads_share_their_b(dtype, P, N, G, H):

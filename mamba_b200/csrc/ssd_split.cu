@@ -1,21 +1,22 @@
-// Stages of the SSD chunked forward for every shape and type, on the tensor cores with products as exact as fp32's.
+// Stages of the SSD chunked forward for every shape and type, on the tensor cores with operands in parts.
 //
 // ssd_tc.cu serves 16-bit calls of headdim 64, dstate 128 and chunk 256 with 16-bit operands throughout: weights, decays and entering
-// states are rounded to the input type.  Here nothing but the result is.  An fp32 operand -- an fp32 input, C.B^T times its decay, a
-// weighted x, an entering state -- is cut into bf16 values that add up to it (three hold all 24 bits), and a half-precision input into two,
-// so that tcgen05.mma of bf16 operands forms the products, which it adds in fp32; terms below 2^-24 of a product are left out.  bf16 has
-// fp32's range: nothing overflows that fp32 holds, whatever the input type.  The tensor core cuts its sums off where fp32 arithmetic
+// states are rounded to the input type.  Here an fp32 operand -- an fp32 input, C.B^T times its decay, a weighted x, an entering state -- is
+// cut into bf16 values that add up to it, and a half-precision input into two, so that tcgen05.mma of bf16 operands forms the products, which
+// it adds in fp32.  Three parts hold all 24 bits, and terms below 2^-24 of a product are left out: so chunk states, C.B^T, and the outputs
+// of half precision and fp32.  bf16 outputs take two parts, 16 to 17 bits, of their entering states and decayed C.B^T, so that about 2^-17 of
+// an operand is left out of a result with 8 bits.  bf16 has fp32's range: nothing overflows that fp32 holds, whatever the input type.  The tensor core cuts its sums off where fp32 arithmetic
 // rounds.  Sums that leave a 16-bit call in fp32 have the small products in a sum of their own; in fp32 calls the tensor core adds the products
 // of 64 steps only, the small ones first, and fp32 additions do the rest: without decays, where the sums are the whole error, states of 256
 // steps are 2.3e-7 from 64 bits, outputs 2.6e-7 (4.0e-7 and 6.4e-7 with two sums over all steps, 3.3e-7 and 4.3e-7 with tiles of fp32 FMAs;
-// 2 x 2048 steps of 8 heads of 64 x 64: 44.4 us for 43.6).  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64:
-// end states 1.6e-6 to 3.4e-6, outputs 1.66e-3 (bf16) and 2.07e-4 (fp16), which is their own rounding; fp32 outputs 0.86e-6 to 2.0e-6.  Tiles
-// of fp32 FMAs gave the same to within 2 %, operands rounded to 16 bits 1.7e-3 / 2.1e-4 and 2.4e-3 / 3.0e-4.
+// 2 x 2048 steps of 8 heads of 64 x 64: 44.4 us for 43.6).  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64, four seeds: outputs 1.66e-3
+// (bf16) and 2.08e-4 (fp16), which is their own rounding, 2.3e-7 to 7.9e-7 in fp32 (tiles of fp32 FMAs: 6.7e-7 to 14e-7); end states 1.3e-7 to
+// 1.7e-6 (1.6e-6 to 4.7e-6).  Operands rounded to 16 bits: outputs 2.4e-3 and 3.0e-4, end states 1.7e-3 and 2.1e-4.
 //
 // A tile loop: 256 threads fetch the next 64 steps of the reduction while the tensor core works on the last ones, form the operand values,
 // cut them and store them.  The tensor core is idle most of the time; what bounds these kernels is that element-wise work and the latencies
 // between it, which two to four CTAs per SM share.  Rows are read with plain loads, so any stride and alignment goes.
-// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states and C.B^T 23, outputs 68; fp32 FMAs took 318 for the call.
+// 2 x 1500 steps of 48 half-precision heads of 64 x 64, us: chunk states and C.B^T 23, outputs 67; fp32 FMAs took 318 for the call.
 #include <algorithm>
 #include <cfloat>
 #include <type_traits>
@@ -39,9 +40,9 @@ template <typename T> constexpr int kInParts = std::is_same<T, __nv_bfloat16>::v
 // to fp32 FMAs like what cannot be cut at all.
 constexpr float kLift = 0x1p17f, kDrop = 0x1p-34f;
 
-// The next tile is requested before the barrier that completes this one, whose cutting takes no time in bf16, or behind it (2 x 3000 steps of
-// 32 heads of 128 x 128 in bf16 187 us behind, 183 before; 2 x 1500 of 48 half-precision heads of 64 x 64 93 / 94.4, 2 x 2048 of 8 fp32
-// heads 44.2 / 45.3).
+// The next tile is requested before the barrier that completes this one, whose cutting takes no time in bf16, or behind it (a call of 2 x 3000
+// steps of 32 heads of 128 x 128 in bf16 173 us behind, 168 before; of 2 x 1500 of 48 half-precision heads of 64 x 64 90.6 / 97.5, of 2 x 2048
+// of 8 fp32 heads 40.5 / 41.4).
 template <typename T> constexpr bool kEarly = kInParts<T> == 1;
 
 enum { kStSplitState = 51, kStSplitCb, kStSplitScan };
@@ -272,8 +273,8 @@ __device__ __forceinline__ int seq_at(const mb200_ssd_args &a, int b, int t) { r
 // each other in a group, and 128 states, of a (batch, chunk) or sequence.  PACKED: the state after the last token of a packed sequence -- its
 // steps in the chunk of that token, plus the state entering the chunk if the sequence began earlier.
 // Two units share B: fetched, cut, stored and read by the tensor core once.  That pays where B is cut, as soon as single units would not all
-// fit the GPU at once (2 x 1500 steps of 48 half-precision heads of 64 x 64: 29 us with one, 23 with two; 2 x 3000 of 32 fp32 heads of 64 x
-// 128: 48 / 45, C.B^T included); in bf16, whose B is stored as it is, two CTAs per SM lose what it saves (2 x 3000 of 32 heads of 128 x 128:
+// fit the GPU at once (2 x 1500 steps of 48 half-precision heads of 64 x 64: 29 us with one, 23 with two; a call of 2 x 3000 of 32 fp32 heads
+// of 64 x 128 181.3 / 179.9, of 128 x 128 336 / 326); in bf16, whose B is stored as it is, two CTAs per SM lose what it saves (2 x 3000 of 32 heads of 128 x 128:
 // 52 / 57), and so do the short sums of packed sequences (46 / 54).
 template <typename T, int U> constexpr uint32_t kStateB = kParts * U * kTileB;
 template <typename T, int U> constexpr uint32_t kStateSmem = kInParts<T> * kTileA + kStateB<T, U> + kTail;      // and the weights of the chunk's steps:
@@ -907,15 +908,15 @@ __device__ __noinline__ void finish_left_out(const mb200_ssd_args a, const float
 }
 
 // ---- 16 bits
-// Two CTAs of 126 registers per SM: three of 80 spill, and took 76 us where this took 69 (2 x 1500 steps of 48 half-precision heads of 64 x
-// 64); a second pair of tiles left L1 so little that C.B^T, which every head reads again, came from L2 each time (72 -> 81 us in bf16); one
-// CTA per SM that keeps C.B^T in tensor memory while the heads pass took 78, with all its warps in step 85.  The kernel for fp32 below,
-// which leaves the MMAs to a warp of their own, takes 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
+// Two CTAs of 121 to 128 registers per SM, of which no more than 12 bytes a thread are spilled: three CTAs of 80 registers spill, and took 76 us
+// where two took 69 and now take 67 (2 x 1500 steps of 48 half-precision heads of 64 x 64); a second pair of tiles left L1 so little that
+// C.B^T, which every head reads again, came from L2 each time (72 -> 81 us in bf16); one CTA per SM that keeps C.B^T in tensor memory while the heads pass took 78, with all its warps in step 85.  A kernel laid out like the one for
+// fp32 below, with a warp for the MMAs alone, took 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
 template <typename T> constexpr uint32_t kScan16A = kOutParts<T> * kTileA;
 template <typename T, int W> constexpr uint32_t kScan16B = kOutParts<T> * W * kTileB;
 static_assert(32768 + kLeftOutBytes <= kScan16A<__nv_bfloat16> + kScan16B<__nv_bfloat16, 1>, "sums and what is added to them");
 // W: tiles of 64 columns that share A, whose forming is most of the work: two of a head that has them, where single ones would not all fit the
-// GPU at once (2 x 3000 steps of 32 bf16 heads of 128 x 128: 154 us with one, 122 with two).
+// GPU at once (a call of 2 x 3000 steps of 32 bf16 heads of 128 x 128: 204 us with one, 168 with two).
 template <typename T, int W>
 __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb200_ssd_args a, const float *dtb, const float *dAb, const float *states, const float *cb,
                                                                      int nchunks, int *status)
@@ -1186,10 +1187,10 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 // has rows 32 (w % 4) .. and one half of the 64 columns; tcgen05.st.16x128b gives a lane four of these rows, and four lanes a row's 16
 // bytes, so that the loads fill whole sectors.  The order within a tile is free: a lane's four consecutive elements go to where its words
 // are, and B's rows (or H's columns) follow.  (A ninth warp for the MMAs alone leaves a thread 96 registers for 128, because a quarter of the
-// SM then has five warps: 600 bytes of spills for 84, 28.0 us for 26.2.)
+// SM then has five warps: 28.0 us for 26.2.  With the 128 nothing is spilled.)
 // What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
 // middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its start, which overlaps the recurrence, included),
-// 2 x 3000 steps of 32 heads of 64 x 128 142; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
+// 2 x 3000 steps of 32 heads of 64 x 128 136; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
 // Shared memory: B, then two stages of C.B^T, 4 KB a warp.  The sums leave through the first of them.
 constexpr uint32_t kScanB = kParts * kTileB, kScanTiles = kScanB + 65536;
 constexpr uint32_t kScanTail = 48;                      // barriers and tensor-memory slot behind the tiles

@@ -506,7 +506,7 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // What bounds it: a head takes the output warps' pass over its accumulators (4200 cycles) plus the MMAs that wait for them (1400); the mask
 // warps have a third of the time to spare.  269 us for the shape above (321 with twelve warps that did both, one after the other), 2.7 ms
 // for 262144 steps of 128 heads (3.28).  C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
-// register comes back from L2: the roles share the block's registers out between them (setmaxnreg).  What is still spilled, 70 bytes a thread,
+// register comes back from L2: the roles share the block's registers out between them (setmaxnreg).  What is still spilled, 72 bytes a thread,
 // is the mask warps' (built with the bodies of the others taken out, 72; the output warps alone 0), who have time to spare.  Instruction fetch is what bounds the
 // roles themselves: loops are rolled, waits short, places advanced without divisions.  The output loop unrolled twice takes 273 us, eight
 // times 320; with the next accumulators requested ahead 289.
@@ -659,13 +659,16 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 left = hpu - w.hv;
                 rows = rb < w.row_blocks(seqlen);
                 dA = dAb + (((int64_t)w.b * nheads + w.h) * nchunks + w.c) * kQ;
+                int lo = 0;                                  // first column of my row's sequence inside the chunk
                 if (rows) {
-                    // first column of my row's sequence inside the chunk
-                    const int lo = seq_start ? seq_start[((int64_t)w.b * nchunks + w.c) * kQ + r] : 0;
+                    if (seq_start) lo = seq_start[((int64_t)w.b * nchunks + w.c) * kQ + r];
                     dA_next = dA[r];
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCb + rb), nunits & 1, status, kStOutCb));      // tcgen05.ld is warp-collective
-                    ++nunits;
-                    if (!ok) break;
+                }
+                // (every unit completes these barriers once, whatever its row blocks, so that nobody falls a phase behind)
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCb + rb), nunits & 1, status, kStOutCb));      // tcgen05.ld is warp-collective
+                ++nunits;
+                if (!ok) break;
+                if (rows) {
                     tc_fence_after_sync();
                     const uint32_t from = tlane + (rb ? kAcc1 : kAcc0);
 #pragma unroll
@@ -686,12 +689,12 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                         }
                     }
                     tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(kBarCbRead + rb));
-                    // the A operand of the lower row block takes the place of C.B^T: no warp may write it while another still reads
-                    if (rb) ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCbRead + rb), (nunits - 1) & 1, status, kStOutCbRead));
-                    if (!ok) break;
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kBarCbRead + rb));
+                // the A operand of the lower row block takes the place of C.B^T: no warp may write it while another still reads
+                if (rb) ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarCbRead + rb), (nunits - 1) & 1, status, kStOutCbRead));
+                if (!ok) break;
             }
             const int s = seq & 1;
             const uint32_t sc = smb + Cfg::kC + 2 * Cfg::kStage + s * Cfg::kScal;
@@ -893,7 +896,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             const uint32_t tm = warp_uniform(tmem), acc = tm + (rb ? kAcc1 : kAcc0);
             auto wait = [&](uint64_t *bar, int phase, int code) { return __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, status, code)) != 0; };
             bool ok = true, rows = true;
-            int nunits = 0, item = 0, cb_done = 0;
+            int nunits = 0, item = 0;
             const uint32_t idesc_cb = instr_desc_f16(128, 128, Fmt<T>::v, 0, 0) + ((uint32_t)(rb ? 128 >> 3 : 0) << 17),      // N = 128 or 256
                            idesc_y1 = instr_desc_f16(128, 64, Fmt<T>::v, 0, h_np ? 1 : 0), idesc_y2 = instr_desc_f16(128, 64, Fmt<T>::v, 0, 1);
             const uint32_t step_H = h_np ? 128 : 2;              // states along the rows of the tile, or along its columns
@@ -903,7 +906,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
             for (int seq = 0; seq < count && ok; ++seq, step()) {
                 if (w.enter) {
                     rows = rb < w.row_blocks(seqlen);
-                    ok = wait(b_unit, nunits, kStOutUnit);       // every unit completes one phase, whatever its row blocks
+                    ok = wait(b_unit, nunits, kStOutUnit);
                     ++nunits;
                     if (!ok) break;
                     if (rows) {
@@ -916,12 +919,13 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                                 mma_steps_ss(4, acc, desc_C + kb * (16384 / 16), 2, desc_x + kb * (Cfg::kStage / 16), 2, idesc_cb, kb > 0);
                             mma_commit(&b_cb[rb]);
                         }
-                        __syncwarp();
-                        ok = wait(&b_cbread[rb], cb_done, kStOutCbRead);
-                        ++cb_done;
-                        if (!ok) break;
-                        tc_fence_after_sync();
+                    } else if (lane == 0) {
+                        mbar_arrive(&b_cb[rb]);
                     }
+                    __syncwarp();
+                    ok = wait(&b_cbread[rb], nunits - 1, kStOutCbRead);
+                    if (!ok) break;
+                    tc_fence_after_sync();
                 }
                 if (!rows) continue;
                 const int s = seq & 1;
@@ -958,7 +962,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 OutWalk w(it0, ngroups, nchunks, hpu);
                 auto step = [&] { w.step(ngroups, nchunks, hpu); };
                 bool ok = true;
-                uint32_t outs = 0, cbs = 0;          // parities of the next completion of each b_out, b_cb
+                uint32_t outs = 0;                   // parities of the next completion of each b_out
                 struct Pending { int b, h, t, nrb; } pend[2] = {};
                 int nunits_requested = 0, seq = 0, done = 0;         // units requested; heads requested, finished
                 // Heads leave in the order in which they came: the one in stage s has its output tiles stored as they are completed.  Then the
@@ -995,10 +999,7 @@ ssd_tc_output_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                             tma_load_4d(st_x(kb), &tm_B, b_unit, kb * 64, w.g, w.c * kQ, w.b);
                         }
 #pragma unroll 1
-                        for (int rb = 0; rb < nrb && ok; ++rb) {
-                            ok = mbar_wait(&b_cb[rb], (cbs >> rb) & 1, status, kStOutCb);        // B has been read
-                            cbs ^= 1u << rb;
-                        }
+                        for (int rb = 0; rb < 2 && ok; ++rb) ok = mbar_wait(&b_cb[rb], (nunits_requested - 1) & 1, status, kStOutCb);        // B has been read
                         if (!ok) break;
                     }
                     mbar_expect_tx(&b_xh[s], 32768 + Cfg::kH);

@@ -24,11 +24,12 @@ def test_lengths_around_row_blocks_and_chunks(L):
 
 
 @pytest.mark.parametrize("has_z", [True, False])
-@pytest.mark.parametrize("L", [356, 257, 384])
-def test_rows_after_a_short_last_chunk(L, has_z):
+@pytest.mark.parametrize("L,G", [(356, 1), (257, 1), (384, 1), (356, 80), (100, 80), (100, 1)])
+def test_rows_after_a_short_last_chunk(L, G, has_z):
     """A last chunk of up to 128 steps has nothing for the warps of its lower row block, which reach the next batch row's first chunk while the
-    heads of the short one are in flight.  Each of 148 CTAs has six or seven heads here, those that come to a new row three or five of the row before."""
-    run_both(make(350 + L, 6, L, 80, 64, 1, 128, torch.bfloat16, has_z=has_z), 256, TOL_BF16, f"L{L} z {has_z}")
+    heads of the short one are in flight.  Each of 148 CTAs has six or seven heads here, those that come to a new row three or five of the row before;
+    with a group per head, every one has its own C and B, and with 100 steps there is nothing for those warps at all."""
+    run_both(make(350 + L, 6, L, 80, 64, G, 128, torch.bfloat16, has_z=has_z), 256, TOL_BF16, f"L{L} G{G} z {has_z}")
 
 
 @pytest.mark.parametrize("Q", [32, 64, 128, 512])

@@ -748,11 +748,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 && U == 1 ? 3 : 2) ss
 // The result is rounded to the input type.  For bf16 two parts, 16 to 17 bits of an operand, leave its error what all three give.
 template <typename T> constexpr int kOutParts = std::is_same<T, __nv_bfloat16>::value ? 2 : 3;
 
-// Decays of the steps a block of rows looks back on, factorised: exp(dA_m - dA_k) dt_k = exp(dA_m - ref) (exp(ref - dA_k) dt_k), ref = dA
-// of the last of 32 steps: an exponential per row and 32 columns instead of one per element.  dA does not increase (A <= 0, dt >= 0), so neither exponent is positive below the diagonal; in the
-// range that holds it the first is bounded.  The two are multiplied with each other before CB, whose product with a column factor of 2^-100
-// may be subnormal; a column factor that is so itself (a step of almost no length) would lose bits as well.  A range for which one of these
-// is not so has its decays formed one by one.
+// Decays of the steps a block of rows looks back on, factorised: exp(dA_m - dA_k) dt_k = exp(dA_m - ref) (exp(ref - dA_k) dt_k), ref = dA of
+// the last of 32 steps: an exponential per row and 32 columns instead of one per element.  dA does not increase (A <= 0, dt >= 0), so neither
+// exponent is positive below the diagonal; in the range that holds it the first is bounded.  The two are multiplied with each other before
+// CB, whose product with a column factor of 2^-100 may be subnormal; a column factor that is so itself (a step of almost no length) would
+// lose bits as well.  A range for which one of these is not so has its decays formed one by one.
 // In that range two exponents of up to 100 replace one that is small where the weight is large, so neither may lose what the other does not
 // give back: the distance of a step from the range's last is summed within the range, not taken from the chunk's sums, which are rounded to
 // 2^-24 of their size, and its rows use the same rounded distances as its columns, so that the exponents of a step's weight on itself cancel.
@@ -908,10 +908,11 @@ __device__ __noinline__ void finish_left_out(const mb200_ssd_args a, const float
 }
 
 // ---- 16 bits
-// Two CTAs of 121 to 128 registers per SM, of which no more than 12 bytes a thread are spilled: three CTAs of 80 registers spill, and took 76 us
-// where two took 69 and now take 67 (2 x 1500 steps of 48 half-precision heads of 64 x 64); a second pair of tiles left L1 so little that
-// C.B^T, which every head reads again, came from L2 each time (72 -> 81 us in bf16); one CTA per SM that keeps C.B^T in tensor memory while the heads pass took 78, with all its warps in step 85.  A kernel laid out like the one for
-// fp32 below, with a warp for the MMAs alone, took 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
+// Two CTAs of 121 to 128 registers per SM, of which no more than 12 bytes a thread are spilled: three CTAs of 80 registers spill, and took 76
+// us where two took 69 and now take 67 (2 x 1500 steps of 48 half-precision heads of 64 x 64); a second pair of tiles left L1 so little that
+// C.B^T, which every head reads again, came from L2 each time (72 -> 81 us in bf16); one CTA per SM that keeps C.B^T in tensor memory while
+// the heads pass took 78, with all its warps in step 85.  A kernel laid out like the one for fp32 below, with a warp for the MMAs alone, took
+// 68 there, but 175 for 155 us in bf16 (2 x 3000 steps of 32 heads of 128 x 128).
 template <typename T> constexpr uint32_t kScan16A = kOutParts<T> * kTileA;
 template <typename T, int W> constexpr uint32_t kScan16B = kOutParts<T> * W * kTileB;
 static_assert(32768 + kLeftOutBytes <= kScan16A<__nv_bfloat16> + kScan16B<__nv_bfloat16, 1>, "sums and what is added to them");
@@ -1189,8 +1190,9 @@ __global__ void __launch_bounds__(kThreads, 2) ssd_split_scan16_kernel(const mb2
 // are, and B's rows (or H's columns) follow.  (A ninth warp for the MMAs alone leaves a thread 96 registers for 128, because a quarter of the
 // SM then has five warps: 28.0 us for 26.2.  With the 128 nothing is spilled.)
 // What bounds it: a CTA is one pass through a chain of latencies -- launch, first loads, operands, MMAs, stores -- with three tiles in the
-// middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its start, which overlaps the recurrence, included),
-// 2 x 3000 steps of 32 heads of 64 x 128 136; 64 x 64 tiles of packed fp32 FMAs took 54 and 245.
+// middle, so everything that can be is requested at the start, and C.B^T two tiles ahead.  2 x 2048 steps of 8 heads of 64 x 64: 27 us (its
+// start, which overlaps the recurrence, included), 2 x 3000 steps of 32 heads of 64 x 128 136; 64 x 64 tiles of packed fp32 FMAs took 54 and
+// 245.
 // Shared memory: B, then two stages of C.B^T, 4 KB a warp.  The sums leave through the first of them.
 constexpr uint32_t kScanB = kParts * kTileB, kScanTiles = kScanB + 65536;
 constexpr uint32_t kScanTail = 48;                      // barriers and tensor-memory slot behind the tiles

@@ -504,12 +504,12 @@ ssd_tc_state_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __gri
 // z in place and leaves through a TMA store.  While a unit starts, B lies in the x parts of the two stages.
 //
 // What bounds it: a head takes the output warps' pass over its accumulators (4200 cycles) plus the MMAs that wait for them (1400); the mask
-// warps have a third of the time to spare.  269 us for the shape above (321 with twelve warps that did both, one after the other), 2.7 ms
-// for 262144 steps of 128 heads (3.28).  C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
-// register comes back from L2: the roles share the block's registers out between them (setmaxnreg).  What is still spilled, 72 bytes a thread,
-// is the mask warps' (built with the bodies of the others taken out, 72; the output warps alone 0), who have time to spare.  Instruction fetch is what bounds the
-// roles themselves: loops are rolled, waits short, places advanced without divisions.  The output loop unrolled twice takes 273 us, eight
-// times 320; with the next accumulators requested ahead 289.
+// warps have a third of the time to spare.  269 us for the shape above (321 with twelve warps that did both, one after the other), 2.7 ms for
+// 262144 steps of 128 heads (3.28).  C.B^T takes 64 registers of a thread, and shared memory leaves the L1 cache nothing, so a spilled
+// register comes back from L2: the roles share the block's registers out between them (setmaxnreg).  What is still spilled, 72 bytes a
+// thread, is the mask warps' (built with the bodies of the others taken out, 72; the output warps alone 0), who have time to spare.
+// Instruction fetch is what bounds the roles themselves: loops are rolled, waits short, places advanced without divisions.  The output loop
+// unrolled twice takes 273 us, eight times 320; with the next accumulators requested ahead 289.
 //
 // Decay mask, per thread one row m and ranges of 8 columns k:
 //   L[m,k] = exp(dA_m - dA_ref) * (exp(dA_ref - dA_k) dt_k), ref = last column of the range

@@ -1,17 +1,18 @@
 // Stages of the SSD chunked forward for every shape and type, on the tensor cores with operands in parts.
 //
-// ssd_tc.cu serves 16-bit calls of headdim 64, dstate 128 and chunk 256 with 16-bit operands throughout: weights, decays and entering
-// states are rounded to the input type.  Here an fp32 operand -- an fp32 input, C.B^T times its decay, a weighted x, an entering state -- is
-// cut into bf16 values that add up to it, and a half-precision input into two, so that tcgen05.mma of bf16 operands forms the products, which
-// it adds in fp32.  Three parts hold all 24 bits, and terms below 2^-24 of a product are left out: so chunk states, C.B^T, and the outputs
-// of half precision and fp32.  bf16 outputs take two parts, 16 to 17 bits, of their entering states and decayed C.B^T, so that about 2^-17 of
-// an operand is left out of a result with 8 bits.  bf16 has fp32's range: nothing overflows that fp32 holds, whatever the input type.  The tensor core cuts its sums off where fp32 arithmetic
-// rounds.  Sums that leave a 16-bit call in fp32 have the small products in a sum of their own; in fp32 calls the tensor core adds the products
-// of 64 steps only, the small ones first, and fp32 additions do the rest: without decays, where the sums are the whole error, states of 256
-// steps are 2.3e-7 from 64 bits, outputs 2.6e-7 (4.0e-7 and 6.4e-7 with two sums over all steps, 3.3e-7 and 4.3e-7 with tiles of fp32 FMAs;
-// 2 x 2048 steps of 8 heads of 64 x 64: 44.4 us for 43.6).  Against 64 bits, 2 x 1500 steps of 16 heads of 64 x 64, four seeds: outputs 1.66e-3
-// (bf16) and 2.08e-4 (fp16), which is their own rounding, 2.3e-7 to 7.9e-7 in fp32 (tiles of fp32 FMAs: 6.7e-7 to 14e-7); end states 1.3e-7 to
-// 1.7e-6 (1.6e-6 to 4.7e-6).  Operands rounded to 16 bits: outputs 2.4e-3 and 3.0e-4, end states 1.7e-3 and 2.1e-4.
+// ssd_tc.cu serves 16-bit calls of headdim 64, dstate 128 and chunk 256 with 16-bit operands throughout: weights, decays and entering states
+// are rounded to the input type.  Here an fp32 operand -- an fp32 input, C.B^T times its decay, a weighted x, an entering state -- is cut
+// into bf16 values that add up to it, and a half-precision input into two, so that tcgen05.mma of bf16 operands forms the products, which it
+// adds in fp32.  Three parts hold all 24 bits, and terms below 2^-24 of a product are left out: so chunk states, C.B^T, and the outputs of
+// half precision and fp32.  bf16 outputs take two parts, 16 to 17 bits, of their entering states and decayed C.B^T, so that about 2^-17 of an
+// operand is left out of a result with 8 bits.  bf16 has fp32's range: nothing overflows that fp32 holds, whatever the input type.  The
+// tensor core cuts its sums off where fp32 arithmetic rounds.  Sums that leave a 16-bit call in fp32 have the small products in a sum of
+// their own; in fp32 calls the tensor core adds the products of 64 steps only, the small ones first, and fp32 additions do the rest: without
+// decays, where the sums are the whole error, states of 256 steps are 2.3e-7 from 64 bits, outputs 2.6e-7 (4.0e-7 and 6.4e-7 with two sums
+// over all steps, 3.3e-7 and 4.3e-7 with tiles of fp32 FMAs; 2 x 2048 steps of 8 heads of 64 x 64: 44.4 us for 43.6).  Against 64 bits, 2 x
+// 1500 steps of 16 heads of 64 x 64, four seeds: outputs 1.66e-3 (bf16) and 2.08e-4 (fp16), which is their own rounding, 2.3e-7 to 7.9e-7 in
+// fp32 (tiles of fp32 FMAs: 6.7e-7 to 14e-7); end states 1.3e-7 to 1.7e-6 (1.6e-6 to 4.7e-6).  Operands rounded to 16 bits: outputs 2.4e-3
+// and 3.0e-4, end states 1.7e-3 and 2.1e-4.
 //
 // A tile loop: 256 threads fetch the next 64 steps of the reduction while the tensor core works on the last ones, form the operand values,
 // cut them and store them.  The tensor core is idle most of the time; what bounds these kernels is that element-wise work and the latencies

@@ -211,6 +211,24 @@ def test_fp32_values_too_large_to_be_cut(name, P, N, lens):
             assert rel(got[:, at + 1:], want[:, at + 1:]) <= F32
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("P,N,L", [(64, 64, 300), (72, 40, 299), (136, 130, 255)])
+def test_gate_and_skip_where_a_tile_is_left_out(dtype, P, N, L):
+    """16 bits: what an infinity in one column does not reach is gated and has its D as everywhere."""
+    t, e = 140, 9
+    inp = make(927 + P, 1, L, 3, P, 1, N, dtype, D_hdim=True, init=True)
+    f = lambda v: v.float()
+    want, _ = oracle.ssd_chunk_scan(f(inp["x"]), f(inp["dt"]), inp["A"], f(inp["B"]), f(inp["C"]), 128, inp["D"], f(inp["z"]), inp["dt_bias"], inp["initial_states"], dt_softplus=True)
+    inp["x"][0, t, 1, e] = float("inf")
+    c = {k: _c(v) for k, v in inp.items()}
+    out = _fn()(c["x"], c["dt"], c["A"], c["B"], c["C"], 128, D=c["D"], z=c["z"], dt_bias=c["dt_bias"], initial_states=c["initial_states"], dt_softplus=True).cpu()
+    keep = torch.arange(P) != e
+    check_out(out[0, :t], want[0, :t], "earlier steps")
+    check_out(out[0, :, 0], want[0, :, 0], "other head")
+    check_out(out[0, :, 1, keep], want[0, :, 1, keep], "other columns")
+    assert not torch.isfinite(out[0, t, 1, e])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("P,N,G,H", [(64, 64, 1, 15), (72, 40, 3, 15), (64, 136, 1, 9)])
 def test_two_heads_share_their_b(dtype, P, N, G, H):
